@@ -38,26 +38,26 @@ def _case(name, model, start, layers, prompts=0, prompt=0, cached=0, decode=0, c
 def listed():
     return [
         # a single chat on two nodes of 14 layers each: what the second node does per token (launches and latency count)
-        _case("chat, one row", "qwen3-0.6b", 14, 14, decode=1, ctx=777),
+        _case("chat-one-row", "qwen3-0.6b", 14, 14, decode=1, ctx=777),
         # a micro-batch of the eight-stage pipeline that serves 512 requests, on a stage of five layers
-        _case("pipeline micro-batch", "qwen3-8b", 13, 5, decode=57, ctx=1280),
+        _case("pipeline-micro-batch", "qwen3-8b", 13, 5, decode=57, ctx=1280),
         # the headline workload: 510 decoding rows beside the prompts that replace finished requests
-        _case("closed loop, mixed", "qwen3-8b", 8, 2, prompts=2, prompt=1024, decode=510, ctx=1280),
+        _case("closed-loop-mixed", "qwen3-8b", 8, 2, prompts=2, prompt=1024, decode=510, ctx=1280),
         # one 8192-token slice of a long prompt
-        _case("long prompt slice", "qwen3-32b", 20, 1, prompts=1, prompt=8192, cached=16384),
+        _case("long-prompt-slice", "qwen3-32b", 20, 1, prompts=1, prompt=8192, cached=16384),
         # decoding with e4m3 pages, chosen where the cache is what limits the batch
-        _case("decode, e4m3 pages", "qwen3-8b", 8, 2, decode=128, ctx=4096, kv="fp8_e4m3"),
+        _case("e4m3-pages-decode", "qwen3-8b", 8, 2, decode=128, ctx=4096, kv="fp8_e4m3"),
         # routed experts: decoding reads almost every expert for a few rows each, prompts fill them
-        _case("experts, decode", "qwen3-30b-a3b", 8, 2, decode=48, ctx=2100),
-        _case("experts, prompts", "qwen3-30b-a3b", 8, 2, prompts=3, prompt=1700),
+        _case("experts-decode", "qwen3-30b-a3b", 8, 2, decode=48, ctx=2100),
+        _case("experts-prompts", "qwen3-30b-a3b", 8, 2, prompts=3, prompt=1700),
         # latent attention with fp8 weights (the dense layers at the front of the model)
-        _case("latent, decode", "deepseek-v3", 1, 2, decode=64, ctx=4096),
-        _case("latent, prompts", "deepseek-v3", 1, 1, prompts=2, prompt=2048),
+        _case("latent-decode", "deepseek-v3", 1, 2, decode=64, ctx=4096),
+        _case("latent-prompts", "deepseek-v3", 1, 1, prompts=2, prompt=2048),
         # latent attention over the indexer's best keys: a slice of a long prompt beside decoding rows
-        _case("indexed, mixed", "deepseek-v3.2", 1, 1, prompts=1, prompt=1000, cached=5000, decode=16, ctx=8192),
+        _case("indexed-mixed", "deepseek-v3.2", 1, 1, prompts=1, prompt=1000, cached=5000, decode=16, ctx=8192),
         # three gated-delta-net layers and one attention layer
-        _case("hybrid, prompts", "hybrid-8b", 4, 4, prompts=2, prompt=3000),
-        _case("hybrid, decode", "hybrid-8b", 4, 4, decode=96, ctx=2048),
+        _case("hybrid-prompts", "hybrid-8b", 4, 4, prompts=2, prompt=3000),
+        _case("hybrid-decode", "hybrid-8b", 4, 4, decode=96, ctx=2048),
     ]
 
 
