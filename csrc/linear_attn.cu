@@ -1,16 +1,10 @@
-// Gated DeltaNet linear-attention layers (Qwen3-Next / Qwen3.5 hybrids): short causal convolution
-// with a carried window, and the gated delta-rule recurrence with a per-request state matrix.
+// Gated DeltaNet linear-attention layers (Qwen3-Next / Qwen3.5 hybrids): short causal convolution with a carried window, and
+// the gates around the mixers (the recurrence itself is in gated_delta.cu).
 //
 //   conv:   y[t, c] = silu( sum_j w[c, j] * u[t - (K-1) + j, c] ),  u = [carried window | x]
-//   delta:  S <- S * exp(g_t);  d = (v_t - S k_t) * beta_t;  S <- S + d k_t^T;  o_t = S q_t
-//           g_t = -exp(A_log) * softplus(a_t + dt_bias),  beta_t = sigmoid(b_t)
-//           q, k are l2-normalised (eps 1e-6 on the sum of squares); q is scaled by Dk^-1/2;
-//           out = rmsnorm(o_t) * norm_w * silu(z_t)
-// State lives in per-request slots (not pages): conv window [slots, C, K-1] bf16, recurrent
-// state [slots, Hv, Dv, Dk] fp32. A sequence whose first token of this step sits at position 0
-// starts from a zero state. The reference runs these layers through mlx-lm's
-// gated_delta_update (src/parallax/models/qwen3_next.py:149-230) and keeps the states in a
-// LinearCache (src/parallax/server/cache/linear_cache.py).
+// The window lives in per-request slots [slots, C, K-1] bf16; a sequence whose first token of this step sits at position 0
+// starts from zeros. The reference runs these layers through mlx-lm (src/parallax/models/qwen3_next.py:149-230) and keeps the
+// states in a LinearCache (src/parallax/server/cache/linear_cache.py).
 #include "common.cuh"
 #include "pxl_api.h"
 
@@ -19,7 +13,8 @@ using namespace pxl;
 
 constexpr int kMaxConvK = 8;
 
-// grid (channel blocks, sequences); thread = one channel, walks the sequence's tokens in order
+// Decoded tokens (and sizes the kernel below does not take): grid (channel blocks, sequences); thread = one channel, walks the
+// sequence's tokens in order
 __global__ void __launch_bounds__(128) conv1d_silu_kernel(const bf16* __restrict__ x, int64_t ldx,
                                                           const bf16* __restrict__ w, const bf16* __restrict__ bias,
                                                           bf16* __restrict__ conv_state, const int* __restrict__ seq_cu,
@@ -50,87 +45,121 @@ __global__ void __launch_bounds__(128) conv1d_silu_kernel(const bf16* __restrict
   for (int j = 0; j < K - 1; ++j) st[j] = __float2bfloat16(win[j]);
 }
 
-// grid (value heads, sequences), Dv threads; thread i owns row i of the state matrix [Dv, Dk]
-template <int DK>
-__global__ void __launch_bounds__(128) gated_delta_kernel(const bf16* __restrict__ qkv, int64_t ld_qkv,
-                                                          const bf16* __restrict__ a_in, const bf16* __restrict__ b_in,
-                                                          int64_t ld_ab, const float* __restrict__ A_log,
-                                                          const float* __restrict__ dt_bias, const bf16* __restrict__ z,
-                                                          int64_t ld_z, const bf16* __restrict__ norm_w,
-                                                          float* __restrict__ rec_state, const int* __restrict__ seq_cu,
-                                                          const int* __restrict__ seq_slots,
-                                                          const int* __restrict__ positions, bf16* __restrict__ out,
-                                                          int64_t ld_out, int Hk, int Hv, int Dv, float eps) {
-  __shared__ float qs[DK], ks[DK];
-  __shared__ float red[32];
-  const int hv = blockIdx.x, b = blockIdx.y;
-  const int i = threadIdx.x;  // row of S / element of v, z, out
-  const int t0 = seq_cu[b], t1 = seq_cu[b + 1];
-  if (t1 <= t0) return;
-  const int hk = hv / (Hv / Hk);
-  const int slot = seq_slots[b];
+// Prompts: a thread walks a run of tokens of 8 channels, weights and last inputs in registers, inputs four tokens ahead. The
+// walk of a whole sequence by one thread (above) is a chain of as many loads as it has tokens (2.0 ms for 5900 tokens x 8192
+// channels); runs make it a streaming pass (57 us, 3.4 TB/s read and written). The slots are rewritten by a launch of its own, because the first tokens of a
+// slice read what its last ones replace.
+template <int K>
+__global__ void __launch_bounds__(128) conv_run_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ w,
+                                                       const bf16* __restrict__ bias, const bf16* __restrict__ conv_state,
+                                                       const int* __restrict__ seq_cu, const int* __restrict__ seq_slots,
+                                                       const int* __restrict__ positions, bf16* __restrict__ out, int64_t ldo,
+                                                       int C, int seqs, int tokens, int run) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
+  if (c >= C) return;
+  const int first = blockIdx.y * run, last = first + run < tokens ? first + run : tokens;
+  int seq = 0;
+  for (int hi = seqs - 1; seq < hi;) {  // the last sequence that starts at or before the run
+    const int mid = (seq + hi + 1) >> 1;
+    if (seq_cu[mid] <= first) seq = mid; else hi = mid - 1;
+  }
+  int end = seq_cu[seq + 1], start = seq_cu[seq];
+  float wk[8][K], b0[8], hist[K - 1][8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) wk[e][j] = __bfloat162float(w[(c + e) * K + j]);
+    b0[e] = bias ? __bfloat162float(bias[c + e]) : 0.f;
+  }
+  auto unpack = [](const bf16x8& v, float (&f)[8]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 p = unpack_bf16x2(v.u[j]);
+      f[2 * j] = p.x, f[2 * j + 1] = p.y;
+    }
+  };
+  constexpr int kAhead = 4;
+  const bf16x8 zero8 = {{0u, 0u, 0u, 0u}};
+  const bf16* cur = x + first * ldx + c;
+  bf16x8 ahead[kAhead];
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) ahead[i] = first + i < last ? ld_bf16x8(cur + i * ldx) : zero8;
+  for (int t4 = first; t4 < last; t4 += kAhead) {
+#pragma unroll
+    for (int i4 = 0; i4 < kAhead; ++i4, cur += ldx) {
+      const int t = t4 + i4;
+      if (t >= last) break;
+      while (end <= t) ++seq, start = end, end = seq_cu[seq + 1];
+      if (t == first || t == start) {  // the inputs before this run, or of this sequence's earlier steps
+        const int li = t - start;
+        const bool fresh = li < K - 1 && positions[start] == 0;
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) {
+          const int back = K - 1 - j;  // hist[j] is the input `back` tokens ago
+          if (back <= li) {
+            unpack(ld_bf16x8(cur - back * ldx), hist[j]);
+          } else {
+            const bf16* st = conv_state + (static_cast<size_t>(seq_slots[seq]) * C + c) * (K - 1) + li + j;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) hist[j][e] = fresh ? 0.f : __bfloat162float(st[e * (K - 1)]);
+          }
+        }
+      }
+      float here[8];
+      unpack(ahead[i4], here);
+      if (t + kAhead < last) ahead[i4] = ld_bf16x8(cur + kAhead * ldx);
+      bf16x8 o;
+      float y[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        y[e] = b0[e] + wk[e][K - 1] * here[e];
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) y[e] += wk[e][j] * hist[j][e];
+#pragma unroll
+        for (int j = 0; j + 1 < K - 1; ++j) hist[j][e] = hist[j + 1][e];
+        hist[K - 2][e] = here[e];
+        y[e] = y[e] / (1.f + __expf(-y[e]));
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o.u[j] = pack_bf16x2(y[2 * j], y[2 * j + 1]);
+      st_bf16x8(out + t * ldo + c, o);
+    }
+  }
+}
+
+// the slots of the prompt slices: the last K - 1 inputs (of older steps where the slice is shorter)
+__global__ void __launch_bounds__(128) conv_window_kernel(const bf16* __restrict__ x, int64_t ldx, bf16* __restrict__ conv_state,
+                                                          const int* __restrict__ seq_cu, const int* __restrict__ seq_slots,
+                                                          const int* __restrict__ positions, int C, int K) {
+  const int c = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  if (c >= C) return;
+  const int t0 = seq_cu[b], n = seq_cu[b + 1] - t0;
+  if (n <= 0) return;
   const bool fresh = positions[t0] == 0;
-  float* Sg = rec_state + ((static_cast<size_t>(slot) * Hv + hv) * Dv + i) * DK;
-  float S[DK];
-  if (i < Dv) {
-#pragma unroll
-    for (int j = 0; j < DK; j += 4) {
-      const float4 v4 = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(Sg + j);
-      S[j] = v4.x; S[j + 1] = v4.y; S[j + 2] = v4.z; S[j + 3] = v4.w;
-    }
+  bf16* st = conv_state + (static_cast<size_t>(seq_slots[b]) * C + c) * (K - 1);
+  for (int j = 0; j < K - 1; ++j) {
+    const int li = n - (K - 1) + j;
+    st[j] = li >= 0 ? x[(t0 + li) * ldx + c] : fresh ? __float2bfloat16(0.f) : st[j + n];
   }
-  const float neg_a = -__expf(A_log[hv]);
-  const float dtb = dt_bias[hv];
-  const float nw = i < Dv ? __bfloat162float(norm_w[i]) : 0.f;
-  const int q_off = hk * DK, k_off = Hk * DK + hk * DK, v_off = 2 * Hk * DK + hv * Dv;
-  const float inv_scale = rsqrtf(static_cast<float>(DK));
-  for (int t = t0; t < t1; ++t) {
-    const bf16* row = qkv + t * ld_qkv;
-    // q, k of this key head: l2-normalise and scale
-    float qv = 0.f, kv = 0.f;
-    if (i < DK) {
-      qv = __bfloat162float(row[q_off + i]);
-      kv = __bfloat162float(row[k_off + i]);
-    }
-    const float q2 = block_reduce_sum(qv * qv, red);
-    const float k2 = block_reduce_sum(kv * kv, red);
-    if (i < DK) {
-      qs[i] = qv * rsqrtf(q2 + 1e-6f) * inv_scale;  // l2-normalised, then scaled by Dk^-1/2
-      ks[i] = kv * rsqrtf(k2 + 1e-6f);
-    }
-    __syncthreads();
-    const float av = __bfloat162float(a_in[t * ld_ab + hv]) + dtb;
-    const float sp = av > 20.f ? av : log1pf(__expf(av));
-    const float decay = __expf(neg_a * sp);
-    const float beta = 1.f / (1.f + __expf(-__bfloat162float(b_in[t * ld_ab + hv])));
-    float o = 0.f;
-    if (i < Dv) {
-      float mem = 0.f;
-#pragma unroll
-      for (int j = 0; j < DK; ++j) {
-        S[j] *= decay;
-        mem = fmaf(S[j], ks[j], mem);
-      }
-      const float d = (__bfloat162float(row[v_off + i]) - mem) * beta;
-#pragma unroll
-      for (int j = 0; j < DK; ++j) {
-        S[j] = fmaf(d, ks[j], S[j]);
-        o = fmaf(S[j], qs[j], o);
-      }
-    }
-    // gated RMSNorm over the head's Dv outputs
-    const float o2 = block_reduce_sum(i < Dv ? o * o : 0.f, red);
-    if (i < Dv) {
-      const float zz = __bfloat162float(z[t * ld_z + hv * Dv + i]);
-      const float y = o * rsqrtf(o2 / Dv + eps) * nw * (zz / (1.f + __expf(-zz)));
-      out[t * ld_out + hv * Dv + i] = __float2bfloat16(y);
-    }
-    __syncthreads();
-  }
-  if (i < Dv) {
-#pragma unroll
-    for (int j = 0; j < DK; j += 4) *reinterpret_cast<float4*>(Sg + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
-  }
+}
+
+// false: sizes or alignments that the kernel above does not take
+bool launch_conv_run(const bf16* x, int64_t ldx, const bf16* w, const bf16* bias, bf16* conv_state, const int* seq_cu,
+                     const int* seq_slots, const int* positions, bf16* out, int64_t ldo, int C, int K, int seqs, int tokens,
+                     cudaStream_t stream) {
+  if (C % 8 || ldx % 8 || ldo % 8 || K > 4 || seqs > 65535 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return false;
+  const int blocks = ceil_div(C, 1024);
+  // enough threads for every SM, runs long enough that a run's first loads do not count
+  int run = ceil_div(tokens * blocks, 8 * pxl_host::num_sms());
+  run = run < 4 ? 4 : run > 64 ? 64 : run;
+  while (ceil_div(tokens, run) > 65535) run *= 2;
+  const dim3 grid(blocks, ceil_div(tokens, run));
+  const auto kern = K == 2 ? conv_run_kernel<2> : K == 3 ? conv_run_kernel<3> : conv_run_kernel<4>;
+  kern<<<grid, 128, 0, stream>>>(x, ldx, w, bias, conv_state, seq_cu, seq_slots, positions, out, ldo, C, seqs, tokens, run);
+  conv_window_kernel<<<dim3(ceil_div(C, 128), seqs), 128, 0, stream>>>(x, ldx, conv_state, seq_cu, seq_slots, positions, C, K);
+  return true;
 }
 
 __global__ void sigmoid_gate_mul_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ gate,
@@ -198,30 +227,20 @@ __global__ void row_dot_kernel(const bf16* __restrict__ x, int64_t ldx, const bf
 
 }  // namespace
 
-PXL_EXPORT int pxl_causal_conv1d_silu(const void* x, int64_t ldx, const void* w, const void* bias, void* conv_state,
-                                      const int* seq_cu, const int* seq_slots, const int* positions, void* out,
-                                      int64_t ldo, int B, int C, int K, cudaStream_t stream) {
+PXL_EXPORT int pxl_causal_conv1d_silu(const void* x_, int64_t ldx, const void* w_, const void* bias_, void* conv_state_,
+                                      const int* seq_cu, const int* seq_slots, const int* positions, void* out_,
+                                      int64_t ldo, int B, int C, int K, int prefill_seqs, int prefill_tokens, cudaStream_t stream) {
   if (B <= 0) return PXL_OK;
   if (K < 2 || K > kMaxConvK) return PXL_ERR_INVALID_ARG;
-  dim3 grid(pxl::ceil_div(C, 128), B);
-  conv1d_silu_kernel<<<grid, 128, 0, stream>>>(static_cast<const pxl::bf16*>(x), ldx, static_cast<const pxl::bf16*>(w),
-                                               static_cast<const pxl::bf16*>(bias), static_cast<pxl::bf16*>(conv_state),
-                                               seq_cu, seq_slots, positions, static_cast<pxl::bf16*>(out), ldo, C, K);
-  return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
-}
-
-PXL_EXPORT int pxl_gated_delta_rule(const void* qkv, int64_t ld_qkv, const void* a, const void* b, int64_t ld_ab,
-                                    const float* A_log, const float* dt_bias, const void* z, int64_t ld_z,
-                                    const void* norm_w, float* rec_state, const int* seq_cu, const int* seq_slots,
-                                    const int* positions, void* out, int64_t ld_out, int B, int Hk, int Hv, int Dk,
-                                    int Dv, float eps, cudaStream_t stream) {
-  if (B <= 0) return PXL_OK;
-  if (Dk != 128 || Dv > 128 || Dv <= 0 || Hk <= 0 || Hv % Hk) return PXL_ERR_INVALID_ARG;
-  dim3 grid(Hv, B);
-  gated_delta_kernel<128><<<grid, 128, 0, stream>>>(
-      static_cast<const pxl::bf16*>(qkv), ld_qkv, static_cast<const pxl::bf16*>(a), static_cast<const pxl::bf16*>(b),
-      ld_ab, A_log, dt_bias, static_cast<const pxl::bf16*>(z), ld_z, static_cast<const pxl::bf16*>(norm_w), rec_state,
-      seq_cu, seq_slots, positions, static_cast<pxl::bf16*>(out), ld_out, Hk, Hv, Dv, eps);
+  const auto *x = static_cast<const pxl::bf16*>(x_), *w = static_cast<const pxl::bf16*>(w_), *bias = static_cast<const pxl::bf16*>(bias_);
+  auto *conv_state = static_cast<pxl::bf16*>(conv_state_), *out = static_cast<pxl::bf16*>(out_);
+  int done = 0;
+  if (prefill_seqs > 0 && prefill_tokens > 0 &&
+      launch_conv_run(x, ldx, w, bias, conv_state, seq_cu, seq_slots, positions, out, ldo, C, K, prefill_seqs, prefill_tokens, stream))
+    done = prefill_seqs;
+  if (done < B)
+    conv1d_silu_kernel<<<dim3(pxl::ceil_div(C, 128), B - done), 128, 0, stream>>>(x, ldx, w, bias, conv_state, seq_cu + done,
+                                                                                 seq_slots + done, positions, out, ldo, C, K);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 

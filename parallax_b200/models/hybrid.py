@@ -202,12 +202,13 @@ class HybridStage(DecoderStage):
         proj = ops.linear(xn, lw.w_in)                                   # [T, qkv | z | b | a]
         n_qkv, n_z = self.qkv_dim, Hv * Dv
         conv = ops.causal_conv1d_silu(proj[:, :n_qkv], lw.conv_w, lw.conv_b, cache.conv_state, fb.seq_cu, fb.seq_slots,
-                                      fb.positions)
+                                      fb.positions, fb.num_prefill_seqs, fb.num_prefill_tokens)
         z = proj[:, n_qkv:n_qkv + n_z]
         b = proj[:, n_qkv + n_z:n_qkv + n_z + Hv]
         a = proj[:, n_qkv + n_z + Hv:n_qkv + n_z + 2 * Hv]
         return ops.gated_delta_rule(conv, a, b, lw.A_log, lw.dt_bias, z, lw.norm_w, cache.rec_state, fb.seq_cu,
-                                    fb.seq_slots, fb.positions, Hk, Hv, Dk, Dv, self.cfg.rms_norm_eps)
+                                    fb.seq_slots, fb.positions, Hk, Hv, Dk, Dv, self.cfg.rms_norm_eps, fb.num_prefill_seqs,
+                                    fb.num_prefill_tokens)
 
     def forward_layers(self, h: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         eps = self.cfg.rms_norm_eps

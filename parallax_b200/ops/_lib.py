@@ -101,9 +101,10 @@ _SIGS = {
     "pxl_gemm_fp8_block_grouped": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P, _P, _P,
                                    c_int, c_int, _P, _P],
     "pxl_quant_fp8_rows": [_P, c_int64, _P, _P, c_int, c_int, _P],
-    "pxl_causal_conv1d_silu": [_P, c_int64, _P, _P, _P, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, _P],
+    "pxl_causal_conv1d_silu": [_P, c_int64, _P, _P, _P, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, c_int, c_int, _P],
     "pxl_gated_delta_rule": [_P, c_int64, _P, _P, c_int64, _P, _P, _P, c_int64, _P, _P, _P, _P, _P, _P, c_int64,
-                             c_int, c_int, c_int, c_int, c_int, c_float, _P],
+                             c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, _P, c_int64, _P],
+    "pxl_gated_delta_workspace": [c_int] * 4,
     "pxl_sigmoid_gate_mul": [_P, c_int64, _P, c_int64, _P, c_int64, c_int, c_int, _P],
     "pxl_gate_mul_grouped": [_P, c_int64, _P, c_int64, _P, c_int64, _P, c_int64, c_int, c_int, c_int, _P],
     "pxl_row_dot": [_P, c_int64, _P, _P, c_int, c_int, _P],
@@ -165,7 +166,7 @@ _SIGS = {
 }
 
 
-_SIZES = {"pxl_delta_rule_workspace"}      # functions that return a number of bytes
+_SIZES = {"pxl_delta_rule_workspace", "pxl_gated_delta_workspace"}      # functions that return a number of bytes
 
 
 @lru_cache(maxsize=1)

@@ -1012,30 +1012,34 @@ def moe_ffn_fp8(x, ids, weights, w1q, w1s, w2q, w2s, num_experts: int, base=None
 
 
 # ---------------------------------------------------------------------------- gated delta net
-def causal_conv1d_silu(x, w, bias, conv_state, seq_cu, seq_slots, positions):
+def causal_conv1d_silu(x, w, bias, conv_state, seq_cu, seq_slots, positions, prefill_seqs: int = 0, prefill_tokens: int = 0):
     T, C = x.shape
     out = torch.empty((T, C), dtype=x.dtype, device=x.device)
     B = seq_slots.shape[0]
     check(_lib.lib().pxl_causal_conv1d_silu(x.data_ptr(), x.stride(0), w.data_ptr(), _ptr(bias), conv_state.data_ptr(),
                                             seq_cu.data_ptr(), seq_slots.data_ptr(), positions.data_ptr(),
-                                            out.data_ptr(), out.stride(0), B, C, w.shape[1], _stream(x.device)),
+                                            out.data_ptr(), out.stride(0), B, C, w.shape[1], prefill_seqs, prefill_tokens,
+                                            _stream(x.device)),
           "pxl_causal_conv1d_silu")
-    _count()
+    _count(1 + (prefill_tokens > 0))
     return out
 
 
 def gated_delta_rule(qkv, a, b, A_log, dt_bias, z, norm_w, rec_state, seq_cu, seq_slots, positions, Hk: int, Hv: int,
-                     Dk: int, Dv: int, eps: float):
+                     Dk: int, Dv: int, eps: float, prefill_seqs: int = 0, prefill_tokens: int = 0):
     T = qkv.shape[0]
     out = torch.empty((T, Hv * Dv), dtype=qkv.dtype, device=qkv.device)
     assert a.stride(0) == b.stride(0)
+    nbytes = _lib.lib().pxl_gated_delta_workspace(Hv, Dv, prefill_seqs, prefill_tokens)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=qkv.device) if nbytes else None
     check(_lib.lib().pxl_gated_delta_rule(qkv.data_ptr(), qkv.stride(0), a.data_ptr(), b.data_ptr(), a.stride(0),
                                           A_log.data_ptr(), dt_bias.data_ptr(), z.data_ptr(), z.stride(0),
                                           norm_w.data_ptr(), rec_state.data_ptr(), seq_cu.data_ptr(),
                                           seq_slots.data_ptr(), positions.data_ptr(), out.data_ptr(), out.stride(0),
-                                          seq_slots.shape[0], Hk, Hv, Dk, Dv, eps, _stream(qkv.device)),
+                                          seq_slots.shape[0], Hk, Hv, Dk, Dv, eps, prefill_seqs, prefill_tokens, _ptr(ws), nbytes,
+                                          _stream(qkv.device)),
           "pxl_gated_delta_rule")
-    _count()
+    _count(3 * (prefill_seqs > 0) + (seq_slots.shape[0] > prefill_seqs))
     return out
 
 

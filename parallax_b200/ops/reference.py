@@ -528,8 +528,10 @@ def moe_ffn_fp8(x, ids, weights, w1q, w1s, w2q, w2s, num_experts: int, base=None
 
 
 # ---------------------------------------------------------------------------- gated delta net
-def causal_conv1d_silu(x, w, bias, conv_state, seq_cu, seq_slots, positions):
-    """Per-channel causal convolution + SiLU with the last K-1 inputs carried per request slot."""
+def causal_conv1d_silu(x, w, bias, conv_state, seq_cu, seq_slots, positions, prefill_seqs: int = 0, prefill_tokens: int = 0):
+    """Per-channel causal convolution + SiLU with the last K-1 inputs carried per request slot. The first ``prefill_seqs``
+    sequences are prompt slices of ``prefill_tokens`` rows together (a hint for the kernels, like in
+    :func:`gated_delta_rule`)."""
     T, C = x.shape
     K = w.shape[1]
     out = torch.empty((T, C), dtype=x.dtype)
@@ -552,7 +554,7 @@ def causal_conv1d_silu(x, w, bias, conv_state, seq_cu, seq_slots, positions):
 
 
 def gated_delta_rule(qkv, a, b, A_log, dt_bias, z, norm_w, rec_state, seq_cu, seq_slots, positions, Hk: int, Hv: int,
-                     Dk: int, Dv: int, eps: float):
+                     Dk: int, Dv: int, eps: float, prefill_seqs: int = 0, prefill_tokens: int = 0):
     """Sequential gated delta rule with a per-request state ``[Hv, Dv, Dk]`` and gated RMSNorm."""
     T = qkv.shape[0]
     out = torch.empty((T, Hv * Dv), dtype=qkv.dtype)
