@@ -9,6 +9,8 @@
 //               rows (page boxes), chunk by chunk. A cache row is key AND value and is loaded once: the chunks this
 //               CTA accumulates as values go to whole-tile V buffers, all others - needed for the scores only - to a
 //               ring of chunk slots that are free again as soon as the scores have read them.
+//               With key lists (attention over an indexer's best keys) a CTA takes one token, whose listed rows are
+//               gathered four at a time (tile::gather4); tokens without a list take the page boxes.
 //   warp 5    : MMA issuer. S = Q K^T over L + R (both operands K-major) into one of two TMEM score buffers, chunk
 //               by chunk as the loads land, so the scores of tile i + 1 are computed while the softmax warps work
 //               on tile i; then O += P V, P from tensor memory, V taken MN-major from the V buffer, all of its
@@ -46,6 +48,8 @@ struct TcArgs {
   const int* ctx_lens;
   bf16* out;            // [T, H, L]
   const float* sinks;
+  const int* topk;      // [T, topk_stride] key positions of every token (first one negative: all keys), or null
+  int topk_k, topk_stride;
   int H, L, D, page, max_blocks, window, vsplit, head_blocks;
   int k_slots, v_bufs;  // ring slots for score-only chunks, buffers for value chunks
   int q_rows;           // rows of the query tile kept in shared memory (decoding: the heads of one token)
@@ -130,6 +134,19 @@ __device__ __forceinline__ void tma_box(uint32_t smem_dst, const CUtensorMap* tm
       : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(leader)
       : "memory");
 }
+// four rows of a tensor map whose box is one row high, one behind the other
+__device__ __forceinline__ void tma_gather4(uint32_t smem_dst, const CUtensorMap* tmap, uint32_t bar, int x, int r0, int r1, int r2,
+                                            int r3, uint32_t leader) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %8, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t"
+      "}\n"
+      :
+      : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(leader)
+      : "memory");
+}
 __device__ __forceinline__ void commit(uint32_t bar, uint32_t leader) {
   asm volatile(
       "{\n\t"
@@ -151,9 +168,10 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
       : "memory");
 }
 
+template <bool LISTS>
 __global__ void __launch_bounds__(kThreads, 1)
 latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
-                      const TcArgs a) {
+                      const __grid_constant__ CUtensorMap tm_row, const TcArgs a) {
   constexpr uint32_t kIdescS = umma_idesc(kRows, NK, 1, 1);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -188,7 +206,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int ctx = a.ctx_lens[b];
   const int h0 = hb * kRows;
   const int heads = a.H - h0 < kRows ? a.H - h0 : kRows;  // heads per token of this tile
-  const int tpt = a.H <= kRows ? kRows / a.H : 1;         // tokens per tile
+  const int tpt = !LISTS && a.H <= kRows ? kRows / a.H : 1;  // tokens per tile
   const int tok0 = tile * tpt;
   if (tok0 >= len) return;  // uniform for the CTA, before any barrier or allocation
   const int ntok = len - tok0 < tpt ? len - tok0 : tpt;
@@ -197,8 +215,14 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int pos0 = ctx - len + tok0;
   const int hi = pos0 + ntok;  // keys [lo, hi) are visible to some row
   const int lo = (a.window > 0 && pos0 - a.window + 1 > 0) ? pos0 - a.window + 1 : 0;
-  const int t_begin = lo / NK;
-  const int n_tiles = __shfl_sync(0xffffffffu, ceil_div(hi, NK) - t_begin, 0);
+  const int* list = nullptr;  // of this CTA's token
+  if constexpr (LISTS) {
+    list = a.topk + static_cast<int64_t>(t0 + tok0) * a.topk_stride;
+    if (list[0] < 0) list = nullptr;
+  }
+  const bool listed = LISTS && list != nullptr;
+  const int t_begin = listed ? 0 : lo / NK;
+  const int n_tiles = __shfl_sync(0xffffffffu, ceil_div(listed ? a.topk_k : hi, NK) - t_begin, 0);
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -268,13 +292,36 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
       return row;
     };
+    auto listed_row = [&](int j) {  // cache row of entry j of the list; entries that name no visible key are masked
+      int kp = j < a.topk_k ? list[j] : 0;
+      if (kp < 0 || kp > pos0) kp = 0;
+      const int bi = kp / a.page;
+      int64_t blk = bi < a.max_blocks ? bt[bi] : -1;
+      if (blk < 0 || blk >= a.num_blocks) {
+        if (a.status) atomicCAS(a.status, 0, PXL_DEV_BAD_BLOCK_PREFILL);
+        blk = 0;
+      }
+      return static_cast<int>(blk * a.page + kp % a.page);
+    };
+    // chunk of 64 columns from column x of the tile's 64 listed rows (two in every lane)
+    auto gather = [&](uint32_t dst, uint32_t bar, int x, int row, int row2) {
+#pragma unroll
+      for (int g = 0; g < NK / 4; ++g) {
+        const int from = g < 8 ? row : row2, l = g % 8 * 4;
+        tma_gather4(dst + g * 512, &tm_row, bar, x, __shfl_sync(0xffffffffu, from, l), __shfl_sync(0xffffffffu, from, l + 1),
+                    __shfl_sync(0xffffffffu, from, l + 2), __shfl_sync(0xffffffffu, from, l + 3), leader);
+      }
+    };
     int slot = 0, slot_use = 0, vb = 0, vb_use = 0;
-    int row = tile_row(0);
+    int row = listed ? listed_row(lane) : tile_row(0), row2 = listed ? listed_row(lane + 32) : 0;
     for (int it = 0; ok && it < n_tiles; ++it) {
-      const int next_row = tile_row(it + 1);  // its table reads are in flight while this tile is issued
+      // its table reads are in flight while this tile is issued
+      const int next_row = listed ? listed_row((it + 1) * NK + lane) : tile_row(it + 1);
+      const int next_row2 = listed ? listed_row((it + 1) * NK + 32 + lane) : 0;
       for (int j = 0; ok && j < nkc; ++j) {
         ok = acquire(k_empty + 8 * slot, k_full + 8 * slot, slot_use, kKvChunk);
-        if (ok)
+        if (ok && listed) gather(sm_k + slot * kKvChunk, k_full + 8 * slot, k_chunk(j) * 64, row, row2);
+        else if (ok)
           for (int p = 0; p < pieces; ++p)
             tma_box(sm_k + slot * kKvChunk + p * box * 128, &tm_kv, k_full + 8 * slot, k_chunk(j) * 64,
                     __shfl_sync(0xffffffffu, row, p), leader);
@@ -285,7 +332,9 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
       if (!ok) break;
       ok = acquire(v_empty + 8 * vb, v_full + 8 * vb, vb_use, nv * kKvChunk);
-      if (ok)
+      if (ok && listed)
+        for (int c = 0; c < nv; ++c) gather(sm_v + (vb * per + c) * kKvChunk, v_full + 8 * vb, (v0 + c) * 64, row, row2);
+      else if (ok)
         for (int p = 0; p < pieces; ++p) {
           const int r = __shfl_sync(0xffffffffu, row, p);
           for (int c = 0; c < nv; ++c)
@@ -296,6 +345,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         ++vb_use;
       }
       row = next_row;
+      row2 = next_row2;
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
@@ -386,6 +436,16 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t lane_sel = static_cast<uint32_t>(warp * 32) << 16;
     float m_run = -INFINITY, l_run = 0.f;
     int failed = 0;
+    // of the listed keys of a tile, those that are visible (a bit each)
+    auto visible = [&](int it, uint32_t (&seen)[2]) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int j = it * NK + half * 32 + lane, kp = j < a.topk_k ? list[j] : -1;
+        seen[half] = __ballot_sync(0xffffffffu, kp >= 0 && kp <= pos0);
+      }
+    };
+    uint32_t seen[2] = {0u, 0u};
+    if (listed) visible(0, seen);
     for (int it = 0; it < n_tiles; ++it) {
       const int par = it & 1;
       failed = mbar_wait_bounded(s_full + 8 * par, (it >> 1) & 1, abort_flag, a.status, PXL_DEV_TIMEOUT_TMEM_FULL) ? 0 : 1;
@@ -398,7 +458,16 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tmem_ld_32x32b_x32(tm_s + par * NK + c + lane_sel, *reinterpret_cast<uint32_t(*)[32]>(&sc[c]));
       tmem_ld_wait();
       const int key0 = (t_begin + it) * NK;
-      const int ma = key_lo - key0, me = key_hi - key0;  // this row sees columns [ma, me)
+      int ma = key_lo - key0, me = key_hi - key0;  // this row sees columns [ma, me)
+      if (listed) {
+        ma = 0, me = NK;
+        if ((seen[0] & seen[1]) != 0xffffffffu) {
+#pragma unroll
+          for (int j = 0; j < NK; ++j)
+            if (!(seen[j >> 5] >> (j & 31) & 1u)) sc[j] = 0xff800000u;  // -inf
+        }
+        if (it + 1 < n_tiles) visible(it + 1, seen);
+      }
       if (!__all_sync(0xffffffffu, ma <= 0 && me >= NK)) {
 #pragma unroll
         for (int j = 0; j < NK; ++j)
@@ -538,9 +607,9 @@ PXL_EXPORT int pxl_latent_attn_tc_supported(int L, int R, int page, float scale)
 }
 
 PXL_EXPORT int pxl_latent_attn_tc(const void* q, const void* cache, const int* block_tables, const int* cu_q,
-                                  const int* ctx_lens, void* out, const float* sinks, int B, int max_q, int total_q, int H,
-                                  int L, int R, int page, int max_blocks, int64_t num_blocks, float scale, int window,
-                                  int* status, cudaStream_t stream) {
+                                  const int* ctx_lens, void* out, const float* sinks, const int* topk, int topk_k, int topk_stride,
+                                  int B, int max_q, int total_q, int H, int L, int R, int page, int max_blocks, int64_t num_blocks,
+                                  float scale, int window, int* status, cudaStream_t stream) {
   if (B <= 0 || max_q <= 0 || total_q <= 0) return PXL_OK;
   if (H <= 0 || B > 65535 || !pxl_latent_attn_tc_supported(L, R, page, scale)) return PXL_ERR_INVALID_ARG;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15)
@@ -549,7 +618,8 @@ PXL_EXPORT int pxl_latent_attn_tc(const void* q, const void* cache, const int* b
   TcArgs a{};
   TilePlan plan;
   // short queries (decoding) leave most of the tile's rows empty: keep only the others, and more keys in flight
-  const int rows = max_q * (H < kRows ? H : kRows);
+  if (topk && (topk_k <= 0 || window > 0)) return PXL_ERR_INVALID_ARG;
+  const int rows = (topk ? 1 : max_q) * (H < kRows ? H : kRows);
   a.q_rows = rows >= kRows ? kRows : pxl::ceil_div(rows, 8) * 8;
   if (!plan_tiles(L, L + R, a.q_rows, page, &plan)) return PXL_ERR_INVALID_ARG;
   a.k_slots = plan.k_slots;
@@ -559,26 +629,31 @@ PXL_EXPORT int pxl_latent_attn_tc(const void* q, const void* cache, const int* b
   a.ctx_lens = ctx_lens;
   a.out = static_cast<pxl::bf16*>(out);
   a.sinks = sinks;
+  a.topk = topk, a.topk_k = topk_k, a.topk_stride = topk_stride;
   a.H = H, a.L = L, a.D = L + R, a.page = page, a.max_blocks = max_blocks, a.window = window, a.num_blocks = num_blocks;
   a.vsplit = pxl::ceil_div(pxl::ceil_div(L, 64), kMaxV);
   a.head_blocks = pxl::ceil_div(H, kRows);
   a.scale_log2 = scale * kLog2eF;
   a.status = status;
-  CUtensorMap tq, tkv;
+  CUtensorMap tq, tkv, trow;
   if (!pxl_host::make_tmap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, static_cast<uint64_t>(total_q) * H, a.D, a.D,
                               a.q_rows, 64) ||
       !pxl_host::make_tmap_2d(&tkv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cache, static_cast<uint64_t>(num_blocks) * page, a.D,
-                              a.D, page < NK ? page : NK, 64))
+                              a.D, page < NK ? page : NK, 64) ||
+      !pxl_host::make_tmap_2d(&trow, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, cache, static_cast<uint64_t>(num_blocks) * page, a.D,
+                              a.D, 1, 64))
     return PXL_ERR_TENSORMAP;
-  const int tpt = H <= kRows ? kRows / H : 1;
+  const int tpt = !topk && H <= kRows ? kRows / H : 1;
   const dim3 grid(pxl::ceil_div(max_q, tpt) * a.vsplit, a.head_blocks, B);
   static bool configured[64] = {false};
   const int dev = pxl_host::current_device_slot();
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess)
+    if (cudaFuncSetAttribute(latent_attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(latent_attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess)
       return PXL_ERR_CUDA;
     configured[dev] = true;
   }
-  pxl_host::launch(latent_attn_tc_kernel, grid, dim3(kThreads), plan.smem, stream, tq, tkv, a);
+  pxl_host::launch(topk ? latent_attn_tc_kernel<true> : latent_attn_tc_kernel<false>, grid, dim3(kThreads), plan.smem, stream, tq, tkv,
+                   trow, a);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

@@ -437,11 +437,13 @@ int pxl_latent_queries(const void* q, int64_t ldq, int heads, int q_width, int q
 int pxl_latent_attn(const void* q, const void* cache, const int* block_tables, const int* cu_q, const int* ctx_lens,
                     void* out, const float* sinks, int B, int max_q, int H, int L, int R, int page, int max_blocks,
                     int64_t num_blocks, float scale, int window, int is_f32, int* status, pxl_stream_t stream);
-// bf16 tensor-core form of pxl_latent_attn (L and R multiples of 8, L + R <= 576, scale > 0; total_q = rows of q).
+// bf16 tensor-core form of pxl_latent_attn (L and R multiples of 8, L + R <= 576, scale > 0; total_q = rows of q). topk (or
+// null) [total_q, topk_stride]: topk_k key positions that a token attends to, all keys where the first is negative; no window.
 int pxl_latent_attn_tc_supported(int L, int R, int page, float scale);
 int pxl_latent_attn_tc(const void* q, const void* cache, const int* block_tables, const int* cu_q, const int* ctx_lens,
-                       void* out, const float* sinks, int B, int max_q, int total_q, int H, int L, int R, int page,
-                       int max_blocks, int64_t num_blocks, float scale, int window, int* status, pxl_stream_t stream);
+                       void* out, const float* sinks, const int* topk, int topk_k, int topk_stride, int B, int max_q,
+                       int total_q, int H, int L, int R, int page, int max_blocks, int64_t num_blocks, float scale, int window,
+                       int* status, pxl_stream_t stream);
 
 // ---- matrix_memory.cu: mLSTM ------------------------------------------------------------------------------
 // q, k [T, H x dk] and v [T, H x dv] are columns of proj; gates [T, ldg] fp32: H input gates | H forget gates before

@@ -4,7 +4,7 @@ DeepSeek-V3.2 / GLM-MoE-DSA (latent attention over the top-k keys of a lightning
 Attention runs in absorbed form for decode and prefill: the per-head up-projections of
 ``kv_b_proj`` are folded into the query (``W_UK``) and the output (``W_UV``), so the paged cache
 holds only ``[latent 512 | rope 64]`` per token and one kernel serves every case
-(:func:`parallax_b200.ops.mla_attn`). The reference keeps the same compressed cache but expands
+(:func:`parallax_b200.ops.latent_attn`; page sizes that it does not take: :func:`parallax_b200.ops.mla_attn`). The reference keeps the same compressed cache but expands
 K/V for prefill (``src/parallax/models/deepseek_v3.py:74-83,158-171``); its indexer and sparse
 attention are ``src/parallax/models/deepseek_v32.py:84-238,376-446``. Per-layer indexer modes
 ("full" layers score keys, "shared" layers reuse the previous full layer's selection) follow
@@ -285,16 +285,40 @@ class DeepseekStage(DecoderStage):
         topk = topk_prev
         if self.dsa and lw.idx_mode == "full":
             topk = self._index_topk(lw, li, qr, kv, fb)
-        q_lat, q_pe = ops.mla_q_absorb(q, lw.w_uk_s, self.cos_sin, fb.positions, H, self.nope, self.L)
         Tp = fb.num_prefill_tokens
-        o_lat = None
+        if not self._rows_form(cache):
+            q_lat, q_pe = ops.mla_q_absorb(q, lw.w_uk_s, self.cos_sin, fb.positions, H, self.nope, self.L)
+            o_lat = None
+            if Tp:
+                o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.p_block_tables, fb.p_cu_q, fb.positions, self.scale, 0, Tp,
+                                     topk=topk)
+            if fb.num_decode:
+                o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.d_block_tables, None, fb.positions, self.scale, Tp,
+                                     fb.num_decode, topk=topk, out=o_lat)
+            return ops.mla_unabsorb(o_lat, lw.w_uv_s, T), topk
+        # token-major rows: the per-head products read and write them in place, without head-major copies or padding
+        L, R, V = self.L, self.R, self.V
+        q_cat = torch.empty((T, H, L + R), dtype=q.dtype, device=q.device)
+        ops.latent_queries(q, H, self.qd, self.nope, self.cos_sin, fb.positions, q_cat, L, R, R)
+        ops.head_linear(q, self.qd, lw.w_uk_s, H, q_cat[:, :, :L])
+        o_lat = torch.empty((T, H, L), dtype=q.dtype, device=q.device)
         if Tp:
-            o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.p_block_tables, fb.p_cu_q, fb.positions, self.scale, 0, Tp,
-                                 topk=topk)
+            ops.latent_attn(q_cat[:Tp], cache, fb.p_block_tables, fb.p_cu_q, fb.p_ctx_lens, self.scale, L, max_q=fb.p_max_q,
+                            max_ctx=fb.p_max_ctx, out=o_lat[:Tp], topk=None if topk is None else topk[:Tp])
         if fb.num_decode:
-            o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.d_block_tables, None, fb.positions, self.scale, Tp,
-                                 fb.num_decode, topk=topk, out=o_lat)
-        return ops.mla_unabsorb(o_lat, lw.w_uv_s, T), topk
+            ops.latent_attn(q_cat[Tp:], cache, fb.d_block_tables, None, fb.d_ctx_lens, self.scale, L, max_ctx=fb.d_max_ctx,
+                            out=o_lat[Tp:], topk=None if topk is None else topk[Tp:])
+        heads = torch.empty((T, H, V), dtype=q.dtype, device=q.device)
+        ops.head_linear(o_lat.view(T, H * L), L, lw.w_uv_s, H, heads)
+        return heads.view(T, H * V), topk
+
+    def _rows_form(self, cache: torch.Tensor) -> bool:
+        """Whether attention runs on token-major rows (the tensor-core kernel takes the page size) or on head-major ones."""
+        if not cache.is_cuda:
+            return True
+        from parallax_b200.ops import cuda as cu
+
+        return cu.latent_attn_takes(self.L, self.R, cache.shape[-2], self.scale)
 
     def forward_layers(self, h: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         eps = self.cfg.rms_norm_eps

@@ -125,8 +125,8 @@ _SIGS = {
     "pxl_latent_attn": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int64, c_float,
                         c_int, c_int, _P, _P],
     "pxl_latent_attn_tc_supported": [c_int, c_int, c_int, c_float],
-    "pxl_latent_attn_tc": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int64,
-                           c_float, c_int, _P, _P],
+    "pxl_latent_attn_tc": [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                           c_int64, c_float, c_int, _P, _P],
     "pxl_gemm_bf16_act_glu": [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int64, c_int, _P, _P],
     "pxl_gemm_simt_grouped": [_P, _P, _P, _P, c_int, c_int, c_int64, c_int64, c_int64, _P, _P, _P, _P, c_int, c_int, _P],
     "pxl_residual_add": [_P, _P, c_int64, _P, c_int64, c_int64, _P, _P, c_int, _P, _P, _P, c_int, c_int, c_float,

@@ -1195,8 +1195,13 @@ def head_linear(x, x_head_stride: int, w, heads: int, out, gate=None):
     return out
 
 
+def latent_attn_takes(latent: int, rot_dim: int, page: int, scale: float) -> bool:
+    """Whether :func:`latent_attn` runs these sizes on the tensor cores (the form that takes key lists)."""
+    return bool(_lib.lib().pxl_latent_attn_tc_supported(latent, rot_dim, page, scale))
+
+
 def latent_attn(q_cat, cache, block_tables, cu_q, ctx_lens, scale: float, latent: int, window: int = 0, sinks=None,
-                max_q: int = 1, max_ctx: int = 0, out=None):
+                max_q: int = 1, max_ctx: int = 0, out=None, topk=None):
     T, H, D = q_cat.shape
     page, B = cache.shape[-2], ctx_lens.numel()
     assert q_cat.is_contiguous() and cache.is_contiguous() and cache.shape[-1] == D and q_cat.dtype == cache.dtype
@@ -1204,14 +1209,18 @@ def latent_attn(q_cat, cache, block_tables, cu_q, ctx_lens, scale: float, latent
         out = torch.empty((T, H, latent), dtype=q_cat.dtype, device=q_cat.device)
     assert out.is_contiguous() and out.shape == (T, H, latent)
     if q_cat.dtype == torch.bfloat16 and not (q_cat.data_ptr() | out.data_ptr() | cache.data_ptr()) & 15 \
-            and _lib.lib().pxl_latent_attn_tc_supported(latent, D - latent, page, scale):
+            and latent_attn_takes(latent, D - latent, page, scale):
+        assert topk is None or (topk.dtype == torch.int32 and topk.shape[0] == T and topk.stride(1) == 1)
         check(_lib.lib().pxl_latent_attn_tc(q_cat.data_ptr(), cache.data_ptr(), block_tables.data_ptr(), _ptr(cu_q),
-                                            ctx_lens.data_ptr(), out.data_ptr(), _ptr(sinks), B, max_q, T, H, latent,
-                                            D - latent, page, block_tables.shape[1], cache.shape[0], float(scale), window,
+                                            ctx_lens.data_ptr(), out.data_ptr(), _ptr(sinks), _ptr(topk),
+                                            0 if topk is None else topk.shape[1], 0 if topk is None else topk.stride(0), B, max_q,
+                                            T, H, latent, D - latent, page, block_tables.shape[1], cache.shape[0], float(scale), window,
                                             status_tensor(q_cat.device).data_ptr(), _stream(q_cat.device)),
               "pxl_latent_attn_tc")
         _count()
         return out
+    if topk is not None:
+        raise ValueError("latent attention over key lists needs bf16 rows and a page size that the tensor-core kernel takes")
     check(_lib.lib().pxl_latent_attn(q_cat.data_ptr(), cache.data_ptr(), block_tables.data_ptr(), _ptr(cu_q),
                                      ctx_lens.data_ptr(), out.data_ptr(), _ptr(sinks), B, max_q, H, latent, D - latent,
                                      page, block_tables.shape[1], cache.shape[0], float(scale), window,

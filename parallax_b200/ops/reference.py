@@ -756,10 +756,11 @@ def head_linear(x, x_head_stride: int, w, heads: int, out, gate=None):
 
 
 def latent_attn(q_cat, cache, block_tables, cu_q, ctx_lens, scale: float, latent: int, window: int = 0, sinks=None,
-                max_q: int = 1, max_ctx: int = 0, out=None):
+                max_q: int = 1, max_ctx: int = 0, out=None, topk=None):
     """Causal attention of ``q_cat [T, H, latent + R]`` over cached rows ``latent | R``; the values are the latent
     parts. ``cu_q`` None: one query per sequence. ``window`` keys per query (0: all); ``sinks [H]`` fp32 add
-    ``exp(sink)`` to the denominator. ``out [T, H, latent]``."""
+    ``exp(sink)`` to the denominator. ``topk [T, k]`` int32: the positions that a token attends to (all where the first is
+    negative; no window). ``out [T, H, latent]``."""
     T, H, _ = q_cat.shape
     page = cache.shape[-2]
     flat = cache.view(-1, cache.shape[-1])
@@ -776,6 +777,11 @@ def latent_attn(q_cat, cache, block_tables, cu_q, ctx_lens, scale: float, latent
         s = torch.einsum("thk,sk->hts", q_cat[t0:t1].float(), rows) * scale
         dist = pos[:, None] - keys[None, :]
         keep = (dist >= 0) & (dist < window) if window > 0 else dist >= 0
+        if topk is not None:
+            lists = topk[t0:t1].long()
+            chosen = torch.zeros((t1 - t0, ctx + 1), dtype=torch.bool, device=s.device)
+            chosen.scatter_(1, torch.where((lists < 0) | (lists >= ctx), ctx, lists), True)      # (entries that name no key: parked)
+            keep = keep & (chosen[:, :ctx] | (lists[:, :1] < 0))
         s = s.masked_fill(~keep, float("-inf"))
         if sinks is not None:
             s = torch.cat([s, sinks.float().view(H, 1, 1).expand(H, t1 - t0, 1)], -1)

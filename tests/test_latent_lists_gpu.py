@@ -1,0 +1,53 @@
+"""Latent attention over key lists (an indexer's choice) on the tensor cores, against the fp32 restatement."""
+
+import pytest
+import torch
+
+from parallax_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,k,page,prompts,decode", [
+    (128, 64, 16, [(5, 300)], [70, 129, 1]),         # whole tiles; a context shorter than the list
+    (128, 200, 64, [(3, 256)], [201]),               # a last tile that is not full
+    (8, 48, 8, [(40, 40), (2, 130)], [64]),          # fewer heads than rows: one token per tile; prompts from the start
+    (192, 96, 128, [], [100, 500]),                  # two blocks of heads, pages longer than a tile
+])
+def test_latent_attention_over_lists(H, k, page, prompts, decode):
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(H + k)
+    L, R, scale = 512, 64, 192 ** -0.5
+    ctx = [c for _n, c in prompts] + decode
+    need = [-(-c // page) for c in ctx]
+    blocks = torch.randperm(sum(need) + 3).int()
+    table = torch.zeros(len(ctx), max(need), dtype=torch.int32)
+    at = 0
+    for i, n in enumerate(need):
+        table[i, :n], at = blocks[at:at + n], at + n
+    cache = torch.randn(sum(need) + 3, 1, page, L + R).bfloat16()
+    lens = [n for n, _c in prompts]
+    for part in ("prompts", "decode"):
+        if not (prompts if part == "prompts" else decode):
+            continue
+        first, seqs = (0, prompts) if part == "prompts" else (len(prompts), [(1, c) for c in decode])
+        T = sum(n for n, _c in seqs)
+        pos = torch.cat([torch.arange(c - n, c) for n, c in seqs])
+        lists = torch.full((T, k), -1, dtype=torch.int32)
+        for t in range(T):
+            n = int(pos[t]) + 1
+            if n > k:
+                lists[t] = torch.randperm(n)[:k].int()
+                if t % 2:       # an empty entry and a key that is not there yet
+                    lists[t, 1], lists[t, 2] = -1, n + 1
+        q = (torch.randn(T, H, L + R) * 0.5).bfloat16()
+        cu_q = torch.tensor([0] + lens).cumsum(0).int() if part == "prompts" else None
+        args = (cache, table[first:first + len(seqs)].contiguous(), cu_q, torch.tensor([c for _n, c in seqs]).int())
+        kw = dict(max_q=max(n for n, _c in seqs), max_ctx=max(c for _n, c in seqs))
+        want = ref.latent_attn(q, *args, scale, L, topk=lists, **kw)
+        gpu = [a if a is None else a.cuda() for a in args]
+        got = cu.latent_attn(q.cuda(), *gpu, scale, L, topk=lists.cuda(), **kw).cpu()
+        cu.check_status(torch.device("cuda", 0))
+        # probabilities and outputs are rounded to bf16 (2^-9 each)
+        assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
