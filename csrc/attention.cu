@@ -630,6 +630,300 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   }
 }
 
+// ---- decode over e4m3 pages, TMA-fed (D = 128; page_size 16, 32 or 64) -------------------------------------
+// The pages stay bytes up to the fragments: a tile of 64 tokens is 8 KB of K and 8 KB of V (one 128-byte swizzled row per
+// token), so the same shared memory holds twice the tiles of the kernel above, and an operand is converted once, by the thread
+// that multiplies it. Widening 8 bytes at a time into shared memory on the way in (the kernel without TMA) took 1170 us for 128
+// rows x 3600 keys x 8 heads, 0.8 TB/s, bound by issue; this one takes 224 us, 4.2 TB/s.
+//
+// e4m3 becomes f16 with one instruction per two values, exactly, and the products are f16 ones. The other operands fit f16
+// without loss that bf16 would not have: a row of q is scaled by a power of two that puts its largest value at 2^13 (undone in
+// the score's scale); probabilities carry a factor of 2^10, so that what bf16 would keep of the small ones is kept, and the
+// rounding of the large ones is 2^-11 instead of 2^-9.
+//   K: which columns a k-step of the MMA takes is free as long as q takes the same. Lane t of a quad takes columns 32 t .. 32 t
+//      + 31 of its token as two 16-byte loads, four per k-step.
+//   V: ldmatrix.trans moves pairs of columns; a byte permutation puts the two tokens of a column side by side, so that one
+//      n-tile holds the even columns of 16 and the next the odd ones.
+constexpr int kE4Stages = 6;
+constexpr int kE4Tile = TILE * 128;  // bytes of K (or V) of a tile
+constexpr float kPShift = 10.f;      // log2 of the factor on the probabilities
+
+__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"(static_cast<unsigned short>(two)));
+  return r;
+}
+__device__ __forceinline__ void mma_m16n8k16_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
+      "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+__global__ void __launch_bounds__(kDecThreads, 2)
+attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                        const bf16* __restrict__ q, int64_t q_stride, const int* __restrict__ block_tables,
+                        const int* __restrict__ ctx_lens, bf16* __restrict__ out, float* __restrict__ workspace,
+                        const float* __restrict__ sinks, int Hq, int Hkv, int page_size, int max_blocks,
+                        int64_t num_blocks, float scale_log2, int window, int keep, int num_splits, float v_scale, int* status) {
+  constexpr int D = 128;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const uint32_t stage0 = smem_u32(smem);  // stage s: K at s * 2 * kE4Tile, V behind it
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kE4Stages * 2 * kE4Tile);  // full[S], empty[S]
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kE4Stages);
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kE4Stages);
+  pdl_wait();
+  pdl_launch_dependents();
+
+  const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
+  const int G = Hq / Hkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int hi = ctx_lens[b];
+  const int lo = (window > 0 && hi > window) ? hi - window : 0;
+  const KeyTiles tiles(lo, hi, keep);
+  const int per_split = ceil_div(tiles.total, num_splits);
+  const int t_begin = split * per_split;
+  const int t_end = min(tiles.total, t_begin + per_split);
+  const int n_tiles = t_end > t_begin ? t_end - t_begin : 0;
+  const int* bt = block_tables + static_cast<size_t>(b) * max_blocks;
+  const int ppt = TILE / page_size;  // pages per tile
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < kE4Stages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 4);  // one arrival per consumer warp
+    }
+    mbar_fence_init();
+    fence_proxy_async_smem();
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  __syncthreads();
+
+  int failed = 0;
+  if (warp == 4) {  // producer: lane p looks up the block of page p of the tile and issues its two boxes
+    for (int it = 0; it < n_tiles; ++it) {
+      const int stage = it % kE4Stages;
+      int blk = 0;
+      if (lane < ppt) {
+        int bi = tiles[t_begin + it] * ppt + lane;
+        if (bi * page_size >= hi) bi = (hi - 1) / page_size;  // beyond the context: re-read the last page (masked)
+        blk = bi < max_blocks ? bt[bi] : -1;
+        if (blk < 0 || blk >= num_blocks) {
+          if (status) atomicCAS(status, 0, PXL_DEV_BAD_BLOCK_DECODE);
+          blk = 0;
+        }
+      }
+      int okf = 1;
+      if (it >= kE4Stages && lane == 0)
+        okf = mbar_wait_bounded(empty0 + 8 * stage, ((it / kE4Stages) - 1) & 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY) ? 1 : 0;
+      okf = __shfl_sync(0xffffffffu, okf, 0);
+      if (!okf) {
+        failed = 1;
+        break;
+      }
+      const uint32_t bar = full0 + 8 * stage, dst = stage0 + stage * 2 * kE4Tile + lane * page_size * 128;
+      if (lane == 0) mbar_arrive_expect_tx(bar, 2 * kE4Tile);
+      __syncwarp();
+      if (lane < ppt) {
+        const int row0 = (blk * Hkv + kvh) * page_size;
+        tma_load_2d(dst, &tm_k, bar, 0, row0);
+        tma_load_2d(dst + kE4Tile, &tm_v, bar, 0, row0);
+      }
+    }
+  }
+
+  // Q fragments: row r of the MMA tile is q head kvh * G + r (rows >= G are zero), scaled per row
+  const int g8 = lane >> 2, t4 = lane & 3;
+  uint32_t qf[D / 16][4];
+  float row_scale[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = g8 + h * 8;
+    float mx = 0.f;
+    if (r < G) {
+      const bf16* row = q + static_cast<size_t>(b) * q_stride + (kvh * G + r) * D + t4 * 32;
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks) {
+        qf[ks][h] = *reinterpret_cast<const uint32_t*>(row + ks * 4);
+        qf[ks][2 + h] = *reinterpret_cast<const uint32_t*>(row + ks * 4 + 2);
+        const float2 x = unpack_bf16x2(qf[ks][h]), y = unpack_bf16x2(qf[ks][2 + h]);
+        mx = fmaxf(fmaxf(fmaxf(mx, fabsf(x.x)), fabsf(x.y)), fmaxf(fabsf(y.x), fabsf(y.y)));
+      }
+    } else {
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks) qf[ks][h] = qf[ks][2 + h] = 0u;
+    }
+    mx = quad_max(mx);
+    int up = 267 - static_cast<int>(__float_as_uint(mx) >> 23);  // exponent bits of the factor: the largest value to [2^13, 2^14)
+    up = up < 1 ? 1 : up > 253 ? 253 : up;
+    const float f = __uint_as_float(static_cast<uint32_t>(up) << 23);
+    row_scale[h] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23) * scale_log2;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const float2 x = unpack_bf16x2(qf[ks][2 * p + h]);
+        qf[ks][2 * p + h] = pack_f16x2(x.x * f, x.y * f);
+      }
+  }
+  float o[D / 8][4];
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  float m_run[2] = {-INFINITY, -INFINITY};
+  float l_run[2] = {0.f, 0.f};
+
+  for (int it = 0; warp < 4 && it < n_tiles; ++it) {
+    const int stage = it % kE4Stages;
+    if (!mbar_wait_bounded(full0 + 8 * stage, (it / kE4Stages) & 1, abort_flag, status, PXL_DEV_TIMEOUT_FULL)) {
+      failed = 1;
+      break;  // reported to the whole CTA at the barrier behind the loop
+    }
+    const uint32_t k_smem = stage0 + stage * 2 * kE4Tile, v_smem = k_smem + kE4Tile;
+    const int r0 = warp * 16;
+    const int tok_base = tiles[t_begin + it] * TILE + r0;
+    if (tok_base < hi && (tok_base + 16 > lo || tok_base < keep)) {  // warp-uniform
+      float s[2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {  // 8 tokens each
+        s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        const int row = r0 + j * 8 + g8;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t w[4];
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                       : "r"(k_smem + row * 128 + (((t4 * 2 + c) ^ (row & 7)) << 4)));
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            mma_m16n8k16_f16(s[j], qf[c * 4 + i], e4m3x2_to_f16x2(w[i] & 0xffffu), e4m3x2_to_f16x2(w[i] >> 16));
+        }
+      }
+      float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int tok = tok_base + j * 8 + 2 * t4 + (e & 1);
+          const bool valid = tok < hi && (tok >= lo || tok < keep);
+          s[j][e] = valid ? s[j][e] * row_scale[e >> 1] : -INFINITY;
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
+        }
+      }
+      float corr[2], m_use[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        mx[h] = quad_max(mx[h]);
+        const float m_new = fmaxf(m_run[h], mx[h]);
+        m_use[h] = (m_new == -INFINITY) ? 0.f : m_new;
+        corr[h] = exp2f(m_run[h] - m_use[h]);
+        m_run[h] = m_new;
+      }
+      float ps[2] = {0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[j][e] = exp2f(s[j][e] - m_use[e >> 1] + kPShift);
+          ps[e >> 1] += s[j][e];
+        }
+      l_run[0] = l_run[0] * corr[0] + ps[0];
+      l_run[1] = l_run[1] * corr[1] + ps[1];
+      if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i) {
+          o[i][0] *= corr[0];
+          o[i][1] *= corr[0];
+          o[i][2] *= corr[1];
+          o[i][3] *= corr[1];
+        }
+      }
+      uint32_t pf[4];
+      pf[0] = pack_f16x2(s[0][0], s[0][1]);
+      pf[1] = pack_f16x2(s[0][2], s[0][3]);
+      pf[2] = pack_f16x2(s[1][0], s[1][1]);
+      pf[3] = pack_f16x2(s[1][2], s[1][3]);
+      const int mi = lane >> 3, row = r0 + (mi & 1) * 8 + (lane & 7);
+#pragma unroll
+      for (int c = 0; c < 8; c += 2) {  // 16 columns per 16-byte chunk
+        uint32_t r[4];  // chunk c: tokens 0-7, 8-15; chunk c + 1: the same
+        ldmatrix_x4_trans(r, v_smem + row * 128 + (((c + (mi >> 1)) ^ (row & 7)) << 4));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);  // even column of both tokens | odd column
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          mma_m16n8k16_f16(o[(c + h) * 2], pf, e4m3x2_to_f16x2(r[2 * h] & 0xffffu), e4m3x2_to_f16x2(r[2 * h + 1] & 0xffffu));
+          mma_m16n8k16_f16(o[(c + h) * 2 + 1], pf, e4m3x2_to_f16x2(r[2 * h] >> 16), e4m3x2_to_f16x2(r[2 * h + 1] >> 16));
+        }
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty0 + 8 * stage);  // this warp is done with the stage
+  }
+  if (__syncthreads_or(failed)) {
+    // loads that are still in flight must land before the CTA's shared memory is released
+    __nanosleep(200000);
+    return;
+  }
+
+  // ---- merge the four warps' partial softmax states through shared memory
+  float* o_sm = reinterpret_cast<float*>(smem);          // [4][16][D]
+  float* m_sm = o_sm + 4 * 16 * D;                       // [4][16]
+  float* l_sm = m_sm + 4 * 16;                           // [4][16]
+  l_run[0] = quad_sum(l_run[0]);
+  l_run[1] = quad_sum(l_run[1]);
+  if (warp < 4) {
+    float* ow = o_sm + warp * 16 * D;
+#pragma unroll
+    for (int i = 0; i < D / 8; i += 2) {  // accumulator columns 2 t, 2 t + 1 of an even and an odd tile: columns 4 t .. 4 t + 3
+      const int c = i * 8 + t4 * 4;
+      *reinterpret_cast<float4*>(ow + g8 * D + c) = make_float4(o[i][0], o[i + 1][0], o[i][1], o[i + 1][1]);
+      *reinterpret_cast<float4*>(ow + (g8 + 8) * D + c) = make_float4(o[i][2], o[i + 1][2], o[i][3], o[i + 1][3]);
+    }
+    if (t4 == 0) {
+      m_sm[warp * 16 + g8] = m_run[0];
+      m_sm[warp * 16 + g8 + 8] = m_run[1];
+      l_sm[warp * 16 + g8] = l_run[0];
+      l_sm[warp * 16 + g8 + 8] = l_run[1];
+    }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; warp < 4 && idx < G * D; idx += 128) {
+    const int r = idx / D, d = idx % D;
+    const int head = kvh * G + r;
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) M = fmaxf(M, m_sm[w * 16 + r]);
+    const float sink = (sinks && num_splits == 1) ? sinks[head] * kLog2e : -INFINITY;
+    const float Mx = fmaxf(M, sink);
+    const float Mu = (Mx == -INFINITY) ? 0.f : Mx;
+    float L = 0.f, acc = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float f = exp2f(m_sm[w * 16 + r] - Mu);
+      L += l_sm[w * 16 + r] * f;
+      acc += o_sm[(w * 16 + r) * D + d] * f;
+    }
+    if (num_splits == 1) {
+      const float denom = L + exp2f(sink - Mu + kPShift);
+      out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(denom > 0.f ? acc / denom * v_scale : 0.f);
+    } else {
+      float* po = workspace;
+      float* plse = workspace + static_cast<size_t>(gridDim.y) * Hq * num_splits * D;
+      const size_t row = (static_cast<size_t>(b) * Hq + head) * num_splits + split;
+      po[row * D + d] = L > 0.f ? acc / L * v_scale : 0.f;
+      if (d == 0) plse[row] = L > 0.f ? Mu + log2f(L) - kPShift : -INFINITY;
+    }
+  }
+}
+
 template <int D, int SM = kPlain>
 __global__ void __launch_bounds__(D)
 attn_decode_reduce_kernel(const float* __restrict__ workspace, const float* __restrict__ sinks,
@@ -909,6 +1203,29 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
     else if (mode == kCapped) PXL_DEC_TMA(kCapped)
     else PXL_DEC_TMA(kPlain)
 #undef PXL_DEC_TMA
+    return check_launch();
+  }
+  if (cache_fp8 && D == 128 && (page_size == 16 || page_size == 32 || page_size == 64) &&
+      num_blocks * Hkv * page_size < (1ll << 31) &&
+      ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0) {
+    CUtensorMap tk, tv;
+    const uint64_t rows = static_cast<uint64_t>(num_blocks) * Hkv * page_size;
+    if (!pxl_host::make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k_cache, rows, 128, 128, page_size, 128) ||
+        !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, v_cache, rows, 128, 128, page_size, 128))
+      return PXL_ERR_TENSORMAP;
+    constexpr int SMEM = 1024 + kE4Stages * 2 * kE4Tile + 128;
+    static bool done[64] = {false}; /* function attributes are per device */
+    const int dev = pxl_host::current_device_slot();
+    if (!done[dev]) {
+      if (set_smem(attn_decode_e4m3_kernel, SMEM)) return PXL_ERR_CUDA;
+      done[dev] = true;
+    }
+    pxl_host::launch(attn_decode_e4m3_kernel, grid, kDecThreads, SMEM, stream, tk, tv, static_cast<const bf16*>(q), q_stride,
+                     block_tables, ctx_lens, static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks,
+                     scale_log2 * k_scale, window, keep_first, num_splits, v_scale, status);
+    if (num_splits > 1)
+      pxl_host::launch(attn_decode_reduce_kernel<128, kPlain>, dim3(Hq, B), 128, 0, stream, workspace, sinks,
+                       static_cast<bf16*>(out), Hq, num_splits);
     return check_launch();
   }
 #define PXL_DEC(DD, F8, M)                                                                       \

@@ -1,0 +1,39 @@
+"""Decode attention over e4m3 pages with f16 products: rows of q far from one, probabilities far below the largest, sinks and
+splits, against the fp32 restatement."""
+
+import pytest
+import torch
+
+from parallax_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("Hq,Hkv,page,window,sinks,splits,q_scale", [
+    (16, 1, 16, 0, False, 1, 1.0),          # sixteen heads of a group: every row of the product
+    (8, 4, 32, 0, True, 1, 1e4),            # scores of hundreds: one key takes all
+    (8, 4, 64, 0, True, 3, 1e-6),           # equal weights
+    (5, 5, 16, 70, False, 2, 3.0),
+])
+def test_decode_over_e4m3_pages(Hq, Hkv, page, window, sinks, splits, q_scale):
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(Hq * page)
+    D, ctx = 128, [1, 15, 64, 65, 129, 700]
+    need = [-(-c // page) for c in ctx]
+    ids, at = torch.randperm(sum(need)).int(), 0
+    table = torch.zeros(len(ctx), max(need), dtype=torch.int32)
+    for i, n in enumerate(need):
+        table[i, :n], at = ids[at:at + n], at + n
+    k, v = (torch.randn(sum(need), Hkv, page, D).to(torch.float8_e4m3fn) for _ in range(2))
+    q = (torch.randn(len(ctx), Hq, D) * q_scale).bfloat16()
+    q[0] = 0.0
+    q[:, 0, 1:] = q[:, 0, 1:] * 2 ** -12    # one large element beside small ones
+    s = torch.randn(Hq) if sinks else None
+    kw = dict(window=window, num_splits=splits, max_ctx=max(ctx), kv_scale=(0.5, 3.0))
+    cl = torch.tensor(ctx).int()
+    got = cu.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), cl.cuda(), D ** -0.5, sinks=None if s is None else s.cuda(), **kw)
+    cu.check_status(torch.device("cuda", 0))
+    want = ref.attn_decode(q, k, v, table, cl, D ** -0.5, window=window, sinks=s, kv_scale=(0.5, 3.0))
+    # one rounding of the output to bf16 (2^-9) on either side; probabilities are rounded to 2^-11
+    assert float((got.cpu().float() - want.float()).norm() / want.float().norm()) < 2 ** -7
