@@ -4,8 +4,8 @@
 //
 // The reference scores one context token per threadgroup (dsa_indexer.metal:34-116, launch in
 // dsa_indexer.cpp:153-196) and selects the top-k with a framework argpartition
-// (parallax_extensions/ops.py:361-367). Here one CTA scores a tile of 64 keys for all index
-// heads with tensor-core MMAs, and a radix select picks the k best positions per query row
+// (parallax_extensions/ops.py:361-367). Here one CTA scores 128 keys for all index
+// heads of a group of tokens with tensor-core MMAs, and a radix select picks the k best positions per query row
 // without sorting.
 #include "common.cuh"
 #include "pxl_api.h"
@@ -15,7 +15,7 @@ using namespace pxl;
 
 constexpr int kDi = 128;          // index head dim
 constexpr int kHiMax = 64;        // index heads handled per CTA (one pass)
-constexpr int kKeyTile = 64;
+constexpr int kKeyTile = 64;      // rows of the score matrix are padded to this
 constexpr int kPitch = kDi + 8;   // smem row pitch (elements)
 
 __device__ __forceinline__ int find_seq(const int* cu_q, int B, int t) {
@@ -27,85 +27,118 @@ __device__ __forceinline__ int find_seq(const int* cu_q, int B, int t) {
   return lo;
 }
 
-// grid (key tiles, T), 128 threads: warp w owns index heads [16w, 16w+16)
-__global__ void __launch_bounds__(128) dsa_scores_kernel(const bf16* __restrict__ q, const float* __restrict__ w,
-                                                         const bf16* __restrict__ cache,
-                                                         const int* __restrict__ block_tables,
-                                                         const int* __restrict__ cu_q,
-                                                         const int* __restrict__ positions,
-                                                         float* __restrict__ scores, int64_t ld_scores, int B,
-                                                         int Hi, int max_blocks, int page) {
-  __shared__ __align__(16) bf16 q_s[kHiMax * kPitch];
-  __shared__ __align__(16) bf16 k_s[kKeyTile * kPitch];
-  __shared__ float acc[kKeyTile];
-  const int t = blockIdx.y;
-  const int j0 = blockIdx.x * kKeyTile;
-  const int pos = positions[t];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float* out = scores + static_cast<size_t>(t) * ld_scores;
-  if (j0 > pos) {  // whole tile beyond the causal limit
-    if (tid < kKeyTile) out[j0 + tid] = -INFINITY;
-    return;
-  }
-  const int seq = cu_q ? find_seq(cu_q, B, t) : t;
-  const int* bt = block_tables + static_cast<size_t>(seq) * max_blocks;
-  for (int c = tid; c < kHiMax * (kDi / 8); c += 128) {
-    const int r = c / (kDi / 8), ch = c % (kDi / 8);
-    cp_async_16(smem_u32(&q_s[r * kPitch + ch * 8]), q + (static_cast<size_t>(t) * Hi + (r < Hi ? r : 0)) * kDi + ch * 8,
-                r < Hi);
-  }
-  for (int c = tid; c < kKeyTile * (kDi / 8); c += 128) {
-    const int r = c / (kDi / 8), ch = c % (kDi / 8);
-    const int kp = j0 + r;
-    const bf16* src = cache;
-    if (kp <= pos) src = cache + (static_cast<size_t>(bt[kp / page]) * page + kp % page) * kDi + ch * 8;
-    cp_async_16(smem_u32(&k_s[r * kPitch + ch * 8]), src, kp <= pos);
-  }
-  cp_async_commit();
-  if (tid < kKeyTile) acc[tid] = 0.f;
-  cp_async_wait<0>();
-  __syncthreads();
+// One CTA scores 128 keys for a group of consecutive tokens. Keys are the rows of the products and index heads the columns: a
+// warp keeps the fragments of its 32 keys in registers for as long as the tokens are of one sequence (a token costs its queries,
+// 16 KB of shared memory, and no key is read again), and the weighted sum over the heads stays inside a thread up to two
+// shuffles. With a CTA per token and 64 keys, queries and keys were loaded anew for each 64 x 64 product and the sum over the
+// heads went through shuffles of every accumulator and shared-memory atomics: 640 us for 1000 tokens x 5500 keys beside 16 x 8000,
+// 324 us this way.
+constexpr int kScoreKeys = 128, kScoreThreads = 128;
 
+struct ScoreSmem {
+  bf16 k[kScoreKeys * kPitch];
+  bf16 q[2][kHiMax * kPitch];
+};
+
+// grid (key tiles, groups of `group` tokens)
+__global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* __restrict__ q, const float* __restrict__ w,
+                                                                   const bf16* __restrict__ cache,
+                                                                   const int* __restrict__ block_tables,
+                                                                   const int* __restrict__ cu_q,
+                                                                   const int* __restrict__ positions,
+                                                                   float* __restrict__ scores, int64_t ld_scores, int T, int B,
+                                                                   int Hi, int max_blocks, int page, int group) {
+  extern __shared__ __align__(16) uint8_t raw[];
+  ScoreSmem& sm = *reinterpret_cast<ScoreSmem*>(raw);
+  const int j0 = blockIdx.x * kScoreKeys;
+  const int first = blockIdx.y * group, last = first + group < T ? first + group : T;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, qd = lane & 3, mi = lane >> 3;
-  float s[8][4];
-#pragma unroll
-  for (int n = 0; n < 8; ++n)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) s[n][k] = 0.f;
-  const uint32_t q_base = smem_u32(&q_s[(warp * 16 + (lane & 15)) * kPitch + (lane >> 4) * 8]);
-#pragma unroll
-  for (int ks = 0; ks < kDi / 16; ++ks) {
-    uint32_t qa[4];
-    ldmatrix_x4(qa, q_base + ks * 32);
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {
-      uint32_t kb[4];
-      ldmatrix_x4(kb, smem_u32(&k_s[(np * 16 + (mi >> 1) * 8 + (lane & 7)) * kPitch + ks * 16 + (mi & 1) * 8]));
-      const uint32_t b0[2] = {kb[0], kb[1]};
-      const uint32_t b1[2] = {kb[2], kb[3]};
-      mma_m16n8k16_bf16(s[2 * np], qa, b0);
-      mma_m16n8k16_bf16(s[2 * np + 1], qa, b1);
+  auto load_q = [&](int t, int buf) {
+    if (t < last) {
+      for (int c = tid; c < kHiMax * (kDi / 8); c += kScoreThreads) {
+        const int r = c / (kDi / 8), ch = c % (kDi / 8);
+        cp_async_16(smem_u32(&sm.q[buf][r * kPitch + ch * 8]), q + (static_cast<size_t>(t) * Hi + (r < Hi ? r : 0)) * kDi + ch * 8,
+                    r < Hi);
+      }
     }
+    cp_async_commit();
+  };
+  int seq = -1, seq_end = first;  // tokens of the sequence in registers: up to seq_end
+  uint32_t kf[2][kDi / 16][4];
+  load_q(first, 0);
+  for (int t = first; t < last; ++t) {
+    const int buf = (t - first) & 1, pos = positions[t];
+    __syncthreads();  // the other buffer's queries were read
+    load_q(t + 1, buf ^ 1);
+    float* out = scores + static_cast<size_t>(t) * ld_scores;
+    const bool seen = j0 <= pos;
+    if (seen && t >= seq_end) {
+      seq = cu_q ? find_seq(cu_q, B, t) : t;
+      seq_end = cu_q ? cu_q[seq + 1] : t + 1;
+      if (seq_end > T) seq_end = T;
+      const int limit = positions[(seq_end < last ? seq_end : last) - 1];  // the group's last token of the sequence sees the most
+      const int* bt = block_tables + static_cast<size_t>(seq) * max_blocks;
+      for (int c = tid; c < kScoreKeys * (kDi / 8); c += kScoreThreads) {
+        const int r = c / (kDi / 8), ch = c % (kDi / 8);
+        const int kp = j0 + r;
+        const bf16* src = cache;
+        if (kp <= limit) src = cache + (static_cast<size_t>(bt[kp / page]) * page + kp % page) * kDi + ch * 8;
+        cp_async_16(smem_u32(&sm.k[r * kPitch + ch * 8]), src, kp <= limit);
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ks = 0; ks < kDi / 16; ++ks)
+          ldmatrix_x4(kf[m][ks], smem_u32(&sm.k[(warp * 32 + m * 16 + (lane & 15)) * kPitch + ks * 16 + (lane >> 4) * 8]));
+    } else {
+      cp_async_wait<1>();
+      __syncthreads();
+    }
+    float part[2][2] = {};
+    if (seen) {
+      const float* wt = w + static_cast<size_t>(t) * Hi;
+#pragma unroll 1
+      for (int np = 0; np < kHiMax / 16; ++np) {  // 16 heads
+        float s[2][2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < kDi / 16; ++ks) {
+          uint32_t qb[4];
+          ldmatrix_x4(qb, smem_u32(&sm.q[buf][(np * 16 + (mi >> 1) * 8 + (lane & 7)) * kPitch + ks * 16 + (mi & 1) * 8]));
+          const uint32_t b0[2] = {qb[0], qb[1]}, b1[2] = {qb[2], qb[3]};
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            mma_m16n8k16_bf16(s[m][0], kf[m][ks], b0);
+            mma_m16n8k16_bf16(s[m][1], kf[m][ks], b1);
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const int h = np * 16 + n * 8 + qd * 2;
+          const float w0 = h < Hi ? wt[h] : 0.f, w1 = h + 1 < Hi ? wt[h + 1] : 0.f;
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              part[m][e] += fmaxf(s[m][n][2 * e], 0.f) * w0 + fmaxf(s[m][n][2 * e + 1], 0.f) * w1;
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float v = part[m][e];
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        const int j = j0 + warp * 32 + m * 16 + e * 8 + g;
+        if (qd == 0 && j < ld_scores) out[j] = j <= pos ? v : -INFINITY;
+      }
   }
-  const int h_lo = warp * 16 + g, h_hi = h_lo + 8;
-  const float w_lo = h_lo < Hi ? w[static_cast<size_t>(t) * Hi + h_lo] : 0.f;
-  const float w_hi = h_hi < Hi ? w[static_cast<size_t>(t) * Hi + h_hi] : 0.f;
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    float c0 = fmaxf(s[n][0], 0.f) * w_lo + fmaxf(s[n][2], 0.f) * w_hi;
-    float c1 = fmaxf(s[n][1], 0.f) * w_lo + fmaxf(s[n][3], 0.f) * w_hi;
-#pragma unroll
-    for (int off = 4; off < 32; off <<= 1) {  // sum over the 8 row groups of the warp
-      c0 += __shfl_xor_sync(0xffffffffu, c0, off);
-      c1 += __shfl_xor_sync(0xffffffffu, c1, off);
-    }
-    if (g == 0) {
-      atomicAdd(&acc[n * 8 + qd * 2], c0);
-      atomicAdd(&acc[n * 8 + qd * 2 + 1], c1);
-    }
-  }
-  __syncthreads();
-  if (tid < kKeyTile) out[j0 + tid] = (j0 + tid <= pos) ? acc[tid] : -INFINITY;
+  cp_async_wait<0>();
 }
 
 __device__ __forceinline__ uint32_t order_key(float x) {
@@ -264,12 +297,23 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
                                     int max_blocks, int page, int max_ctx, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (Di != kDi || Hi <= 0 || Hi > kHiMax || max_ctx <= 0) return PXL_ERR_INVALID_ARG;
-  const int tiles = pxl::ceil_div(max_ctx, kKeyTile);
-  if (static_cast<int64_t>(tiles) * kKeyTile > ld_scores) return PXL_ERR_INVALID_ARG;
-  dim3 grid(tiles, T);
-  dsa_scores_kernel<<<grid, 128, 0, stream>>>(static_cast<const pxl::bf16*>(q), w,
-                                              static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q,
-                                              positions, scores, ld_scores, B, Hi, max_blocks, page);
+  if (static_cast<int64_t>(pxl::ceil_div(max_ctx, kKeyTile)) * kKeyTile > ld_scores) return PXL_ERR_INVALID_ARG;
+  static bool done[64] = {false};
+  const int dev = pxl_host::current_device_slot();
+  if (!done[dev]) {
+    if (cudaFuncSetAttribute(dsa_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ScoreSmem)) != cudaSuccess)
+      return PXL_ERR_CUDA;
+    done[dev] = true;
+  }
+  const int tiles = pxl::ceil_div(max_ctx, kScoreKeys);
+  // prompts: as many tokens per CTA as still leave every SM three of them, and no more than bring anything; decoded tokens have
+  // a sequence each
+  int group = cu_q ? static_cast<int>(static_cast<int64_t>(T) * tiles / (3 * pxl_host::num_sms())) : 1;
+  group = group < 1 ? 1 : group > 16 ? 16 : group;
+  while (pxl::ceil_div(T, group) > 65535) group *= 2;
+  dsa_scores_kernel<<<dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream>>>(
+      static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
+      ld_scores, T, B, Hi, max_blocks, page, group);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
