@@ -27,3 +27,22 @@ def test_fp8_product_and_row_quantisation(M, N, K):
     got, want = cu.linear_fp8(x.cuda(), w.cuda(), s.cuda()).cpu(), ref.linear_fp8(x, w, s)
     cu.check_status(torch.device("cuda", 0))
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (64, 256, 4096), (100, 128, 2304), (130, 256, 2176)])
+@pytest.mark.parametrize("epi", ["plain", "residual", "glu"])
+def test_fp8_product_split_over_a_cluster(M, N, K, epi):
+    """Few output tiles: K in ranges (also of unequal lengths), the rows of a tile shared out over the CTAs that add them."""
+    from parallax_b200.loader.quant import quantize_fp8_block
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(M + N + K)
+    x, r = torch.randn(M, K).bfloat16(), torch.randn(M, N).bfloat16()
+    w, s = quantize_fp8_block(torch.randn(N, K) * 0.05, (64, 128))
+    kw = dict(residual=r) if epi == "residual" else dict(epi=ref.EPI_SILU_MUL) if epi == "glu" else {}
+    want = ref.linear_fp8(x, w, s, **kw)
+    kw = {n: v.cuda() if isinstance(v, torch.Tensor) else v for n, v in kw.items()}
+    got = [cu.linear_fp8(x.cuda(), w.cuda(), s.cuda(), **kw).cpu() for _ in range(2)]
+    cu.check_status(torch.device("cuda", 0))
+    assert float((got[0].float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+    assert torch.equal(*got)        # added in K order
