@@ -268,6 +268,96 @@ qk_norm_rope_cache_kernel(bf16* __restrict__ qkv, const bf16* __restrict__ q_nor
   }
 }
 
+// The same by 16-byte vectors: 8 elements per lane, D / 8 lanes per head, a block per token whose lane groups take its heads in
+// turn with the token's cosines and sines in registers. A rotation pairs lane l with l +- rot_dim / 16, so nothing goes through
+// shared memory. 5903 rows x 48 heads: 50 us, 2.9 TB/s read and written (86 us with a warp per head and four 2-byte accesses a lane).
+template <int D, bool FP8>
+__global__ void __launch_bounds__(256)
+qk_norm_rope_rows_kernel(bf16* __restrict__ qkv, const bf16* __restrict__ q_norm_w, const bf16* __restrict__ k_norm_w,
+                         const float* __restrict__ cos_sin, const int* __restrict__ positions,
+                         const int64_t* __restrict__ slot_mapping, void* __restrict__ k_cache, void* __restrict__ v_cache, int Hq,
+                         int Hkv, int rot_dim, int page_size, int64_t num_slots, float eps, float w_offset, float k_inv_scale,
+                         float v_inv_scale, int max_pos, int* status) {
+  constexpr int LPH = D / 8, kGroups = 256 / LPH;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, group = threadIdx.x / LPH, l = threadIdx.x % LPH, e0 = l * 8;
+  const int heads = Hq + 2 * Hkv, half = rot_dim >> 1;
+  bf16* row = qkv + static_cast<size_t>(t) * heads * D;
+  const int64_t slot = slot_mapping ? slot_mapping[t] : -1;
+  if (slot >= num_slots && status && threadIdx.x == 0) atomicCAS(status, 0, PXL_DEV_BAD_SLOT);
+  const int p = rot_dim > 0 ? positions[t] : 0;
+  const bool p_ok = p >= 0 && (max_pos <= 0 || p < max_pos);
+  if (rot_dim > 0 && !p_ok && status && threadIdx.x == 0) atomicCAS(status, 0, PXL_DEV_BAD_POSITION);
+  const bool turned = rot_dim > 0 && p_ok;  // a position outside the table is reported, its row is left unrotated
+  const bool mine = turned && e0 < rot_dim, low = e0 < half;
+  float cs[8], sn[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) cs[j] = sn[j] = 0.f;
+  if (mine) {
+    const float* c = cos_sin + static_cast<size_t>(p) * rot_dim + (low ? e0 : e0 - half);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cs[j] = c[j], sn[j] = c[half + j];
+  }
+  const int lane = threadIdx.x & 31, partner = mine ? (low ? lane + half / 8 : lane - half / 8) : lane;
+  int64_t cache_row = -1;  // of head 0
+  if (slot >= 0 && slot < num_slots) cache_row = (slot / page_size * Hkv) * page_size + slot % page_size;
+  for (int h0 = 0; h0 < heads; h0 += kGroups) {  // (every lane of a warp stays in for the shuffles)
+    const int hs = h0 + group;
+    const bool in = hs < heads, is_q = hs < Hq, is_k = !is_q && hs < Hq + Hkv;
+    const bf16x8 zero8 = {{0u, 0u, 0u, 0u}};
+    const bf16x8 x = in ? ld_bf16x8(row + hs * D + e0) : zero8;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16x2(x.u[j]);
+      v[2 * j] = f.x, v[2 * j + 1] = f.y;
+    }
+    const bf16* nw = is_q ? q_norm_w : is_k ? k_norm_w : nullptr;
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+#pragma unroll
+    for (int o = 1; o < LPH; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (nw) {
+      const float inv = rsqrtf(ss / static_cast<float>(D) + eps);
+      const bf16x8 w = ld_bf16x8(nw + e0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {  // match a bf16 module: the normalised value is rounded before RoPE
+        const float2 f = unpack_bf16x2(w.u[j]);
+        v[2 * j] = __bfloat162float(__float2bfloat16(v[2 * j] * inv * (f.x + w_offset)));
+        v[2 * j + 1] = __bfloat162float(__float2bfloat16(v[2 * j + 1] * inv * (f.y + w_offset)));
+      }
+    }
+    if (turned) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float other = __shfl_sync(0xffffffffu, v[j], partner);
+        if (mine && (is_q || is_k)) v[j] = v[j] * cs[j] + (low ? -other : other) * sn[j];
+      }
+    }
+    if (!in) continue;
+    bf16x8 o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.u[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+    if (is_q) {
+      st_bf16x8(row + hs * D + e0, o);
+      continue;
+    }
+    if (cache_row < 0) continue;
+    const int64_t at = (cache_row + static_cast<int64_t>(is_k ? hs - Hq : hs - Hq - Hkv) * page_size) * D + e0;
+    if constexpr (FP8) {
+      const float inv = is_k ? k_inv_scale : v_inv_scale;
+      uint32_t b[2] = {0u, 0u};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[j >> 2] |= static_cast<uint32_t>(to_e4m3(v[j] * inv)) << (8 * (j & 3));
+      *reinterpret_cast<uint2*>(static_cast<uint8_t*>(is_k ? k_cache : v_cache) + at) = make_uint2(b[0], b[1]);
+    } else {
+      st_bf16x8(static_cast<bf16*>(is_k ? k_cache : v_cache) + at, o);
+    }
+  }
+}
+
 // ------------------------------------------------------------ plain cache scatter
 template <bool FP8>
 __global__ void __launch_bounds__(256)
@@ -425,6 +515,27 @@ int qk_norm_rope_cache_impl(void* qkv, const void* q_norm_w, const void* k_norm_
                             float v_inv_scale, int max_pos, int* status, pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
   if (rot_dim > D || (rot_dim & 1)) return PXL_ERR_INVALID_ARG;
+  // vectors of 16 bytes: whole lanes on either side of a rotation, rows, weights and pages aligned
+  const auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  if ((D == 64 || D == 128 || D == 256) && rot_dim % 16 == 0 && !off16(qkv) && !off16(q_norm_w) && !off16(k_norm_w) &&
+      !off16(k_cache) && !off16(v_cache)) {
+#define PXL_QKROWS(DD, F8)                                                                                                    \
+  pxl_host::launch(qk_norm_rope_rows_kernel<DD, F8>, T, 256, 0, stream, static_cast<bf16*>(qkv),                              \
+                   static_cast<const bf16*>(q_norm_w), static_cast<const bf16*>(k_norm_w), cos_sin, positions, slot_mapping,  \
+                   k_cache, v_cache, Hq, Hkv, rot_dim, page_size, num_slots, eps, norm_w_offset, k_inv_scale, v_inv_scale,    \
+                   max_pos, status)
+    if (cache_fp8) {
+      if (D == 64) PXL_QKROWS(64, true);
+      else if (D == 128) PXL_QKROWS(128, true);
+      else PXL_QKROWS(256, true);
+    } else {
+      if (D == 64) PXL_QKROWS(64, false);
+      else if (D == 128) PXL_QKROWS(128, false);
+      else PXL_QKROWS(256, false);
+    }
+#undef PXL_QKROWS
+    return check_launch();
+  }
   const int64_t warps = static_cast<int64_t>(T) * (Hq + 2 * Hkv);
   const unsigned grid = static_cast<unsigned>((warps + 7) / 8);
 #define PXL_QKROPE(DD)                                                                        \
