@@ -15,6 +15,7 @@
 #include <cuda_fp8.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "attention_score.cuh"
 #include "common.cuh"
@@ -376,10 +377,60 @@ attn_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const void* __r
 // of its own (warp 4) and the stages are handed back through "empty" mbarriers (one arrival per
 // consumer warp), so the consumer warps never meet at a CTA-wide barrier inside the loop: with the
 // producer inside warp 0 and a __syncthreads per tile the top stall was that barrier.
+// ---- split-KV results met inside a thread-block cluster (2 to 8 splits): the CTAs of a (sequence, key head) leave their partial
+// outputs, maxima and sums in shared memory, and each adds a share of the columns over all of them. Saves the workspace's round
+// trip and a kernel whose launch is most of its 4 to 5 us, once per layer of a chat.
+constexpr int kMaxClusterSplits = 8;
+
+__device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_map_shared(smem_u32(p), rank)) : "memory");
+  return v;
+}
+
+// part_o [G][128] relative to the maxima part_m [G], sums part_l [G] (scaled by 2^shift, like part_o). Every thread of every CTA of
+// the cluster calls this, also after a failed wait.
+template <int SM>
+__device__ __forceinline__ void add_splits(const float* part_o, const float* part_m, const float* part_l, int splits, int rank, int G,
+                                           int head0, const float* sinks, float shift, float v_scale, bf16* out) {
+  constexpr int D = 128;
+  cluster_sync_all();
+  const int share = ceil_div(G * D, splits), end = min(G * D, (rank + 1) * share);
+  for (int idx = rank * share + threadIdx.x; threadIdx.x < 128 && idx < end; idx += 128) {
+    const int r = idx / D, head = head0 + r;
+    float acc = 0.f;
+    if constexpr (SM == kSigmoid) {
+      for (int s = 0; s < splits; ++s) acc += ld_cluster_f32(part_o + idx, s);
+      out[static_cast<size_t>(head) * D + idx % D] = __float2bfloat16(acc);
+    } else {
+      const float sink = sinks ? sinks[head] * kLog2e : -INFINITY;
+      float m[kMaxClusterSplits], M = sink;
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s) {
+        m[s] = s < splits ? ld_cluster_f32(part_m + r, s) : -INFINITY;
+        M = fmaxf(M, m[s]);
+      }
+      const float Mu = (M == -INFINITY) ? 0.f : M;
+      float denom = exp2f(sink - Mu + shift);
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s) {
+        if (s >= splits) break;
+        const float f = exp2f(m[s] - Mu);
+        denom += ld_cluster_f32(part_l + r, s) * f;
+        acc += ld_cluster_f32(part_o + idx, s) * f;
+      }
+      out[static_cast<size_t>(head) * D + idx % D] = __float2bfloat16(denom > 0.f ? acc / denom * v_scale : 0.f);
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // nobody leaves while its parts are being read
+}
+
 constexpr int kDecStages = 3;
 constexpr int kDecThreads = 160;  // 4 consumer warps + 1 producer warp
 
-template <int SM>
+// CLUSTER: the splits of a (sequence, key head) are a cluster and add their results (add_splits); else through the workspace
+template <int SM, bool CLUSTER>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const bf16* __restrict__ q, int64_t q_stride, const int* __restrict__ block_tables,
@@ -565,6 +616,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   if (__syncthreads_or(failed)) {
     // loads that are still in flight must land before the CTA's shared memory is released
     __nanosleep(200000);
+    if constexpr (CLUSTER) {  // the other CTAs of the cluster wait for this one
+      cluster_sync_all();
+      cluster_sync_all();
+    }
     return;
   }
 
@@ -592,6 +647,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       l_sm[warp * 16 + r_hi] = l_run[1];
     }
   }
+  float* part_o = l_sm + 4 * 16;  // [16][D]: behind the warps' results
+  float *part_m = part_o + 16 * D, *part_l = part_m + 16;
   __syncthreads();
   for (int idx = threadIdx.x; warp < 4 && idx < G * D; idx += 128) {
     const int r = idx / D, d = idx % D;
@@ -600,6 +657,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       float acc = 0.f;
 #pragma unroll
       for (int w = 0; w < 4; ++w) acc += o_sm[(w * 16 + r) * D + d];
+      if constexpr (CLUSTER) {
+        part_o[idx] = acc;
+        continue;
+      }
       if (num_splits == 1) out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(acc);
       else workspace[((static_cast<size_t>(b) * Hq + head) * num_splits + split) * D + d] = acc;
       continue;
@@ -607,7 +668,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < 4; ++w) M = fmaxf(M, m_sm[w * 16 + r]);
-    const float sink = (sinks && num_splits == 1) ? sinks[head] * kLog2e : -INFINITY;
+    const float sink = (!CLUSTER && sinks && num_splits == 1) ? sinks[head] * kLog2e : -INFINITY;
     const float Mx = fmaxf(M, sink);
     const float Mu = (Mx == -INFINITY) ? 0.f : Mx;
     float L = 0.f, acc = 0.f;
@@ -617,7 +678,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       L += l_sm[w * 16 + r] * f;
       acc += o_sm[(w * 16 + r) * D + d] * f;
     }
-    if (num_splits == 1) {
+    if constexpr (CLUSTER) {
+      part_o[idx] = acc;
+      if (d == 0) part_m[r] = M, part_l[r] = L;
+    } else if (num_splits == 1) {
       const float denom = L + exp2f(sink - Mu);
       out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(denom > 0.f ? acc / denom : 0.f);
     } else {
@@ -627,6 +691,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       po[row * D + d] = L > 0.f ? acc / L : 0.f;
       if (d == 0) plse[row] = L > 0.f ? Mu + log2f(L) : -INFINITY;
     }
+  }
+  if constexpr (CLUSTER) {
+    __syncwarp();
+    add_splits<SM>(part_o, part_m, part_l, num_splits, split, G, kvh * G, sinks, 0.f, 1.f, out + static_cast<size_t>(b) * Hq * D);
   }
 }
 
@@ -665,6 +733,7 @@ __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                         const bf16* __restrict__ q, int64_t q_stride, const int* __restrict__ block_tables,
@@ -870,6 +939,10 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   if (__syncthreads_or(failed)) {
     // loads that are still in flight must land before the CTA's shared memory is released
     __nanosleep(200000);
+    if constexpr (CLUSTER) {  // the other CTAs of the cluster wait for this one
+      cluster_sync_all();
+      cluster_sync_all();
+    }
     return;
   }
 
@@ -894,6 +967,8 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       l_sm[warp * 16 + g8 + 8] = l_run[1];
     }
   }
+  float* part_o = l_sm + 4 * 16;  // [16][D]: behind the warps' results
+  float *part_m = part_o + 16 * D, *part_l = part_m + 16;
   __syncthreads();
   for (int idx = threadIdx.x; warp < 4 && idx < G * D; idx += 128) {
     const int r = idx / D, d = idx % D;
@@ -901,7 +976,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < 4; ++w) M = fmaxf(M, m_sm[w * 16 + r]);
-    const float sink = (sinks && num_splits == 1) ? sinks[head] * kLog2e : -INFINITY;
+    const float sink = (!CLUSTER && sinks && num_splits == 1) ? sinks[head] * kLog2e : -INFINITY;
     const float Mx = fmaxf(M, sink);
     const float Mu = (Mx == -INFINITY) ? 0.f : Mx;
     float L = 0.f, acc = 0.f;
@@ -911,7 +986,10 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       L += l_sm[w * 16 + r] * f;
       acc += o_sm[(w * 16 + r) * D + d] * f;
     }
-    if (num_splits == 1) {
+    if constexpr (CLUSTER) {
+      part_o[idx] = acc;
+      if (d == 0) part_m[r] = M, part_l[r] = L;
+    } else if (num_splits == 1) {
       const float denom = L + exp2f(sink - Mu + kPShift);
       out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(denom > 0.f ? acc / denom * v_scale : 0.f);
     } else {
@@ -921,6 +999,10 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       po[row * D + d] = L > 0.f ? acc / L * v_scale : 0.f;
       if (d == 0) plse[row] = L > 0.f ? Mu + log2f(L) - kPShift : -INFINITY;
     }
+  }
+  if constexpr (CLUSTER) {
+    __syncwarp();
+    add_splits<kPlain>(part_o, part_m, part_l, num_splits, split, G, kvh * G, sinks, kPShift, v_scale, out + static_cast<size_t>(b) * Hq * D);
   }
 }
 
@@ -1160,6 +1242,38 @@ PXL_EXPORT int pxl_attn_decode_splits(int B, int Hkv, int max_ctx) {
 }
 
 namespace {
+// One kernel of the splits (grid.z): alone, as clusters that add their results, or with the reduction behind it.
+template <auto Alone, auto Together, auto Reduce, typename... Args>
+int launch_decode_splits(dim3 grid, int smem, int B, int Hq, const float* workspace, const float* sinks, void* out, cudaStream_t stream,
+                         Args... args) {
+  const int splits = static_cast<int>(grid.z);
+  static bool done[64] = {false};  // function attributes are per device
+  const int dev = pxl_host::current_device_slot();
+  if (!done[dev]) {
+    if (set_smem(Alone, smem) || set_smem(Together, smem)) return PXL_ERR_CUDA;
+    done[dev] = true;
+  }
+  if (splits == 1 || splits > kMaxClusterSplits) {
+    pxl_host::launch(Alone, grid, kDecThreads, smem, stream, args...);
+    if (splits > 1) pxl_host::launch(Reduce, dim3(Hq, B), 128, 0, stream, workspace, sinks, static_cast<bf16*>(out), Hq, splits);
+    return check_launch();
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kDecThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = static_cast<unsigned>(splits);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pxl_host::pdl_flag() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, Together, args...) == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
+}
+
 int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
                      const int* block_tables, const int* ctx_lens, void* out, float* workspace,
                      const float* sinks, int B, int Hq, int Hkv, int D, int page_size, int max_blocks,
@@ -1184,26 +1298,16 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v_cache, rows, 128, 128, page_size, 64))
       return PXL_ERR_TENSORMAP;
     constexpr int SMEM = 1024 + kDecStages * 2 * TILE * 128 * 2 + 128;
-#define PXL_DEC_TMA(M)                                                                                                  \
-  {                                                                                                                     \
-    static bool done[64] = {false}; /* function attributes are per device */                                            \
-    const int dev = pxl_host::current_device_slot();                                                                    \
-    if (!done[dev]) {                                                                                                   \
-      if (set_smem(attn_decode_tma_kernel<M>, SMEM)) return PXL_ERR_CUDA;                                               \
-      done[dev] = true;                                                                                                 \
-    }                                                                                                                   \
-    pxl_host::launch(attn_decode_tma_kernel<M>, grid, kDecThreads, SMEM, stream, tk, tv, static_cast<const bf16*>(q),   \
-                     q_stride, block_tables, ctx_lens, static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size,   \
-                     max_blocks, num_blocks, scale_log2, window, keep_first, num_splits, sa, status);                   \
-    if (num_splits > 1)                                                                                                 \
-      pxl_host::launch(attn_decode_reduce_kernel<128, M>, dim3(Hq, B), 128, 0, stream, workspace, sinks,                \
-                       static_cast<bf16*>(out), Hq, num_splits);                                                        \
-  }
-    if (mode == kSigmoid) PXL_DEC_TMA(kSigmoid)
-    else if (mode == kCapped) PXL_DEC_TMA(kCapped)
-    else PXL_DEC_TMA(kPlain)
-#undef PXL_DEC_TMA
-    return check_launch();
+    auto go = [&](auto sm) {
+      constexpr int M = decltype(sm)::value;
+      return launch_decode_splits<attn_decode_tma_kernel<M, false>, attn_decode_tma_kernel<M, true>, attn_decode_reduce_kernel<128, M>>(
+          grid, SMEM, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
+          static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2, window, keep_first,
+          num_splits, sa, status);
+    };
+    if (mode == kSigmoid) return go(std::integral_constant<int, kSigmoid>{});
+    if (mode == kCapped) return go(std::integral_constant<int, kCapped>{});
+    return go(std::integral_constant<int, kPlain>{});
   }
   if (cache_fp8 && D == 128 && (page_size == 16 || page_size == 32 || page_size == 64) &&
       num_blocks * Hkv * page_size < (1ll << 31) &&
@@ -1214,19 +1318,10 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, v_cache, rows, 128, 128, page_size, 128))
       return PXL_ERR_TENSORMAP;
     constexpr int SMEM = 1024 + kE4Stages * 2 * kE4Tile + 128;
-    static bool done[64] = {false}; /* function attributes are per device */
-    const int dev = pxl_host::current_device_slot();
-    if (!done[dev]) {
-      if (set_smem(attn_decode_e4m3_kernel, SMEM)) return PXL_ERR_CUDA;
-      done[dev] = true;
-    }
-    pxl_host::launch(attn_decode_e4m3_kernel, grid, kDecThreads, SMEM, stream, tk, tv, static_cast<const bf16*>(q), q_stride,
-                     block_tables, ctx_lens, static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks,
-                     scale_log2 * k_scale, window, keep_first, num_splits, v_scale, status);
-    if (num_splits > 1)
-      pxl_host::launch(attn_decode_reduce_kernel<128, kPlain>, dim3(Hq, B), 128, 0, stream, workspace, sinks,
-                       static_cast<bf16*>(out), Hq, num_splits);
-    return check_launch();
+    return launch_decode_splits<attn_decode_e4m3_kernel<false>, attn_decode_e4m3_kernel<true>, attn_decode_reduce_kernel<128, kPlain>>(
+        grid, SMEM, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
+        static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2 * k_scale, window, keep_first,
+        num_splits, v_scale, status);
   }
 #define PXL_DEC(DD, F8, M)                                                                       \
   {                                                                                              \

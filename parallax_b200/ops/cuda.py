@@ -429,6 +429,12 @@ def _attn_on_tensor_cores(q, k_cache, scale: float, max_group: int) -> bool:
     return q.dtype == torch.bfloat16 and q.shape[2] in (64, 128) and q.shape[1] // k_cache.shape[1] <= max_group and scale > 0
 
 
+def _decode_launches(splits: int, D: int, page: int) -> int:
+    """Kernels of one decode attention: a few splits add their results inside a cluster, more in a kernel of their own."""
+    together = D == 128 and page in (16, 32, 64) and splits <= 8
+    return 1 if splits == 1 or together else 2
+
+
 def attn_decode(
     q: torch.Tensor,
     k_cache: torch.Tensor,
@@ -475,7 +481,7 @@ def attn_decode(
                 float(kv_scale[0]), float(kv_scale[1]), status_tensor(q.device).data_ptr(), _stream(q.device)),
             "pxl_attn_decode_fp8",
         )
-        _count(2 if num_splits > 1 else 1)
+        _count(_decode_launches(num_splits, D, page))
         return out
     check(
         _lib.lib().pxl_attn_decode(
@@ -486,7 +492,7 @@ def attn_decode(
             softcap, _ptr(sigmoid_bias), status_tensor(q.device).data_ptr(), _stream(q.device)),
         "pxl_attn_decode",
     )
-    _count(2 if num_splits > 1 else 1)
+    _count(_decode_launches(num_splits, D, page))
     return out
 
 
