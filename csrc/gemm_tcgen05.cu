@@ -1427,6 +1427,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
        reinterpret_cast<uintptr_t>(C)) & 15)
     return PXL_ERR_INVALID_ARG;
   if (epi == PXL_EPI_RESIDUAL && residual == nullptr) return PXL_ERR_INVALID_ARG;
+  if (bn == 0 && pxl_gemv_bf16_takes(M, N, K, epi)) return pxl_gemv_bf16(A, W, C, residual, bias, M, N, K, lda, ldw, ldc, epi, stream);
   if (bn == 0 && pxl_gemm_bf16_uses_small_m(M, N, K, epi) &&
       !((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(bias)) & 15))
     return gemm_small_m(A, W, C, epi == PXL_EPI_F32, epi == PXL_EPI_RESIDUAL ? residual : nullptr, bias, M, N, K,

@@ -1,0 +1,219 @@
+// C[m, n] = sum_k A[m, k] W[n, k] for a handful of rows (one to a few requests decoding), bf16 with fp32 sums.
+//
+// Every weight is read once and used M times: bound by memory, so nothing of a tensor-core product helps and its costs remain
+// (tiles of 128 rows for M = 1, partial sums exchanged between the K ranges, TMA and TMEM set up per launch). Here a warp takes
+// R rows of W over the whole of K, 16 bytes a lane and eight such loads in flight, and the sums of its lanes meet in one
+// transposing shuffle reduction. The rows of A are shared by all warps and come from L1. Weights are not written by the kernel
+// before, so the first loads go out ahead of the wait for it (programmatic dependent launch): in a chain of small layers they
+// run under its tail.
+#include "common.cuh"
+#include "pxl_api.h"
+
+namespace {
+using namespace pxl;
+
+constexpr int kWarps = 4;
+
+struct GemvArgs {
+  const bf16 *A, *W, *residual, *bias;
+  void* C;
+  int M, N, K, lda, ldw, ldc;
+  const bf16* norm_w;  // NORM: [K]; rows of A times norm_w + norm_offset over their root mean square, rounded to bf16
+  float norm_eps, norm_offset;
+};
+
+__device__ __forceinline__ uint64_t widen(uint32_t two) {  // two bf16 -> two fp32 in a register pair
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(two << 16), "r"(two & 0xffff0000u));
+  return v;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// MM rows of A (the last ones repeated where M is smaller), R rows of W per warp, U steps of 256 columns in flight.
+// EPI: PXL_EPI_NONE, _RESIDUAL, _F32 or _SILU_MUL (R rows = R / 2 gate / up pairs, 64 rows apart in groups of 128)
+template <int MM, int R, int U, int EPI, bool NORM>
+__global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
+  constexpr bool kGlu = EPI == PXL_EPI_SILU_MUL;
+  const int lane = threadIdx.x & 31, wid = blockIdx.x * kWarps + (threadIdx.x >> 5);
+  const int n0 = wid * R;  // first row of W; pairs: 2 x first output column
+  if (n0 >= a.N) return;
+  int row[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int c = n0 / 2 + r / 2;
+    row[r] = kGlu ? c / 64 * 128 + c % 64 + (r & 1) * 64 : n0 + r;
+  }
+  uint4 w[U][R];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * 256 + lane * 8;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        w[u][r] = k < a.K ? __ldcs(reinterpret_cast<const uint4*>(a.W + static_cast<int64_t>(row[r]) * a.ldw + k)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  load(0);
+  pdl_wait();
+  pdl_launch_dependents();
+  float inv[MM];
+  if constexpr (NORM) {
+#pragma unroll
+    for (int m = 0; m < MM; ++m) {
+      const bf16* x = a.A + static_cast<int64_t>(m < a.M ? m : a.M - 1) * a.lda;
+      float ss = 0.f;
+      for (int k = lane * 8; k < a.K; k += 256) {
+        const bf16x8 v = ld_bf16x8(x + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = unpack_bf16x2(v.u[j]);
+          ss += f.x * f.x + f.y * f.y;
+        }
+      }
+      inv[m] = rsqrtf(warp_reduce_sum(ss) / static_cast<float>(a.K) + a.norm_eps);
+    }
+  }
+  uint64_t acc[MM][R] = {};
+  for (int k0 = 0; k0 < a.K; k0 += U * 256) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * 256 + lane * 8;
+      if (k >= a.K) break;
+      uint64_t wv[R][4];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        wv[r][0] = widen(w[u][r].x), wv[r][1] = widen(w[u][r].y), wv[r][2] = widen(w[u][r].z), wv[r][3] = widen(w[u][r].w);
+#pragma unroll
+      for (int m = 0; m < MM; ++m) {
+        uint4 xr = *reinterpret_cast<const uint4*>(a.A + static_cast<int64_t>(m < a.M ? m : a.M - 1) * a.lda + k);
+        if constexpr (NORM) {
+          const bf16x8 nw = ld_bf16x8(a.norm_w + k);
+          uint32_t* xw = &xr.x;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = unpack_bf16x2(xw[j]), g = unpack_bf16x2(nw.u[j]);
+            xw[j] = pack_bf16x2(f.x * inv[m] * (g.x + a.norm_offset), f.y * inv[m] * (g.y + a.norm_offset));
+          }
+        }
+        const uint64_t x[4] = {widen(xr.x), widen(xr.y), widen(xr.z), widen(xr.w)};
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[m][r] = fma2(wv[r][j], x[j], acc[m][r]);
+      }
+    }
+    if (k0 + U * 256 < a.K) load(k0 + U * 256);
+  }
+  // sums over the lanes: every exchange halves the numbers a lane holds, lanes V = MM * R apart end with the same one
+  constexpr int V = MM * R;
+  float v[V];
+#pragma unroll
+  for (int m = 0; m < MM; ++m)
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[m * R + r] = __uint_as_float(static_cast<uint32_t>(acc[m][r])) + __uint_as_float(static_cast<uint32_t>(acc[m][r] >> 32));
+  int o = 16;
+#pragma unroll
+  for (int n = V; n > 1; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n / 2; ++i) {
+      const float give = up ? v[i] : v[i + n / 2], keep = up ? v[i + n / 2] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  constexpr int kSpan = 32 / V;  // number i is in lanes [i * kSpan, (i + 1) * kSpan)
+  const int i = lane / kSpan, m = i / R, r = i % R;
+  float sum = v[0];
+  int col = n0 + r;
+  if constexpr (kGlu) {  // the up product sits kSpan lanes further
+    const float up = __shfl_down_sync(0xffffffffu, sum, kSpan);
+    sum = sum / (1.f + __expf(-sum)) * up;
+    col = (n0 + r) / 2;
+  }
+  if (lane % kSpan || m >= a.M || (kGlu && (r & 1))) return;
+  if (!kGlu && a.bias) sum += __bfloat162float(a.bias[col]);
+  const int64_t at = static_cast<int64_t>(m) * a.ldc + col;
+  if constexpr (EPI == PXL_EPI_F32) {
+    static_cast<float*>(a.C)[at] = sum;
+  } else {
+    if constexpr (EPI == PXL_EPI_RESIDUAL) sum += __bfloat162float(a.residual[at]);
+    static_cast<bf16*>(a.C)[at] = __float2bfloat16(sum);
+  }
+}
+
+template <int MM, int R, int U>
+int launch_epi(const GemvArgs& a, int epi, cudaStream_t stream) {
+  const dim3 grid(ceil_div(ceil_div(a.N, R), kWarps)), block(kWarps * 32);
+  auto go = [&](auto kern) {
+    pxl_host::launch(kern, grid, block, 0, stream, a);
+    return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
+  };
+  if (a.norm_w) {
+    if constexpr (MM <= PXL_GEMV_NORM_MAX_M) {
+      if (epi == PXL_EPI_NONE) return go(gemv_kernel<MM, R, U, PXL_EPI_NONE, true>);
+      if constexpr (R > 1)
+        if (epi == PXL_EPI_SILU_MUL) return go(gemv_kernel<MM, R, U, PXL_EPI_SILU_MUL, true>);
+    }
+    return PXL_ERR_INVALID_ARG;
+  }
+  switch (epi) {
+    case PXL_EPI_NONE: return go(gemv_kernel<MM, R, U, PXL_EPI_NONE, false>);
+    case PXL_EPI_RESIDUAL: return go(gemv_kernel<MM, R, U, PXL_EPI_RESIDUAL, false>);
+    case PXL_EPI_F32: return go(gemv_kernel<MM, R, U, PXL_EPI_F32, false>);
+    case PXL_EPI_SILU_MUL:
+      if constexpr (R > 1) return go(gemv_kernel<MM, R, U, PXL_EPI_SILU_MUL, false>);
+    default: return PXL_ERR_INVALID_ARG;
+  }
+}
+
+template <int MM>
+int launch_rows(const GemvArgs& a, int epi, cudaStream_t stream) {
+  // rows of W per warp: as many as still give every SM a dozen warps
+  const int want = 12 * pxl_host::num_sms();
+  if (a.N >= 4 * want) return launch_epi<MM, 4, 2>(a, epi, stream);
+  if (a.N >= 2 * want || epi == PXL_EPI_SILU_MUL) return launch_epi<MM, 2, 4>(a, epi, stream);
+  return launch_epi<MM, 1, 8>(a, epi, stream);
+}
+
+int run(const GemvArgs& a, int epi, cudaStream_t stream) {
+  if (!pxl_gemv_bf16_takes(a.M, a.N, a.K, epi) || ((a.lda | a.ldw) & 7) ||
+      ((reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.W) | reinterpret_cast<uintptr_t>(a.norm_w)) & 15))
+    return PXL_ERR_INVALID_ARG;
+  if (epi == PXL_EPI_RESIDUAL && a.residual == nullptr) return PXL_ERR_INVALID_ARG;
+  if (a.M == 1) return launch_rows<1>(a, epi, stream);
+  if (a.M == 2) return launch_rows<2>(a, epi, stream);
+  return launch_rows<4>(a, epi, stream);
+}
+}  // namespace
+
+// Where it beats the tensor cores: the rows of A cost it a load and an unpacking each per 16 bytes of W, so it is ahead for one
+// row (4096 x 4096: 9.0 us against 11.8; 151936 x 1024: 46 against 63) and stays so up to four where K is short (4096 x 1024, four
+// rows: 4.4 against 7.2) but not where the split along K of the other kernel pays (6144 x 4096, four rows: 17.3 against 15.2).
+// Gated products have no such split: four rows at 24576 x 4096 take 41 us against 50, six 67 against 49.
+PXL_EXPORT int pxl_gemv_bf16_takes(int M, int N, int K, int epi) {
+  if (M <= 0 || M > PXL_GEMV_MAX_M || N % 8 || K % 8) return 0;
+  if (epi == PXL_EPI_SILU_MUL) return N % 128 == 0;
+  return (epi == PXL_EPI_NONE || epi == PXL_EPI_RESIDUAL || epi == PXL_EPI_F32) && M * K <= 14336;
+}
+
+// contract of pxl_gemm_bf16, for the sizes that pxl_gemv_bf16_takes() names
+PXL_EXPORT int pxl_gemv_bf16(const void* A, const void* W, void* C, const void* residual, const void* bias, int M, int N, int K,
+                             int lda, int ldw, int ldc, int epi, cudaStream_t stream) {
+  return run(GemvArgs{static_cast<const pxl::bf16*>(A), static_cast<const pxl::bf16*>(W), static_cast<const pxl::bf16*>(residual),
+                      static_cast<const pxl::bf16*>(bias), C, M, N, K, lda, ldw, ldc, nullptr, 0.f, 0.f},
+             epi, stream);
+}
+
+PXL_EXPORT int pxl_gemv_bf16_norm(const void* A, const void* norm_w, float eps, float offset, const void* W, void* C, const void* bias,
+                                  int M, int N, int K, int lda, int ldw, int ldc, int epi, cudaStream_t stream) {
+  if (norm_w == nullptr || M > PXL_GEMV_NORM_MAX_M) return PXL_ERR_INVALID_ARG;
+  return run(GemvArgs{static_cast<const pxl::bf16*>(A), static_cast<const pxl::bf16*>(W), nullptr, static_cast<const pxl::bf16*>(bias),
+                      C, M, N, K, lda, ldw, ldc, static_cast<const pxl::bf16*>(norm_w), eps, offset},
+             epi, stream);
+}

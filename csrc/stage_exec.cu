@@ -119,13 +119,20 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
     explicit PdlScope(bool on) : prev(pxl_host::pdl_flag()) { pxl_host::pdl_flag() = on; }
     ~PdlScope() { pxl_host::pdl_flag() = prev; }
   } pdl_scope(!no_pdl && !stage_debug());
+  // one or two rows: the norms are part of the products behind them
+  auto normed = [&](int N, int epi) { return T <= PXL_GEMV_NORM_MAX_M && pxl_gemv_bf16_takes(T, N, H, epi) && H % 8 == 0; };
   for (int li = 0; li < st->n_layers; ++li) {
     const PxlDenseLayer& L = st->layers[li];
     int op_ = 0;  // 1 norm, 2 qkv, 3 rope+cache, 4 prefill, 5 decode (4 if no prefill), then o_proj, norm, gate_up, down
     void* h_mid = (h == ws->h_a) ? ws->h_b : ws->h_a;
-    PXL_TRY(pxl_rmsnorm(h, L.ln1, ws->xn, nullptr, T, H, st->eps, st->norm_offset, stream));
-    PXL_TRY(pxl_gemm_bf16(ws->xn, L.w_qkv, qkv, nullptr, L.b_qkv, T, qkv_n, H, H, H, qkv_n, PXL_EPI_NONE, 0, status,
-                          stream));
+    if (normed(qkv_n, PXL_EPI_NONE)) {
+      PXL_TRY(pxl_gemv_bf16_norm(h, L.ln1, st->eps, st->norm_offset, L.w_qkv, qkv, L.b_qkv, T, qkv_n, H, H, H, qkv_n, PXL_EPI_NONE,
+                                 stream));
+      --n;
+    } else {
+      PXL_TRY(pxl_rmsnorm(h, L.ln1, ws->xn, nullptr, T, H, st->eps, st->norm_offset, stream));
+      PXL_TRY(pxl_gemm_bf16(ws->xn, L.w_qkv, qkv, nullptr, L.b_qkv, T, qkv_n, H, H, H, qkv_n, PXL_EPI_NONE, 0, status, stream));
+    }
     PXL_TRY(pxl_qk_norm_rope_cache(qkv, L.q_norm, L.k_norm, st->cos_sin, sp->positions, sp->slots, L.k_cache,
                                    L.v_cache, T, Hq, Hkv, D, st->rot_dim, st->page, num_slots, st->eps,
                                    st->norm_offset, st->max_pos, status, stream));
@@ -153,9 +160,14 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
     }
     PXL_TRY(pxl_gemm_bf16(attn, L.w_o, h_mid, h, L.b_o, T, H, Hq * D, Hq * D, Hq * D, H, PXL_EPI_RESIDUAL, 0, status,
                           stream));
-    PXL_TRY(pxl_rmsnorm(h_mid, L.ln2, ws->xn, nullptr, T, H, st->eps, st->norm_offset, stream));
-    PXL_TRY(pxl_gemm_bf16(ws->xn, L.w_gu, ws->act, nullptr, nullptr, T, 2 * I, H, H, H, I, PXL_EPI_SILU_MUL, 0, status,
-                          stream));
+    if (normed(2 * I, PXL_EPI_SILU_MUL)) {
+      PXL_TRY(pxl_gemv_bf16_norm(h_mid, L.ln2, st->eps, st->norm_offset, L.w_gu, ws->act, nullptr, T, 2 * I, H, H, H, I,
+                                 PXL_EPI_SILU_MUL, stream));
+      --n;
+    } else {
+      PXL_TRY(pxl_rmsnorm(h_mid, L.ln2, ws->xn, nullptr, T, H, st->eps, st->norm_offset, stream));
+      PXL_TRY(pxl_gemm_bf16(ws->xn, L.w_gu, ws->act, nullptr, nullptr, T, 2 * I, H, H, H, I, PXL_EPI_SILU_MUL, 0, status, stream));
+    }
     void* h_next = (h_mid == ws->h_a) ? ws->h_b : ws->h_a;
     PXL_TRY(pxl_gemm_bf16(ws->act, L.w_down, h_next, h_mid, nullptr, T, H, I, I, I, H, PXL_EPI_RESIDUAL, 0, status,
                           stream));

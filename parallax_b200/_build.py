@@ -53,13 +53,13 @@ def _nvcc() -> str:
 # Sources a model family needs when nothing has been built yet (the whole library otherwise): a fresh checkout
 # that only runs this family compiles these into a library of their own.
 FAMILY_SOURCES = {
-    "latent": ["elementwise", "gemm_simt", "gemm_tcgen05", "latent_attn", "latent_attn_tc", "residual", "sampler"],
-    "looped": ["attention", "attention_any", "attention_prefill_tc", "attn_prep", "elementwise", "gemm_simt", "gemm_tcgen05",
+    "latent": ["elementwise", "gemm_simt", "gemm_tcgen05", "gemv", "latent_attn", "latent_attn_tc", "residual", "sampler"],
+    "looped": ["attention", "attention_any", "attention_prefill_tc", "attn_prep", "elementwise", "gemm_simt", "gemm_tcgen05", "gemv",
                "latent_attn", "latent_attn_tc", "matrix_memory", "moe", "residual", "sampler", "tanh_norm"],
     "prenorm_mix": ["attention", "attention_any", "attention_prefill_tc", "attn_prep", "delta_rule", "elementwise", "gemm_simt",
-                    "gemm_tcgen05", "matrix_memory", "moe", "residual", "sampler", "short_conv"],
+                    "gemm_tcgen05", "gemv", "matrix_memory", "moe", "residual", "sampler", "short_conv"],
     "parallel_block": ["attention", "attention_any", "attention_prefill_tc", "attn_prep", "elementwise", "gemm_simt",
-                       "gemm_tcgen05", "lightning_attn", "moe", "residual", "sampler"],
+                       "gemm_tcgen05", "gemv", "lightning_attn", "moe", "residual", "sampler"],
 }
 
 
