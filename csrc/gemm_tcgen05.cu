@@ -1360,6 +1360,29 @@ MidPlan mid_m_plan(int M, int N, int K) {
   return best;
 }
 
+// Rows that go ahead of the last wave of 128-row tiles: M itself, or as many as fill the SMs a whole number of times when the
+// rows behind them cost less on their own (split along K over all SMs, or streamed once for a few rows) than the nearly empty
+// wave that they would add. 5903 rows x 4096 columns are 752 tiles of 128 x 256, 5.08 waves of 148: 5888 rows take five.
+int rows_ahead_of_the_tail(int M, int N, int K) {
+  const int sms = pxl_host::num_sms(), num_kb = pxl::ceil_div(K, BK);
+  auto plain = [&](int rows) {
+    const int bns[2] = {256, 192};
+    const double t_kb[2] = {0.43, 0.36};
+    double best = 1e300;
+    for (int i = 0; i < 2; ++i) {
+      const double c = pxl::ceil_div(pxl::ceil_div(rows, BM) * pxl::ceil_div(N, bns[i]), sms) * (num_kb * t_kb[i]) + 7.0;
+      best = c < best ? c : best;
+    }
+    return best;
+  };
+  const int num_n = pxl::ceil_div(N, 256);
+  const int ahead = pxl::ceil_div(M, BM) * num_n / sms * sms / num_n * BM;
+  const int tail = M - ahead;
+  if (ahead <= 0 || tail <= 0 || tail > kMidMaxM) return M;
+  const double alone = tail <= kSmallMaxM ? 2.0 * N * K / 5.0e6 + 8.0 : mid_m_plan(tail, N, K).cost;
+  return plain(ahead) + alone < 0.97 * plain(M) ? ahead : M;
+}
+
 bool mid_m_disabled() {
   static const bool off = getenv("PXL_NO_MID_M_GEMM") != nullptr;
   return off;
@@ -1437,6 +1460,19 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
     if (plan > 0 && (plan & 15) > 1)
       return gemm_mid_m(A, W, C, epi == PXL_EPI_F32, epi == PXL_EPI_RESIDUAL ? residual : nullptr, bias, M, N, K, lda,
                         ldw, ldc, plan >> 4, plan & 15, status, stream);
+  }
+  if (bn == 0 && M > kMidMaxM && (epi == PXL_EPI_NONE || epi == PXL_EPI_RESIDUAL || epi == PXL_EPI_F32) && !mid_m_disabled()) {
+    const int ahead = rows_ahead_of_the_tail(M, N, K);
+    if (ahead < M) {
+      const int rc = pxl_gemm_bf16(A, W, C, residual, bias, ahead, N, K, lda, ldw, ldc, epi, pxl_gemm_bf16_pick_bn(ahead, N, epi), status,
+                                   stream);
+      if (rc != PXL_OK) return rc;
+      const size_t out = static_cast<size_t>(ahead) * ldc;
+      return pxl_gemm_bf16(static_cast<const pxl::bf16*>(A) + static_cast<size_t>(ahead) * lda, W,
+                           static_cast<char*>(C) + out * (epi == PXL_EPI_F32 ? sizeof(float) : sizeof(pxl::bf16)),
+                           epi == PXL_EPI_RESIDUAL ? static_cast<const pxl::bf16*>(residual) + out : residual, bias, M - ahead, N, K,
+                           lda, ldw, ldc, epi, 0, status, stream);
+    }
   }
   if (bn == 0) bn = pxl_gemm_bf16_pick_bn(M, N, epi);
   if (epi == PXL_EPI_SILU_MUL && ((N % bn) != 0 || bn < 128)) return PXL_ERR_INVALID_ARG;
