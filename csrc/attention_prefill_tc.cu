@@ -22,6 +22,7 @@
 //
 // Reference counterpart: the MLX SDPA call with a gathered KV prefix
 // (src/parallax/server/cache/prefix_cache_utils.py:11-91, src/parallax/models/qwen3.py:84-120).
+#include "attention_rows.cuh"
 #include "attention_score.cuh"
 #include "common.cuh"
 #include "pxl_api.h"
@@ -426,27 +427,6 @@ constexpr uint32_t kIdescPairPV = umma_idesc(kQ, kD, 1, 1) | (1u << 16);  // B (
 __device__ __forceinline__ uint64_t desc_v128(uint32_t addr) {
   return (umma_desc_k_sw128(addr) & ~(0x3fffull << 16)) | (static_cast<uint64_t>(kHalf >> 4) << 16);
 }
-__device__ __forceinline__ uint64_t pair2(float a, float b) {
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-  return v;
-}
-__device__ __forceinline__ float2 unpair2(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 template <int SM>
 __global__ void __launch_bounds__(kPairThreads, 1)
 attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -632,84 +612,13 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       failed = __any_sync(0xffffffffu, failed);  // warp-uniform: the TMEM accesses below are warp-wide
       if (failed) break;
       tc_fence_after_sync();
-      uint32_t sc[kT];
-#pragma unroll
-      for (int c = 0; c < kT; c += 32) tmem_ld_32x32b_x32(my_s + c, *reinterpret_cast<uint32_t(*)[32]>(&sc[c]));
-      tmem_ld_wait();
       const int key0 = tile_of(it) * kT;
       // interior tile: every key is visible to every row of the block, no masking needed
       const bool interior = key0 + kT - 1 <= pos0 && (window <= 0 || key0 >= pos0 + kQ - window || key0 + kT <= keep);
-      if constexpr (SM == kCapped) {
-#pragma unroll
-        for (int j = 0; j < kT; ++j) sc[j] = __float_as_uint(score_log2<SM>(__uint_as_float(sc[j]), 0.f, sa));
-      }
-      if (!interior) {
-        // keys this row sees among the 128 columns: [a, e), and those before f
-        const int a = key_lo - key0, e = (row_valid ? q_pos + 1 : 0) - key0, f = keep - key0;
-#pragma unroll
-        for (int j = 0; j < kT; ++j)
-          if ((j < a && j >= f) || j >= e) sc[j] = 0xff800000u;  // -inf
-      }
-      if constexpr (SM != kSigmoid) {
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-        for (int j = 0; j < kT; j += 8) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) m4[k] = fmaxf(fmaxf(m4[k], __uint_as_float(sc[j + k])), __uint_as_float(sc[j + 4 + k]));
-        }
-        const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * (SM == kCapped ? 1.f : scale_log2);  // scale > 0
-        const float m_new = fmaxf(m_run, mx);
-        // O accumulates relative to m_run, which only moves when a row of the warp grew by more than 2^8 (see above)
-        if (it == 0) {
-          m_run = m_new;
-        } else if (__any_sync(0xffffffffu, m_new > m_run + 8.f)) {
-          const float corr = fast_exp2(m_run - (m_new == -INFINITY ? 0.f : m_new));
-          m_run = m_new;
-          const uint64_t c2 = pair2(corr, corr);
-          l2[0] = fma2(l2[0], c2, 0ull), l2[1] = fma2(l2[1], c2, 0ull);
-#pragma unroll
-          for (int c = 0; c < kD; c += 16) {
-            uint32_t v[16];
-            tmem_ld_32x32b_x16(my_o + c, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
-            tmem_st_32x32b_x16(my_o + c, v);
-          }
-        }
-      }
-      const float m_use = (m_run == -INFINITY) ? 0.f : m_run;
-      const uint64_t scale2 = pair2(scale_log2, scale_log2), neg_m2 = pair2(-m_use, -m_use);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int c = h * 64; c < h * 64 + 64; c += 32) {
-          uint32_t pk[16];
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float s0 = __uint_as_float(sc[c + j]), s1 = __uint_as_float(sc[c + j + 1]);
-            float p0, p1;
-            if constexpr (SM == kSigmoid) {
-              p0 = sigmoid_weight(s0, scale_log2, bias2);  // (a masked score, -inf, gives 0)
-              p1 = sigmoid_weight(s1, scale_log2, bias2);
-            } else if constexpr (SM == kCapped) {
-              p0 = fast_exp2(s0 - m_use);
-              p1 = fast_exp2(s1 - m_use);
-            } else {
-              const float2 x = unpair2(fma2(pair2(s0, s1), scale2, neg_m2));
-              p0 = fast_exp2(x.x);
-              p1 = fast_exp2(x.y);
-            }
-            l2[(j >> 1) & 1] = add2(l2[(j >> 1) & 1], pair2(p0, p1));
-            pk[j >> 1] = pack_bf16x2(p0, p1);
-          }
-          tmem_st_32x32b_x16(my_s + c / 2, pk);
-        }
-        tmem_st_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready + 16 * u + 8 * h);
-      }
+      // keys this row sees among the 128 columns: [a, e), and those before f
+      const int a = key_lo - key0, e = (row_valid ? q_pos + 1 : 0) - key0, f = keep - key0;
+      softmax_tile<SM>(my_s, my_o, it == 0, interior, [&](int j) { return (j < a && j >= f) || j >= e; }, scale_log2, sa, bias2, m_run,
+                       l2, p_ready + 16 * u);
     }
     if (!failed) failed = mbar_wait_bounded(o_full + 8 * u, 0, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_FULL) ? 0 : 1;
     failed = __any_sync(0xffffffffu, failed);
@@ -725,20 +634,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       const float inv = SM == kSigmoid ? 1.f : denom > 0.f ? f / denom : 0.f;
       bf16* dst = out + static_cast<size_t>(q_begin + q0 + r) * out_stride + head * kD;
       tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < kD; c += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(my_o + c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int c8 = 0; c8 < 32; c8 += 8) {
-          bf16x8 ov;
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            ov.u[j] = pack_bf16x2(__uint_as_float(v[c8 + 2 * j]) * inv, __uint_as_float(v[c8 + 2 * j + 1]) * inv);
-          if (row_valid) st_bf16x8(dst + c + c8, ov);
-        }
-      }
+      store_row(my_o, inv, dst, row_valid);
       tc_fence_before_sync();
     }
   }

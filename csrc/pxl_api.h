@@ -301,6 +301,15 @@ int pxl_ep_combine(const void* comb, const float* w, const void* base, int64_t l
                    int64_t ld_out, const void* ret_flag, int ep, uint32_t epoch, int n_rows, int k, int H,
                    int* status, pxl_stream_t stream);
 
+// ---- mla_prefill.cu: prompts from their first token, keys and values expanded per head ------------------------
+// q [T, H * (nope + rot)]: rotates the last `rot` columns of every head in place (interleaved pairs).
+int pxl_mla_rotate(void* q, int64_t ld, const float* cos_sin, const int* positions, int max_pos, int T, int H, int nope, int rot,
+                   int* status, pxl_stream_t stream);
+// out [T, H * vdim] = causal attention of the rotated q within the sequences cu_q [B + 1]; kv [T, H * (nope + vdim)]: k | v per head,
+// rows [T, latent + rot]: latent | rotated key columns, the same for all heads. nope = vdim = 128, rot = 64, latent = 512.
+int pxl_mla_prefill(const void* q, const void* kv, const void* rows, const int* cu_q, void* out, int B, int max_q, int T, int H,
+                    int nope, int rot, int vdim, int latent, float scale, int* status, pxl_stream_t stream);
+
 // ---- linear_attn.cu: gated delta-net layers (per-request state slots) ---------------------------
 // y = silu(causal_conv(x)) per channel with the last K-1 inputs carried in conv_state [slots, C, K-1];
 // sequence b covers tokens [seq_cu[b], seq_cu[b+1]) and uses slot seq_slots[b]; a sequence whose

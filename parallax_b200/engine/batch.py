@@ -30,6 +30,7 @@ class ForwardBatch:
     p_block_tables: Optional[torch.Tensor] = None  # int32 [Bp, MB]
     p_max_q: int = 0
     p_max_ctx: int = 0
+    p_total_ctx: int = 0                          # sum of p_ctx_lens; num_prefill_tokens if no prompt has a cached prefix
     # decode part
     d_ctx_lens: Optional[torch.Tensor] = None     # int32 [Bd]
     d_block_tables: Optional[torch.Tensor] = None  # int32 [Bd, MB]
@@ -150,6 +151,7 @@ class BatchBuilder:
             fb.p_block_tables = view("p_bt").view(Bp, -1)
             fb.p_max_q = int(max(p_q_lens))
             fb.p_max_ctx = int(max(p_ctx_lens))
+            fb.p_total_ctx = int(sum(p_ctx_lens))
         if Bd:
             fb.d_ctx_lens = view("d_ctx")
             fb.d_block_tables = view("d_bt").view(Bd, -1)

@@ -3,8 +3,9 @@ DeepSeek-V3.2 / GLM-MoE-DSA (latent attention over the top-k keys of a lightning
 
 Attention runs in absorbed form for decode and prefill: the per-head up-projections of
 ``kv_b_proj`` are folded into the query (``W_UK``) and the output (``W_UV``), so the paged cache
-holds only ``[latent 512 | rope 64]`` per token and one kernel serves every case
-(:func:`parallax_b200.ops.latent_attn`; page sizes that it does not take: :func:`parallax_b200.ops.mla_attn`). The reference keeps the same compressed cache but expands
+holds only ``[latent 512 | rope 64]`` per token (:func:`parallax_b200.ops.latent_attn`; page sizes that it does not take:
+:func:`parallax_b200.ops.mla_attn`). On a GPU, prompts without a cached prefix expand their keys and values instead
+(:func:`parallax_b200.ops.mla_prefill`). The reference keeps the same compressed cache but expands
 K/V for prefill (``src/parallax/models/deepseek_v3.py:74-83,158-171``); its indexer and sparse
 attention are ``src/parallax/models/deepseek_v32.py:84-238,376-446``. Per-layer indexer modes
 ("full" layers score keys, "shared" layers reuse the previous full layer's selection) follow
@@ -39,7 +40,7 @@ def derive_indexer_types(cfg: ModelConfig) -> list[str]:
 
 
 class MLALayer:
-    __slots__ = ("ln1", "ln2", "w_q_a", "q_a_norm", "w_q_b", "w_kv_a", "kv_a_norm", "w_uk_s", "w_uv_s", "w_o",
+    __slots__ = ("ln1", "ln2", "w_q_a", "q_a_norm", "w_q_b", "w_kv_a", "kv_a_norm", "w_uk_s", "w_uv_s", "w_kvb", "w_o",
                  "idx_wq_b", "idx_k_norm_w", "idx_k_norm_b", "idx_mode", "w_gu", "w_down", "moe", "layer_idx",
                  "n_kv_a")
 
@@ -84,6 +85,9 @@ class DeepseekStage(DecoderStage):
         kvb = kv_b.view(H, nope + V, L)
         lw.w_uk_s = kvb[:, :nope].transpose(1, 2).reshape(H * L, nope).contiguous()   # q_lat = W_UK^T q_nope
         lw.w_uv_s = kvb[:, nope:].reshape(H * V, L).contiguous()                        # o = W_UV o_lat
+        # k | v of every head, for prompts that start at their first token (see _attention)
+        expand = kv_b.is_cuda and kv_b.dtype == torch.bfloat16 and (nope, self.R, V, L) == (128, 64, 128, 512)
+        lw.w_kvb = kv_b.contiguous() if expand else None
         lw.w_o = w_o.contiguous()
 
     def init_random(self, seed: int = 0, std: float = 0.02) -> None:
@@ -296,21 +300,42 @@ class DeepseekStage(DecoderStage):
                 o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.d_block_tables, None, fb.positions, self.scale, Tp,
                                      fb.num_decode, topk=topk, out=o_lat)
             return ops.mla_unabsorb(o_lat, lw.w_uv_s, T), topk
-        # token-major rows: the per-head products read and write them in place, without head-major copies or padding
         L, R, V = self.L, self.R, self.V
-        q_cat = torch.empty((T, H, L + R), dtype=q.dtype, device=q.device)
-        ops.latent_queries(q, H, self.qd, self.nope, self.cos_sin, fb.positions, q_cat, L, R, R)
-        ops.head_linear(q, self.qd, lw.w_uk_s, H, q_cat[:, :, :L])
-        o_lat = torch.empty((T, H, L), dtype=q.dtype, device=q.device)
-        if Tp:
-            ops.latent_attn(q_cat[:Tp], cache, fb.p_block_tables, fb.p_cu_q, fb.p_ctx_lens, self.scale, L, max_q=fb.p_max_q,
-                            max_ctx=fb.p_max_ctx, out=o_lat[:Tp], topk=None if topk is None else topk[:Tp])
-        if fb.num_decode:
-            ops.latent_attn(q_cat[Tp:], cache, fb.d_block_tables, None, fb.d_ctx_lens, self.scale, L, max_ctx=fb.d_max_ctx,
-                            out=o_lat[Tp:], topk=None if topk is None else topk[Tp:])
         heads = torch.empty((T, H, V), dtype=q.dtype, device=q.device)
-        ops.head_linear(o_lat.view(T, H * L), L, lw.w_uv_s, H, heads)
+        done = 0
+        if self._expands(lw, fb) and topk is None:
+            # no prompt has a cached prefix: keys and values expanded once per token, 320 instead of 1088 columns per pair
+            rows = ops.gather_rows(cache.view(-1, L + R), fb.slot_mapping[:Tp])
+            ops.mla_prefill(q[:Tp], rows, lw.w_kvb, self.cos_sin, fb.positions[:Tp], fb.p_cu_q, H, self.nope, V, L, self.scale,
+                            fb.p_max_q, out=heads[:Tp])
+            done = Tp
+        if done < T:
+            # token-major rows: the per-head products read and write them in place, without head-major copies or padding
+            q, n = q[done:], T - done
+            q_cat = torch.empty((n, H, L + R), dtype=q.dtype, device=q.device)
+            ops.latent_queries(q, H, self.qd, self.nope, self.cos_sin, fb.positions[done:], q_cat, L, R, R)
+            ops.head_linear(q, self.qd, lw.w_uk_s, H, q_cat[:, :, :L])
+            o_lat = torch.empty((n, H, L), dtype=q.dtype, device=q.device)
+            if Tp > done:
+                ops.latent_attn(q_cat[:Tp], cache, fb.p_block_tables, fb.p_cu_q, fb.p_ctx_lens, self.scale, L, max_q=fb.p_max_q,
+                                max_ctx=fb.p_max_ctx, out=o_lat[:Tp], topk=None if topk is None else topk[:Tp])
+            if fb.num_decode:
+                ops.latent_attn(q_cat[Tp - done:], cache, fb.d_block_tables, None, fb.d_ctx_lens, self.scale, L,
+                                max_ctx=fb.d_max_ctx, out=o_lat[Tp - done:], topk=None if topk is None else topk[Tp:])
+            ops.head_linear(o_lat.view(n, H * L), L, lw.w_uv_s, H, heads[done:])
         return heads.view(T, H * V), topk
+
+    # Expanded keys and values: a pair of (query, key) costs 320 columns instead of 1088, but every token's keys and values
+    # are written and read once, and the kernel's query tiles are a prompt's own. Of a layer with 128 heads (us, absorbed and
+    # expanded): 2 x 2048 tokens 6940 and 4340, 1 x 1024 1702 and 1095, 4 x 64 486 and 461, 16 x 32 577 and 577, 16 x 16 448
+    # and 475. Below 256 rows either form is mostly weights (1 x 128: 365 and 330), and a prompt keeps the form of the
+    # decoding rows.
+    _EXPAND_MIN_ROWS = 256
+    _EXPAND_MIN_PROMPT = 64
+
+    def _expands(self, lw: MLALayer, fb: ForwardBatch) -> bool:
+        return lw.w_kvb is not None and fb.num_prefill_tokens >= max(self._EXPAND_MIN_ROWS, self._EXPAND_MIN_PROMPT * fb.num_prefill_seqs) \
+            and fb.p_total_ctx == fb.num_prefill_tokens
 
     def _rows_form(self, cache: torch.Tensor) -> bool:
         """Whether attention runs on token-major rows (the tensor-core kernel takes the page size) or on head-major ones."""

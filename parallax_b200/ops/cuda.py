@@ -913,6 +913,23 @@ def mla_unabsorb(o_lat_hm, w_uv_s, T: int):
     return o.view(H, Tpad, V)[:, :T].transpose(0, 1).reshape(T, H * V)
 
 
+def mla_prefill(q, rows, w_kvb, cos_sin, positions, cu_q, H: int, nope: int, vdim: int, latent: int, scale, max_q: int, out=None):
+    T = q.shape[0]
+    rot = q.shape[1] // H - nope
+    assert q.is_contiguous() and rows.is_contiguous() and rows.shape == (T, latent + rot) and w_kvb.shape == (H * (nope + vdim), latent)
+    if out is None:
+        out = torch.empty((T, H * vdim), dtype=q.dtype, device=q.device)
+    assert out.is_contiguous() and out.numel() == T * H * vdim
+    status, stream = status_tensor(q.device).data_ptr(), _stream(q.device)
+    check(_lib.lib().pxl_mla_rotate(q.data_ptr(), q.stride(0), cos_sin.data_ptr(), positions.data_ptr(), cos_sin.shape[0], T, H, nope, rot,
+                                    status, stream), "pxl_mla_rotate")
+    kv = linear(rows[:, :latent], w_kvb)
+    check(_lib.lib().pxl_mla_prefill(q.data_ptr(), kv.data_ptr(), rows.data_ptr(), cu_q.data_ptr(), out.data_ptr(), cu_q.numel() - 1, max_q,
+                                     T, H, nope, rot, vdim, latent, float(scale), status, stream), "pxl_mla_prefill")
+    _count(2)
+    return out
+
+
 def store_rows(src, slot_mapping, cache):
     T, D = src.shape
     num_slots = cache.numel() // D

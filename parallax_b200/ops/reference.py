@@ -434,6 +434,25 @@ def mla_unabsorb(o_lat_hm, w_uv_s, T: int):
     return o.reshape(T, -1).to(o_lat_hm.dtype)
 
 
+def mla_prefill(q, rows, w_kvb, cos_sin, positions, cu_q, H: int, nope: int, vdim: int, latent: int, scale, max_q: int, out=None):
+    """Latent attention of prompts from their first token, keys and values expanded per head: ``q [T, H*(nope+R)]`` (its last R
+    columns per head are rotated in place), ``rows [T, latent+R]`` latent | rotated key columns, ``w_kvb [H*(nope+vdim), latent]``
+    -> ``[T, H*vdim]``."""
+    T = q.shape[0]
+    qh = q.view(T, H, -1)
+    qh[..., nope:] = _rope_interleaved(qh[..., nope:], cos_sin, positions).to(q.dtype)
+    kv = (rows[:, :latent].float() @ w_kvb.float().t()).to(q.dtype).view(T, H, nope + vdim)
+    if out is None:
+        out = torch.empty((T, H * vdim), dtype=q.dtype, device=q.device)
+    o, cu = out.view(T, H, vdim), cu_q.tolist()
+    for a, b in zip(cu, cu[1:]):
+        k = torch.cat([kv[a:b, :, :nope], rows[a:b, None, latent:].expand(b - a, H, -1)], -1).float()
+        s = torch.einsum("thd,shd->hts", qh[a:b].float(), k) * scale
+        s = s.masked_fill(torch.ones(b - a, b - a, dtype=torch.bool, device=q.device).triu(1), float("-inf"))
+        o[a:b] = torch.einsum("hts,shd->thd", torch.softmax(s, -1), kv[a:b, :, nope:].float()).to(q.dtype)
+    return out
+
+
 def store_rows(src, slot_mapping, cache):
     flat = cache.view(-1, cache.shape[-1])
     ok = slot_mapping >= 0

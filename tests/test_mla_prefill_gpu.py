@@ -1,0 +1,29 @@
+"""Latent attention of prompts with expanded keys and values, against the fp32 restatement."""
+
+import pytest
+import torch
+
+from parallax_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,lens", [
+    (128, [65]), (2, [128, 1, 129]), (3, [256, 257, 383]), (8, [700, 90]),      # ends on and off tiles, one and two blocks of queries
+])
+def test_expanded_prompts(H, lens):
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(H)
+    T, nope, R, V, L = sum(lens), 128, 64, 128, 512
+    q, rows = torch.randn(T, H * (nope + R)).bfloat16(), torch.randn(T, L + R).bfloat16()
+    w = (torch.randn(H * (nope + V), L) * 0.05).bfloat16()
+    cs, pos = ref.build_cos_sin(800, R, 1e4), torch.cat([torch.arange(n) for n in lens]).int()
+    cu_q = torch.tensor([0] + lens).cumsum(0).int()
+    a, b = q.clone(), q.cuda()
+    want = ref.mla_prefill(a, rows, w, cs, pos, cu_q, H, nope, V, L, 192 ** -0.5, max(lens))
+    got = cu.mla_prefill(b, rows.cuda(), w.cuda(), cs.cuda(), pos.cuda(), cu_q.cuda(), H, nope, V, L, 192 ** -0.5, max(lens)).cpu()
+    cu.check_status(torch.device("cuda", 0))
+    assert float((b.cpu().float() - a.float()).norm() / a.float().norm()) < 2 ** -8      # rotated in place
+    # probabilities, expanded values and outputs are rounded to bf16 (2^-9 each)
+    assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
