@@ -11,11 +11,11 @@
 //               ring of chunk slots that are free again as soon as the scores have read them.
 //               With key lists (attention over an indexer's best keys) a CTA takes one token, whose listed rows are
 //               gathered four at a time (tile::gather4); tokens without a list take the page boxes.
-//   warp 6    : with key lists only, a second producer, for the value buffers. A full query tile leaves room for one of
-//               them (64 keys x 256 columns), so the gathers of a tile's values wait for the product of the tile before;
-//               a warp of their own lets the scores' gathers of the next tiles go out meanwhile. 1024 tokens x 2048 of
-//               their keys, 128 heads: 1.02 ms instead of 1.39 (gathering with cp.async by four warps: 1.75; tiles of 32
-//               keys with three buffers: 1.19, as narrow products cost almost as much as wide ones). Page boxes are
+//   warp 6    : with key lists only, a second producer, for the value buffers. A full query tile leaves room for few
+//               of them (64 keys x 256 columns), so the gathers of a tile's values wait for the product of a tile before;
+//               a warp of their own lets the scores' gathers of the next tiles go out meanwhile. 1000 tokens x 2048 of
+//               their keys, 128 heads, with one buffer: 2.0 ms instead of 2.8 (gathering with cp.async by four warps:
+//               3.5; tiles of 32 keys with three buffers: 2.4, as narrow products cost almost as much as wide ones). Page boxes are
 //               few, and gain nothing from it.
 //   warp 5    : MMA issuer. S = Q K^T over L + R (both operands K-major) into one of two TMEM score buffers, chunk
 //               by chunk as the loads land, so the scores of tile i + 1 are computed while the softmax warps work
@@ -61,6 +61,8 @@ struct TcArgs {
   int H, L, D, page, max_blocks, window, vsplit, head_blocks;
   int k_slots, v_bufs;  // ring slots for score-only chunks, buffers for value chunks
   int q_rows;           // rows of the query tile kept in shared memory (decoding: the heads of one token)
+  int q_tmem;           // first column chunks of a full query tile that are kept in tensor memory instead
+  const bf16* q;
   int64_t num_blocks;
   float scale_log2;
   int* status;
@@ -72,7 +74,7 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
 }
 template <bool LISTS>
 __global__ void __launch_bounds__(kThreads<LISTS>, 1)
-latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
+latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid_constant__ CUtensorMap tm_kv,
                       const __grid_constant__ CUtensorMap tm_row, const TcArgs a) {
   constexpr uint32_t kIdescS = umma_idesc(kRows, NK, 1, 1);
   extern __shared__ uint8_t smem_raw[];
@@ -82,6 +84,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // key ring): those rows' scores are masked and their outputs never stored.
   const uint32_t q_chunk = a.q_rows * 128;
   const uint32_t sm_q = smem_u32(smem);
+  const int nqs = nck - a.q_tmem;  // query chunks in shared memory
   // latent chunks of this CTA
   const int vs = blockIdx.x % a.vsplit, tile = blockIdx.x / a.vsplit;
   const int ncv = ceil_div(a.L, 64), per = ceil_div(ncv, a.vsplit);
@@ -89,9 +92,9 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int nv = ncv - v0 < per ? ncv - v0 : per;
   const int nkc = nck - nv;                                   // chunks that only the scores read
   auto k_chunk = [&](int j) { return j < v0 ? j : j + nv; };  // their column chunks
-  const uint32_t sm_v = sm_q + nck * q_chunk;
+  const uint32_t sm_v = sm_q + nqs * q_chunk;
   const uint32_t sm_k = sm_v + a.v_bufs * per * kKvChunk;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + nck * q_chunk + (a.v_bufs * per + a.k_slots) * kKvChunk);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + nqs * q_chunk + (a.v_bufs * per + a.k_slots) * kKvChunk);
   // q_full | v_full, v_empty [kMaxVBufs] | k_full, k_empty [kMaxSlots] | s_full, p_ready, o_full [2]
   const uint32_t q_full = smem_u32(bars), v_full = q_full + 8, v_empty = v_full + 8 * kMaxVBufs,
                  k_full = v_empty + 8 * kMaxVBufs, k_empty = k_full + 8 * kMaxSlots, s_full = k_empty + 8 * kMaxSlots,
@@ -128,7 +131,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    mbar_init(q_full, 1);
+    mbar_init(q_full, a.q_tmem > 0 ? 5 : 1);  // the TMA producer, and the warps that write the chunks in tensor memory
     for (int s = 0; s < a.v_bufs; ++s) {
       mbar_init(v_full + 8 * s, 1);
       mbar_init(v_empty + 8 * s, 1);
@@ -144,10 +147,10 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
     mbar_fence_init();
     fence_proxy_async_smem();
-    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_q_map);
     tma_prefetch_desc(&tm_kv);
   }
-  const uint32_t tmem_cols = 64 * per + 3 * NK <= 256 ? 256 : 512;  // O | two score | two probability buffers
+  const uint32_t tmem_cols = 64 * per + 3 * NK + 32 * a.q_tmem <= 256 ? 256 : 512;  // O | two score | two probability buffers | q
   if (warp == kMmaWarp) {
     tmem_alloc(smem_u32(tmem_slot), tmem_cols);
     tmem_relinquish();
@@ -158,6 +161,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const uint32_t tm_o = *tmem_slot;             // O: 64 columns per latent chunk
   const uint32_t tm_s = tm_o + 64 * per;        // two score buffers of NK columns
   const uint32_t tm_p = tm_s + 2 * NK;          // two probability buffers of NK / 2 columns
+  const uint32_t tm_q = tm_p + NK;              // 32 columns per query chunk
 
   if (warp == kProducerWarp || warp == kValueWarp) {
     // ------------------------------------------------------------------ TMA producers
@@ -165,9 +169,9 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t leader = elect_leader();
     const bool keys = warp == kProducerWarp, values = !LISTS || warp == kValueWarp;
     if (keys) {
-      if (leader) mbar_arrive_expect_tx(q_full, nck * q_chunk);
+      if (leader) mbar_arrive_expect_tx(q_full, nqs * q_chunk);
       __syncwarp();
-      for (int c = 0; c < nck; ++c) tma_box(sm_q + c * q_chunk, &tm_q, q_full, c * 64, static_cast<int>(row0), leader);
+      for (int c = 0; c < nqs; ++c) tma_box(sm_q + c * q_chunk, &tm_q_map, q_full, (a.q_tmem + c) * 64, static_cast<int>(row0), leader);
     }
     const int* bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     const int box = a.page < NK ? a.page : NK;
@@ -260,10 +264,17 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // descriptors advance by 16-byte units: 2 per k-step inside a chunk (columns past D are zeros on both sides)
       auto ready = [](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test(bar, parity)) != 0; };
       auto s_chunk = [&](int it, int col_chunk, uint32_t rows_addr, bool first) {  // S[it % 2] (+)= Q[:, chunk] K[:, chunk]^T
-        const uint64_t dq = dq0 + static_cast<uint64_t>(col_chunk) * (q_chunk >> 4), dk = umma_desc_k_sw128(rows_addr);
+        const uint64_t dk = umma_desc_k_sw128(rows_addr);
+        const uint32_t d = tm_s + (it & 1) * NK;
+        if (col_chunk < a.q_tmem) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          mma_ss(tm_s + (it & 1) * NK, dq + 2 * ks, dk + 2 * ks, kIdescS, first && ks == 0 ? 0u : 1u, leader);
+          for (int ks = 0; ks < 4; ++ks)
+            mma_ts(d, tm_q + col_chunk * 32 + ks * 8, dk + 2 * ks, kIdescS, first && ks == 0 ? 0u : 1u, leader);
+        } else {
+          const uint64_t dq = dq0 + static_cast<uint64_t>(col_chunk - a.q_tmem) * (q_chunk >> 4);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) mma_ss(d, dq + 2 * ks, dk + 2 * ks, kIdescS, first && ks == 0 ? 0u : 1u, leader);
+        }
       };
       // Whichever is ready goes next: the product of a tile whose probabilities are written, or the next chunk of the
       // scores (at most one tile ahead of the products: two score buffers). A load in flight never holds back a
@@ -340,6 +351,25 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t lane_sel = static_cast<uint32_t>(warp * 32) << 16;
     float m_run = -INFINITY, l_run = 0.f;
     int failed = 0;
+    if (a.q_tmem > 0) {  // this row's part of the query chunks in tensor memory, two columns per word
+      const bf16* src = a.q + (row0 + r) * a.D;
+      for (int c = 0; c < a.q_tmem; ++c) {
+        uint32_t v[32] = {};
+        if (row_valid) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const bf16x8 x = ld_bf16x8(src + c * 64 + j * 8);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[j * 4 + k] = x.u[k];
+          }
+        }
+        tmem_st_32x32b_x32(tm_q + c * 32 + lane_sel, v);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
     // of the listed keys of a tile, those that are visible (a bit each)
     auto visible = [&](int it, uint32_t (&seen)[2]) {
 #pragma unroll
@@ -476,18 +506,20 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 }
 
 struct TilePlan {
-  int k_slots, v_bufs, smem;
+  int k_slots, v_bufs, q_tmem, smem;
 };
 
-// Ring slots and V buffers beside a query tile of q_rows rows; false when the sizes do not fit.
-bool plan_tiles(int L, int D, int q_rows, int page, TilePlan* p) {
+// Ring slots and V buffers beside a query tile of q_rows rows, q_tmem chunks of which are in tensor memory; false when the sizes
+// do not fit.
+bool plan_tiles(int L, int D, int q_rows, int page, int q_tmem, TilePlan* p) {
   if (page % 8 != 0 || (page % NK != 0 && NK % page != 0)) return false;
   const int nck = ceil_div(D, 64), ncv = ceil_div(L, 64);
   const int vsplit = ceil_div(ncv, kMaxV), per = ceil_div(ncv, vsplit);
   const int nkc = nck - (ncv - (vsplit - 1) * per);  // score-only chunks of the CTA that has most of them
-  const int q_bytes = nck * q_rows * 128;
+  const int q_bytes = (nck - q_tmem) * q_rows * 128;
   const int slots = (kMaxSmem - 1024 - kBarBytes - q_bytes) / kKvChunk;
   p->k_slots = 0;
+  p->q_tmem = q_tmem;
   for (int vb = kMaxVBufs; vb >= 1; --vb) {
     const int ks = slots - vb * per;
     if (ks >= (vb > 1 ? nkc + 1 : (nkc > 0 ? 1 : 0))) {
@@ -495,12 +527,23 @@ bool plan_tiles(int L, int D, int q_rows, int page, TilePlan* p) {
       p->k_slots = ks < kMaxSlots ? ks : kMaxSlots;
       if (p->k_slots < 1) p->k_slots = 1;
       const int tiles = q_bytes + (vb * per + p->k_slots) * kKvChunk;
-      const int reach = (nck - 1) * q_rows * 128 + kQChunk;  // what the MMA reads of the query tile
+      const int reach = (nck - q_tmem - 1) * q_rows * 128 + kQChunk;  // what the MMA reads of the query tile
       p->smem = 1024 + (tiles > reach ? tiles : reach) + kBarBytes;
       return p->smem <= kMaxSmem;
     }
   }
   return false;
+}
+
+// A full query tile of 576 columns (144 KB) leaves room for one V buffer: the loads of a tile's values then wait for the product of
+// the tile before it, a load latency per tile. O, scores and probabilities leave 64 columns of tensor memory, which hold two of the
+// nine query chunks: room for a second buffer. 128 heads, one layer: 64 sequences decoding behind 4096 tokens 196 -> 182 us, 1000
+// tokens x 2048 listed keys 2.01 -> 1.73 ms.
+bool plan_tiles(int L, int D, int q_rows, int page, TilePlan* p) {
+  const bool fits = plan_tiles(L, D, q_rows, page, 0, p);
+  TilePlan other;
+  if (fits && p->v_bufs == 1 && q_rows == kRows && D >= 192 && plan_tiles(L, D, q_rows, page, 2, &other) && other.v_bufs > 1) *p = other;
+  return fits;
 }
 }  // namespace
 
@@ -528,6 +571,8 @@ PXL_EXPORT int pxl_latent_attn_tc(const void* q, const void* cache, const int* b
   if (!plan_tiles(L, L + R, a.q_rows, page, &plan)) return PXL_ERR_INVALID_ARG;
   a.k_slots = plan.k_slots;
   a.v_bufs = plan.v_bufs;
+  a.q_tmem = plan.q_tmem;
+  a.q = static_cast<const pxl::bf16*>(q);
   a.block_tables = block_tables;
   a.cu_q = cu_q;
   a.ctx_lens = ctx_lens;

@@ -51,3 +51,30 @@ def test_latent_attention_over_lists(H, k, page, prompts, decode):
         cu.check_status(torch.device("cuda", 0))
         # probabilities and outputs are rounded to bf16 (2^-9 each)
         assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("H,page,prompts", [
+    (128, 64, [(1, 130), (1, 64), (1, 1)]),     # decoding, one token per tile
+    (24, 16, [(11, 75), (7, 7)]),               # five tokens and rows that are left over
+    (192, 8, [(3, 70)]),                        # a second block of heads that fills half a tile
+])
+def test_wide_rows_with_a_part_of_the_query_in_tensor_memory(H, page, prompts):
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(H)
+    L, R = 512, 64
+    need = [-(-c // page) for _n, c in prompts]
+    table = torch.zeros(len(prompts), max(need), dtype=torch.int32)
+    blocks, at = torch.randperm(sum(need)).int(), 0
+    for i, n in enumerate(need):
+        table[i, :n], at = blocks[at:at + n], at + n
+    cache = torch.randn(sum(need), 1, page, L + R).bfloat16()
+    q = (torch.randn(sum(n for n, _c in prompts), H, L + R) * 0.5).bfloat16()
+    cu_q = torch.tensor([0] + [n for n, _c in prompts]).cumsum(0).int()
+    args = (cache, table, cu_q, torch.tensor([c for _n, c in prompts]).int())
+    kw = dict(max_q=max(n for n, _c in prompts), max_ctx=max(c for _n, c in prompts))
+    want = ref.latent_attn(q, *args, 192 ** -0.5, L, **kw)
+    got = cu.latent_attn(q.cuda(), *[a.cuda() for a in args], 192 ** -0.5, L, **kw).cpu()
+    cu.check_status(torch.device("cuda", 0))
+    # probabilities and outputs are rounded to bf16 (2^-9 each)
+    assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
