@@ -11,12 +11,13 @@
 //               ring of chunk slots that are free again as soon as the scores have read them.
 //               With key lists (attention over an indexer's best keys) a CTA takes one token, whose listed rows are
 //               gathered four at a time (tile::gather4); tokens without a list take the page boxes.
-//   warp 6    : with key lists only, a second producer, for the value buffers. A full query tile leaves room for few
-//               of them (64 keys x 256 columns), so the gathers of a tile's values wait for the product of a tile before;
-//               a warp of their own lets the scores' gathers of the next tiles go out meanwhile. 1000 tokens x 2048 of
-//               their keys, 128 heads, with one buffer: 2.0 ms instead of 2.8 (gathering with cp.async by four warps:
-//               3.5; tiles of 32 keys with three buffers: 2.4, as narrow products cost almost as much as wide ones). Page boxes are
-//               few, and gain nothing from it.
+//   warp 6    : the same for the value buffers. A full query tile leaves room for few of them (64 keys x 256 columns), so the loads
+//               of a tile's values wait for the product of a tile before; in a warp of their own they don't hold back the loads
+//               for the scores of the next tiles, and boxes of short pages and gathers are issued twice as fast. 64 sequences
+//               of 4096 keys, 128 heads, pages of 16: 189 -> 150 us (pages of 64: 146 and 148); 1000 tokens x 2048 listed
+//               keys, with one value buffer: 2.8 -> 2.0 ms (gathering with cp.async by four warps: 3.5; tiles of 32 keys with
+//               three buffers: 2.4). What is left is the scores' products: 128 x 64 x 16 costs the reads of its 128 rows of
+//               queries, about 96 clocks of the 2.2 us that a tile takes 36 times, whatever the number of heads.
 //   warp 5    : MMA issuer. S = Q K^T over L + R (both operands K-major) into one of two TMEM score buffers, chunk
 //               by chunk as the loads land, so the scores of tile i + 1 are computed while the softmax warps work
 //               on tile i; then O += P V, P from tensor memory, V taken MN-major from the V buffer, all of its
@@ -44,8 +45,7 @@ constexpr int NK = 64;                 // keys per tile
 constexpr int kKvChunk = NK * 128;     // bytes of 64 columns of a key tile
 constexpr int kMaxSlots = 16, kMaxVBufs = 3;
 constexpr int kProducerWarp = 4, kMmaWarp = 5, kValueWarp = 6;
-template <bool LISTS>
-constexpr int kThreads = LISTS ? 224 : 192;
+constexpr int kThreads = 224;
 constexpr int kBarBytes = 512;
 constexpr int kMaxSmem = 227 * 1024;
 constexpr float kLog2eF = 1.4426950408889634f;
@@ -73,7 +73,7 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
   return (umma_desc_k_sw128(addr) & ~(0x3fffull << 16)) | (static_cast<uint64_t>(kKvChunk >> 4) << 16);
 }
 template <bool LISTS>
-__global__ void __launch_bounds__(kThreads<LISTS>, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid_constant__ CUtensorMap tm_kv,
                       const __grid_constant__ CUtensorMap tm_row, const TcArgs a) {
   constexpr uint32_t kIdescS = umma_idesc(kRows, NK, 1, 1);
@@ -167,7 +167,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
     // ------------------------------------------------------------------ TMA producers
     // Lane p looks up the block of piece p of the tile; one lane issues all boxes.
     const uint32_t leader = elect_leader();
-    const bool keys = warp == kProducerWarp, values = !LISTS || warp == kValueWarp;
+    const bool keys = warp == kProducerWarp, values = !keys;
     if (keys) {
       if (leader) mbar_arrive_expect_tx(q_full, nqs * q_chunk);
       __syncwarp();
@@ -537,7 +537,7 @@ bool plan_tiles(int L, int D, int q_rows, int page, int q_tmem, TilePlan* p) {
 
 // A full query tile of 576 columns (144 KB) leaves room for one V buffer: the loads of a tile's values then wait for the product of
 // the tile before it, a load latency per tile. O, scores and probabilities leave 64 columns of tensor memory, which hold two of the
-// nine query chunks: room for a second buffer. 128 heads, one layer: 64 sequences decoding behind 4096 tokens 196 -> 182 us, 1000
+// nine query chunks: room for a second buffer. 128 heads, one layer: 64 sequences decoding behind 4096 tokens (pages of 16) 196 -> 182 us, 1000
 // tokens x 2048 listed keys 2.01 -> 1.73 ms.
 bool plan_tiles(int L, int D, int q_rows, int page, TilePlan* p) {
   const bool fits = plan_tiles(L, D, q_rows, page, 0, p);
@@ -602,7 +602,7 @@ PXL_EXPORT int pxl_latent_attn_tc(const void* q, const void* cache, const int* b
       return PXL_ERR_CUDA;
     configured[dev] = true;
   }
-  pxl_host::launch(topk ? latent_attn_tc_kernel<true> : latent_attn_tc_kernel<false>, grid, dim3(topk ? kThreads<true> : kThreads<false>), plan.smem, stream, tq, tkv,
+  pxl_host::launch(topk ? latent_attn_tc_kernel<true> : latent_attn_tc_kernel<false>, grid, dim3(kThreads), plan.smem, stream, tq, tkv,
                    trow, a);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
