@@ -919,6 +919,16 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       pf[1] = pack_f16x2(s[0][2], s[0][3]);
       pf[2] = pack_f16x2(s[1][0], s[1][1]);
       pf[3] = pack_f16x2(s[1][2], s[1][3]);
+      if (tok_base + 16 > hi || (tok_base < lo && tok_base + 16 > keep)) {
+        // The pages come whole. A probability of 0 times a NaN byte of a token that is not seen (what the page's last owner left
+        // behind the context) would be NaN: this warp's rows of such tokens become zeros, in the first and last tiles only.
+        for (int i = lane; i < 16 * 8; i += 32) {
+          const int tok = tok_base + (i >> 3);
+          if (!(tok < hi && (tok >= lo || tok < keep))) st_shared_zero16(v_smem + (r0 + (i >> 3)) * 128 + (i & 7) * 16);
+        }
+        fence_proxy_async_smem();  // the stage is loaded again
+        __syncwarp();
+      }
       const int mi = lane >> 3, row = r0 + (mi & 1) * 8 + (lane & 7);
 #pragma unroll
       for (int c = 0; c < 8; c += 2) {  // 16 columns per 16-byte chunk

@@ -37,3 +37,32 @@ def test_decode_over_e4m3_pages(Hq, Hkv, page, window, sinks, splits, q_scale):
     want = ref.attn_decode(q, k, v, table, cl, D ** -0.5, window=window, sinks=s, kv_scale=(0.5, 3.0))
     # one rounding of the output to bf16 (2^-9) on either side; probabilities are rounded to 2^-11
     assert float((got.cpu().float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("page,window,splits,byte", [(16, 0, 1, 0x7F), (32, 0, 3, 0xFF), (64, 70, 1, 0x7F), (16, 70, 9, 0xFF)])
+def test_bytes_of_tokens_that_are_not_seen(page, window, splits, byte):
+    """NaN bytes behind the contexts (a freed page keeps its contents) and ahead of the window change no bit."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(page + splits)
+    Hq, Hkv, D, ctx = 8, 2, 128, [1, 15, 17, 64, 65, 130, 700]
+    need = [-(-c // page) for c in ctx]
+    ids, at = torch.randperm(sum(need)), 0
+    table = torch.zeros(len(ctx), max(need), dtype=torch.int32)
+    seen = torch.zeros(sum(need), page, dtype=torch.bool)
+    for i, (n, c) in enumerate(zip(need, ctx)):
+        mine, at = ids[at:at + n], at + n
+        table[i, :n] = mine.int()
+        rows = torch.zeros(n * page, dtype=torch.bool)
+        rows[max(0, c - window) if window else 0:c] = True
+        seen[mine] = rows.view(n, page)
+    k, v = (torch.randn(sum(need), Hkv, page, D).to(torch.float8_e4m3fn).view(torch.uint8) for _ in range(2))
+    q = torch.randn(len(ctx), Hq, D).bfloat16().cuda()
+    out = []
+    for fill in (0, byte):
+        hidden = [t.masked_fill(~seen[:, None, :, None], fill).view(torch.float8_e4m3fn).cuda() for t in (k, v)]
+        out.append(cu.attn_decode(q, *hidden, table.cuda(), torch.tensor(ctx).int().cuda(), D ** -0.5, window=window, num_splits=splits,
+                                  max_ctx=max(ctx)))
+    cu.check_status(torch.device("cuda", 0))
+    assert bool(torch.isfinite(out[0].float()).all())
+    assert torch.equal(*out)
