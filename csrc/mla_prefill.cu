@@ -139,6 +139,13 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       for (int it = 0; ok && it < n_all; ++it) {
         ok = wait(v_full, it & 1, PXL_DEV_TIMEOUT_FULL);
         if (ok && it + 1 < n_all) ok = k_ready(it + 1);
+        if (const int seen = L - it * kT; ok && seen < kT) {
+          // The last tile ends in the next prompt of the batch: a probability of 0 times what is no number there would be NaN
+          for (int i = lane; i < (kT - seen) * 16; i += 32)
+            st_shared_zero16(sm0 + kOffV + ((i >> 3) & 1) * kHalf + (seen + (i >> 4)) * 128 + (i & 7) * 16);
+          fence_proxy_async_smem();
+          __syncwarp();
+        }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           if (!ok || it >= tiles(u)) continue;

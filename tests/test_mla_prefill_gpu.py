@@ -27,3 +27,25 @@ def test_expanded_prompts(H, lens):
     assert float((b.cpu().float() - a.float()).norm() / a.float().norm()) < 2 ** -8      # rotated in place
     # probabilities, expanded values and outputs are rounded to bf16 (2^-9 each)
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("lens", [[65, 63], [1, 300], [129, 1, 127], [255, 2], [383, 200]])     # last tiles of either block of queries
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_prompts_do_not_see_the_next_one(lens, bad):
+    """Keys and values of the next prompt of the batch that are no numbers change no bit of the prompts before it."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(sum(lens))
+    H, T, nope, R, V, L = 3, sum(lens), 128, 64, 128, 512
+    q, rows = torch.randn(T, H * (nope + R)).bfloat16().cuda(), torch.randn(T, L + R).bfloat16().cuda()
+    w = (torch.randn(H * (nope + V), L) * 0.05).bfloat16().cuda()
+    cs, pos = ref.build_cos_sin(800, R, 1e4).cuda(), torch.cat([torch.arange(n) for n in lens]).int().cuda()
+    cu_q = torch.tensor([0] + lens).cumsum(0).int().cuda()
+    out = []
+    for value in (0.0, bad):
+        other = rows.clone()
+        other[lens[0]:] = value
+        out.append(cu.mla_prefill(q.clone(), other, w, cs, pos, cu_q, H, nope, V, L, 192 ** -0.5, max(lens))[:lens[0]])
+    cu.check_status(torch.device("cuda", 0))
+    assert bool(torch.isfinite(out[0].float()).all())
+    assert torch.equal(*out)
