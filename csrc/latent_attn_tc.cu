@@ -72,6 +72,19 @@ struct TcArgs {
 __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
   return (umma_desc_k_sw128(addr) & ~(0x3fffull << 16)) | (static_cast<uint64_t>(kKvChunk >> 4) << 16);
 }
+// Zeros over the rows of a value buffer (`chunks` of NK rows x 128 bytes) whose bits are set, by 128 threads. A function of its own
+// and not inlined: each CTA calls it once ahead of its tiles with no bit set, while the first loads are on their way, so that its
+// instructions are at hand in the last tile (inlined and cold it cost 2.5 us of 141 for 64 sequences of 4096 keys; 0 this way).
+__device__ __noinline__ void clear_rows(uint32_t v, int chunks, uint32_t rows, uint32_t rows2) {
+#pragma unroll 1
+  for (int k = threadIdx.x >> 3; k < NK; k += 16) {
+    if (!((k < 32 ? rows : rows2) >> (k & 31) & 1u)) continue;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) st_shared_zero16(v + c * kKvChunk + k * 128 + (threadIdx.x & 7) * 16);
+  }
+  fence_proxy_async_smem();
+}
+
 template <bool LISTS>
 __global__ void __launch_bounds__(kThreads, 1)
 latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid_constant__ CUtensorMap tm_kv,
@@ -371,17 +384,17 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
       if (lane == 0) mbar_arrive(q_full);
     }
     // of the listed keys of a tile, those that are visible (a bit each)
-    auto visible = [&](int it, uint32_t (&seen)[2]) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int j = it * NK + half * 32 + lane, kp = j < a.topk_k ? list[j] : -1;
-        seen[half] = __ballot_sync(0xffffffffu, kp >= 0 && kp <= pos0);
-      }
-    };
     uint32_t seen[2] = {0u, 0u};
-    if (listed) visible(0, seen);
+    auto entry = [&](int j) { return listed && j < a.topk_k ? list[j] : -1; };
+    auto visible = [&](int kp, int kp2) {
+      seen[0] = __ballot_sync(0xffffffffu, kp >= 0 && kp <= pos0);
+      seen[1] = __ballot_sync(0xffffffffu, kp2 >= 0 && kp2 <= pos0);
+    };
+    if (listed) visible(entry(lane), entry(32 + lane));
+    clear_rows(sm_v, nv, 0u, 0u);
     for (int it = 0; it < n_tiles; ++it) {
       const int par = it & 1;
+      const int next = entry((it + 1) * NK + lane), next2 = entry((it + 1) * NK + 32 + lane);
       failed = mbar_wait_bounded(s_full + 8 * par, (it >> 1) & 1, abort_flag, a.status, PXL_DEV_TIMEOUT_TMEM_FULL) ? 0 : 1;
       failed = __any_sync(0xffffffffu, failed);  // warp-uniform: the TMEM accesses below are warp-wide
       if (failed) break;
@@ -400,7 +413,6 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
           for (int j = 0; j < NK; ++j)
             if (!(seen[j >> 5] >> (j & 31) & 1u)) sc[j] = 0xff800000u;  // -inf
         }
-        if (it + 1 < n_tiles) visible(it + 1, seen);
       }
       if (!__all_sync(0xffffffffu, ma <= 0 && me >= NK)) {
 #pragma unroll
@@ -459,9 +471,20 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
       for (int c = 0; c < NK / 2; c += 16)
         tmem_st_32x32b_x16(tm_p + par * (NK / 2) + c + lane_sel, *reinterpret_cast<uint32_t(*)[16]>(&pk[c]));
       tmem_st_wait();
+      if (listed ? (seen[0] & seen[1]) != 0xffffffffu : key0 < lo || key0 + NK > hi) {
+        // Rows that no query of the tile sees (behind the context, ahead of the window, stand-ins of a list's empty entries): a
+        // probability of 0 times what is no number there would be NaN. The scores have read these buffers, the product has not.
+        if (!listed) {
+          auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; };
+          const int from = lo - key0, to = hi - key0;
+          seen[0] = below(to) & ~below(from), seen[1] = below(to - 32) & ~below(from - 32);
+        }
+        clear_rows(sm_v + it % a.v_bufs * per * kKvChunk, nv, ~seen[0], ~seen[1]);
+      }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_ready + 8 * par);
+      if (listed) visible(next, next2);
     }
     if (!failed)
       failed = mbar_wait_bounded(o_full + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, abort_flag, a.status,

@@ -78,3 +78,51 @@ def test_wide_rows_with_a_part_of_the_query_in_tensor_memory(H, page, prompts):
     cu.check_status(torch.device("cuda", 0))
     # probabilities and outputs are rounded to bf16 (2^-9 each)
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("H,page,prompts,k,window", [
+    (128, 64, [(1, 130), (1, 64), (1, 1)], 0, 0),       # decoding; a context that ends with its page
+    (128, 16, [(1, 700), (1, 77)], 0, 100),             # keys ahead of the window, in the first tile's pages
+    (24, 16, [(11, 75), (7, 7)], 0, 0),                 # tokens that share a tile: rows behind the last one's
+    (192, 128, [(3, 70)], 0, 0),
+    (16, 8, [(40, 130)], 48, 0),                        # lists, with entries that name no key
+    (128, 64, [(1, 300), (1, 65)], 100, 0),             # a last tile of lists that is not full
+])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_rows_that_are_not_seen(H, page, prompts, k, window, bad):
+    """Cache rows behind a context, ahead of a window or off the lists that are no numbers change no bit."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(H + page)
+    L, R, T = 512, 64, sum(n for n, _c in prompts)
+    need = [-(-c // page) for _n, c in prompts]
+    table = torch.zeros(len(prompts), max(need), dtype=torch.int32)
+    blocks, at, t = torch.randperm(sum(need)), 0, 0
+    seen = torch.zeros(sum(need), page, dtype=torch.bool)
+    lists = torch.full((T, k), -1, dtype=torch.int32) if k else None
+    for i, (n, (new, c)) in enumerate(zip(need, prompts)):
+        mine, at = blocks[at:at + n], at + n
+        table[i, :n] = mine.int()
+        rows = torch.zeros(n * page, dtype=torch.bool)
+        if k:       # a list per token out of the sequence's keys but the first one, short of a few entries
+            for pos in range(c - new, c):
+                keys = 1 + torch.randperm(pos)[:k]
+                keys = keys if len(keys) < k else keys[:k - 3]
+                lists[t, :len(keys)] = keys.int()
+                rows[keys] = True
+                t += 1
+        else:
+            rows[max(0, c - new - window + 1) if window else 0:c] = True
+        seen[mine] = rows.view(n, page)
+    cache = torch.randn(sum(need), 1, page, L + R).bfloat16()
+    q = (torch.randn(T, H, L + R) * 0.5).bfloat16().cuda()
+    cu_q = torch.tensor([0] + [n for n, _c in prompts]).cumsum(0).int().cuda()
+    out = []
+    for value in (0.0, bad):
+        hidden = cache.masked_fill(~seen[:, None, :, None], value).cuda()
+        out.append(cu.latent_attn(q, hidden, table.cuda(), cu_q, torch.tensor([c for _n, c in prompts]).int().cuda(), 192 ** -0.5, L,
+                                  window=window, max_q=max(n for n, _c in prompts), max_ctx=max(c for _n, c in prompts),
+                                  topk=None if lists is None else lists.cuda()))
+    cu.check_status(torch.device("cuda", 0))
+    assert bool(torch.isfinite(out[0].float()).all())
+    assert torch.equal(*out)
