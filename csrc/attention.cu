@@ -377,9 +377,9 @@ attn_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const void* __r
 // of its own (warp 4) and the stages are handed back through "empty" mbarriers (one arrival per
 // consumer warp), so the consumer warps never meet at a CTA-wide barrier inside the loop: with the
 // producer inside warp 0 and a __syncthreads per tile the top stall was that barrier.
-// ---- split-KV results met inside a thread-block cluster (2 to 8 splits): the CTAs of a (sequence, key head) leave their partial
-// outputs, maxima and sums in shared memory, and each adds a share of the columns over all of them. Saves the workspace's round
-// trip and a kernel whose launch is most of its 4 to 5 us, once per layer of a chat.
+// ---- split-KV results met inside a thread-block cluster (2 to 8 splits of few sequences: splits_together): the CTAs of a
+// (sequence, key head) leave their partial outputs, maxima and sums in shared memory, and each adds a share of the columns over all
+// of them. Saves the workspace's round trip and a kernel whose launch is most of its 4 to 5 us, once per layer of a chat.
 constexpr int kMaxClusterSplits = 8;
 
 __device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
@@ -1252,6 +1252,42 @@ PXL_EXPORT int pxl_attn_decode_splits(int B, int Hkv, int max_ctx) {
 }
 
 namespace {
+constexpr int kDecSmem = 1024 + kDecStages * 2 * TILE * 128 * 2 + 128, kE4Smem = 1024 + kE4Stages * 2 * kE4Tile + 128;
+
+// Clusters of `splits` CTAs of a kernel that are on the chip at once; asked for once per device and size.
+template <auto Kernel>
+int resident_clusters(int splits, int smem) {
+  static std::atomic<int> known[64][kMaxClusterSplits + 1];  // count + 1
+  std::atomic<int>& entry = known[pxl_host::current_device_slot()][splits];
+  if (const int n = entry.load(std::memory_order_relaxed)) return n - 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1, 1, splits);
+  cfg.blockDim = dim3(kDecThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = static_cast<unsigned>(splits);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (set_smem(Kernel, smem) || cudaOccupancyMaxActiveClusters(&n, Kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  entry.store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+// Whether the splits of `pairs` (sequence, key head) pairs add their results inside clusters: where all of them are on the chip at
+// once. Then the reduction's launch is saved (8 rows x 8 key heads x 777 keys in 4 splits: 10.9 us for the two kernels, 9.9 for the
+// one). A cluster that has to wait waits for as many places at once, which costs more than that: 8 rows x 8 key heads x 2100 keys
+// in 5 splits 20.8 and 24.5 us, 48 x 4 in 2 splits 48.0 and 49.7.
+template <auto Together>
+bool splits_together(int64_t pairs, int splits, int smem) {
+  return splits > 1 && splits <= kMaxClusterSplits && pairs <= resident_clusters<Together>(splits, smem);
+}
+
 // One kernel of the splits (grid.z): alone, as clusters that add their results, or with the reduction behind it.
 template <auto Alone, auto Together, auto Reduce, typename... Args>
 int launch_decode_splits(dim3 grid, int smem, int B, int Hq, const float* workspace, const float* sinks, void* out, cudaStream_t stream,
@@ -1263,7 +1299,7 @@ int launch_decode_splits(dim3 grid, int smem, int B, int Hq, const float* worksp
     if (set_smem(Alone, smem) || set_smem(Together, smem)) return PXL_ERR_CUDA;
     done[dev] = true;
   }
-  if (splits == 1 || splits > kMaxClusterSplits) {
+  if (!splits_together<Together>(static_cast<int64_t>(grid.x) * grid.y, splits, smem)) {
     pxl_host::launch(Alone, grid, kDecThreads, smem, stream, args...);
     if (splits > 1) pxl_host::launch(Reduce, dim3(Hq, B), 128, 0, stream, workspace, sinks, static_cast<bf16*>(out), Hq, splits);
     return check_launch();
@@ -1307,11 +1343,10 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
     if (!pxl_host::make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k_cache, rows, 128, 128, page_size, 64) ||
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v_cache, rows, 128, 128, page_size, 64))
       return PXL_ERR_TENSORMAP;
-    constexpr int SMEM = 1024 + kDecStages * 2 * TILE * 128 * 2 + 128;
     auto go = [&](auto sm) {
       constexpr int M = decltype(sm)::value;
       return launch_decode_splits<attn_decode_tma_kernel<M, false>, attn_decode_tma_kernel<M, true>, attn_decode_reduce_kernel<128, M>>(
-          grid, SMEM, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
+          grid, kDecSmem, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
           static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2, window, keep_first,
           num_splits, sa, status);
     };
@@ -1327,9 +1362,8 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
     if (!pxl_host::make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k_cache, rows, 128, 128, page_size, 128) ||
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, v_cache, rows, 128, 128, page_size, 128))
       return PXL_ERR_TENSORMAP;
-    constexpr int SMEM = 1024 + kE4Stages * 2 * kE4Tile + 128;
     return launch_decode_splits<attn_decode_e4m3_kernel<false>, attn_decode_e4m3_kernel<true>, attn_decode_reduce_kernel<128, kPlain>>(
-        grid, SMEM, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
+        grid, kE4Smem, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
         static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2 * k_scale, window, keep_first,
         num_splits, v_scale, status);
   }
@@ -1369,6 +1403,18 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
   return check_launch();
 }
 }  // namespace
+
+PXL_EXPORT int pxl_attn_decode_launches(int B, int Hkv, int D, int page_size, int num_splits, int cache_fp8, float softcap,
+                                        int sigmoid) {
+  if (num_splits <= 1) return 1;
+  if (D != 128 || (page_size != 16 && page_size != 32 && page_size != 64)) return 2;
+  const int64_t pairs = static_cast<int64_t>(B) * Hkv;
+  const bool one = cache_fp8       ? splits_together<attn_decode_e4m3_kernel<true>>(pairs, num_splits, kE4Smem)
+                   : sigmoid       ? splits_together<attn_decode_tma_kernel<kSigmoid, true>>(pairs, num_splits, kDecSmem)
+                   : softcap > 0.f ? splits_together<attn_decode_tma_kernel<kCapped, true>>(pairs, num_splits, kDecSmem)
+                                   : splits_together<attn_decode_tma_kernel<kPlain, true>>(pairs, num_splits, kDecSmem);
+  return one ? 1 : 2;
+}
 
 PXL_EXPORT int pxl_attn_decode(const void* q, int64_t q_stride, const void* k_cache,
                                const void* v_cache,

@@ -155,8 +155,7 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
                               sp->d_ctx, attn + static_cast<size_t>(sp->Tp) * Hq * D, ws->decode, L.sinks, sp->Bd, Hq,
                               Hkv, D, st->page, sp->d_max_blocks, st->num_blocks, st->scale, L.window, 0, splits,
                               sp->d_max_ctx, 0.f, nullptr, status, stream));
-      // (a few splits add their results inside a cluster)
-      n += splits == 1 || (splits <= 8 && D == 128 && (st->page == 16 || st->page == 32 || st->page == 64)) ? 1 : 2;
+      n += pxl_attn_decode_launches(sp->Bd, Hkv, D, st->page, splits, 0, 0.f, 0);
     }
     PXL_TRY(pxl_gemm_bf16(attn, L.w_o, h_mid, h, L.b_o, T, H, Hq * D, Hq * D, Hq * D, H, PXL_EPI_RESIDUAL, 0, status,
                           stream));

@@ -80,6 +80,7 @@ _SIGS = {
     "pxl_attn_decode": [_P, c_int64, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
                         c_int64, c_float, c_int, c_int, c_int, c_int, c_float, _P, _P, _P],
     "pxl_attn_decode_splits": [c_int, c_int, c_int],
+    "pxl_attn_decode_launches": [c_int] * 6 + [c_float, c_int],
     "pxl_attn_prefill": [_P, c_int64, _P, _P, _P, _P, _P, _P, c_int64, _P, c_int, c_int, c_int,
                          c_int, c_int, c_int, c_int, c_int64, c_float, c_int, c_int, c_float, _P, _P, _P],
     "pxl_attn_prefill_tc": [_P, c_int64, _P, _P, _P, _P, _P, _P, c_int64, _P, c_int, c_int, c_int, c_int,

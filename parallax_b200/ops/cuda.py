@@ -429,12 +429,6 @@ def _attn_on_tensor_cores(q, k_cache, scale: float, max_group: int) -> bool:
     return q.dtype == torch.bfloat16 and q.shape[2] in (64, 128) and q.shape[1] // k_cache.shape[1] <= max_group and scale > 0
 
 
-def _decode_launches(splits: int, D: int, page: int) -> int:
-    """Kernels of one decode attention: a few splits add their results inside a cluster, more in a kernel of their own."""
-    together = D == 128 and page in (16, 32, 64) and splits <= 8
-    return 1 if splits == 1 or together else 2
-
-
 def attn_decode(
     q: torch.Tensor,
     k_cache: torch.Tensor,
@@ -481,7 +475,7 @@ def attn_decode(
                 float(kv_scale[0]), float(kv_scale[1]), status_tensor(q.device).data_ptr(), _stream(q.device)),
             "pxl_attn_decode_fp8",
         )
-        _count(_decode_launches(num_splits, D, page))
+        _count(_lib.lib().pxl_attn_decode_launches(B, Hkv, D, page, num_splits, 1, 0.0, 0))
         return out
     check(
         _lib.lib().pxl_attn_decode(
@@ -492,7 +486,7 @@ def attn_decode(
             softcap, _ptr(sigmoid_bias), status_tensor(q.device).data_ptr(), _stream(q.device)),
         "pxl_attn_decode",
     )
-    _count(_decode_launches(num_splits, D, page))
+    _count(_lib.lib().pxl_attn_decode_launches(B, Hkv, D, page, num_splits, 0, softcap, sigmoid_bias is not None))
     return out
 
 

@@ -1,0 +1,35 @@
+"""Decode attention in splits: added inside clusters where all of them are on the chip at once, through the workspace otherwise."""
+
+import pytest
+import torch
+
+from parallax_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,splits,kernels", [(1, 8, 1), (2, 9, 2), (74, 2, 1), (80, 2, 2), (40, 5, 2)])
+@pytest.mark.parametrize("fp8,kw", [(False, {}), (False, dict(softcap=20.0)), (False, dict(sigmoid=True)), (False, dict(sinks=True)),
+                                    (True, dict(sinks=True))])
+def test_splits(B, splits, kernels, fp8, kw):
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(B + splits)
+    Hq, Hkv, D, page, kw = 8, 2, 128, 16, dict(kw)
+    ctx = torch.tensor([1 + 37 * i % 640 for i in range(B)]).int()      # some splits have no keys
+    if kw.pop("sinks", False):
+        kw["sinks"] = torch.randn(Hq)
+    if kw.pop("sigmoid", False):
+        kw["sigmoid_bias"] = torch.randn(Hq) - 3.0
+    table = torch.randperm(B * 40).int().view(B, 40)
+    k, v = (torch.randn(B * 40, Hkv, page, D).to(torch.float8_e4m3fn if fp8 else torch.bfloat16) for _ in range(2))
+    q = torch.randn(B, Hq, D).bfloat16()
+    to = lambda a: a.cuda() if isinstance(a, torch.Tensor) else a  # noqa: E731
+    before = cu.launch_count
+    got = cu.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), ctx.cuda(), D ** -0.5, max_ctx=640, num_splits=splits,
+                         **{n: to(a) for n, a in kw.items()})
+    assert cu.launch_count - before == kernels
+    cu.check_status(torch.device("cuda", 0))
+    want = ref.attn_decode(q, k, v, table, ctx, D ** -0.5, **kw)
+    # probabilities and outputs are rounded to bf16 (2^-9 each)
+    assert float((got.cpu().float() - want.float()).norm() / want.float().norm()) < 2 ** -7
