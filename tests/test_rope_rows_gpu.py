@@ -34,3 +34,23 @@ def test_norm_rotation_cache(D, rot, Hq, Hkv, fp8):
     for x, y, lim in ((a[0][:, :Hq * D], b[0][:, :Hq * D], 2 ** -7), (a[1], b[1], 2 ** -4 if fp8 else 2 ** -7), (a[2], b[2], 0.0)):
         d = (x.float() - y.cpu().float()).norm() / x.float().norm()
         assert float(d) <= lim
+
+
+@pytest.mark.parametrize("T", [1, 100, 197, 300, 700])      # a token's heads over three blocks, two and one
+@pytest.mark.parametrize("D,Hq,Hkv", [(128, 32, 4), (64, 7, 30), (256, 9, 4)])
+def test_blocks_per_token(T, D, Hq, Hkv):
+    """However the heads of a token are shared out, every row comes out as in a batch of another size."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(T + D)
+    n, page = 2000, 16
+    qkv, pos = torch.randn(n, (Hq + 2 * Hkv) * D).bfloat16().cuda(), torch.randint(0, 300, (n,)).int().cuda()
+    w, cs, slots = torch.randn(2, D).bfloat16().cuda(), ref.build_cos_sin(300, D, 1e4).cuda(), torch.randperm(n).cuda()
+    out = []
+    for rows in (n, T):
+        x = [qkv[:rows].clone()] + [torch.zeros(n // page, Hkv, page, D, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        cu.qk_norm_rope_cache(x[0], w[0], w[1], cs, pos[:rows], slots[:rows], x[1], x[2], Hq, Hkv, D, D)
+        at = slots[:T]
+        out.append([x[0][:T]] + [c[at // page, :, at % page] for c in x[1:]])
+    cu.check_status(torch.device("cuda", 0))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
