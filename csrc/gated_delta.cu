@@ -18,10 +18,12 @@
 //    The first makes X and P of every chunk and head in parallel, the second walks the chunks of a (sequence, head, 32 columns
 //    of v) with S in registers, the third norms and gates the heads. Because the decay is one number per token it stays out of
 //    the products with q, k and v, which enter the tensor cores as the bf16 numbers they are; what is fp32 (S, X, P, u)
-//    enters as the sum of two bf16 numbers (rounding 2^-17), the triangular system is solved in fp32, and o stays fp32 up to
-//    the norm. No exponent is positive. The walk is a chain of chunks, bound by the latency of its four products and three
-//    barriers; everything it reads is one chunk ahead. Two prompts of 2950 tokens, 32 heads: 109 + 314 + 46 us for the three
-//    kernels (8.0 ms token by token); their working space is at most 256 MB, longer prompts go through it in runs.
+//    enters as the sum of three bf16 numbers, with every partial product above 2^-24, the triangular system is solved in fp32,
+//    and o stays fp32 up to the norm. No exponent is positive. The kept state's error against 64 bits after 16 slices of 257
+//    tokens is 0.8e-7 to 3.0e-7 for decays of 0.0025 to 7 per token (sums of two bf16 numbers: 3.4e-6 to 6.6e-6, and 314 us for the
+//    walk). The walk is a chain of chunks, bound by the latency of its four products and three barriers; everything it reads is
+//    one chunk ahead. Two prompts of 2950 tokens, 32 heads: 107 + 474 + 47 us for the three kernels (8.0 ms token by token);
+//    their working space is at most 256 MB, longer prompts go through it in runs.
 //
 // This file is compiled without fast math: what enters the recurrence uses the accurate functions.
 #include "common.cuh"
@@ -169,19 +171,28 @@ __global__ void __launch_bounds__(256, 2) delta_step_kernel(const GdArgs a, int 
 }
 
 // ---- chunks ------------------------------------------------------------------------------------------------
-// What the kernels hand on, per (chunk, head), in bytes: high and low parts of X and P [64][64] bf16, factors of the rows, o
+// What the kernels hand on, per (chunk, head), in bytes: X and P [64][64] fp32, factors of the rows, o
 struct Record {
-  static constexpr int XH = 0, XL = XH + kChunk * kChunk * 2, PH = XL + kChunk * kChunk * 2, PL = PH + kChunk * kChunk * 2;
-  static constexpr int F = PL + kChunk * kChunk * 2;  // fp32: e^G ik | e^G iq | e^(G_n - G) ik | e^(G_n), padded to 256
+  static constexpr int X = 0, P = X + kChunk * kChunk * 4;
+  static constexpr int F = P + kChunk * kChunk * 4;  // fp32: e^G ik | e^G iq | e^(G_n - G) ik | e^(G_n), padded to 256
   static constexpr int kFactors = 4 * kChunk;
   static constexpr int O = F + kFactors * 4;  // [64][Dv] fp32
   __host__ __device__ static int64_t bytes(int Dv) { return O + static_cast<int64_t>(kChunk) * Dv * 4; }
 };
 
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
-  hi = pack_bf16x2(a, b);
-  const float2 f = unpack_bf16x2(hi);
-  lo = pack_bf16x2(a - f.x, b - f.y);
+// Two fp32 numbers as sums of three bf16 numbers each (rounding 2^-27: none that fp32 does not have).
+struct Parts {
+  uint32_t v[3];
+};
+__device__ __forceinline__ Parts split3(float a, float b) {
+  Parts p;
+  p.v[0] = pack_bf16x2(a, b);
+  float2 f = unpack_bf16x2(p.v[0]);
+  a -= f.x, b -= f.y;
+  p.v[1] = pack_bf16x2(a, b);
+  f = unpack_bf16x2(p.v[1]);
+  p.v[2] = pack_bf16x2(a - f.x, b - f.y);
+  return p;
 }
 
 // chunk number `id` of the prompt slices: sequence and number within it; false past the last one. Warp-collective.
@@ -327,14 +338,8 @@ __global__ void __launch_bounds__(kMakeThreads) delta_make_kernel(const GdArgs a
             const float decay = in ? expf((s.gh[t] - s.gh[j + c]) + (s.gl[t] - s.gl[j + c])) : 0.f;
             w[c] = d[cb][u][2 * e + c] * decay * s.ik[j + c] * (score ? s.iq[t] : s.b[t] * s.ik[t]);
           }
-          if (score) {
-            uint32_t hi, lo;
-            split2(w[0], w[1], hi, lo);
-            *reinterpret_cast<uint32_t*>(rec + Record::PH + (t * kChunk + j) * 2) = hi;
-            *reinterpret_cast<uint32_t*>(rec + Record::PL + (t * kChunk + j) * 2) = lo;
-          } else {
-            *reinterpret_cast<float2*>(&s.A[t][j]) = make_float2(w[0], w[1]);
-          }
+          *reinterpret_cast<float2*>(score ? reinterpret_cast<float*>(rec + Record::P) + t * kChunk + j : &s.A[t][j]) =
+              make_float2(w[0], w[1]);
         }
     }
   }
@@ -394,27 +399,60 @@ __global__ void __launch_bounds__(kMakeThreads) delta_make_kernel(const GdArgs a
     const int t = i / (kChunk / 4), j = i % (kChunk / 4) * 4;
     if (j / kBlock > t / kBlock) continue;  // (the walk does not use the blocks above the diagonal)
     const float4 v = *reinterpret_cast<const float4*>(&s.X[t][j]);
-    uint2 hi, lo;
-    split2(v.x * s.b[j], v.y * s.b[j + 1], hi.x, lo.x);
-    split2(v.z * s.b[j + 2], v.w * s.b[j + 3], hi.y, lo.y);
-    *reinterpret_cast<uint2*>(rec + Record::XH + (t * kChunk + j) * 2) = hi;
-    *reinterpret_cast<uint2*>(rec + Record::XL + (t * kChunk + j) * 2) = lo;
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(rec + Record::X) + t * kChunk + j) =
+        make_float4(v.x * s.b[j], v.y * s.b[j + 1], v.z * s.b[j + 2], v.w * s.b[j + 3]);
   }
 }
 
+constexpr int kPitchM = kChunk + 8;  // pairs of a quarter warp's rows hit distinct banks
+
 struct WalkStage {
   bf16 q[kChunk][kPitch], k[kChunk][kPitch];
-  bf16 xh[kChunk][kChunk + 8], xl[kChunk][kChunk + 8], ph[kChunk][kChunk + 8], pl[kChunk][kChunk + 8];
+  float x[kChunk][kPitchM], p[kChunk][kPitchM];
   bf16 v[kChunk][kSlice + 8];
   float f[Record::kFactors];
 };
-struct WalkSmem {
+struct WalkSmem {  // [3]: the parts of fp32 numbers
   WalkStage st[2];
-  bf16 s_hi[DK][kSlice + 8], s_lo[DK][kSlice + 8];
-  bf16 r_hi[kChunk][kSlice + 8], r_lo[kChunk][kSlice + 8];  // v - e^G K S
-  bf16 u_hi[kChunk][kSlice + 8], u_lo[kChunk][kSlice + 8];
-  bf16 d_hi[kChunk][kSlice + 8], d_lo[kChunk][kSlice + 8];  // e^(G_n - G) ik u
+  bf16 s[3][DK][kSlice + 8];
+  bf16 r[3][kChunk][kSlice + 8];  // v - e^G K S
+  bf16 u[3][kChunk][kSlice + 8];
+  bf16 d[3][kChunk][kSlice + 8];  // e^(G_n - G) ik u
 };
+static_assert(sizeof(WalkSmem) <= 227 * 1024, "shared memory of a CTA");
+
+template <int ROWS>
+__device__ __forceinline__ void put_parts(bf16 (&dst)[3][ROWS][kSlice + 8], int r, int c, float a, float b) {
+  const Parts p = split3(a, b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&dst[i][r][c]) = p.v[i];
+}
+
+// acc[0] + acc[1] + acc[2] += M B for 16 rows of an fp32 matrix and 16 rows x 16 columns of an operand in parts: the six products
+// that are not below fp32's rounding, those of a size in an accumulator of their own.
+template <int ROWS>
+__device__ __forceinline__ void mul_parts(float (&acc)[3][2][4], const float (&m)[kChunk][kPitchM], int row, int col,
+                                          const bf16 (&b)[3][ROWS][kSlice + 8], int k0, int c0) {
+  const int lane = threadIdx.x & 31, mi = lane >> 3, r8 = lane & 7, g8 = lane >> 2, t2 = (lane & 3) * 2;
+  uint32_t a[3][4], bp[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = *reinterpret_cast<const float2*>(&m[row + g8 + (i & 1) * 8][col + t2 + (i >> 1) * 8]);
+    const Parts p = split3(v.x, v.y);
+    a[0][i] = p.v[0], a[1][i] = p.v[1], a[2][i] = p.v[2];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) ldmatrix_x4_trans(bp[i], smem_u32(&b[i][k0 + (mi & 1) * 8 + r8][c0 + (mi >> 1) * 8]));
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; i + j < 3; ++j)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const uint32_t b2[2] = {bp[j][2 * n], bp[j][2 * n + 1]};
+        mma_m16n8k16_bf16(acc[i + j][n], a[i], b2);
+      }
+}
 
 // Warps 0 to 7 make u and keep the state, warps 8 to 15 make the outputs.
 constexpr int kHalf = 8, kWalkThreads = 2 * kHalf * 32;
@@ -444,15 +482,12 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
       cp_async_16(smem_u32(&st.q[r][c]), row + hk * DK + c, r < n);
       cp_async_16(smem_u32(&st.k[r][c]), row + (a.Hk + hk) * DK + c, r < n);
     }
-    {  // 512 pieces of 16 bytes in each of the four matrices
-      const int r = tid / (kChunk / 8), c = tid % (kChunk / 8) * 8;
-      if (c / kBlock <= r / kBlock) {
-        const int at = (r * kChunk + c) * 2;
-        cp_async_16(smem_u32(&st.xh[r][c]), rec + Record::XH + at, true);
-        cp_async_16(smem_u32(&st.xl[r][c]), rec + Record::XL + at, true);
-        cp_async_16(smem_u32(&st.ph[r][c]), rec + Record::PH + at, true);
-        cp_async_16(smem_u32(&st.pl[r][c]), rec + Record::PL + at, true);
-      }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {  // pieces of 16 bytes, 1024 in each of the two matrices
+      const int r = tid / (kChunk / 4) + j * (kChunk / 2), c = tid % (kChunk / 4) * 4;
+      if (c / kBlock > r / kBlock) continue;
+      cp_async_16(smem_u32(&st.x[r][c]), rec + Record::X + (r * kChunk + c) * 4, true);
+      cp_async_16(smem_u32(&st.p[r][c]), rec + Record::P + (r * kChunk + c) * 4, true);
     }
     if (tid < kChunk * (kSlice / 8)) {
       const int r = tid / (kSlice / 8), c = tid % (kSlice / 8) * 8;
@@ -462,7 +497,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
       cp_async_16(smem_u32(&st.f[c]), rec + Record::F + c * 4, true);
     }
   };
-  static_assert(kChunk * kChunk / 8 == kWalkThreads, "one piece of X and P per thread");
+  static_assert(kChunk * kChunk / 4 == 2 * kWalkThreads, "two pieces of X and P per thread");
   load(first);
   cp_async_commit();
   if (first + 1 < last) load(first + 1);
@@ -476,12 +511,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        uint32_t hi, lo;
-        split2(S[j][2 * e], S[j][2 * e + 1], hi, lo);
-        *reinterpret_cast<uint32_t*>(&s.s_hi[w8 * 16 + g8 + e * 8][j * 8 + t2]) = hi;
-        *reinterpret_cast<uint32_t*>(&s.s_lo[w8 * 16 + g8 + e * 8][j * 8 + t2]) = lo;
-      }
+      for (int e = 0; e < 2; ++e) put_parts(s.s, w8 * 16 + g8 + e * 8, j * 8 + t2, S[j][2 * e], S[j][2 * e + 1]);
   };
   if (keeper) {
 #pragma unroll
@@ -497,27 +527,27 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
     cp_async_wait<1>();
     __syncthreads();
     // ---- K S and Q S: 16 tokens x 16 columns per warp
-    float o[2][4] = {}, o1[2][4] = {};
+    float o[2][4], part[3][2][4] = {};
     {
       const uint32_t rows = smem_u32(keeper ? &st.k[rg * 16 + (lane & 15)][(lane >> 4) * 8] : &st.q[rg * 16 + (lane & 15)][(lane >> 4) * 8]);
 #pragma unroll
       for (int kk = 0; kk < DK / 16; ++kk) {
-        uint32_t x[4], sh[4], sl[4];
+        uint32_t x[4], sp[4];
         ldmatrix_x4(x, rows + kk * 32);
-        ldmatrix_x4_trans(sh, smem_u32(&s.s_hi[kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
-        ldmatrix_x4_trans(sl, smem_u32(&s.s_lo[kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t bh[2] = {sh[2 * j], sh[2 * j + 1]}, bl[2] = {sl[2 * j], sl[2 * j + 1]};
-          mma_m16n8k16_bf16(o[j], x, bh);
-          mma_m16n8k16_bf16(o1[j], x, bl);
+        for (int i = 0; i < 3; ++i) {
+          ldmatrix_x4_trans(sp, smem_u32(&s.s[i][kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
+          const uint32_t b0[2] = {sp[0], sp[1]}, b1[2] = {sp[2], sp[3]};
+          mma_m16n8k16_bf16(part[i][0], x, b0);
+          mma_m16n8k16_bf16(part[i][1], x, b1);
         }
       }
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[j][e] = (o[j][e] + o1[j][e]) * st.f[(keeper ? 0 : kChunk) + rg * 16 + g8 + (e >> 1) * 8];
+      for (int e = 0; e < 4; ++e)
+        o[j][e] = (part[0][j][e] + (part[1][j][e] + part[2][j][e])) * st.f[(keeper ? 0 : kChunk) + rg * 16 + g8 + (e >> 1) * 8];
     if (keeper) {
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -525,61 +555,33 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
         for (int e = 0; e < 2; ++e) {
           const int r = rg * 16 + g8 + e * 8, c = ch * 16 + j * 8 + t2;
           const float2 v = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&st.v[r][c]));
-          uint32_t hi, lo;
-          split2(v.x - o[j][2 * e], v.y - o[j][2 * e + 1], hi, lo);
-          *reinterpret_cast<uint32_t*>(&s.r_hi[r][c]) = hi;
-          *reinterpret_cast<uint32_t*>(&s.r_lo[r][c]) = lo;
+          put_parts(s.r, r, c, v.x - o[j][2 * e], v.y - o[j][2 * e + 1]);
         }
       asm volatile("bar.sync 1, 256;" ::: "memory");  // the keepers
       // ---- u = X (v - e^G K S)
-      float u[2][4] = {}, u1[2][4] = {}, u2[2][4] = {};
-      for (int kk = 0; kk <= rg; ++kk) {
-        uint32_t xh[4], xl[4], bh[4], bl[4];
-        ldmatrix_x4(xh, smem_u32(&st.xh[rg * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]));
-        ldmatrix_x4(xl, smem_u32(&st.xl[rg * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]));
-        ldmatrix_x4_trans(bh, smem_u32(&s.r_hi[kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
-        ldmatrix_x4_trans(bl, smem_u32(&s.r_lo[kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t h2[2] = {bh[2 * j], bh[2 * j + 1]}, l2[2] = {bl[2 * j], bl[2 * j + 1]};
-          mma_m16n8k16_bf16(u[j], xh, h2);
-          mma_m16n8k16_bf16(u1[j], xh, l2);
-          mma_m16n8k16_bf16(u2[j], xl, h2);
-        }
-      }
+      float u[3][2][4] = {};
+      for (int kk = 0; kk <= rg; ++kk) mul_parts(u, st.x, rg * 16, kk * 16, s.r, kk * 16, ch * 16);
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int r = rg * 16 + g8 + e * 8, c = ch * 16 + j * 8 + t2;
           const float w = st.f[2 * kChunk + r];
-          const float x = u[j][2 * e] + (u1[j][2 * e] + u2[j][2 * e]), y = u[j][2 * e + 1] + (u1[j][2 * e + 1] + u2[j][2 * e + 1]);
-          uint32_t hi, lo;
-          split2(x, y, hi, lo);
-          *reinterpret_cast<uint32_t*>(&s.u_hi[r][c]) = hi;
-          *reinterpret_cast<uint32_t*>(&s.u_lo[r][c]) = lo;
-          split2(x * w, y * w, hi, lo);
-          *reinterpret_cast<uint32_t*>(&s.d_hi[r][c]) = hi;
-          *reinterpret_cast<uint32_t*>(&s.d_lo[r][c]) = lo;
+          const float x = u[0][j][2 * e] + (u[1][j][2 * e] + u[2][j][2 * e]);
+          const float y = u[0][j][2 * e + 1] + (u[1][j][2 * e + 1] + u[2][j][2 * e + 1]);
+          put_parts(s.u, r, c, x, y);
+          put_parts(s.d, r, c, x * w, y * w);
         }
     }
     __syncthreads();
     if (!keeper) {
       // ---- o += P u (blocks up to this one)
-      for (int kk = 0; kk <= rg; ++kk) {
-        uint32_t ph[4], pl[4], bh[4], bl[4];
-        ldmatrix_x4(ph, smem_u32(&st.ph[rg * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]));
-        ldmatrix_x4(pl, smem_u32(&st.pl[rg * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]));
-        ldmatrix_x4_trans(bh, smem_u32(&s.u_hi[kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
-        ldmatrix_x4_trans(bl, smem_u32(&s.u_lo[kk * 16 + (mi & 1) * 8 + r8][ch * 16 + (mi >> 1) * 8]));
+      float pu[3][2][4] = {};
+      for (int kk = 0; kk <= rg; ++kk) mul_parts(pu, st.p, rg * 16, kk * 16, s.u, kk * 16, ch * 16);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t h2[2] = {bh[2 * j], bh[2 * j + 1]}, l2[2] = {bl[2 * j], bl[2 * j + 1]};
-          mma_m16n8k16_bf16(o[j], ph, h2);
-          mma_m16n8k16_bf16(o[j], ph, l2);
-          mma_m16n8k16_bf16(o[j], pl, h2);
-        }
-      }
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] += pu[0][j][e] + (pu[1][j][e] + pu[2][j][e]);
       float* og = reinterpret_cast<float*>(record(i) + Record::O) + v0;
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -590,27 +592,26 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
     } else {
       // ---- S = e^(G_n) S + K^T (e^(G_n - G) ik u)
       const float gn = st.f[3 * kChunk];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) S[j][e] *= gn;
+      float add[3][4][4] = {};
 #pragma unroll
       for (int kk = 0; kk < kChunk / 16; ++kk) {
         uint32_t k[4];
         ldmatrix_x4_trans(k, smem_u32(&st.k[kk * 16 + (mi >> 1) * 8 + r8][w8 * 16 + (mi & 1) * 8]));
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t bh[4], bl[4];
-          ldmatrix_x4_trans(bh, smem_u32(&s.d_hi[kk * 16 + (mi & 1) * 8 + r8][c * 16 + (mi >> 1) * 8]));
-          ldmatrix_x4_trans(bl, smem_u32(&s.d_lo[kk * 16 + (mi & 1) * 8 + r8][c * 16 + (mi >> 1) * 8]));
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const uint32_t h2[2] = {bh[2 * j], bh[2 * j + 1]}, l2[2] = {bl[2 * j], bl[2 * j + 1]};
-            mma_m16n8k16_bf16(S[2 * c + j], k, h2);
-            mma_m16n8k16_bf16(S[2 * c + j], k, l2);
+          for (int i = 0; i < 3; ++i) {
+            uint32_t dp[4];
+            ldmatrix_x4_trans(dp, smem_u32(&s.d[i][kk * 16 + (mi & 1) * 8 + r8][c * 16 + (mi >> 1) * 8]));
+            const uint32_t b0[2] = {dp[0], dp[1]}, b1[2] = {dp[2], dp[3]};
+            mma_m16n8k16_bf16(add[i][2 * c], k, b0);
+            mma_m16n8k16_bf16(add[i][2 * c + 1], k, b1);
           }
-        }
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j][e] = fmaf(gn, S[j][e], add[0][j][e] + (add[1][j][e] + add[2][j][e]));
       publish();  // every read of the old state happened before the last barrier
     }
     __syncthreads();

@@ -110,3 +110,31 @@ def test_convolution_in_runs(K, C, bias):
                                 prefill_seqs=prompts, prefill_tokens=sum(lens[:prompts]))
     assert torch.equal(s1.cpu(), s0)                    # inputs are copied as they are
     assert _rel(got, want) < 2 ** -7                    # one rounding to bf16 on either side
+
+
+@pytest.mark.parametrize("log_a", [-6.0, -2.0, 0.0])
+def test_kept_state_over_slices(log_a):
+    """The state behind several slices of a prompt stays as close to 64 bits in chunks as token by token: both hold fp32 numbers
+    and add fp32 products, in another order (a factor of two), and the chunks' factors take a few more roundings of 2^-24."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(int(-log_a))
+    Hk, Hv, D, T = 1, 2, 128, 150
+    A, dt, w = torch.full((Hv,), log_a).cuda(), torch.linspace(-2, 1, Hv).cuda(), torch.ones(D).bfloat16().cuda()
+    cu_t, slot = torch.tensor([0, T]).int().cuda(), torch.zeros(1).int().cuda()
+    want = torch.zeros(Hv, D, D, dtype=torch.float64, device="cuda")
+    states = [torch.zeros(1, Hv, D, D, device="cuda") for _ in range(2)]
+    for s in range(4):
+        rows, z, ab = (torch.randn(T, n).bfloat16().cuda() for n in (2 * Hk * D + Hv * D, Hv * D, 2 * Hv))
+        for st, prompts in zip(states, (1, 0)):
+            cu.gated_delta_rule(rows, ab[:, :Hv], ab[:, Hv:], A, dt, z, w, st, cu_t, slot, (torch.arange(T) + s * T).int().cuda(), Hk, Hv,
+                                D, D, 1e-6, prefill_seqs=prompts, prefill_tokens=T * prompts)
+        k, v = rows[:, D:2 * D].double(), rows[:, 2 * D:].double().view(T, Hv, D)
+        k = k / (k.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+        g = torch.exp(-torch.exp(A.double()) * torch.nn.functional.softplus(ab[:, :Hv].double() + dt.double()))
+        b = torch.sigmoid(ab[:, Hv:].double())
+        for t in range(T):
+            want *= g[t, :, None, None]
+            want += ((v[t] - want @ k[t]) * b[t, :, None])[:, :, None] * k[t]
+    chunks, steps = (float((st[0].double() - want).norm() / want.norm()) for st in states)
+    assert chunks < 2 * steps + 2 ** -22, (chunks, steps)
