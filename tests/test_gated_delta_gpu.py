@@ -138,3 +138,29 @@ def test_kept_state_over_slices(log_a):
             want += ((v[t] - want @ k[t]) * b[t, :, None])[:, :, None] * k[t]
     chunks, steps = (float((st[0].double() - want).norm() / want.norm()) for st in states)
     assert chunks < 2 * steps + 2 ** -22, (chunks, steps)
+
+
+def test_steps_of_a_long_memory():
+    """Decays of about 0.002 per token: a state remembers some 500 tokens, each of which rounds it twice (2^-25 each, independent)."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(5)
+    Hv, D, T, slices = 2, 128, 257, 8
+    A, dt, w = torch.full((Hv,), -6.0).cuda(), torch.linspace(-2, 1, Hv).cuda(), torch.ones(D).bfloat16().cuda()
+    cu_t, slot = torch.tensor([0, T]).int().cuda(), torch.zeros(1).int().cuda()
+    want, st = torch.zeros(Hv, D, D, dtype=torch.float64, device="cuda"), torch.zeros(1, Hv, D, D, device="cuda")
+    common = torch.randn(1, 2 * D + Hv * D)
+    for s in range(slices):
+        rows = (common * 0.9 + torch.randn(T, 2 * D + Hv * D) * 0.4).bfloat16().cuda()
+        z, ab = (torch.randn(T, n).bfloat16().cuda() for n in (Hv * D, 2 * Hv))
+        cu.gated_delta_rule(rows, ab[:, :Hv], ab[:, Hv:], A, dt, z, w, st, cu_t, slot, (torch.arange(T) + s * T).int().cuda(), 1, Hv, D, D,
+                            1e-6)
+        k, v = rows[:, D:2 * D].double(), rows[:, 2 * D:].double().view(T, Hv, D)
+        k = k / (k.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+        g = torch.exp(-torch.exp(A.double()) * torch.nn.functional.softplus(ab[:, :Hv].double() + dt.double()))
+        b = torch.sigmoid(ab[:, Hv:].double())
+        for t in range(T):
+            want *= g[t, :, None, None]
+            want += ((v[t] - want @ k[t]) * b[t, :, None])[:, :, None] * k[t]
+    err = float((st[0].double() - want).norm() / want.norm())
+    assert err < 2 ** -25 * (2 * 500) ** 0.5, err
