@@ -15,7 +15,7 @@ attention are ``src/parallax/models/deepseek_v32.py:84-238,376-446``. Per-layer 
 from __future__ import annotations
 
 import math
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -37,6 +37,14 @@ def derive_indexer_types(cfg: ModelConfig) -> list[str]:
     off = freq - 1 if off is None else int(off)
     k0 = cfg.first_k_dense_replace
     return ["full" if (i < k0 or (i - k0) % freq == off) else "shared" for i in range(n)]
+
+
+class KeyLists(NamedTuple):
+    """An indexer's choice: key positions per token (a row of -1: all keys), and for which part of the batch there are any. A part
+    whose contexts all fit the choice has none and attends densely."""
+    rows: torch.Tensor        # int32 [T, index_topk]; rows of a part without lists are not set
+    prompts: bool
+    decode: bool
 
 
 class MLALayer:
@@ -249,8 +257,8 @@ class DeepseekStage(DecoderStage):
 
     # ------------------------------------------------------------------ forward
     def _index_topk(self, lw: MLALayer, li: int, qr: torch.Tensor, kv: torch.Tensor, fb: ForwardBatch):
-        """Run the lightning indexer of a "full" layer: store this step's index keys, score the
-        context and select the top-k key positions per query token (-1 rows = attend densely)."""
+        """Run the lightning indexer of a "full" layer: store this step's index keys, score the context and select the top-k
+        key positions per query token: :class:`KeyLists`, or None when no context is longer than the choice."""
         cfg, T, Hi, Di, R = self.cfg, qr.shape[0], self.Hi, self.Di, self.R
         k_top = cfg.index_topk
         cache = self.kv_caches[li].index_k
@@ -264,7 +272,7 @@ class DeepseekStage(DecoderStage):
         need_d = fb.num_decode > 0 and fb.d_max_ctx > k_top
         if not (need_p or need_d):
             return None
-        topk = torch.full((T, k_top), -1, dtype=torch.int32, device=qr.device)
+        topk = torch.empty((T, k_top), dtype=torch.int32, device=qr.device)
         if need_p:
             sc = ops.dsa_index_scores(iq[:Tp], iw[:Tp], cache, fb.p_block_tables, fb.p_cu_q, fb.positions[:Tp],
                                       fb.p_max_ctx)
@@ -273,9 +281,9 @@ class DeepseekStage(DecoderStage):
             sc = ops.dsa_index_scores(iq[Tp:], iw[Tp:], cache, fb.d_block_tables, None, fb.positions[Tp:],
                                       fb.d_max_ctx)
             topk[Tp:] = ops.topk_select(sc, fb.positions[Tp:], k_top)
-        return topk
+        return KeyLists(topk, need_p, need_d)
 
-    def _attention(self, lw: MLALayer, li: int, xn: torch.Tensor, fb: ForwardBatch, topk_prev):
+    def _attention(self, lw: MLALayer, li: int, xn: torch.Tensor, fb: ForwardBatch, lists_prev: Optional[KeyLists]):
         cfg, T, H = self.cfg, xn.shape[0], self.H
         eps = cfg.rms_norm_eps
         if lw.w_q_a is not None:
@@ -286,24 +294,26 @@ class DeepseekStage(DecoderStage):
         kv = ops.linear(xn, lw.w_kv_a)
         cache = self.kv_caches[li].k
         ops.mla_kv_prep(kv[:, :lw.n_kv_a], lw.kv_a_norm, self.cos_sin, fb.positions, fb.slot_mapping, cache, eps, self.L)
-        topk = topk_prev
+        lists = lists_prev
         if self.dsa and lw.idx_mode == "full":
-            topk = self._index_topk(lw, li, qr, kv, fb)
+            lists = self._index_topk(lw, li, qr, kv, fb)
+        topk_p = lists.rows if lists is not None and lists.prompts else None
+        topk_d = lists.rows if lists is not None and lists.decode else None
         Tp = fb.num_prefill_tokens
         if not self._rows_form(cache):
             q_lat, q_pe = ops.mla_q_absorb(q, lw.w_uk_s, self.cos_sin, fb.positions, H, self.nope, self.L)
             o_lat = None
             if Tp:
                 o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.p_block_tables, fb.p_cu_q, fb.positions, self.scale, 0, Tp,
-                                     topk=topk)
+                                     topk=topk_p)
             if fb.num_decode:
                 o_lat = ops.mla_attn(q_lat, q_pe, cache, fb.d_block_tables, None, fb.positions, self.scale, Tp,
-                                     fb.num_decode, topk=topk, out=o_lat)
-            return ops.mla_unabsorb(o_lat, lw.w_uv_s, T), topk
+                                     fb.num_decode, topk=topk_d, out=o_lat)
+            return ops.mla_unabsorb(o_lat, lw.w_uv_s, T), lists
         L, R, V = self.L, self.R, self.V
         heads = torch.empty((T, H, V), dtype=q.dtype, device=q.device)
         done = 0
-        if self._expands(lw, fb) and topk is None:
+        if self._expands(lw, fb) and topk_p is None:
             # no prompt has a cached prefix: keys and values expanded once per token, 320 instead of 1088 columns per pair
             rows = ops.gather_rows(cache.view(-1, L + R), fb.slot_mapping[:Tp])
             ops.mla_prefill(q[:Tp], rows, lw.w_kvb, self.cos_sin, fb.positions[:Tp], fb.p_cu_q, H, self.nope, V, L, self.scale,
@@ -318,12 +328,12 @@ class DeepseekStage(DecoderStage):
             o_lat = torch.empty((n, H, L), dtype=q.dtype, device=q.device)
             if Tp > done:
                 ops.latent_attn(q_cat[:Tp], cache, fb.p_block_tables, fb.p_cu_q, fb.p_ctx_lens, self.scale, L, max_q=fb.p_max_q,
-                                max_ctx=fb.p_max_ctx, out=o_lat[:Tp], topk=None if topk is None else topk[:Tp])
+                                max_ctx=fb.p_max_ctx, out=o_lat[:Tp], topk=None if topk_p is None else topk_p[:Tp])
             if fb.num_decode:
                 ops.latent_attn(q_cat[Tp - done:], cache, fb.d_block_tables, None, fb.d_ctx_lens, self.scale, L,
-                                max_ctx=fb.d_max_ctx, out=o_lat[Tp - done:], topk=None if topk is None else topk[Tp:])
+                                max_ctx=fb.d_max_ctx, out=o_lat[Tp - done:], topk=None if topk_d is None else topk_d[Tp:])
             ops.head_linear(o_lat.view(n, H * L), L, lw.w_uv_s, H, heads[done:])
-        return heads.view(T, H * V), topk
+        return heads.view(T, H * V), lists
 
     # Expanded keys and values: a pair of (query, key) costs 320 columns instead of 1088, but every token's keys and values
     # are written and read once, and the kernel's query tiles are a prompt's own. Of a layer with 128 heads (us, absorbed and
@@ -347,10 +357,10 @@ class DeepseekStage(DecoderStage):
 
     def forward_layers(self, h: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         eps = self.cfg.rms_norm_eps
-        topk = None
+        lists = None
         for li, lw in enumerate(self.layers):
             xn = ops.rmsnorm(h, lw.ln1, eps)
-            a, topk = self._attention(lw, li, xn, fb, topk)
+            a, lists = self._attention(lw, li, xn, fb, lists)
             h = self._lin(a.contiguous(), lw.w_o, residual=h)
             xn = ops.rmsnorm(h, lw.ln2, eps)
             h = self._mlp(lw, xn, h)

@@ -187,7 +187,7 @@ class TPDeepseekStage(FamilyTPMixin, DeepseekStage):
         pass                                        # attention was cut when it was installed
 
     def _tp_attention(self, lw, li, xn, fb, state):
-        a, state["topk"] = self._attention(lw, li, xn, fb, state.get("topk"))
+        a, state["lists"] = self._attention(lw, li, xn, fb, state.get("lists"))
         return a
 
     def _tp_out_weight(self, lw):

@@ -109,3 +109,38 @@ def test_topk_select_and_index_scores_reference():
     top = ref.topk_select(sc, pos, 8)
     assert (top[1] == -1).all()
     assert set(top[0].tolist()) == set(torch.topk(sc[0, :41], 8).indices.tolist())
+
+
+def test_key_lists_only_where_contexts_outgrow_them(monkeypatch):
+    """A long decoding row gives a short prompt beside it no lists (they would keep it from the dense and expanded forms), and a
+    long prompt none to a short decoding row; tokens as in the restatement either way."""
+    from parallax_b200 import ops
+
+    cfg = named_config("tiny-dsa")
+    calls, plain = [], ops.latent_attn
+
+    def recorded(q, cache, tables, cu_q, *a, **kw):
+        calls.append(("decode" if cu_q is None else "prompt", kw.get("topk") is not None, kw["max_ctx"] > cfg.index_topk))
+        return plain(q, cache, tables, cu_q, *a, **kw)
+
+    monkeypatch.setattr(ops, "latent_attn", recorded)
+    g = torch.Generator().manual_seed(4)
+    for first, second in ((41, 9), (5, 40)):
+        eng = Engine(cfg, device="cpu", num_blocks=64, page_size=16, max_batch_size=4, max_num_tokens_per_batch=256, max_total_length=256)
+        prompts = [torch.randint(0, cfg.vocab_size, (n,), generator=g).tolist() for n in (first, second)]
+        reqs = [Request(input_ids=p, sampling_params=SamplingParams(max_new_tokens=4, temperature=0.0, ignore_eos=True),
+                        max_total_length=256) for p in prompts]
+        eng.add_request(reqs[0])
+        eng.step()
+        eng.add_request(reqs[1])
+        mixed = len(calls)
+        eng.step()
+        assert {c[0] for c in calls[mixed:]} == {"decode", "prompt"}
+        while eng.has_work():
+            eng.step()
+        for p, r in zip(prompts, reqs):
+            seq = list(p)
+            for tok in r.output_ids:
+                assert int(oracle_last_logits(eng.stages[0].model, seq).argmax()) == tok
+                seq.append(tok)
+    assert all(lists == longer for _kind, lists, longer in calls)
