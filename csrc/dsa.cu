@@ -40,14 +40,14 @@ struct ScoreSmem {
   bf16 q[2][kHiMax * kPitch];
 };
 
-// grid (key tiles, groups of `group` tokens)
+// grid (key tiles, groups of `group` tokens); columns [0, width) of a row of scores are written
 __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* __restrict__ q, const float* __restrict__ w,
                                                                    const bf16* __restrict__ cache,
                                                                    const int* __restrict__ block_tables,
                                                                    const int* __restrict__ cu_q,
                                                                    const int* __restrict__ positions,
-                                                                   float* __restrict__ scores, int64_t ld_scores, int T, int B,
-                                                                   int Hi, int max_blocks, int page, int group) {
+                                                                   float* __restrict__ scores, int64_t ld_scores, int width, int T,
+                                                                   int B, int Hi, int max_blocks, int page, int group) {
   extern __shared__ __align__(16) uint8_t raw[];
   ScoreSmem& sm = *reinterpret_cast<ScoreSmem*>(raw);
   const int j0 = blockIdx.x * kScoreKeys;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
         v += __shfl_xor_sync(0xffffffffu, v, 1);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
         const int j = j0 + warp * 32 + m * 16 + e * 8 + g;
-        if (qd == 0 && j < ld_scores) out[j] = j <= pos ? v : -INFINITY;
+        if (qd == 0 && j < width) out[j] = j <= pos ? v : -INFINITY;
       }
   }
   cp_async_wait<0>();
@@ -297,7 +297,8 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
                                     int max_blocks, int page, int max_ctx, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (Di != kDi || Hi <= 0 || Hi > kHiMax || max_ctx <= 0) return PXL_ERR_INVALID_ARG;
-  if (static_cast<int64_t>(pxl::ceil_div(max_ctx, kKeyTile)) * kKeyTile > ld_scores) return PXL_ERR_INVALID_ARG;
+  const int width = pxl::ceil_div(max_ctx, kKeyTile) * kKeyTile;  // (the last tile of 128 keys may reach past it)
+  if (width > ld_scores) return PXL_ERR_INVALID_ARG;
   static bool done[64] = {false};
   const int dev = pxl_host::current_device_slot();
   if (!done[dev]) {
@@ -313,7 +314,7 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
   while (pxl::ceil_div(T, group) > 65535) group *= 2;
   dsa_scores_kernel<<<dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream>>>(
       static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
-      ld_scores, T, B, Hi, max_blocks, page, group);
+      ld_scores, width, T, B, Hi, max_blocks, page, group);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 

@@ -31,3 +31,22 @@ def test_scores_of_ragged_prompts(Hi, page):
     assert torch.equal(torch.isfinite(got), seen)
     # bf16 products are exact in fp32; sums of 128 and of Hi terms in another order
     assert float((got[seen] - want[seen]).norm() / want[seen].norm()) < 1e-5
+
+
+@pytest.mark.parametrize("max_ctx,width", [(40, 64), (65, 128), (129, 192), (320, 320)])
+def test_columns_beyond_the_keys_stay(max_ctx, width):
+    """Rows of scores inside a wider buffer: columns up to the next multiple of 64 are written, those behind are someone else's."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(max_ctx)
+    T, Hi, page = 3, 8, 16
+    q, w = torch.randn(T, Hi, 128).bfloat16().cuda(), torch.randn(T, Hi).cuda()
+    cache, table = torch.randn(20, 1, page, 128).bfloat16().cuda(), torch.arange(20).int().view(1, 20).cuda()
+    pos, cu_q = torch.arange(max_ctx - T, max_ctx).int().cuda(), torch.tensor([0, T]).int().cuda()
+    wide = torch.full((T, 512), 7.0, device="cuda")
+    code = cu._lib.lib().pxl_dsa_index_scores(q.data_ptr(), w.data_ptr(), cache.data_ptr(), table.data_ptr(), cu_q.data_ptr(),
+                                              pos.data_ptr(), wide.data_ptr(), 512, T, 1, Hi, 128, 20, page, max_ctx,
+                                              torch.cuda.current_stream().cuda_stream)
+    assert code == 0
+    assert torch.equal(wide[:, :width], cu.dsa_index_scores(q, w, cache, table, cu_q, pos, max_ctx))
+    assert bool((wide[:, width:] == 7.0).all())
