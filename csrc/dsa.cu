@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
       seq = cu_q ? find_seq(cu_q, B, t) : t;
       seq_end = cu_q ? cu_q[seq + 1] : t + 1;
       if (seq_end > T) seq_end = T;
-      const int limit = positions[(seq_end < last ? seq_end : last) - 1];  // the group's last token of the sequence sees the most
+      int limit = pos;  // what the group's tokens of the sequence see, in whatever order they are
+      for (int i = t + 1; i < seq_end && i < last; ++i) limit = max(limit, positions[i]);
       const int* bt = block_tables + static_cast<size_t>(seq) * max_blocks;
       for (int c = tid; c < kScoreKeys * (kDi / 8); c += kScoreThreads) {
         const int r = c / (kDi / 8), ch = c % (kDi / 8);

@@ -50,3 +50,21 @@ def test_columns_beyond_the_keys_stay(max_ctx, width):
     assert code == 0
     assert torch.equal(wide[:, :width], cu.dsa_index_scores(q, w, cache, table, cu_q, pos, max_ctx))
     assert bool((wide[:, width:] == 7.0).all())
+
+
+def test_tokens_in_any_order():
+    """Positions of a sequence that do not rise from token to token."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(9)
+    lens, ctx, page, Hi = [70, 200], [300, 513], 16, 16
+    table = torch.randperm(2 * 33).int().view(2, 33)
+    cache = torch.randn(66, 1, page, 128).bfloat16()
+    pos = torch.cat([c - 1 - torch.randperm(n) for n, c in zip(lens, ctx)]).int()
+    q, w = torch.randn(sum(lens), Hi, 128).bfloat16(), torch.randn(sum(lens), Hi)
+    cu_q = torch.tensor([0, 70, 270]).int()
+    got = cu.dsa_index_scores(*[t.cuda() for t in (q, w, cache, table, cu_q, pos)], max(ctx)).cpu()
+    want = ref.dsa_index_scores(q, w, cache, table, cu_q, pos, max(ctx))
+    seen = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), seen)
+    assert float((got[seen] - want[seen]).norm() / want[seen].norm()) < 1e-5      # fp32 sums in another order
