@@ -357,7 +357,13 @@ __global__ void __launch_bounds__(256) quant_fp8_rows_kernel(const bf16* __restr
     packed[j >> 2] |= static_cast<uint32_t>(b) << (8 * (j & 3));
   }
   if (!in) return;
-  *reinterpret_cast<uint2*>(q + i * 128 + l * 8) = make_uint2(packed[0], packed[1]);
+  uint8_t* dst = q + i * 128 + l * 8;
+  if ((reinterpret_cast<uintptr_t>(q) & 7) == 0) {
+    *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
+  } else {  // (q starts on 4 bytes)
+    reinterpret_cast<uint32_t*>(dst)[0] = packed[0];
+    reinterpret_cast<uint32_t*>(dst)[1] = packed[1];
+  }
   if (l == 0) s[i] = scale;
 }
 

@@ -46,3 +46,18 @@ def test_fp8_product_split_over_a_cluster(M, N, K, epi):
     cu.check_status(torch.device("cuda", 0))
     assert float((got[0].float() - want.float()).norm() / want.float().norm()) < 2 ** -7
     assert torch.equal(*got)        # added in K order
+
+
+def test_row_quantisation_into_words():
+    """A result that starts on 4 bytes, not on 8."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(2)
+    T, K = 5, 256
+    x = torch.randn(T, K).bfloat16().cuda()
+    want, scales = cu.quant_fp8_rows(x)
+    buf, s = torch.zeros(T * K + 8, dtype=torch.uint8, device="cuda"), torch.empty_like(scales)
+    assert cu._lib.lib().pxl_quant_fp8_rows(x.data_ptr(), K, buf.data_ptr() + 4, s.data_ptr(), T, K,
+                                            torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(buf[4:-4], want.view(torch.uint8).flatten()) and torch.equal(s, scales)
+    assert int(buf[:4].sum()) == 0 and int(buf[-4:].sum()) == 0
