@@ -15,6 +15,7 @@
 //
 // Covers the dense projections reached through the reference's GPU backend
 // (src/parallax/sglang/model_runner.py:358-366; the reference itself ships no GPU GEMM).
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 
@@ -1335,57 +1336,52 @@ struct MidPlan {
   int bn, splitk;
   double cost;
 };
+constexpr int kPlanBns[3] = {256, 128, 192};
+constexpr double kPlanKb[3] = {0.43, 0.29, 0.36};  // t_kb
+
+double plain_cost(int M, int N, int K, int i) {  // tiles of kPlanBns[i] columns
+  const int tiles = pxl::ceil_div(M, BM) * pxl::ceil_div(N, kPlanBns[i]);
+  return pxl::ceil_div(tiles, pxl_host::num_sms()) * (pxl::ceil_div(K, BK) * kPlanKb[i]) + 7.0;
+}
 
 MidPlan mid_m_plan(int M, int N, int K) {
   const int num_kb = pxl::ceil_div(K, BK);
   const int num_m = pxl::ceil_div(M, BM);
-  const int sms = pxl_host::num_sms();
   MidPlan best{0, 1, 1e300};
-  const int bns[3] = {256, 128, 192};
-  const double t_kb[3] = {0.43, 0.29, 0.36};
   for (int i = 0; i < 3; ++i) {
-    const int tiles = num_m * pxl::ceil_div(N, bns[i]);
-    const double plain = pxl::ceil_div(tiles, sms) * (num_kb * t_kb[i]) + 7.0;
-    if (plain < best.cost) best = MidPlan{bns[i], 1, plain};
-    if (bns[i] == 192) continue;  // the cluster variant exists for 128- and 256-wide tiles
+    const int bn = kPlanBns[i], tiles = num_m * pxl::ceil_div(N, bn);
+    const double plain = plain_cost(M, N, K, i);
+    if (plain < best.cost) best = MidPlan{bn, 1, plain};
+    if (bn == 192) continue;  // the cluster variant exists for 128- and 256-wide tiles
     for (int sk = 2; sk <= 4; sk += 2) {
       if (num_kb / sk < 4) break;
       const int kb_per = pxl::ceil_div(num_kb, sk);
       if (pxl::ceil_div(num_kb, kb_per) != sk) continue;  // no empty K range
-      if (tiles > mid_m_max_clusters(bns[i], sk)) continue;
-      const double cost = kb_per * t_kb[i] + 8.0 + sk * (bns[i] / 128);
-      if (cost < best.cost) best = MidPlan{bns[i], sk, cost};
+      if (tiles > mid_m_max_clusters(bn, sk)) continue;
+      const double cost = kb_per * kPlanKb[i] + 8.0 + sk * (bn / 128);
+      if (cost < best.cost) best = MidPlan{bn, sk, cost};
     }
   }
   return best;
 }
 
+bool mid_m_disabled() {
+  static const bool off = getenv("PXL_NO_MID_M_GEMM") != nullptr;
+  return off;
+}
+
 // Rows that go ahead of the last wave of 128-row tiles: M itself, or as many as fill the SMs a whole number of times when the
 // rows behind them cost less on their own (split along K over all SMs, or streamed once for a few rows) than the nearly empty
 // wave that they would add. 5903 rows x 4096 columns are 752 tiles of 128 x 256, 5.08 waves of 148: 5888 rows take five.
-int rows_ahead_of_the_tail(int M, int N, int K) {
-  const int sms = pxl_host::num_sms(), num_kb = pxl::ceil_div(K, BK);
-  auto plain = [&](int rows) {
-    const int bns[2] = {256, 192};
-    const double t_kb[2] = {0.43, 0.36};
-    double best = 1e300;
-    for (int i = 0; i < 2; ++i) {
-      const double c = pxl::ceil_div(pxl::ceil_div(rows, BM) * pxl::ceil_div(N, bns[i]), sms) * (num_kb * t_kb[i]) + 7.0;
-      best = c < best ? c : best;
-    }
-    return best;
-  };
-  const int num_n = pxl::ceil_div(N, 256);
+int rows_ahead_of_the_tail(int M, int N, int K, int epi) {
+  if (M <= kMidMaxM || (epi != PXL_EPI_NONE && epi != PXL_EPI_RESIDUAL && epi != PXL_EPI_F32) || mid_m_disabled()) return M;
+  const int sms = pxl_host::num_sms(), num_n = pxl::ceil_div(N, 256);
+  auto plain = [&](int rows) { return std::min(plain_cost(rows, N, K, 0), plain_cost(rows, N, K, 2)); };
   const int ahead = pxl::ceil_div(M, BM) * num_n / sms * sms / num_n * BM;
   const int tail = M - ahead;
   if (ahead <= 0 || tail <= 0 || tail > kMidMaxM) return M;
   const double alone = tail <= kSmallMaxM ? 2.0 * N * K / 5.0e6 + 8.0 : mid_m_plan(tail, N, K).cost;
   return plain(ahead) + alone < 0.97 * plain(M) ? ahead : M;
-}
-
-bool mid_m_disabled() {
-  static const bool off = getenv("PXL_NO_MID_M_GEMM") != nullptr;
-  return off;
 }
 
 int gemm_mid_m(const void* A, const void* W, void* C, bool f32_out, const void* residual, const void* bias, int M,
@@ -1441,6 +1437,10 @@ PXL_EXPORT int pxl_gemm_bf16_small_m(const void* A, const void* W, void* C, cons
   return gemm_small_m(A, W, C, false, residual, bias, M, N, K, lda, ldw, ldc, splitk, mode, status, stream);
 }
 
+PXL_EXPORT int pxl_gemm_bf16_launches(int M, int N, int K, int epi) {
+  return M > 0 && N > 0 && K > 0 && rows_ahead_of_the_tail(M, N, K, epi) < M ? 2 : 1;
+}
+
 PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* residual,
                              const void* bias, int M, int N, int K, int lda, int ldw, int ldc,
                              int epi, int bn, int* status, cudaStream_t stream) {
@@ -1461,8 +1461,8 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
       return gemm_mid_m(A, W, C, epi == PXL_EPI_F32, epi == PXL_EPI_RESIDUAL ? residual : nullptr, bias, M, N, K, lda,
                         ldw, ldc, plan >> 4, plan & 15, status, stream);
   }
-  if (bn == 0 && M > kMidMaxM && (epi == PXL_EPI_NONE || epi == PXL_EPI_RESIDUAL || epi == PXL_EPI_F32) && !mid_m_disabled()) {
-    const int ahead = rows_ahead_of_the_tail(M, N, K);
+  if (bn == 0) {
+    const int ahead = rows_ahead_of_the_tail(M, N, K, epi);
     if (ahead < M) {
       const int rc = pxl_gemm_bf16(A, W, C, residual, bias, ahead, N, K, lda, ldw, ldc, epi, pxl_gemm_bf16_pick_bn(ahead, N, epi), status,
                                    stream);

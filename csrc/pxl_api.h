@@ -39,6 +39,11 @@ typedef struct CUstream_st* pxl_stream_t;
 // C[M,N] = A[M,K] * W[N,K]^T. lda/ldw/ldc in elements. `bn` = tile width (64/128/256)
 // or 0 to pick automatically. For PXL_EPI_SILU_MUL the rows of W must be arranged in
 // groups of 128: 64 gate rows followed by the 64 up rows of the same outputs (bn >= 128).
+int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* residual, const void* bias,
+                  int M, int N, int K, int lda, int ldw, int ldc, int epi, int bn, int* status,
+                  pxl_stream_t stream);
+// kernels that pxl_gemm_bf16 launches with bn = 0: two where the rows of a nearly empty last wave go on their own
+int pxl_gemm_bf16_launches(int M, int N, int K, int epi);
 // M <= PXL_GEMV_MAX_M rows without tensor cores (gemv.cu); pxl_gemm_bf16 takes it by itself.
 #define PXL_GEMV_MAX_M 4
 int pxl_gemv_bf16_takes(int M, int N, int K, int epi);
@@ -48,9 +53,6 @@ int pxl_gemv_bf16(const void* A, const void* W, void* C, const void* residual, c
 #define PXL_GEMV_NORM_MAX_M 2
 int pxl_gemv_bf16_norm(const void* A, const void* norm_w, float eps, float offset, const void* W, void* C, const void* bias, int M,
                        int N, int K, int lda, int ldw, int ldc, int epi, pxl_stream_t stream);
-int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* residual, const void* bias,
-                  int M, int N, int K, int lda, int ldw, int ldc, int epi, int bn, int* status,
-                  pxl_stream_t stream);
 int pxl_gemm_bf16_pick_bn(int M, int N, int epi);
 // Small-M (decode) GEMM, M <= 128: the weight matrix takes the 128-row operand slot of the tensor
 // core, the few activation rows the narrow one, and K is split over `splitk` CTAs per 128 output

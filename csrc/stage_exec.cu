@@ -136,7 +136,7 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
     PXL_TRY(pxl_qk_norm_rope_cache(qkv, L.q_norm, L.k_norm, st->cos_sin, sp->positions, sp->slots, L.k_cache,
                                    L.v_cache, T, Hq, Hkv, D, st->rot_dim, st->page, num_slots, st->eps,
                                    st->norm_offset, st->max_pos, status, stream));
-    n += 3;
+    n += 2 + pxl_gemm_bf16_launches(T, qkv_n, H, PXL_EPI_NONE);
     if (sp->Tp > 0) {
       if (prefill_tc) {
         PXL_TRY(pxl_attn_prefill_tc(qkv, qkv_n, L.k_cache, L.v_cache, sp->p_bt, sp->p_cu_q, sp->p_ctx, attn,
@@ -170,7 +170,8 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
     void* h_next = (h_mid == ws->h_a) ? ws->h_b : ws->h_a;
     PXL_TRY(pxl_gemm_bf16(ws->act, L.w_down, h_next, h_mid, nullptr, T, H, I, I, I, H, PXL_EPI_RESIDUAL, 0, status,
                           stream));
-    n += 4;
+    n += 1 + pxl_gemm_bf16_launches(T, H, Hq * D, PXL_EPI_RESIDUAL) + pxl_gemm_bf16_launches(T, 2 * I, H, PXL_EPI_SILU_MUL) +
+         pxl_gemm_bf16_launches(T, H, I, PXL_EPI_RESIDUAL);
     h = h_next;
   }
   *h_out = const_cast<void*>(h);
