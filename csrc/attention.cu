@@ -1429,8 +1429,9 @@ PXL_EXPORT int pxl_attn_decode(const void* q, int64_t q_stride, const void* k_ca
 }
 
 // Decode attention over e4m3 caches written by pxl_qk_norm_rope_cache_fp8 / pxl_reshape_and_cache_fp8
-// with the same scales. The cache bytes are widened to bf16 on their way into shared memory, the K
-// scale is folded into the score scale and the V scale into the output normalisation.
+// with the same scales, which are folded into the score scale (K) and the output normalisation (V). Head dim 128 and pages of 16, 32 or
+// 64: bytes up to the fragments, f16 products (attn_decode_e4m3_kernel); other sizes widen the bytes to bf16 on their way into
+// shared memory.
 PXL_EXPORT int pxl_attn_decode_fp8(const void* q, int64_t q_stride, const void* k_cache,
                                    const void* v_cache, const int* block_tables,
                                    const int* ctx_lens, void* out, float* workspace,

@@ -105,6 +105,13 @@ __device__ __forceinline__ void st_bf16x8(bf16* p, const bf16x8& v) {
   *reinterpret_cast<bf16x8*>(p) = v;
 }
 
+// a * b + c for two fp32 numbers in a register pair
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // ---------------------------------------------------------------------------
 // shared-memory address / mbarrier / TMA / tcgen05 PTX wrappers
 // ---------------------------------------------------------------------------

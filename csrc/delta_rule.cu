@@ -299,11 +299,6 @@ __device__ __forceinline__ float2 unpair(uint64_t v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
   return f;
 }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
 // What the first kernel hands to the second, per (chunk, head), in 32-bit words
 template <int DK>

@@ -27,11 +27,6 @@ __device__ __forceinline__ uint64_t widen(uint32_t two) {  // two bf16 -> two fp
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(two << 16), "r"(two & 0xffff0000u));
   return v;
 }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
 // MM rows of A (the last ones repeated where M is smaller), R rows of W per warp, U steps of 256 columns in flight.
 // EPI: PXL_EPI_NONE, _RESIDUAL, _F32 or _SILU_MUL (R rows = R / 2 gate / up pairs, 64 rows apart in groups of 128)

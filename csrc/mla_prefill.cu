@@ -3,13 +3,15 @@
 // A prompt that starts at its first token finds no keys but its own. For those the up-projection can be done once per token -
 // [k | v] of every head = latent x W_kvb^T, one plain product - and attention runs on 192 key and 128 value columns per head: 320
 // multiply-adds per (query, key) pair where the absorbed form, which scores and sums 576 and 512 latent columns, takes 1088.
-// (Slices behind a cached prefix, key lists and decoding stay absorbed: there the expansion is paid per cached token and step.)
+// (Decoding and key lists stay absorbed: there the expansion would be paid per cached token for a row or two. Slices behind a cached
+// prefix stay absorbed, too, though only because nothing expands the prefix: 1024 rows would pay for it.)
 //
 // One CTA = two blocks of 128 queries of one head, which share the tiles of 128 keys and take turns on the tensor pipe as the two
 // heads of attn_prefill_pair_kernel do: P_u V, then S_u of the next tile, u = 0, 1, while the other block's softmax runs; P
 // replaces S in tensor memory. The first block ends a tile earlier than the second. Shared memory holds both query tiles, two
 // key tiles and one value tile (224 KB); rotated key columns are the same for all heads and are read from the latent rows.
-// Bound: 4 x 128 x 128 x 320 multiply-adds against 2 x 128 x 128 exponentials per tile pair, 2560 and 2048 clocks.
+// Bound: 2 x 128 x 128 x 320 multiply-adds (4096 a clock) against 2 x 128 x 128 exponentials (16 a clock) per tile of keys, 2560 and
+// 2048 clocks.
 // 2 prompts of 2048 tokens, 128 heads: 371 us (0.93 PFLOP/s) beside 25 us for the rotation and the rows and 75 us for the
 // expansion; the absorbed form's kernel takes 2770 us.
 #include "attention_rows.cuh"
