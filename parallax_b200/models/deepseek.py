@@ -338,8 +338,9 @@ class DeepseekStage(DecoderStage):
     # Expanded keys and values: a pair of (query, key) costs 320 columns instead of 1088, but every token's keys and values
     # are written and read once, and the kernel's query tiles are a prompt's own. Of a layer with 128 heads (us, absorbed and
     # expanded): 2 x 2048 tokens 6940 and 4340, 1 x 1024 1702 and 1095, 4 x 64 486 and 461, 16 x 32 577 and 577, 16 x 16 448
-    # and 475. Below 256 rows either form is mostly weights (1 x 128: 365 and 330), and a prompt keeps the form of the
-    # decoding rows.
+    # and 475: hence the 64 tokens per prompt. The 256 rows are no matter of speed, one prompt of 128 tokens takes 365 and 330. The
+    # two forms round at different places (equally far from 64 bits), so a routed choice near a tie falls differently between
+    # them; batches of few prompt rows, which gain a tenth, keep the rounding that their decoding rows have.
     _EXPAND_MIN_ROWS = 256
     _EXPAND_MIN_PROMPT = 64
 
