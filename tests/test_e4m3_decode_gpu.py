@@ -66,3 +66,24 @@ def test_bytes_of_tokens_that_are_not_seen(page, window, splits, byte):
     cu.check_status(torch.device("cuda", 0))
     assert bool(torch.isfinite(out[0].float()).all())
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("splits", [1, 3, 9])
+def test_small_probabilities_keep_their_bits(splits):
+    """Where the values of the keys that carry the softmax vanish, the others' make the output: here those of 2^-28.9."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(splits)
+    Hkv, D, page, ctx = 2, 128, 16, 600
+    nb = -(-ctx // page)
+    table, cl = torch.randperm(nb).int().view(1, nb), torch.tensor([ctx]).int()
+    k, v = torch.zeros(nb, Hkv, page, D), torch.randn(nb, Hkv, page, D)
+    k[..., 0::2, 0], v[..., 1::2, :] = -0.9375, 0.0         # every other key scores -28.9 in powers of two, the rest 0
+    k, v = k.to(torch.float8_e4m3fn), v.to(torch.float8_e4m3fn)
+    q = torch.zeros(1, Hkv, D).bfloat16()
+    q[..., 0] = 32.0
+    scale = 28.9 / 30 * 0.6931471805599453
+    got = cu.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), cl.cuda(), scale, max_ctx=ctx, num_splits=splits).cpu()
+    want = ref.attn_decode(q, k, v, table, cl, scale)
+    # outputs are rounded to bf16 (2^-8 at most, 2^-9 of a norm) on either side, probabilities to 2^-11
+    assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -8
