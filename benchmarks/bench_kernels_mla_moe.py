@@ -52,51 +52,40 @@ def bench_fp8(rows):
 
 def bench_mla(rows):
     hbm, tf, tag = peaks()
-    H, L, R, page = 128, 512, 64, 16
-    scale = (128 + R) ** -0.5
-    # decode: B sequences of ctx tokens; traffic = the latent cache once per sequence
-    for B, ctx in [(64, 4096), (256, 2048)]:
-        nb = (ctx + page - 1) // page
-        cache = torch.randn(B * nb, 1, page, L + R, device=DEV, dtype=torch.bfloat16) * 0.3
-        bt = torch.randperm(B * nb, device=DEV).to(torch.int32).view(B, nb)
-        pos = torch.full((B,), ctx - 1, dtype=torch.int32, device=DEV)
-        Tpad = (B + 127) // 128 * 128
-        q_lat = torch.randn(H, Tpad, L, device=DEV, dtype=torch.bfloat16) * 0.3
-        q_pe = torch.randn(B, H, R, device=DEV, dtype=torch.bfloat16) * 0.3
-        try:
-            ms = time_fn(lambda: cu.mla_attn(q_lat, q_pe, cache, bt, None, pos, scale, 0, B), iters=5)
-        except Exception as exc:      # layout of q_lat differs: record and go on
-            rows.append({"kernel": "mla_attn decode", "B": B, "ctx": ctx, "error": str(exc)[:200]})
-            print(rows[-1], flush=True)
-            continue
-        byts = 2.0 * B * ctx * (L + R)
-        flops = 2.0 * B * H * ctx * (L + R + L)
-        rows.append({"kernel": "mla_attn decode", "B": B, "ctx": ctx, "heads": H, "ms": round(ms, 4),
-                     "gbs": round(byts / ms / 1e6, 1), "tflops": round(flops / ms / 1e9, 1),
+    H, L, R, nope, V, page = 128, 512, 64, 128, 128, 16
+    scale = (nope + R) ** -0.5
+
+    def rnd(*s):
+        return torch.randn(*s, device=DEV, dtype=torch.bfloat16) * 0.3
+
+    def row(kernel, ms, flops, byts, **kw):
+        rows.append({"kernel": kernel, **kw, "heads": H, "ms": round(ms, 4), "gbs": round(byts / ms / 1e6, 1),
+                     "tflops": round(flops / ms / 1e9, 1),
                      "roofline_frac": round(max(byts / (hbm * 1e9), flops / (tf * 1e12)) * 1e3 / ms, 3), "tag": tag})
         print(rows[-1], flush=True)
+
+    # absorbed form: decode (B sequences of ctx tokens) and a slice behind a cached prefix; traffic = the latent cache once per sequence
+    for B, n, ctx in [(64, 1, 4096), (256, 1, 2048), (1, 1024, 4096)]:
+        nb = (ctx + page - 1) // page
+        cache = rnd(B * nb, 1, page, L + R)
+        bt = torch.randperm(B * nb, device=DEV).to(torch.int32).view(B, nb)
+        lens = torch.full((B,), ctx, dtype=torch.int32, device=DEV)
+        cu_q = torch.tensor([0, n], dtype=torch.int32, device=DEV) if n > 1 else None
+        q, out = rnd(B * n, H, L + R), torch.empty((B * n, H, L), device=DEV, dtype=torch.bfloat16)
+        ms = time_fn(lambda: cu.latent_attn(q, cache, bt, cu_q, lens, scale, L, max_q=n, max_ctx=ctx, out=out), iters=5)
+        pairs = B * (n * (ctx - n) + n * (n + 1) / 2)
+        row("latent_attn (absorbed form)", ms, 2.0 * pairs * H * (2 * L + R), 2.0 * B * ctx * (L + R), B=B, rows=n, ctx=ctx)
         del cache
-    # prefill: one 4096-token prompt, causal
-    for Lq in (1024, 4096):
-        nb = (Lq + page - 1) // page
-        cache = torch.randn(nb, 1, page, L + R, device=DEV, dtype=torch.bfloat16) * 0.3
-        bt = torch.arange(nb, device=DEV, dtype=torch.int32).view(1, nb)
-        pos = torch.arange(Lq, device=DEV, dtype=torch.int32)
-        cu_q = torch.tensor([0, Lq], dtype=torch.int32, device=DEV)
-        Tpad = (Lq + 127) // 128 * 128
-        q_lat = torch.randn(H, Tpad, L, device=DEV, dtype=torch.bfloat16) * 0.3
-        q_pe = torch.randn(Lq, H, R, device=DEV, dtype=torch.bfloat16) * 0.3
-        try:
-            ms = time_fn(lambda: cu.mla_attn(q_lat, q_pe, cache, bt, cu_q, pos, scale, 0, Lq), iters=3, warmup=2)
-        except Exception as exc:
-            rows.append({"kernel": "mla_attn prefill", "L": Lq, "error": str(exc)[:200]})
-            print(rows[-1], flush=True)
-            continue
-        flops = 2.0 * H * (Lq * (Lq + 1) / 2) * (L + R + L)
-        rows.append({"kernel": "mla_attn prefill (absorbed form)", "L": Lq, "heads": H, "ms": round(ms, 4),
-                     "tflops": round(flops / ms / 1e9, 1), "roofline_frac": round(flops / (tf * 1e12) * 1e3 / ms, 3),
-                     "tag": tag})
-        print(rows[-1], flush=True)
+    # fresh prompts: rotation, expansion of keys and values and attention
+    for B, n in ((1, 1024), (1, 4096), (2, 2048)):
+        T = B * n
+        q, latent_rows, w = rnd(T, H * (nope + R)), rnd(T, L + R), rnd(H * (nope + V), L) * 0.1
+        cs, pos = ref.build_cos_sin(n, R, 1e4).to(DEV), torch.arange(n, dtype=torch.int32, device=DEV).repeat(B)
+        cu_q = torch.arange(0, T + 1, n, dtype=torch.int32, device=DEV)
+        out = torch.empty((T, H * V), device=DEV, dtype=torch.bfloat16)
+        ms = time_fn(lambda: cu.mla_prefill(q, latent_rows, w, cs, pos, cu_q, H, nope, V, L, scale, n, out=out), iters=3, warmup=2)
+        flops = 2.0 * B * n * (n + 1) / 2 * H * (nope + R + V) + 2.0 * T * L * H * (nope + V)
+        row("mla_prefill (expanded form)", ms, flops, 2.0 * T * (H * (nope + R + V) + L + R), B=B, rows=n)
     cu.check_status(torch.device(DEV))
 
 

@@ -192,14 +192,25 @@ def kernel_rows(stack: Stack, fb, label: str, keys: int, kv_tokens: int) -> list
         kv, q = cu.linear(x, lw.w_kv_a), cu.linear(x, lw.w_q_b)
         add("cache rows", lambda: cu.mla_kv_prep(kv, lw.kv_a_norm, st.cos_sin, fb.positions, fb.slot_mapping, cache, 1e-6, L),
             0, 2.0 * T * 2 * (L + R))
-        add("query rotation + key up-projection of q", lambda: cu.mla_q_absorb(q, lw.w_uk_s, st.cos_sin, fb.positions, H, dim, L),
-            up_flops * dim, uk_bytes)
-        q_lat, q_pe = cu.mla_q_absorb(q, lw.w_uk_s, st.cos_sin, fb.positions, H, dim, L)
-        o_lat = torch.empty_like(q_lat)
-        bt, cq = (fb.p_block_tables, fb.p_cu_q) if Tp else (fb.d_block_tables, None)
-        add("attention", lambda: cu.mla_attn(q_lat, q_pe, cache, bt, cq, fb.positions, scale, 0, T, out=o_lat), attn_flops,
-            attn_bytes)
-        add("value up-projection", lambda: cu.mla_unabsorb(o_lat, lw.w_uv_s, T), up_flops * V, uv_bytes)
+        heads = torch.empty((T, H, V), dtype=bf, device=stack.dev)
+        if Tp == T and st._expands(lw, fb):      # fresh prompts: keys and values expanded per head
+            add("prompts' cache rows", lambda: cu.gather_rows(cache.view(-1, L + R), fb.slot_mapping), 0, 4.0 * T * (L + R))
+            latent_rows = cu.gather_rows(cache.view(-1, L + R), fb.slot_mapping)
+            gemm("key and value expansion", latent_rows[:, :L], lw.w_kvb)
+            per = 2.0 * keys * H * (dim + R + V) + 2.0 * T * L * H * (dim + V)
+            add("query rotation, expansion and attention", lambda: cu.mla_prefill(
+                q, latent_rows, lw.w_kvb, st.cos_sin, fb.positions, fb.p_cu_q, H, dim, V, L, scale, fb.p_max_q, out=heads), per,
+                2.0 * (T * H * (2 * dim + R + 2 * V) + T * (L + R)))
+        else:
+            q_cat, o_lat = (torch.empty((T, H, n), dtype=bf, device=stack.dev) for n in (L + R, L))
+            add("query rotation", lambda: cu.latent_queries(q, H, st.qd, dim, st.cos_sin, fb.positions, q_cat, L, R, R), 0,
+                4.0 * T * H * R)
+            add("key up-projection of q", lambda: cu.head_linear(q, st.qd, lw.w_uk_s, H, q_cat[:, :, :L]), up_flops * dim, uk_bytes)
+            bt, cq, ctx, mq, mc = (fb.p_block_tables, fb.p_cu_q, fb.p_ctx_lens, fb.p_max_q, fb.p_max_ctx) if Tp else \
+                (fb.d_block_tables, None, fb.d_ctx_lens, 1, fb.d_max_ctx)
+            add("attention", lambda: cu.latent_attn(q_cat, cache, bt, cq, ctx, scale, L, max_q=mq, max_ctx=mc, out=o_lat), attn_flops,
+                attn_bytes)
+            add("value up-projection", lambda: cu.head_linear(o_lat.view(T, -1), L, lw.w_uv_s, H, heads), up_flops * V, uv_bytes)
         gemm("output projection (+ residual)", rnd(T, H * V), lw.w_o, residual=x)
         add("norm", lambda: cu.rmsnorm(x, lw.ln1, 1e-6), 0, T * W * 4.0)
         gemm("gate / up (+ SwiGLU)", x, lw.w_gu, epi=cu.EPI_SILU_MUL)

@@ -168,14 +168,16 @@ def twin_linear_rows(r: Rows) -> None:
     proj = cu.linear(x, lw.w_in)
 
     def conv():
-        return cu.causal_conv1d_silu(proj[:, :n], lw.conv_w, lw.conv_b, lc.conv_state, fb.seq_cu, fb.seq_slots, fb.positions)
+        return cu.causal_conv1d_silu(proj[:, :n], lw.conv_w, lw.conv_b, lc.conv_state, fb.seq_cu, fb.seq_slots, fb.positions,
+                                       fb.num_prefill_seqs, fb.num_prefill_tokens)
 
     r.add("convolution", conv, 0, 4.0 * T * n + (4.0 * 3 * T * n if fb.num_decode else 0))
     c, nz = conv(), Hv * Dv
     z, b, a = proj[:, n:n + nz], proj[:, n + nz:n + nz + Hv], proj[:, n + nz + Hv:n + nz + 2 * Hv]
     carried = 4.0 * (2 if fb.num_decode else 1) * seqs * Hv * Dk * Dv
     r.add("linear attention", lambda: cu.gated_delta_rule(c, a, b, lw.A_log, lw.dt_bias, z, lw.norm_w, lc.rec_state, fb.seq_cu,
-                                                          fb.seq_slots, fb.positions, Hk, Hv, Dk, Dv, 1e-6),
+                                                          fb.seq_slots, fb.positions, Hk, Hv, Dk, Dv, 1e-6,
+                                                          fb.num_prefill_seqs, fb.num_prefill_tokens),
           6.0 * T * Hv * Dk * Dv, 2.0 * T * (n + 2 * nz) + carried)
     heads, act = r.rnd(T, nz), r.rnd(T, lw.w_down.shape[1])
     r.gemm("output projection (+ residual)", heads, lw.w_out, lambda: cu.linear(heads, lw.w_out, residual=x))
