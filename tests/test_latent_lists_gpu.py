@@ -126,3 +126,28 @@ def test_rows_that_are_not_seen(H, page, prompts, k, window, bad):
     cu.check_status(torch.device("cuda", 0))
     assert bool(torch.isfinite(out[0].float()).all())
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("q_scale,bound", [(0.05, 2.3e-3), (1.0, 2.3e-3), (3.0, 1.95e-3)])
+@pytest.mark.parametrize("lists", [False, True])
+def test_error_against_64_bits(q_scale, bound, lists):
+    """From flat to sharp distributions. Outputs are rounded to bf16 (1.66e-3 in the norm for random ones), and so are probabilities:
+    another 1.4e-3 of the result as long as several keys count (2.2e-3 together), half of it or less once one key carries a row,
+    whose rounding is above and below the line (1.8e-3)."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(3)
+    B, H, L, R, page, ctx = 2, 128, 512, 64, 64, 2000
+    nb, scale = -(-ctx // page), 192 ** -0.5
+    cache, table = torch.randn(B * nb, 1, page, L + R).bfloat16().cuda(), torch.randperm(B * nb).int().view(B, nb).cuda()
+    q, ctx_lens = (torch.randn(B, H, L + R) * q_scale).bfloat16().cuda(), torch.full((B,), ctx).int().cuda()
+    topk = torch.stack([torch.randperm(ctx)[:1024] for _ in range(B)]).int().cuda() if lists else None
+    got = cu.latent_attn(q, cache, table, None, ctx_lens, scale, L, max_ctx=ctx, topk=topk).double()
+    cu.check_status(torch.device("cuda", 0))
+    kv = cache.view(B * nb, page, L + R)[table.long()].view(B, nb * page, L + R)[:, :ctx].double()
+    if lists:
+        kv = torch.stack([k[t.long()] for k, t in zip(kv, topk)])
+    p = torch.softmax(torch.einsum("bhd,bkd->bhk", q.double(), kv) * scale, -1)
+    want = torch.einsum("bhk,bkd->bhd", p, kv[..., :L])
+    err = float((got - want).norm() / want.norm())
+    assert err < bound, err
