@@ -16,9 +16,10 @@ namespace {
 using namespace pxl;
 
 // ----------------------------------------------------------------------------- RMSNorm
+// Rows of any length: read twice (the second time from L1 / L2).
 template <bool HAS_RES>
 __global__ void __launch_bounds__(256)
-rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out,
+rmsnorm_long_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out,
                bf16* __restrict__ residual, int H, float eps, float w_offset) {
   __shared__ float red[32];
   pdl_wait();
@@ -64,8 +65,85 @@ rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
   }
 }
 
+// One block per row, the row and the weights held in registers: one read and one write of every element, one block-wide
+// sum. NV = 16-byte vectors per thread. Bound by latency up to a few hundred rows (load, reduction, store), by memory beyond:
+// the weights are on their way before the row's sum is known, and a row is spread over as many threads as a block of NV vectors
+// per thread takes, so that all SMs have rows already at a batch of about a hundred. (One warp per row, eight rows per block,
+// left 8 of 148 SMs at work for 64 rows: 64 x 7168 took 10.8 us and takes 2.3, 128 x 4096 6.5 and 2.1, 4096 x 7168 40.2 and 22.4,
+// 5.2 TB/s.)
+template <bool HAS_RES, int NV>
+__global__ void __launch_bounds__(1024)
+rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out, bf16* __restrict__ residual,
+               int H, float eps, float w_offset) {
+  __shared__ float red[32];
+  const size_t row = blockIdx.x;
+  const bf16* xr = x + row * H;
+  bf16* rr = HAS_RES ? residual + row * H : nullptr;
+  bf16* outr = out + row * H;
+  const int nvec = H >> 3;
+  bf16x8 a[NV], g[NV];
+  pdl_wait();
+  pdl_launch_dependents();
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < nvec) a[i] = ld_bf16x8(xr + v * 8);
+  }
+  if constexpr (HAS_RES) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
+      if (v < nvec) {
+        const bf16x8 b = ld_bf16x8(rr + v * 8);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 fa = unpack_bf16x2(a[i].u[j]);
+          const float2 fb = unpack_bf16x2(b.u[j]);
+          a[i].u[j] = pack_bf16x2(fa.x + fb.x, fa.y + fb.y);
+        }
+        st_bf16x8(rr + v * 8, a[i]);  // the sum (rounded to bf16) is the new residual stream
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < nvec) g[i] = ld_bf16x8(w + v * 8);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    if (threadIdx.x + i * blockDim.x < nvec) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(a[i].u[j]);
+        ss += f.x * f.x + f.y * f.y;
+      }
+    }
+  }
+  ss = warp_reduce_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = warp_reduce_sum((threadIdx.x & 31) < (blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.f);
+  const float inv = rsqrtf(ss / static_cast<float>(H) + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < nvec) {
+      bf16x8 o;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(a[i].u[j]);
+        const float2 gg = unpack_bf16x2(g[i].u[j]);
+        o.u[j] = pack_bf16x2(f.x * inv * (gg.x + w_offset), f.y * inv * (gg.y + w_offset));
+      }
+      st_bf16x8(outr + v * 8, o);
+    }
+  }
+}
+
 // One warp per row, the row held in registers between the sum of squares and the scaling: one read
-// and one write of every element, no block-wide barrier. NV = 16-byte vectors per lane (H <= NV * 256).
+// and one write of every element, no block-wide barrier, eight rows per block. NV = 16-byte vectors per lane (H <= NV * 256).
 template <bool HAS_RES, int NV>
 __global__ void __launch_bounds__(256)
 rmsnorm_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out,
@@ -474,26 +552,39 @@ PXL_EXPORT int pxl_rmsnorm(const void* x, const void* weight, void* out, void* r
   const bf16* wp = static_cast<const bf16*>(weight);
   bf16* op = static_cast<bf16*>(out);
   bf16* rp = static_cast<bf16*>(residual);
-  if (H <= 8192 && T >= 64) {
-    // many rows: one warp per row with the row in registers
+  if (H <= 2048 && T >= 2048) {
+    // short rows by the thousand: blocks of eight rows, a block for each would be bound by their number (8192 x 1024: 7.2 us
+    // against 9.6; 4096 x 1536: 5.9 against 6.1; 1024 rows are better off with a block each, 2.5 against 3.2)
     const unsigned grid = static_cast<unsigned>((T + 7) / 8);
-#define PXL_RMS_WARP(NV)                                                                          \
-  do {                                                                                            \
-    if (residual)                                                                                 \
-      pxl_host::launch(rmsnorm_warp_kernel<true, NV>, grid, 256, 0, stream, xp, wp, op, rp, T, H, eps, w_offset); \
-    else                                                                                          \
-      pxl_host::launch(rmsnorm_warp_kernel<false, NV>, grid, 256, 0, stream, xp, wp, op, rp, T, H, eps, w_offset); \
+    if (residual)
+      pxl_host::launch(rmsnorm_warp_kernel<true, 8>, grid, 256, 0, stream, xp, wp, op, rp, T, H, eps, w_offset);
+    else
+      pxl_host::launch(rmsnorm_warp_kernel<false, 8>, grid, 256, 0, stream, xp, wp, op, rp, T, H, eps, w_offset);
+    return check_launch();
+  }
+  const int nvec = H >> 3;
+  if (H <= 16384) {
+    // vectors per thread: two for the shortest chain while the SMs are not full, four once throughput counts (128 x 4096: 2.1 us
+    // with two, 2.3 with four; 1016 x 7168: 8.6 and 6.9; 8192 x 4096: 28.7 and 23.2)
+    int nv = T < 512 ? 2 : 4;
+    while (nvec > nv * 1024) nv *= 2;
+    const int threads = pxl::ceil_div(pxl::ceil_div(nvec, nv), 32) * 32;
+#define PXL_RMS(NV)                                                                                                      \
+  do {                                                                                                                   \
+    if (residual)                                                                                                        \
+      pxl_host::launch(rmsnorm_kernel<true, NV>, T, threads, 0, stream, xp, wp, op, rp, H, eps, w_offset);               \
+    else                                                                                                                 \
+      pxl_host::launch(rmsnorm_kernel<false, NV>, T, threads, 0, stream, xp, wp, op, rp, H, eps, w_offset);              \
   } while (0)
-    if (H <= 2048) PXL_RMS_WARP(8);
-    else if (H <= 4096) PXL_RMS_WARP(16);
-    else PXL_RMS_WARP(32);
-#undef PXL_RMS_WARP
+    if (nv == 2) PXL_RMS(2);
+    else PXL_RMS(4);
+#undef PXL_RMS
     return check_launch();
   }
   if (residual)
-    pxl_host::launch(rmsnorm_kernel<true>, T, 256, 0, stream, xp, wp, op, rp, H, eps, w_offset);
+    pxl_host::launch(rmsnorm_long_kernel<true>, T, 256, 0, stream, xp, wp, op, rp, H, eps, w_offset);
   else
-    pxl_host::launch(rmsnorm_kernel<false>, T, 256, 0, stream, xp, wp, op, static_cast<bf16*>(nullptr), H, eps, w_offset);
+    pxl_host::launch(rmsnorm_long_kernel<false>, T, 256, 0, stream, xp, wp, op, static_cast<bf16*>(nullptr), H, eps, w_offset);
   return check_launch();
 }
 

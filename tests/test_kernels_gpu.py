@@ -147,6 +147,28 @@ def test_rmsnorm_many_rows(cu, T, H):
     assert _rel_err(r1, r2) < 1e-3
 
 
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 1032), (64, 7168), (511, 8192), (512, 8200), (9, 16384), (600, 16384), (5, 16392),
+                                 (2047, 2048), (2048, 2048), (2049, 2056)])
+def test_rmsnorm_forms(cu, T, H):
+    """Edges of the forms: vectors per thread, rows in registers and longer ones, blocks of one and of eight rows."""
+    g = torch.Generator(device=_dev()).manual_seed(T * 31 + H)
+    x, r = (torch.randn(T, H, device=_dev(), dtype=torch.bfloat16, generator=g) for _ in range(2))
+    w = torch.randn(H, device=_dev(), dtype=torch.bfloat16, generator=g)
+
+    def exact(v, off):
+        v = v.double()
+        return v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + 1e-5) * (w.double() + off)
+
+    # one rounding to bf16 (eight significant bits: half a unit is at most 2^-8 of the value) and fp32 sums
+    y, want = cu.rmsnorm(x, w, 1e-5), exact(x, 0.0)
+    assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 1e-5) + 1e-9).all()
+    r1 = r.clone()
+    y = cu.rmsnorm(x, w, 1e-5, residual=r1, w_offset=1.0)
+    assert torch.equal(r1, (x.float() + r.float()).to(torch.bfloat16))
+    want = exact(r1, 1.0)
+    assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 1e-5) + 1e-9).all()
+
+
 @pytest.mark.parametrize("D,rot", [(128, 128), (64, 64), (128, 64)])
 def test_qk_norm_rope_cache(cu, D, rot):
     torch.manual_seed(3)
