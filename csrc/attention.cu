@@ -1318,7 +1318,7 @@ int launch_decode_splits(dim3 grid, int smem, int B, int Hq, const float* worksp
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pxl_host::pdl_flag() ? 2 : 1;
+  cfg.numAttrs = pxl_host::chained() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, Together, args...) == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
@@ -1384,8 +1384,8 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
         static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks,   \
         scale_log2 * k_scale, window, keep_first, num_splits, v_scale, sa, status);              \
     if (num_splits > 1)                                                                          \
-      attn_decode_reduce_kernel<DD, M><<<dim3(Hq, B), DD, 0, stream>>>(                          \
-          workspace, sinks, static_cast<bf16*>(out), Hq, num_splits);                            \
+      pxl_host::launch(attn_decode_reduce_kernel<DD, M>, dim3(Hq, B), DD, 0, stream, workspace,  \
+                       sinks, static_cast<bf16*>(out), Hq, num_splits);                          \
   }
   if (D != 64 && D != 128) return PXL_ERR_INVALID_ARG;
   if (cache_fp8) {

@@ -84,7 +84,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   pdl_wait();
-  pdl_launch_dependents();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.z, head = blockIdx.y;
@@ -128,6 +127,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tm_o = tmem_base + 2 * kT;
 
@@ -445,7 +445,6 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kSlots + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   pdl_wait();
-  pdl_launch_dependents();
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int b = blockIdx.z, head0 = blockIdx.y * 2;
@@ -490,6 +489,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_launch_dependents();
   const uint32_t tm_s = *tmem_slot, tm_o = tm_s + 2 * kT;
 
   // a softmax thread holds 128 scores: 384 threads x 168 registers at launch cover 256 x 208 + 128 x 80

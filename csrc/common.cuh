@@ -451,7 +451,9 @@ __device__ __forceinline__ bool flag_wait_bounded(const uint32_t* flag, uint32_t
 // kernel before it in the stream is still draining. pdl_wait() blocks until that kernel has
 // completed and its writes are visible (a no-op for launches without the attribute), so it must
 // run before the first access to global memory that an earlier kernel wrote or still reads.
-// pdl_launch_dependents() lets the next kernel of the stream begin its own prologue early.
+// pdl_launch_dependents() lets the next kernel of the stream begin its own prologue early. It comes after pdl_wait(), so that
+// what the kernels before the last one wrote is visible without a wait, and in kernels with tensor memory after their allocation:
+// the next kernel's blocks take theirs as soon as they run, and would keep it from a block of this one that still needs some.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -494,11 +496,20 @@ __device__ __forceinline__ void cp_async_wait() {
 // ---------------------------------------------------------------------------
 namespace pxl_host {
 
-// Launches issued by this thread while the flag is set carry the programmatic-stream-serialization
-// attribute (the stage executor sets it around a layer sequence whose kernels all call pdl_wait()).
-inline bool& pdl_flag() {
-  static thread_local bool on = false;
-  return on;
+// Launch chain of the calling thread: a sequence of layers whose launches carry the programmatic-stream-serialization attribute
+// (every kernel started through launch() waits with pdl_wait()). The first launch of a chain goes without it: it follows whatever
+// the caller had in the stream, so that weights and batch arrays are complete before any kernel of the chain starts.
+enum Chain : int { kNoChain = 0, kChainBegun = 1, kInChain = 2 };
+inline int& launch_chain() {
+  static thread_local int state = kNoChain;
+  return state;
+}
+// whether the next launch carries the attribute
+inline bool chained() {
+  int& s = launch_chain();
+  const bool in = s == kInChain;
+  if (s == kChainBegun) s = kInChain;
+  return in;
 }
 
 template <typename... KArgs, typename... Args>
@@ -513,7 +524,7 @@ inline cudaError_t launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_flag() ? 1 : 0;
+  cfg.numAttrs = chained() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 

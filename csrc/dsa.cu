@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
                                                                    const int* __restrict__ positions,
                                                                    float* __restrict__ scores, int64_t ld_scores, int width, int T,
                                                                    int B, int Hi, int max_blocks, int page, int group) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t raw[];
   ScoreSmem& sm = *reinterpret_cast<ScoreSmem*>(raw);
   const int j0 = blockIdx.x * kScoreKeys;
@@ -151,6 +153,8 @@ __device__ __forceinline__ uint32_t order_key(float x) {
 __global__ void __launch_bounds__(512) topk_select_kernel(const float* __restrict__ scores, int64_t ld,
                                                           const int* __restrict__ positions, int k,
                                                           int* __restrict__ out, int64_t ld_out) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ int hist[256];
   __shared__ uint32_t s_prefix, s_mask;
   __shared__ int s_remaining, s_gt, s_eq;
@@ -208,6 +212,8 @@ __global__ void __launch_bounds__(512) topk_select_kernel(const float* __restric
 
 __global__ void store_rows_kernel(const bf16* __restrict__ src, int64_t ld, const int64_t* __restrict__ slots,
                                   bf16* __restrict__ cache, int D, int64_t num_slots, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x;
   const int64_t slot = slots[t];
   if (slot < 0) return;
@@ -231,6 +237,8 @@ dsa_index_prep_kernel(bf16* __restrict__ q_idx, int64_t ldq, const bf16* __restr
                       const float* __restrict__ cos_sin, const int* __restrict__ positions, int max_pos,
                       const int64_t* __restrict__ slots, bf16* __restrict__ cache, int64_t num_slots,
                       float* __restrict__ w_out, float w_scale, int Hi, int R, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[32];
   __shared__ float y_s[kDi];
   const int t = blockIdx.x, d = threadIdx.x;
@@ -284,7 +292,7 @@ PXL_EXPORT int pxl_dsa_index_prep(void* q_idx, int64_t ldq, const void* kv, int6
                                   int* status, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (Di != kDi || Hi <= 0 || Hi > 128 || R <= 0 || R > Di || (R & 1)) return PXL_ERR_INVALID_ARG;
-  dsa_index_prep_kernel<<<T, 128, 0, stream>>>(static_cast<pxl::bf16*>(q_idx), ldq, static_cast<const pxl::bf16*>(kv),
+  pxl_host::launch(dsa_index_prep_kernel, T, 128, 0, stream, static_cast<pxl::bf16*>(q_idx), ldq, static_cast<const pxl::bf16*>(kv),
                                                ldkv, k_off, w_off, static_cast<const pxl::bf16*>(ln_w),
                                                static_cast<const pxl::bf16*>(ln_b), ln_eps, cos_sin, positions,
                                                max_pos, slots, static_cast<pxl::bf16*>(cache), num_slots, w_out,
@@ -313,8 +321,7 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
   int group = cu_q ? static_cast<int>(static_cast<int64_t>(T) * tiles / (3 * pxl_host::num_sms())) : 1;
   group = group < 1 ? 1 : group > 16 ? 16 : group;
   while (pxl::ceil_div(T, group) > 65535) group *= 2;
-  dsa_scores_kernel<<<dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream>>>(
-      static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
+  pxl_host::launch(dsa_scores_kernel, dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream, static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
       ld_scores, width, T, B, Hi, max_blocks, page, group);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
@@ -323,7 +330,7 @@ PXL_EXPORT int pxl_topk_select(const float* scores, int64_t ld, const int* posit
                                int64_t ld_out, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (k <= 0 || ld_out < k) return PXL_ERR_INVALID_ARG;
-  topk_select_kernel<<<T, 512, 0, stream>>>(scores, ld, positions, k, out, ld_out);
+  pxl_host::launch(topk_select_kernel, T, 512, 0, stream, scores, ld, positions, k, out, ld_out);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
@@ -331,7 +338,7 @@ PXL_EXPORT int pxl_store_rows(const void* src, int64_t ld, const int64_t* slots,
                               int64_t num_slots, int* status, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (D % 8 || ld % 8) return PXL_ERR_INVALID_ARG;
-  store_rows_kernel<<<T, 64, 0, stream>>>(static_cast<const pxl::bf16*>(src), ld, slots,
+  pxl_host::launch(store_rows_kernel, T, 64, 0, stream, static_cast<const pxl::bf16*>(src), ld, slots,
                                           static_cast<pxl::bf16*>(cache), D, num_slots, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

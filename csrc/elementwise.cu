@@ -214,6 +214,8 @@ rmsnorm_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16
 __global__ void __launch_bounds__(256)
 rmsnorm_strided_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ w, bf16* __restrict__ out,
                        int64_t ldo, int H, float eps, float w_offset) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[32];
   const size_t row = blockIdx.x;
   const bf16* xr = x + row * ldx;
@@ -444,6 +446,8 @@ reshape_and_cache_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v,
                          void* __restrict__ k_cache_v, void* __restrict__ v_cache_v, int Hkv, int Dk,
                          int Dv, int page_size, int64_t num_slots, float k_inv_scale,
                          float v_inv_scale, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   using CT = typename std::conditional<FP8, uint8_t, bf16>::type;
   CT* k_cache = static_cast<CT*>(k_cache_v);
   CT* v_cache = static_cast<CT*>(v_cache_v);
@@ -491,6 +495,8 @@ __device__ __forceinline__ float act_mul(float g, float u, int mode, float limit
 
 __global__ void __launch_bounds__(256)
 act_mul_kernel(const bf16* __restrict__ x, bf16* __restrict__ out, int I, int mode, float limit) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t row = blockIdx.x;
   const bf16* g = x + row * 2 * I;
   const bf16* u = g + I;
@@ -514,6 +520,8 @@ template <typename IdT>
 __global__ void __launch_bounds__(128)
 gather_rows_kernel(const bf16* __restrict__ table, const IdT* __restrict__ ids,
                    bf16* __restrict__ out, int H, int64_t num_rows, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t t = blockIdx.x;
   int64_t id = static_cast<int64_t>(ids[t]);
   if (id < 0 || id >= num_rows) {
@@ -527,6 +535,8 @@ gather_rows_kernel(const bf16* __restrict__ table, const IdT* __restrict__ ids,
 }
 
 __global__ void __launch_bounds__(256) add_inplace_kernel(bf16* y, const bf16* x, int64_t nvec) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= nvec) return;
   bf16x8 a = ld_bf16x8(y + i * 8);
@@ -592,7 +602,7 @@ PXL_EXPORT int pxl_rmsnorm_strided(const void* x, int64_t ldx, const void* weigh
                                    int H, float eps, float w_offset, pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
   if ((H % 8) || (ldx % 8) || (ldo % 8)) return PXL_ERR_INVALID_ARG;
-  rmsnorm_strided_kernel<<<T, 256, 0, stream>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(weight),
+  pxl_host::launch(rmsnorm_strided_kernel, T, 256, 0, stream, static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(weight),
                                                 static_cast<bf16*>(out), ldo, H, eps, w_offset);
   return check_launch();
 }
@@ -689,6 +699,8 @@ __global__ void patch_i32_kernel(int* __restrict__ dst, const int* __restrict__ 
                                  const int* __restrict__ src_idx, int n, int dst_len, int src_len, int* status) {
   pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
+  pdl_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int d = dst_idx[i], s = src_idx[i];
@@ -716,7 +728,7 @@ PXL_EXPORT int pxl_selftest_bounded_wait(const uint32_t* flag, uint32_t epoch, i
 PXL_EXPORT int pxl_patch_i32(int* dst, const int* dst_idx, const int* src, const int* src_idx, int n, int dst_len,
                              int src_len, int* status, pxl_stream_t stream) {
   if (n <= 0) return PXL_OK;
-  patch_i32_kernel<<<(n + 255) / 256, 256, 0, stream>>>(dst, dst_idx, src, src_idx, n, dst_len, src_len, status);
+  pxl_host::launch(patch_i32_kernel, (n + 255) / 256, 256, 0, stream, dst, dst_idx, src, src_idx, n, dst_len, src_len, status);
   return check_launch();
 }
 
@@ -725,8 +737,7 @@ PXL_EXPORT int pxl_reshape_and_cache(const void* k, const void* v, int64_t k_str
                                      void* v_cache, int T, int Hkv, int Dk, int Dv, int page_size,
                                      int64_t num_slots, int* status, pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
-  reshape_and_cache_kernel<false><<<T, 256, 0, stream>>>(
-      static_cast<const bf16*>(k), static_cast<const bf16*>(v), k_stride, v_stride, slot_mapping,
+  pxl_host::launch(reshape_and_cache_kernel<false>, T, 256, 0, stream, static_cast<const bf16*>(k), static_cast<const bf16*>(v), k_stride, v_stride, slot_mapping,
       k_cache, v_cache, Hkv, Dk, Dv, page_size, num_slots, 1.f, 1.f, status);
   return check_launch();
 }
@@ -738,8 +749,7 @@ PXL_EXPORT int pxl_reshape_and_cache_fp8(const void* k, const void* v, int64_t k
                                          float v_scale, int* status, pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
   if (!(k_scale > 0.f) || !(v_scale > 0.f)) return PXL_ERR_INVALID_ARG;
-  reshape_and_cache_kernel<true><<<T, 256, 0, stream>>>(
-      static_cast<const bf16*>(k), static_cast<const bf16*>(v), k_stride, v_stride, slot_mapping,
+  pxl_host::launch(reshape_and_cache_kernel<true>, T, 256, 0, stream, static_cast<const bf16*>(k), static_cast<const bf16*>(v), k_stride, v_stride, slot_mapping,
       k_cache, v_cache, Hkv, Dk, Dv, page_size, num_slots, 1.f / k_scale, 1.f / v_scale, status);
   return check_launch();
 }
@@ -748,7 +758,7 @@ PXL_EXPORT int pxl_act_mul(const void* x, void* out, int T, int I, int mode, flo
                            pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
   if (I % 8) return PXL_ERR_INVALID_ARG;
-  act_mul_kernel<<<T, 256, 0, stream>>>(static_cast<const bf16*>(x), static_cast<bf16*>(out), I,
+  pxl_host::launch(act_mul_kernel, T, 256, 0, stream, static_cast<const bf16*>(x), static_cast<bf16*>(out), I,
                                         mode, limit);
   return check_launch();
 }
@@ -759,12 +769,12 @@ PXL_EXPORT int pxl_gather_rows(const void* table, const void* ids, void* out, in
   if (T <= 0) return PXL_OK;
   if (H % 8) return PXL_ERR_INVALID_ARG;
   if (ids_are_i64)
-    gather_rows_kernel<int64_t><<<T, 128, 0, stream>>>(static_cast<const bf16*>(table),
+    pxl_host::launch(gather_rows_kernel<int64_t>, T, 128, 0, stream, static_cast<const bf16*>(table),
                                                        static_cast<const int64_t*>(ids),
                                                        static_cast<bf16*>(out), H, num_rows,
                                                        status);
   else
-    gather_rows_kernel<int><<<T, 128, 0, stream>>>(static_cast<const bf16*>(table),
+    pxl_host::launch(gather_rows_kernel<int>, T, 128, 0, stream, static_cast<const bf16*>(table),
                                                    static_cast<const int*>(ids),
                                                    static_cast<bf16*>(out), H, num_rows, status);
   return check_launch();
@@ -774,7 +784,6 @@ PXL_EXPORT int pxl_add_inplace(void* y, const void* x, int64_t n, pxl_stream_t s
   if (n <= 0) return PXL_OK;
   if (n % 8) return PXL_ERR_INVALID_ARG;
   const int64_t nvec = n / 8;
-  add_inplace_kernel<<<static_cast<unsigned>((nvec + 255) / 256), 256, 0, stream>>>(
-      static_cast<bf16*>(y), static_cast<const bf16*>(x), nvec);
+  pxl_host::launch(add_inplace_kernel, static_cast<unsigned>((nvec + 255) / 256), 256, 0, stream, static_cast<bf16*>(y), static_cast<const bf16*>(x), nvec);
   return check_launch();
 }

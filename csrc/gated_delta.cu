@@ -81,6 +81,8 @@ __device__ __forceinline__ void load4(const bf16* p, float* v) {
 // VEC: rows of q and k start on 8 bytes.
 template <bool VEC>
 __global__ void __launch_bounds__(256, 2) delta_step_kernel(const GdArgs a, int seq0) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[2][8];
   const int hv = blockIdx.x, seq = seq0 + blockIdx.y, hk = hv / (a.Hv / a.Hk);
   const int l = threadIdx.x & 7, r0 = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -248,6 +250,8 @@ constexpr int kMakeThreads = 256;
 
 // grid (chunks, heads). Warps 0 to 3: 16 rows of A each, warps 4 to 7: of P.
 __global__ void __launch_bounds__(kMakeThreads) delta_make_kernel(const GdArgs a, int seqs, int chunk0, uint8_t* __restrict__ work) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t raw[];
   MakeSmem& s = *reinterpret_cast<MakeSmem*>(raw);
   const int h = blockIdx.y, hk = h / (a.Hv / a.Hk), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -466,6 +470,8 @@ constexpr int kHalf = 8, kWalkThreads = 2 * kHalf * 32;
 
 // grid (slices of v, heads, sequences): the chunks [chunk0, chunk0 + chunks) of one sequence, in order
 __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArgs a, int chunk0, int chunks, uint8_t* __restrict__ work) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t raw[];
   WalkSmem& s = *reinterpret_cast<WalkSmem*>(raw);
   const int h = blockIdx.y, hk = h / (a.Hv / a.Hk), seq = blockIdx.z, v0 = blockIdx.x * kSlice;
@@ -636,6 +642,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) delta_walk_kernel(const GdArg
 
 // grid (chunks, heads), a warp per token: out = rmsnorm(o) * norm_w * silu(z)
 __global__ void __launch_bounds__(256) delta_norm_kernel(const GdArgs a, int seqs, int chunk0, const uint8_t* __restrict__ work) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int seq, index;
   if (!find_chunk(a.seq_cu, seqs, chunk0 + blockIdx.x, seq, index)) return;
@@ -681,9 +689,9 @@ int launch_chunked(const GdArgs& a, int seqs, int tokens, uint8_t* work, int64_t
   const int run = fit < bound ? static_cast<int>(fit) : bound;
   for (int c0 = 0; c0 < bound; c0 += run) {
     const int n = bound - c0 < run ? bound - c0 : run;
-    delta_make_kernel<<<dim3(n, a.Hv), kMakeThreads, sizeof(MakeSmem), stream>>>(a, seqs, c0, work);
-    delta_walk_kernel<<<dim3(a.Dv / kSlice, a.Hv, seqs), kWalkThreads, sizeof(WalkSmem), stream>>>(a, c0, n, work);
-    delta_norm_kernel<<<dim3(n, a.Hv), 256, 0, stream>>>(a, seqs, c0, work);
+    pxl_host::launch(delta_make_kernel, dim3(n, a.Hv), kMakeThreads, sizeof(MakeSmem), stream, a, seqs, c0, work);
+    pxl_host::launch(delta_walk_kernel, dim3(a.Dv / kSlice, a.Hv, seqs), kWalkThreads, sizeof(WalkSmem), stream, a, c0, n, work);
+    pxl_host::launch(delta_norm_kernel, dim3(n, a.Hv), 256, 0, stream, a, seqs, c0, work);
   }
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
@@ -723,8 +731,8 @@ PXL_EXPORT int pxl_gated_delta_rule(const void* qkv, int64_t ld_qkv, const void*
   const bool vec = ld_qkv % 4 == 0 && aligned(qkv, 8);
   for (; done < B; done += 65535) {
     const dim3 grid(Hv, B - done < 65535 ? B - done : 65535);
-    if (vec) delta_step_kernel<true><<<grid, 256, 0, stream>>>(a, done);
-    else delta_step_kernel<false><<<grid, 256, 0, stream>>>(a, done);
+    if (vec) pxl_host::launch(delta_step_kernel<true>, grid, 256, 0, stream, a, done);
+    else pxl_host::launch(delta_step_kernel<false>, grid, 256, 0, stream, a, done);
   }
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

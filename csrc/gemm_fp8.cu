@@ -69,6 +69,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const uint32_t pfull0 = smem_u32(bars + 2 * F_STAGES), pempty0 = smem_u32(bars + 2 * F_STAGES + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  if (g.num_mt != nullptr) pdl_wait();  // the list of tiles comes from the kernels before
   // ---- tile coordinates
   const int num_n = ceil_div(g.N, FN);
   int a_row, b_row, row_end, n_blk;
@@ -116,17 +117,28 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // weights of the first stages, under the tail of the kernel before (no kernel of a launch chain writes weights)
+  if (warp == 0 && lane == 0) {
+    for (int kb = 0; kb < F_STAGES && kb < num_kb; ++kb) {
+      mbar_arrive_expect_tx(full0 + 8 * kb, F_STAGE_BYTES);
+      tma_load_2d(smem_u32(smem + kb * F_STAGE_BYTES + FM * FK), &tmap_b, full0 + 8 * kb, (kb_base + kb) * FK, b_row);
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY)) break;
         const uint32_t fb = full0 + 8 * stage;
-        mbar_arrive_expect_tx(fb, F_STAGE_BYTES);
+        if (kb >= F_STAGES) {
+          if (!mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY)) break;
+          mbar_arrive_expect_tx(fb, F_STAGE_BYTES);
+          tma_load_2d(smem_u32(smem + stage * F_STAGE_BYTES + FM * FK), &tmap_b, fb, (kb_base + kb) * FK, b_row);
+        }
         tma_load_2d(smem_u32(smem + stage * F_STAGE_BYTES), &tmap_a, fb, (kb_base + kb) * FK, a_row);
-        tma_load_2d(smem_u32(smem + stage * F_STAGE_BYTES + FM * FK), &tmap_b, fb, (kb_base + kb) * FK, b_row);
         if (++stage == F_STAGES) {
           stage = 0;
           phase ^= 1;
@@ -325,6 +337,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 __global__ void __launch_bounds__(256) quant_fp8_rows_kernel(const bf16* __restrict__ x, int64_t ld,
                                                              uint8_t* __restrict__ q, float* __restrict__ s, int64_t total,
                                                              int groups) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4);
   const int l = threadIdx.x & 15;
   const bool in = i < total;  // (whole half warps; the other half takes part in the shuffles)
@@ -387,15 +401,17 @@ int launch_fp8(const void* A, const void* W, const Fp8Args& g, uint64_t a_rows, 
     cfg.blockDim = dim3(F_THREADS);
     cfg.dynamicSmemBytes = F_SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = static_cast<unsigned>(g.splits);
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pxl_host::chained() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gemm_fp8_kernel<true>, ta, tb, g, status) == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
   }
-  gemm_fp8_kernel<false><<<tiles, F_THREADS, F_SMEM, stream>>>(ta, tb, g, status);
+  pxl_host::launch(gemm_fp8_kernel<false>, tiles, F_THREADS, F_SMEM, stream, ta, tb, g, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
@@ -453,7 +469,6 @@ PXL_EXPORT int pxl_quant_fp8_rows(const void* x, int64_t ld, void* q, float* sca
   if (T <= 0) return PXL_OK;
   if (K % 128) return PXL_ERR_INVALID_ARG;
   const int64_t total = static_cast<int64_t>(T) * (K / 128);
-  quant_fp8_rows_kernel<<<static_cast<unsigned>((total + 15) / 16), 256, 0, stream>>>(
-      static_cast<const pxl::bf16*>(x), ld, static_cast<uint8_t*>(q), scales, total, K / 128);
+  pxl_host::launch(quant_fp8_rows_kernel, static_cast<unsigned>((total + 15) / 16), 256, 0, stream, static_cast<const pxl::bf16*>(x), ld, static_cast<uint8_t*>(q), scales, total, K / 128);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

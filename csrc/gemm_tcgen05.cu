@@ -280,6 +280,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     return;
   }
 
+  if (grp.num_mt != nullptr) pdl_wait();  // the list of tiles comes from the kernels before
   const int num_m = grp.num_mt != nullptr ? *grp.num_mt : ceil_div(M, BM);
   const int num_n = ceil_div(N, BN);
   const int num_tiles = num_m * num_n * (grp.heads > 0 ? grp.heads : 1);
@@ -319,8 +320,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // everything above touched only this CTA's shared and tensor memory: with a programmatic dependent
-  // launch it overlaps the tail of the previous kernel, whose results are needed from here on
+  // Everything above touched only this CTA's shared and tensor memory: with a programmatic dependent launch it overlaps the tail
+  // of the previous kernel. So do the first loads of weights, which no kernel of a launch chain writes: what the ring of stages
+  // takes. A product of a few rows is bound by these bytes, and the SMs that the previous kernel (a norm, a rotation, the tail
+  // of an attention) leaves idle fetch them: five layers of 57 rows 800 -> 780 us, a layer's weights 59 us of each 160. (More of
+  // the tile into L2 by prefetches brings nothing, or delays the rows that queue behind them: 8 boxes 780, 24 boxes 803 us.)
+  constexpr bool kSwapped = EPI == PXL_EPI_SPLITK_T || EPI == PXL_EPI_SPLITK_C;  // the weights take A's slot
+  int ahead = 0;
+  if (warp == 0 && lane == 0 && grp.num_mt == nullptr && comm.tp <= 1 && static_cast<int>(blockIdx.x) < num_items) {
+    const TileCoord tc = tile_coord<BN>(item_tile(blockIdx.x), num_m, num_n, M, grp, comm);
+    const int kb0 = item_ks(blockIdx.x) * kb_per, kb1 = kb0 + kb_per < num_kb ? kb0 + kb_per : num_kb;
+    for (int kb = kb0; kb < kb1 && ahead < STAGES; ++kb, ++ahead) {
+      const uint32_t fb = full0 + 8 * ahead;
+      mbar_arrive_expect_tx(fb, A_STAGE_BYTES + Cfg::B_STAGE_BYTES);
+      if constexpr (kSwapped) tma_load_2d(smem_u32(smem_a + ahead * A_STAGE_BYTES), &tmap_a, fb, kb * BK, tc.a_row);
+      else tma_load_2d(smem_u32(smem_b + ahead * Cfg::B_STAGE_BYTES), &tmap_b, fb, kb * BK, tc.b_row);
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
 
@@ -344,15 +360,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           fence_proxy_async_all();
         }
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status,
-                                 PXL_DEV_TIMEOUT_EMPTY);
-          if (!ok) break;
+          const bool begun = ahead > 0;  // this stage's weights are on their way
+          if (begun) {
+            --ahead;
+          } else {
+            ok = mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status,
+                                   PXL_DEV_TIMEOUT_EMPTY);
+            if (!ok) break;
+          }
           const uint32_t fb = full0 + 8 * stage;
-          mbar_arrive_expect_tx(fb, A_STAGE_BYTES + Cfg::B_STAGE_BYTES);
-          tma_load_2d(smem_u32(smem_a + stage * A_STAGE_BYTES), &tmap_a, fb, tc.a_col + kb * BK,
-                      tc.a_row);
-          tma_load_2d(smem_u32(smem_b + stage * Cfg::B_STAGE_BYTES), &tmap_b, fb, kb * BK,
-                      tc.b_row);
+          if (!begun) mbar_arrive_expect_tx(fb, A_STAGE_BYTES + Cfg::B_STAGE_BYTES);
+          if (!begun || !kSwapped)
+            tma_load_2d(smem_u32(smem_a + stage * A_STAGE_BYTES), &tmap_a, fb, tc.a_col + kb * BK,
+                        tc.a_row);
+          if (!begun || kSwapped)
+            tma_load_2d(smem_u32(smem_b + stage * Cfg::B_STAGE_BYTES), &tmap_b, fb, kb * BK,
+                        tc.b_row);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -744,18 +767,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // Every thread of every CTA passes both cluster barriers, also after a failed wait (all other
     // waits are bounded). Barrier 1: all accumulators of the cluster are complete, so nobody's
     // pipeline stages are in use any more and can receive partial sums: CTA r collects, from every
-    // CTA of the cluster, the tokens [r*S, (r+1)*S) as [source][S][128 columns] floats. Barrier 2:
-    // the partial sums have landed; each CTA adds its tokens in K order and writes the result.
+    // CTA of the cluster, the tokens [r*S, (r+1)*S) as [source][S / 4][128 columns][4 tokens] floats (S a multiple
+    // of four: 16-byte remote stores, and a warp writes 512 contiguous bytes). Barrier 2: the partial sums have
+    // landed; each CTA adds its tokens in K order and writes the result, a warp's lanes neighbouring columns.
     __syncwarp();
     cluster_sync_all();
     const uint32_t my_rank = cluster_cta_rank();
     const int n_tok = N;
-    const int S = ceil_div(n_tok, splitk);
+    const int S4 = ceil_div(n_tok, 4 * splitk), S = 4 * S4;
     const uint32_t recv0 = smem_u32(smem);
     if (warp >= 2 && acc_ready) {
       const int q = warp & 3;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-      const uint32_t col_off = (my_rank * S * 128 + q * 32 + lane) * 4;
+      const uint32_t col_off = (my_rank * S4 * 128 + q * 32 + lane) * 16;
       int owner = 0, tl = 0;
       uint32_t dst = cluster_map_shared(recv0, 0) + col_off;
 #pragma unroll 1
@@ -764,10 +788,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tmem_ld_32x32b_x32(t_row + c0, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (c0 + j < n_tok) {
-            st_shared_cluster_f32(dst + tl * 512, __uint_as_float(r[j]));
-            if (++tl == S) {
+        for (int j = 0; j < 32; j += 4) {
+          if (c0 + j < n_tok) {  // (columns past the last token hold sums of zero rows)
+            st_shared_cluster_f32x4(dst + tl * 2048, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                    __uint_as_float(r[j + 3]));
+            if (++tl == S4) {
               tl = 0;
               ++owner;
               if (owner < splitk) dst = cluster_map_shared(recv0, owner) + col_off;
@@ -784,34 +809,30 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int n0 = tile * BM;  // first output column of the tile (num_n == 1)
       const int t0 = my_rank * S;
       const int s_valid = n_tok - t0 < S ? n_tok - t0 : S;
-      for (int i = threadIdx.x - 64; i < s_valid * 32; i += 128) {
-        const int tl = i >> 5, c4 = (i & 31) * 4;
-        const int n = n0 + c4;
-        if (n < M) {
-          const uint32_t src = recv0 + (tl * 128 + c4) * 4;
+      const int col = threadIdx.x - 64, n = n0 + col;
+      if (n < M) {
+        const float bias = ep.bias ? __bfloat162float(ep.bias[n]) : 0.f;
+        for (int q4 = 0; q4 * 4 < s_valid; ++q4) {
+          const uint32_t src = recv0 + (q4 * 128 + col) * 16;
+          const size_t c_off = static_cast<size_t>(t0 + q4 * 4) * ep.ldc + n;
+          const int left = s_valid - q4 * 4;
+          float res[4] = {};
+          if (ep.residual) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (e < left) res[e] = __bfloat162float(ep.residual[c_off + static_cast<size_t>(e) * ep.ldc]);
+          }
           float4 a = ld_shared_f32x4(src);
           for (int r = 1; r < splitk; ++r) {
             const float4 b = ld_shared_f32x4(src + r * S * 512);
             a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w;
           }
-          const size_t c_off = static_cast<size_t>(t0 + tl) * ep.ldc + n;
-          if (ep.bias) {
-            const uint2 b = *reinterpret_cast<const uint2*>(ep.bias + n);
-            const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y);
-            a.x += b0.x, a.y += b0.y, a.z += b1.x, a.w += b1.y;
-          }
-          if (ep.residual) {
-            const uint2 b = *reinterpret_cast<const uint2*>(ep.residual + c_off);
-            const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y);
-            a.x += b0.x, a.y += b0.y, a.z += b1.x, a.w += b1.y;
-          }
-          if (ep.C_f32 != nullptr) {
-            *reinterpret_cast<float4*>(ep.C_f32 + c_off) = a;
-          } else {
-            uint2 o;
-            o.x = pack_bf16x2(a.x, a.y);
-            o.y = pack_bf16x2(a.z, a.w);
-            *reinterpret_cast<uint2*>(ep.C + c_off) = o;
+          const float o[4] = {a.x + bias + res[0], a.y + bias + res[1], a.z + bias + res[2], a.w + bias + res[3]};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (e >= left) break;
+            if (ep.C_f32 != nullptr) ep.C_f32[c_off + static_cast<size_t>(e) * ep.ldc] = o[e];
+            else ep.C[c_off + static_cast<size_t>(e) * ep.ldc] = __float2bfloat16(o[e]);
           }
         }
       }
@@ -1056,7 +1077,7 @@ int launch_gemm_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = (pxl_host::pdl_flag() && max_clusters == nullptr) ? 2 : 1;
+  cfg.numAttrs = max_clusters == nullptr && pxl_host::chained() ? 2 : 1;
   if (max_clusters != nullptr) {
     cfg.gridDim = dim3(static_cast<unsigned>(cluster) * 64u, 1, 1);  // the query only needs a legal grid
     int n = 0;

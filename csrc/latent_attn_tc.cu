@@ -116,7 +116,6 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kMaxVBufs + 2 * kMaxSlots + 6);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   pdl_wait();
-  pdl_launch_dependents();
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int b = blockIdx.z, hb = blockIdx.y;
@@ -172,6 +171,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_launch_dependents();
   const uint32_t tm_o = *tmem_slot;             // O: 64 columns per latent chunk
   const uint32_t tm_s = tm_o + 64 * per;        // two score buffers of NK columns
   const uint32_t tm_p = tm_s + 2 * NK;          // two probability buffers of NK / 2 columns

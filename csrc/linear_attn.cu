@@ -21,6 +21,8 @@ __global__ void __launch_bounds__(128) conv1d_silu_kernel(const bf16* __restrict
                                                           const int* __restrict__ seq_slots,
                                                           const int* __restrict__ positions, bf16* __restrict__ out,
                                                           int64_t ldo, int C, int K) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (c >= C) return;
@@ -55,6 +57,8 @@ __global__ void __launch_bounds__(128) conv_run_kernel(const bf16* __restrict__ 
                                                        const int* __restrict__ seq_cu, const int* __restrict__ seq_slots,
                                                        const int* __restrict__ positions, bf16* __restrict__ out, int64_t ldo,
                                                        int C, int seqs, int tokens, int run) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
   if (c >= C) return;
   const int first = blockIdx.y * run, last = first + run < tokens ? first + run : tokens;
@@ -131,6 +135,8 @@ __global__ void __launch_bounds__(128) conv_run_kernel(const bf16* __restrict__ 
 __global__ void __launch_bounds__(128) conv_window_kernel(const bf16* __restrict__ x, int64_t ldx, bf16* __restrict__ conv_state,
                                                           const int* __restrict__ seq_cu, const int* __restrict__ seq_slots,
                                                           const int* __restrict__ positions, int C, int K) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int c = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
   if (c >= C) return;
   const int t0 = seq_cu[b], n = seq_cu[b + 1] - t0;
@@ -157,13 +163,15 @@ bool launch_conv_run(const bf16* x, int64_t ldx, const bf16* w, const bf16* bias
   while (ceil_div(tokens, run) > 65535) run *= 2;
   const dim3 grid(blocks, ceil_div(tokens, run));
   const auto kern = K == 2 ? conv_run_kernel<2> : K == 3 ? conv_run_kernel<3> : conv_run_kernel<4>;
-  kern<<<grid, 128, 0, stream>>>(x, ldx, w, bias, conv_state, seq_cu, seq_slots, positions, out, ldo, C, seqs, tokens, run);
-  conv_window_kernel<<<dim3(ceil_div(C, 128), seqs), 128, 0, stream>>>(x, ldx, conv_state, seq_cu, seq_slots, positions, C, K);
+  pxl_host::launch(kern, grid, 128, 0, stream, x, ldx, w, bias, conv_state, seq_cu, seq_slots, positions, out, ldo, C, seqs, tokens, run);
+  pxl_host::launch(conv_window_kernel, dim3(ceil_div(C, 128), seqs), 128, 0, stream, x, ldx, conv_state, seq_cu, seq_slots, positions, C, K);
   return true;
 }
 
 __global__ void sigmoid_gate_mul_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ gate,
                                         int64_t ldg, bf16* __restrict__ out, int64_t ldo, int n8) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x;
   for (int v = threadIdx.x; v < n8; v += blockDim.x) {
     const bf16x8 a = ld_bf16x8(x + t * ldx + v * 8), g = ld_bf16x8(gate + t * ldg + v * 8);
@@ -182,6 +190,8 @@ __global__ void sigmoid_gate_mul_kernel(const bf16* __restrict__ x, int64_t ldx,
 __global__ void gate_mul_grouped_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ gate,
                                         int64_t ldg, const bf16* __restrict__ res, int64_t ldr,
                                         bf16* __restrict__ out, int64_t ldo, int n8, int group8) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x;
   for (int v = threadIdx.x; v < n8; v += blockDim.x) {
     const float g = __bfloat162float(gate[t * ldg + v / group8]);
@@ -208,6 +218,8 @@ __global__ void gate_mul_grouped_kernel(const bf16* __restrict__ x, int64_t ldx,
 // out[t] = x[t, :] . w  (one warp per row; the one-column projection of a scalar gate is too thin for a GEMM tile)
 __global__ void row_dot_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ w,
                                bf16* __restrict__ out, int T, int k8) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   if (t >= T) return;
   const int lane = threadIdx.x % 32;
@@ -239,7 +251,7 @@ PXL_EXPORT int pxl_causal_conv1d_silu(const void* x_, int64_t ldx, const void* w
       launch_conv_run(x, ldx, w, bias, conv_state, seq_cu, seq_slots, positions, out, ldo, C, K, prefill_seqs, prefill_tokens, stream))
     done = prefill_seqs;
   if (done < B)
-    conv1d_silu_kernel<<<dim3(pxl::ceil_div(C, 128), B - done), 128, 0, stream>>>(x, ldx, w, bias, conv_state, seq_cu + done,
+    pxl_host::launch(conv1d_silu_kernel, dim3(pxl::ceil_div(C, 128), B - done), 128, 0, stream, x, ldx, w, bias, conv_state, seq_cu + done,
                                                                                  seq_slots + done, positions, out, ldo, C, K);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
@@ -248,7 +260,7 @@ PXL_EXPORT int pxl_sigmoid_gate_mul(const void* x, int64_t ldx, const void* gate
                                     int64_t ldo, int T, int N, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (N % 8) return PXL_ERR_INVALID_ARG;
-  sigmoid_gate_mul_kernel<<<T, 128, 0, stream>>>(static_cast<const pxl::bf16*>(x), ldx,
+  pxl_host::launch(sigmoid_gate_mul_kernel, T, 128, 0, stream, static_cast<const pxl::bf16*>(x), ldx,
                                                  static_cast<const pxl::bf16*>(gate), ldg,
                                                  static_cast<pxl::bf16*>(out), ldo, N / 8);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
@@ -259,7 +271,7 @@ PXL_EXPORT int pxl_gate_mul_grouped(const void* x, int64_t ldx, const void* gate
                                     cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (N % 8 || group <= 0 || group % 8 || N % group) return PXL_ERR_INVALID_ARG;
-  gate_mul_grouped_kernel<<<T, 128, 0, stream>>>(static_cast<const pxl::bf16*>(x), ldx,
+  pxl_host::launch(gate_mul_grouped_kernel, T, 128, 0, stream, static_cast<const pxl::bf16*>(x), ldx,
                                                  static_cast<const pxl::bf16*>(gate), ldg,
                                                  static_cast<const pxl::bf16*>(res), ldr,
                                                  static_cast<pxl::bf16*>(out), ldo, N / 8, group / 8);
@@ -269,7 +281,7 @@ PXL_EXPORT int pxl_gate_mul_grouped(const void* x, int64_t ldx, const void* gate
 PXL_EXPORT int pxl_row_dot(const void* x, int64_t ldx, const void* w, void* out, int T, int K, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (K % 8) return PXL_ERR_INVALID_ARG;
-  row_dot_kernel<<<pxl::ceil_div(T, 4), 128, 0, stream>>>(static_cast<const pxl::bf16*>(x), ldx,
+  pxl_host::launch(row_dot_kernel, pxl::ceil_div(T, 4), 128, 0, stream, static_cast<const pxl::bf16*>(x), ldx,
                                                           static_cast<const pxl::bf16*>(w),
                                                           static_cast<pxl::bf16*>(out), T, K / 8);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;

@@ -63,6 +63,8 @@ __device__ __forceinline__ int find_seq(const int* cu_q, int B, int t) {
 }
 
 __global__ void __launch_bounds__(kMlaThreads, 1) mla_attn_kernel(const MlaArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   MlaSmem& sm = *reinterpret_cast<MlaSmem*>(smem_raw);
   const int t = a.tok_begin + blockIdx.x;  // token index in the batch-wide activation matrices
@@ -256,6 +258,8 @@ __global__ void __launch_bounds__(128) mla_kv_prep_kernel(const bf16* __restrict
                                                           const int64_t* __restrict__ slots,
                                                           bf16* __restrict__ cache, int64_t num_slots,
                                                           float eps, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[32];
   const int t = blockIdx.x;
   const int64_t slot = slots[t];
@@ -296,6 +300,8 @@ __global__ void __launch_bounds__(128) mla_q_prep_kernel(const bf16* __restrict_
                                                          bf16* __restrict__ q_nope_hm,
                                                          bf16* __restrict__ q_pe, int T, int Tpad, int H,
                                                          int nope) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x;
   const bf16* src = q + t * ld;
   const float* cs = cos_sin + static_cast<size_t>(positions[t]) * kR;
@@ -347,7 +353,7 @@ PXL_EXPORT int pxl_mla_attn(const void* q_lat, const void* q_pe, const void* cac
   a.topk_k = topk_k; a.topk_stride = topk_stride;
   a.scale_log2 = scale * 1.4426950408889634f;
   dim3 grid(n_tok, pxl::ceil_div(H, kHB));
-  mla_attn_kernel<<<grid, kMlaThreads, sizeof(MlaSmem), stream>>>(a);
+  pxl_host::launch(mla_attn_kernel, grid, kMlaThreads, sizeof(MlaSmem), stream, a);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
@@ -356,7 +362,7 @@ PXL_EXPORT int pxl_mla_kv_prep(const void* ckv, int64_t ld, const void* norm_w, 
                                int rope, int64_t num_slots, float eps, int* status, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (latent != kL || rope != kR) return PXL_ERR_INVALID_ARG;
-  mla_kv_prep_kernel<<<T, 128, 0, stream>>>(static_cast<const pxl::bf16*>(ckv), ld,
+  pxl_host::launch(mla_kv_prep_kernel, T, 128, 0, stream, static_cast<const pxl::bf16*>(ckv), ld,
                                             static_cast<const pxl::bf16*>(norm_w), cos_sin, positions, slots,
                                             static_cast<pxl::bf16*>(cache), num_slots, eps, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
@@ -367,7 +373,7 @@ PXL_EXPORT int pxl_mla_q_prep(const void* q, int64_t ld, const float* cos_sin, c
                               cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (rope != kR || (nope % 2)) return PXL_ERR_INVALID_ARG;
-  mla_q_prep_kernel<<<T, 128, 0, stream>>>(static_cast<const pxl::bf16*>(q), ld, cos_sin, positions,
+  pxl_host::launch(mla_q_prep_kernel, T, 128, 0, stream, static_cast<const pxl::bf16*>(q), ld, cos_sin, positions,
                                            static_cast<pxl::bf16*>(q_nope_hm), static_cast<pxl::bf16*>(q_pe), T,
                                            Tpad, H, nope);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;

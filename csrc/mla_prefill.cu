@@ -45,6 +45,7 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  pdl_wait();
   const int b = blockIdx.z, head = blockIdx.y;
   const int t0 = cu_q[b], L = cu_q[b + 1] - t0;
   // heavy blocks (late queries see the most keys) are scheduled first
@@ -81,6 +82,7 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_launch_dependents();
   const uint32_t tm_s = *tmem_slot, tm_o = tm_s + 2 * kT;
 
   // a softmax thread holds 128 scores: 384 threads x 168 registers at launch cover 256 x 208 + 128 x 80
@@ -213,6 +215,8 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // interleaved rotation of the last 64 of every head's 192 columns, in place
 __global__ void __launch_bounds__(256) mla_rotate_kernel(bf16* __restrict__ q, int64_t ld, const float* __restrict__ cos_sin,
                                                          const int* __restrict__ positions, int max_pos, int H, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x, p = positions[t];
   if (p < 0 || p >= max_pos) {
     if (threadIdx.x == 0 && status) atomicCAS(status, 0, PXL_DEV_BAD_POSITION);
@@ -239,7 +243,7 @@ PXL_EXPORT int pxl_mla_rotate(void* q, int64_t ld, const float* cos_sin, const i
                               int rot, int* status, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (nope != kNope || rot != kRot || H <= 0 || (ld % 8) || (reinterpret_cast<uintptr_t>(q) & 15)) return PXL_ERR_INVALID_ARG;
-  mla_rotate_kernel<<<T, 256, 0, stream>>>(static_cast<pxl::bf16*>(q), ld, cos_sin, positions, max_pos, H, status);
+  pxl_host::launch(mla_rotate_kernel, T, 256, 0, stream, static_cast<pxl::bf16*>(q), ld, cos_sin, positions, max_pos, H, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
@@ -263,7 +267,7 @@ PXL_EXPORT int pxl_mla_prefill(const void* q, const void* kv, const void* rows, 
     if (cudaFuncSetAttribute(mla_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return PXL_ERR_CUDA;
     configured[dev] = true;
   }
-  mla_prefill_kernel<<<dim3(pxl::ceil_div(max_q, 2 * kQ), H, B), kThreads, kSmem, stream>>>(
+  pxl_host::launch(mla_prefill_kernel, dim3(pxl::ceil_div(max_q, 2 * kQ), H, B), kThreads, kSmem, stream, 
       tq, tkv, trows, cu_q, static_cast<pxl::bf16*>(out), H, scale * kLog2eF, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

@@ -33,6 +33,8 @@ __global__ void __launch_bounds__(128)
 moe_route_kernel(const void* __restrict__ logits, int64_t ld, const float* __restrict__ e_bias, int T, int E,
                  int k, int mode, int renorm, int n_group, int topk_group, int group_top, float routed_scale,
                  int* __restrict__ out_ids, float* __restrict__ out_w) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
   if (t >= T) return;
@@ -159,6 +161,8 @@ moe_route_kernel(const void* __restrict__ logits, int64_t ld, const float* __res
 // counts[e] = number of (token, slot) pairs routed to expert e (ids < 0 or >= E are skipped)
 __global__ void moe_count_kernel(const int* __restrict__ ids, int n, int E, int e_lo, int e_hi,
                                  int* __restrict__ counts) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int e = ids[i];
@@ -172,6 +176,8 @@ __global__ void __launch_bounds__(1024)
 moe_scan_kernel(const int* __restrict__ counts, int E, int* __restrict__ offsets,
                 int* __restrict__ cursor, int* __restrict__ mt_expert, int* __restrict__ mt_row0,
                 int* __restrict__ mt_row_end, int* __restrict__ num_mt, int max_mt) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ int s_off[1025];
   __shared__ int s_mt[1025];
   const int tid = threadIdx.x;
@@ -208,6 +214,8 @@ moe_scan_kernel(const int* __restrict__ counts, int E, int* __restrict__ offsets
 __global__ void moe_place_kernel(const int* __restrict__ ids, int n, int k, int E, int e_lo,
                                  int e_hi, int* __restrict__ cursor, int* __restrict__ pos_of,
                                  int* __restrict__ src_tok) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int e = ids[i];
@@ -224,6 +232,8 @@ __global__ void moe_place_kernel(const int* __restrict__ ids, int n, int k, int 
 __global__ void __launch_bounds__(128)
 moe_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ src_tok,
                   const int* __restrict__ n_rows, bf16* __restrict__ x_perm, int H) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int p = blockIdx.x;
   if (p >= *n_rows) return;
   const bf16* src = x + static_cast<size_t>(src_tok[p]) * H;
@@ -237,6 +247,8 @@ moe_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ src_tok,
 template <typename T, int VEC>
 __global__ void __launch_bounds__(512) moe_scatter_rows_kernel(const T* __restrict__ x, int64_t ldx, const int* __restrict__ pos_of,
                                                                const float* __restrict__ w, T* __restrict__ x_perm, int k, int H) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ int rows[32];
   __shared__ float factors[32];
   const int64_t t = blockIdx.x;
@@ -278,6 +290,8 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ pos_of,
                    const float* __restrict__ w, const bf16* __restrict__ base,
                    bf16* __restrict__ out, int k, int H) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t t = blockIdx.x;
   for (int v = threadIdx.x; v < (H >> 3); v += blockDim.x) {
     float acc[8];
@@ -325,7 +339,7 @@ PXL_EXPORT int pxl_moe_route(const void* logits, int64_t ld, int logits_bf16, co
   const unsigned grid = (T + 3) / 4;
   const int epl = (E + 31) / 32;
 #define PXL_ROUTE(B16, EPL)                                                                                        \
-  moe_route_kernel<B16, EPL><<<grid, 128, 0, stream>>>(logits, ld, e_bias, T, E, k, mode, renorm, n_group, topk_group, \
+  pxl_host::launch(moe_route_kernel<B16, EPL>, grid, 128, 0, stream, logits, ld, e_bias, T, E, k, mode, renorm, n_group, topk_group, \
                                                        group_top, routed_scale, out_ids, out_w)
 #define PXL_ROUTE_EPL(B16)          \
   if (epl <= 1) PXL_ROUTE(B16, 1);  \
@@ -354,10 +368,10 @@ PXL_EXPORT int pxl_moe_align(const int* ids, int T, int k, int E, int e_lo, int 
   const int n_local = e_hi - e_lo;
   if (n <= 0 || n_local <= 0 || n_local > 1024) return PXL_ERR_INVALID_ARG;
   const unsigned grid = (n + 255) / 256;
-  moe_count_kernel<<<grid, 256, 0, stream>>>(ids, n, E, e_lo, e_hi, counts);
-  moe_scan_kernel<<<1, 1024, 0, stream>>>(counts, n_local, offsets, cursor, mt_expert, mt_row0,
+  pxl_host::launch(moe_count_kernel, grid, 256, 0, stream, ids, n, E, e_lo, e_hi, counts);
+  pxl_host::launch(moe_scan_kernel, 1, 1024, 0, stream, counts, n_local, offsets, cursor, mt_expert, mt_row0,
                                           mt_row_end, num_mt, max_mt);
-  moe_place_kernel<<<grid, 256, 0, stream>>>(ids, n, k, E, e_lo, e_hi, cursor, pos_of, src_tok);
+  pxl_host::launch(moe_place_kernel, grid, 256, 0, stream, ids, n, k, E, e_lo, e_hi, cursor, pos_of, src_tok);
   return check_launch();
 }
 
@@ -365,7 +379,7 @@ PXL_EXPORT int pxl_moe_gather(const void* x, const int* src_tok, const int* n_ro
                               int max_rows, int H, pxl_stream_t stream) {
   if (max_rows <= 0) return PXL_OK;
   if (H % 8) return PXL_ERR_INVALID_ARG;
-  moe_gather_kernel<<<max_rows, 128, 0, stream>>>(static_cast<const bf16*>(x), src_tok, n_rows,
+  pxl_host::launch(moe_gather_kernel, max_rows, 128, 0, stream, static_cast<const bf16*>(x), src_tok, n_rows,
                                                   static_cast<bf16*>(x_perm), H);
   return check_launch();
 }
@@ -377,13 +391,13 @@ PXL_EXPORT int pxl_moe_scatter_rows(const void* x, int64_t ldx, const int* pos_o
   const int threads = H >= 4096 ? 512 : H >= 2048 ? 256 : 128;
   const bool vec = !is_f32 && !((ldx | H) & 7) && !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_perm)) & 15);
   if (is_f32)
-    moe_scatter_rows_kernel<float, 1><<<T, threads, 0, stream>>>(static_cast<const float*>(x), ldx, pos_of, w,
+    pxl_host::launch(moe_scatter_rows_kernel<float, 1>, T, threads, 0, stream, static_cast<const float*>(x), ldx, pos_of, w,
                                                              static_cast<float*>(x_perm), k, H);
   else if (vec)
-    moe_scatter_rows_kernel<bf16, 8><<<T, threads, 0, stream>>>(static_cast<const bf16*>(x), ldx, pos_of, w,
+    pxl_host::launch(moe_scatter_rows_kernel<bf16, 8>, T, threads, 0, stream, static_cast<const bf16*>(x), ldx, pos_of, w,
                                                             static_cast<bf16*>(x_perm), k, H);
   else
-    moe_scatter_rows_kernel<bf16, 1><<<T, threads, 0, stream>>>(static_cast<const bf16*>(x), ldx, pos_of, w,
+    pxl_host::launch(moe_scatter_rows_kernel<bf16, 1>, T, threads, 0, stream, static_cast<const bf16*>(x), ldx, pos_of, w,
                                                             static_cast<bf16*>(x_perm), k, H);
   return check_launch();
 }
@@ -393,7 +407,7 @@ PXL_EXPORT int pxl_moe_combine(const void* y_perm, const int* pos_of, const floa
                                pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
   if (H % 8) return PXL_ERR_INVALID_ARG;
-  moe_combine_kernel<<<T, 256, 0, stream>>>(static_cast<const bf16*>(y_perm), pos_of, w,
+  pxl_host::launch(moe_combine_kernel, T, 256, 0, stream, static_cast<const bf16*>(y_perm), pos_of, w,
                                             static_cast<const bf16*>(base),
                                             static_cast<bf16*>(out), k, H);
   return check_launch();

@@ -87,6 +87,14 @@ static int stage_probe(int* status, cudaStream_t stream, int layer, int op) {
     if (pr_ != PXL_OK) return pr_;                     \
   } while (0)
 
+PXL_EXPORT int pxl_launch_chain(int on) {
+  int& s = pxl_host::launch_chain();
+  const int prev = s != pxl_host::kNoChain;
+  static const bool no_pdl = getenv("PXL_NO_PDL") != nullptr;
+  s = on && !no_pdl ? pxl_host::kChainBegun : pxl_host::kNoChain;
+  return prev;
+}
+
 // h_in [T, H] -> returns the pointer that holds the stage's output hidden states in *h_out (one of
 // the workspace's ping/pong buffers). *launches receives the number of kernels launched.
 PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc* sp, const PxlStageWorkspace* ws,
@@ -114,11 +122,13 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
   // every kernel of the sequence waits (griddepcontrol.wait) before it touches global memory, so each
   // launch may overlap its prologue with the tail of the kernel before it
   static const bool no_pdl = getenv("PXL_NO_PDL") != nullptr;
-  struct PdlScope {
-    bool prev;
-    explicit PdlScope(bool on) : prev(pxl_host::pdl_flag()) { pxl_host::pdl_flag() = on; }
-    ~PdlScope() { pxl_host::pdl_flag() = prev; }
-  } pdl_scope(!no_pdl && !stage_debug());
+  struct ChainScope {
+    int prev;
+    explicit ChainScope(bool on) : prev(pxl_host::launch_chain()) {
+      pxl_host::launch_chain() = on ? pxl_host::kChainBegun : pxl_host::kNoChain;
+    }
+    ~ChainScope() { pxl_host::launch_chain() = prev; }
+  } chain_scope(!no_pdl && !stage_debug());
   // one or two rows: the norms are part of the products behind them
   auto normed = [&](int N, int epi) { return T <= PXL_GEMV_NORM_MAX_M && pxl_gemv_bf16_takes(T, N, H, epi) && H % 8 == 0; };
   for (int li = 0; li < st->n_layers; ++li) {

@@ -359,10 +359,11 @@ class DeepseekStage(DecoderStage):
     def forward_layers(self, h: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         eps = self.cfg.rms_norm_eps
         lists = None
-        for li, lw in enumerate(self.layers):
-            xn = ops.rmsnorm(h, lw.ln1, eps)
-            a, lists = self._attention(lw, li, xn, fb, lists)
-            h = self._lin(a.contiguous(), lw.w_o, residual=h)
-            xn = ops.rmsnorm(h, lw.ln2, eps)
-            h = self._mlp(lw, xn, h)
+        with self.chained(h):
+            for li, lw in enumerate(self.layers):
+                xn = ops.rmsnorm(h, lw.ln1, eps)
+                a, lists = self._attention(lw, li, xn, fb, lists)
+                h = self._lin(a.contiguous(), lw.w_o, residual=h)
+                xn = ops.rmsnorm(h, lw.ln2, eps)
+                h = self._mlp(lw, xn, h)
         return h

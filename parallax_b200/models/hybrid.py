@@ -212,15 +212,16 @@ class HybridStage(DecoderStage):
 
     def forward_layers(self, h: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         eps = self.cfg.rms_norm_eps
-        for li, lw in enumerate(self.layers):
-            xn = ops.rmsnorm(h, lw.ln1, eps, w_offset=self.norm_offset)
-            if lw.kind == LINEAR:
-                a = self._linear_attention(lw, li, xn, fb)
-                h = ops.linear(a, lw.w_out, residual=h)
-            else:
-                a = self._attention(lw, li, xn, fb)                      # q/k norm, partial RoPE, paged attention
-                gate = ops.linear(xn, lw.w_gate)
-                h = ops.linear(ops.sigmoid_gate_mul(a, gate), lw.w_o, residual=h)
-            xn = ops.rmsnorm(h, lw.ln2, eps, w_offset=self.norm_offset)
-            h = self._mlp(lw, xn, h)
+        with self.chained(h):
+            for li, lw in enumerate(self.layers):
+                xn = ops.rmsnorm(h, lw.ln1, eps, w_offset=self.norm_offset)
+                if lw.kind == LINEAR:
+                    a = self._linear_attention(lw, li, xn, fb)
+                    h = ops.linear(a, lw.w_out, residual=h)
+                else:
+                    a = self._attention(lw, li, xn, fb)                  # q/k norm, partial RoPE, paged attention
+                    gate = ops.linear(xn, lw.w_gate)
+                    h = ops.linear(ops.sigmoid_gate_mul(a, gate), lw.w_o, residual=h)
+                xn = ops.rmsnorm(h, lw.ln2, eps, w_offset=self.norm_offset)
+                h = self._mlp(lw, xn, h)
         return h

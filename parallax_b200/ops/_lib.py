@@ -51,6 +51,7 @@ def check(code: int, what: str) -> None:
 
 _P = c_void_p
 _SIGS = {
+    "pxl_launch_chain": [c_int],
     "pxl_gemm_bf16_launches": [c_int] * 4,
     "pxl_gemm_bf16": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "pxl_gemm_bf16_pick_bn": [c_int, c_int, c_int],

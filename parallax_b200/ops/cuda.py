@@ -108,6 +108,20 @@ def workspace(device: torch.device, tag: str, nbytes: int) -> torch.Tensor:
     return t
 
 
+class launch_chain:
+    """``with launch_chain():`` - the kernels that this thread launches inside overlap their prologue, and the first loads of
+    weights, with the tail of the kernel before them on the stream (programmatic dependent launch; every kernel waits before it
+    touches anything else). Weights and the step's index arrays are written before the chain, on the same stream."""
+
+    def __enter__(self):
+        self.before = _lib.lib().pxl_launch_chain(1)
+        return self
+
+    def __exit__(self, *exc):
+        _lib.lib().pxl_launch_chain(self.before)
+        return False
+
+
 # ----------------------------------------------------------------------------- GEMM
 def _tma_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether bf16 operands ``x [M, K]``, ``w [N, K]`` fit the tensor-core GEMM (16-byte rows and bases)."""
