@@ -151,3 +151,42 @@ def test_error_against_64_bits(q_scale, bound, lists):
     want = torch.einsum("bhk,bkd->bhd", p, kv[..., :L])
     err = float((got - want).norm() / want.norm())
     assert err < bound, err
+
+
+@pytest.mark.parametrize("L,R,H,k,page,ctx", [
+    (512, 32, 128, 130, 16, [400, 131]),    # a last column chunk that the rows do not fill; a last tile of two rows
+    (480, 64, 128, 64, 64, [257, 64]),      # values that end inside a chunk; a context of one list's length
+    (512, 8, 16, 200, 8, [1000]),           # few heads
+    (448, 64, 128, 96, 16, [300]),          # eight column chunks
+])
+def test_lists_of_other_widths(L, R, H, k, page, ctx):
+    """Rows off the lists are no numbers, also those that follow a listed row in memory."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(L + R)
+    need = [-(-c // page) for c in ctx]
+    table, at = torch.zeros(len(ctx), max(need), dtype=torch.int32), 0
+    order = torch.randperm(sum(need)).int()
+    for i, n in enumerate(need):
+        table[i, :n], at = order[at:at + n], at + n
+    cache = torch.randn(sum(need), 1, page, L + R).bfloat16()
+    lists = torch.full((len(ctx), k), -1, dtype=torch.int32)
+    for i, c in enumerate(ctx):
+        if c > k:
+            lists[i] = torch.randperm(c)[:k].int()
+        keys = (lists[i] if c > k else torch.arange(c)).long()
+        keep = torch.zeros(need[i] * page, dtype=torch.bool)
+        keep[keys] = True
+        rows = cache[table[i, :need[i]].long(), 0]
+        rows.view(-1, L + R)[~keep] = float("nan")
+        cache[table[i, :need[i]].long(), 0] = rows
+    q = (torch.randn(len(ctx), H, L + R) * 0.5).bfloat16()
+    lens, scale = torch.tensor(ctx).int(), 192 ** -0.5
+    got = cu.latent_attn(q.cuda(), cache.cuda(), table.cuda(), None, lens.cuda(), scale, L, max_ctx=max(ctx), topk=lists.cuda()).cpu()
+    cu.check_status(torch.device("cuda", 0))
+    for i, c in enumerate(ctx):
+        keys = (lists[i] if c > k else torch.arange(c)).long()
+        rows = cache[table[i].long(), 0].reshape(-1, L + R)[keys].double()
+        want = (q[i].double() @ rows.t() * scale).softmax(-1) @ rows[:, :L]
+        # probabilities and outputs are rounded to bf16 (2^-9 each)
+        assert float((got[i].double() - want).norm() / want.norm()) < 2 ** -7
