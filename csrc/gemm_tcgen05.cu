@@ -4,6 +4,8 @@
 //   warp 0   : TMA producer. One elected lane streams 128xBK A tiles and BNxBK W
 //              tiles (both K-major, 128-byte swizzle) through a ring of shared-memory
 //              stages guarded by full/empty mbarriers.
+//              (Both issuing warps run their loops with all lanes, which keeps addresses and descriptors uniform: 128 rows x 6144 x
+//              4096 split over clusters 20.0 -> 17.7 us, 512 rows x 4096 x 4096 24.8 -> 18.9, large products the same.)
 //   warp 1   : MMA issuer. One elected lane issues tcgen05.mma (M=128, N=BN, K=16)
 //              straight from shared memory into a TMEM accumulator; tcgen05.commit
 //              releases the smem stage / publishes the finished accumulator.
@@ -21,6 +23,7 @@
 
 #include "common.cuh"
 #include "pxl_api.h"
+#include "tc_issue.cuh"
 
 namespace {
 using namespace pxl;
@@ -57,6 +60,7 @@ struct GemmEpilogueArgs {
   const bf16* bias;      // optional, length N (pre-activation columns)
   float* C_f32;          // EPI_F32 output
   int ldc;
+  int a_rows;            // rows of A that a stage loads (0: all 128)
   bf16* const* row_ptrs; // EPI_SCATTER: destination of every output row (null = drop), N elements each
   uint32_t* done_counter;  // EPI_SCATTER: local counter for the "last CTA publishes the flags" step
   float act_limit;           // EPI_CLIP_GLU
@@ -182,7 +186,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const uint32_t tfull0 = smem_u32(bars + 2 * STAGES);
   const uint32_t tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
 
   const int gemm_ctas = gridDim.x - comm.ag_ncopy;
@@ -325,6 +329,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   // takes. A product of a few rows is bound by these bytes, and the SMs that the previous kernel (a norm, a rotation, the tail
   // of an attention) leaves idle fetch them: five layers of 57 rows 800 -> 780 us, a layer's weights 59 us of each 160. (More of
   // the tile into L2 by prefetches brings nothing, or delays the rows that queue behind them: 8 boxes 780, 24 boxes 803 us.)
+  const uint32_t stage_bytes = (ep.a_rows > 0 ? ep.a_rows * BK * 2 : A_STAGE_BYTES) + Cfg::B_STAGE_BYTES;
   constexpr bool kSwapped = EPI == PXL_EPI_SPLITK_T || EPI == PXL_EPI_SPLITK_C;  // the weights take A's slot
   int ahead = 0;
   if (warp == 0 && lane == 0 && grp.num_mt == nullptr && comm.tp <= 1 && static_cast<int>(blockIdx.x) < num_items) {
@@ -332,7 +337,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int kb0 = item_ks(blockIdx.x) * kb_per, kb1 = kb0 + kb_per < num_kb ? kb0 + kb_per : num_kb;
     for (int kb = kb0; kb < kb1 && ahead < STAGES; ++kb, ++ahead) {
       const uint32_t fb = full0 + 8 * ahead;
-      mbar_arrive_expect_tx(fb, A_STAGE_BYTES + Cfg::B_STAGE_BYTES);
+      mbar_arrive_expect_tx(fb, stage_bytes);
       if constexpr (kSwapped) tma_load_2d(smem_u32(smem_a + ahead * A_STAGE_BYTES), &tmap_a, fb, kb * BK, tc.a_row);
       else tma_load_2d(smem_u32(smem_b + ahead * Cfg::B_STAGE_BYTES), &tmap_b, fb, kb * BK, tc.b_row);
     }
@@ -342,7 +347,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
+      ahead = __shfl_sync(0xffffffffu, ahead, 0);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -354,28 +361,26 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (comm.ag_ncopy > 0 && tc.a_row / comm.rows_per_rank != comm.rank) {
           // rows of another rank: wait until the copy CTAs have landed this tile locally
           const uint32_t* tf = comm.ag_tile_flags + (tc.a_row / BM) * kAgChunksPerTile;
-          for (int ch = 0; ok && ch < kAgChunksPerTile; ++ch)
-            ok = flag_wait_bounded<false>(tf + ch, comm.epoch, abort_flag, status);
+          if (lane == 0) {
+            for (int ch = 0; ok && ch < kAgChunksPerTile; ++ch)
+              ok = flag_wait_bounded<false>(tf + ch, comm.epoch, abort_flag, status);
+            fence_proxy_async_all();
+          }
+          ok = __all_sync(0xffffffffu, ok) != 0;
           if (!ok) break;
-          fence_proxy_async_all();
         }
         for (int kb = kb0; kb < kb1; ++kb) {
           const bool begun = ahead > 0;  // this stage's weights are on their way
+          const uint32_t fb = full0 + 8 * stage;
           if (begun) {
             --ahead;
           } else {
-            ok = mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status,
-                                   PXL_DEV_TIMEOUT_EMPTY);
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY)) != 0;
             if (!ok) break;
+            expect_tx(fb, stage_bytes, leader);
           }
-          const uint32_t fb = full0 + 8 * stage;
-          if (!begun) mbar_arrive_expect_tx(fb, A_STAGE_BYTES + Cfg::B_STAGE_BYTES);
-          if (!begun || !kSwapped)
-            tma_load_2d(smem_u32(smem_a + stage * A_STAGE_BYTES), &tmap_a, fb, tc.a_col + kb * BK,
-                        tc.a_row);
-          if (!begun || kSwapped)
-            tma_load_2d(smem_u32(smem_b + stage * Cfg::B_STAGE_BYTES), &tmap_b, fb, kb * BK,
-                        tc.b_row);
+          if (!begun || !kSwapped) tma_box(smem_u32(smem_a) + stage * A_STAGE_BYTES, &tmap_a, fb, tc.a_col + kb * BK, tc.a_row, leader);
+          if (!begun || kSwapped) tma_box(smem_u32(smem_b) + stage * Cfg::B_STAGE_BYTES, &tmap_b, fb, kb * BK, tc.b_row, leader);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -385,8 +390,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_leader();
       constexpr uint32_t idesc = umma_idesc(BM, BN, 1, 1);
+      const uint64_t da0 = umma_desc_k_sw128(smem_u32(smem_a)), db0 = umma_desc_k_sw128(smem_u32(smem_b));
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -395,32 +402,26 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       for (int item = blockIdx.x; ok && item < num_items; item += gemm_ctas) {
         const int kb0 = item_ks(item) * kb_per;
         const int kb1 = kb0 + kb_per < num_kb ? kb0 + kb_per : num_kb;
-        ok = mbar_wait_bounded(tempty0 + 8 * acc, acc_phase ^ 1, abort_flag, status,
-                               PXL_DEV_TIMEOUT_TMEM_EMPTY);
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(tempty0 + 8 * acc, acc_phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_EMPTY)) != 0;
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait_bounded(full0 + 8 * stage, phase, abort_flag, status,
-                                 PXL_DEV_TIMEOUT_FULL);
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(full0 + 8 * stage, phase, abort_flag, status, PXL_DEV_TIMEOUT_FULL)) != 0;
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem_a + stage * A_STAGE_BYTES);
-          const uint32_t b_addr = smem_u32(smem_b + stage * Cfg::B_STAGE_BYTES);
+          const uint64_t da = da0 + stage * (A_STAGE_BYTES >> 4), db = db0 + stage * (Cfg::B_STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = umma_desc_k_sw128(a_addr + k * UMMA_K * 2);
-            const uint64_t db = umma_desc_k_sw128(b_addr + k * UMMA_K * 2);
-            tc_mma_f16(d_tmem, da, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          }
-          tc_commit(empty0 + 8 * stage);  // stage reusable once these MMAs retire
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            mma_ss(d_tmem, da + k * (UMMA_K * 2 >> 4), db + k * (UMMA_K * 2 >> 4), idesc, (kb > kb0 || k > 0) ? 1u : 0u, leader);
+          commit(empty0 + 8 * stage, leader);  // stage reusable once these MMAs retire
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
         if (!ok) break;
-        tc_commit(tfull0 + 8 * acc);  // accumulator complete
+        commit(tfull0 + 8 * acc, leader);  // accumulator complete
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
@@ -1118,6 +1119,12 @@ int dispatch_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 
 }  // namespace
 
+namespace {
+// Rows of the box that loads A: fewer than a tile where the matrix has fewer. (The product reads what an earlier kernel left in the
+// others' place, for accumulator rows that are not stored.)
+int box_rows(int M) { return M < BM ? pxl::ceil_div(M, 8) * 8 : BM; }
+}  // namespace
+
 // Tile width heuristic: estimated time = waves over the SMs x tile width / relative throughput of
 // that width (measured on compute-bound shapes: a 256-wide tile keeps the tensor pipe busiest, a
 // 64-wide one reaches about a third of it). Large problems take the width that wastes the least of
@@ -1499,7 +1506,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
   if (epi == PXL_EPI_SILU_MUL && ((N % bn) != 0 || bn < 128)) return PXL_ERR_INVALID_ARG;
 
   CUtensorMap ta, tb;
-  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, BM, BK))
+  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, box_rows(M), BK))
     return PXL_ERR_TENSORMAP;
   if (!pxl_host::make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, N, K, ldw, bn, BK))
     return PXL_ERR_TENSORMAP;
@@ -1509,6 +1516,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
   ep.residual = static_cast<const pxl::bf16*>(residual);
   ep.bias = static_cast<const pxl::bf16*>(bias);
   ep.ldc = ldc;
+  ep.a_rows = box_rows(M);
   GemmGroupArgs grp{};
   switch (bn) {
     case 256: return dispatch_epi<256>(epi, ta, tb, ep, grp, GemmCommArgs{}, 0, M, N, K, status, stream);
@@ -1540,11 +1548,12 @@ int gemm_glu(const void* A, const void* W, void* C, int M, int N, int K, int lda
   if (bn == 0) bn = pxl_gemm_bf16_pick_bn(M, N, PXL_EPI_SILU_MUL);
   if ((bn != 128 && bn != 256) || (N % bn)) return PXL_ERR_INVALID_ARG;
   CUtensorMap ta, tb;
-  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, BM, BK) ||
+  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, box_rows(M), BK) ||
       !pxl_host::make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, N, K, ldw, bn, BK))
     return PXL_ERR_TENSORMAP;
   ep.C = static_cast<pxl::bf16*>(C);
   ep.ldc = ldc;
+  ep.a_rows = box_rows(M);
   GemmGroupArgs grp{};
   if (bn == 256) return launch_gemm<256, EPI>(ta, tb, ep, grp, GemmCommArgs{}, 0, M, N, K, status, stream);
   return launch_gemm<128, EPI>(ta, tb, ep, grp, GemmCommArgs{}, 0, M, N, K, status, stream);
@@ -1580,12 +1589,13 @@ PXL_EXPORT int pxl_gemm_bf16_act(const void* A, const void* W, void* C, int M, i
     return PXL_ERR_INVALID_ARG;
   const int bn = pxl_gemm_bf16_pick_bn(M, N, PXL_EPI_ACT);
   CUtensorMap ta, tb;
-  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, BM, BK) ||
+  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, box_rows(M), BK) ||
       !pxl_host::make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, N, K, ldw, bn, BK))
     return PXL_ERR_TENSORMAP;
   GemmEpilogueArgs ep{};
   ep.C = static_cast<pxl::bf16*>(C);
   ep.ldc = ldc;
+  ep.a_rows = box_rows(M);
   ep.act = act;
   ep.table = static_cast<const pxl::bf16*>(table);
   ep.ids = ids;

@@ -91,17 +91,6 @@ __device__ __noinline__ void clear_rows(uint32_t v, int chunks, uint32_t rows, u
   fence_proxy_async_smem();
 }
 
-// A wait that did not pass at once: out of line, so that the loops of the roles stay short (see the kernel).
-__device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  return mbar_wait_bounded(bar, parity, abort_flag, status, code);
-}
-// Warp-collective, the same result in every lane.
-__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  bool there = __all_sync(0xffffffffu, mbar_test(bar, parity)) != 0;
-  if (!there) there = __all_sync(0xffffffffu, wait_slow(bar, parity, abort_flag, status, code)) != 0;
-  return there;
-}
-
 // WIDE: nine column chunks, eight of them values (L = 512 and up to 64 columns more), in two CTAs of four value chunks.
 constexpr int kWideKeys = 5, kWideFirst = 3, kWideVBufs = 3;  // score-only chunks, those of the first group, value buffers
 constexpr int kWideSlots = 2 * kWideFirst;

@@ -20,6 +20,16 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {  // n
       : "memory");
   return ok != 0;
 }
+// A wait that did not pass at once: out of line, so that the loops of the warps that issue stay short.
+static __device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return mbar_wait_bounded(bar, parity, abort_flag, status, code);
+}
+// Warp-collective, the same result in every lane.
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  bool there = __all_sync(0xffffffffu, mbar_test(bar, parity)) != 0;
+  if (!there) there = __all_sync(0xffffffffu, wait_slow(bar, parity, abort_flag, status, code)) != 0;
+  return there;
+}
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -87,6 +97,30 @@ __device__ __forceinline__ void tma_gather4(uint32_t smem_dst, const CUtensorMap
       "}\n"
       :
       : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void mma_f8_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate,
+                                          uint32_t leader) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes, uint32_t leader) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"
+      "}\n"
+      :
+      : "r"(bar), "r"(bytes), "r"(leader)
       : "memory");
 }
 __device__ __forceinline__ void commit(uint32_t bar, uint32_t leader) {
