@@ -31,7 +31,9 @@ constexpr int F_SMEM = 1024 + F_STAGES * F_STAGE_BYTES + 256;
 // Scales of four K blocks, fetched one group of four ahead by the thread that uses them (no barrier): a scale per row of A and
 // two per 64 rows of W. Read where they are needed, they were most of the kernel: a load of every thread's own line per K block
 // between "the product is there" and its promotion (44 % of the warps' cycles waiting for L1, 24 % hits). The four products of a
-// dense layer of 4000 tokens (7168 wide, 18432 inside): 4.38 -> 2.88 ms, 1.53 PFLOP/s.
+// dense layer of 4000 tokens (7168 wide, 18432 inside): 4.38 -> 2.88 ms, and 2.65 (1.7 PFLOP/s) with the sums promoted in pairs.
+// A thread without a row fetches none: copies of one address by many lanes go out one by one, and with 64 of 128 rows they took
+// longer than the product (36864 x 7168, 64 rows: 97 -> 48 us; one row, whose three idle warps no longer promote either: 155 -> 45).
 constexpr int F_GROUP = 4;
 constexpr int F_THREADS = 192;
 
@@ -49,6 +51,7 @@ struct Fp8Args {
   int w_rows_per_expert;
   // SPLIT: CTAs of a cluster, one per K range; K blocks per range (a multiple of F_GROUP)
   int splits, kb_per;
+  int stage_bytes;  // of a stage that are loaded
 };
 
 constexpr int kPartPitch = FN + 4;  // floats of a row of partial sums: 16-byte stores of a quarter warp hit distinct banks
@@ -67,7 +70,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + F_STAGES);
   const uint32_t pfull0 = smem_u32(bars + 2 * F_STAGES), pempty0 = smem_u32(bars + 2 * F_STAGES + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (g.num_mt != nullptr) pdl_wait();  // the list of tiles comes from the kernels before
   // ---- tile coordinates
@@ -120,55 +123,59 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   // weights of the first stages, under the tail of the kernel before (no kernel of a launch chain writes weights)
   if (warp == 0 && lane == 0) {
     for (int kb = 0; kb < F_STAGES && kb < num_kb; ++kb) {
-      mbar_arrive_expect_tx(full0 + 8 * kb, F_STAGE_BYTES);
+      mbar_arrive_expect_tx(full0 + 8 * kb, g.stage_bytes);
       tma_load_2d(smem_u32(smem + kb * F_STAGE_BYTES + FM * FK), &tmap_b, full0 + 8 * kb, (kb_base + kb) * FK, b_row);
     }
   }
   pdl_wait();
   pdl_launch_dependents();
 
+  // (the issuing loops run with all lanes, so that their addresses and descriptors are uniform; see tc_issue.cuh)
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const uint32_t fb = full0 + 8 * stage;
-        if (kb >= F_STAGES) {
-          if (!mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY)) break;
-          mbar_arrive_expect_tx(fb, F_STAGE_BYTES);
-          tma_load_2d(smem_u32(smem + stage * F_STAGE_BYTES + FM * FK), &tmap_b, fb, (kb_base + kb) * FK, b_row);
-        }
-        tma_load_2d(smem_u32(smem + stage * F_STAGE_BYTES), &tmap_a, fb, (kb_base + kb) * FK, a_row);
-        if (++stage == F_STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
+    const uint32_t leader = elect_leader(), s0 = smem_u32(smem);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      const uint32_t fb = full0 + 8 * stage, at = s0 + stage * F_STAGE_BYTES;
+      if (kb >= F_STAGES) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY))) break;
+        expect_tx(fb, g.stage_bytes, leader);
+        tma_box(at + FM * FK, &tmap_b, fb, (kb_base + kb) * FK, b_row, leader);
+      }
+      tma_box(at, &tmap_a, fb, (kb_base + kb) * FK, a_row, leader);
+      if (++stage == F_STAGES) {
+        stage = 0;
+        phase ^= 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(FM, FN, 0, 0);  // e4m3 x e4m3 -> fp32
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int part = kb & 1;
-        const uint32_t pphase = (kb >> 1) & 1;
-        if (!mbar_wait_bounded(pempty0 + 8 * part, pphase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_EMPTY)) break;
-        if (!mbar_wait_bounded(full0 + 8 * stage, phase, abort_flag, status, PXL_DEV_TIMEOUT_FULL)) break;
-        tc_fence_after_sync();
-        const uint32_t a_addr = smem_u32(smem + stage * F_STAGE_BYTES);
-        const uint32_t b_addr = a_addr + FM * FK;
+    constexpr uint32_t idesc = umma_idesc(FM, FN, 0, 0);  // e4m3 x e4m3 -> fp32
+    const uint32_t leader = elect_leader();
+    const uint64_t da0 = umma_desc_k_sw128(smem_u32(smem)), db0 = umma_desc_k_sw128(smem_u32(smem) + FM * FK);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      const int part = kb & 1;
+      const uint32_t pphase = (kb >> 1) & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(pempty0 + 8 * part, pphase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_EMPTY))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(full0 + 8 * stage, phase, abort_flag, status, PXL_DEV_TIMEOUT_FULL))) break;
+      tc_fence_after_sync();
+      const uint64_t da = da0 + stage * (F_STAGE_BYTES >> 4), db = db0 + stage * (F_STAGE_BYTES >> 4);
 #pragma unroll
-        for (int k = 0; k < FK / 32; ++k)
-          tc_mma_f8(tmem_base + part * FN, umma_desc_k_sw128(a_addr + k * 32), umma_desc_k_sw128(b_addr + k * 32),
-                    idesc, k > 0 ? 1u : 0u);
-        tc_commit(empty0 + 8 * stage);
-        tc_commit(pfull0 + 8 * part);
-        if (++stage == F_STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
+      for (int k = 0; k < FK / 32; ++k) mma_f8_ss(tmem_base + part * FN, da + 2 * k, db + 2 * k, idesc, k > 0 ? 1u : 0u, leader);
+      commit(empty0 + 8 * stage, leader);
+      commit(pfull0 + 8 * part, leader);
+      if (++stage == F_STAGES) {
+        stage = 0;
+        phase ^= 1;
       }
+    }
+  } else if (a_row + (warp & 3) * 32 >= row_end) {
+    // ---- an epilogue warp whose rows are all behind the tile's last one hands the partial sums back as they come
+    bool ok = true;
+    for (int kb = 0; ok && kb < num_kb; ++kb) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(pfull0 + 8 * (kb & 1), (kb >> 1) & 1, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_FULL)) != 0;
+      if (ok && lane == 0) mbar_arrive(pempty0 + 8 * (kb & 1));
     }
   } else {
     // ---- epilogue warps: thread = one accumulator row
@@ -189,15 +196,15 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
       };
       if (kb < num_kb) {
-        copy(scales[buf][q][lane], as_row);
+        if (row_ok) copy(scales[buf][q][lane], as_row);
         if (lane < 2) copy(w_scales[buf][q][lane], ws0 + lane * kb_total);
       }
       cp_async_commit();
     };
     fetch(0);
-    float acc[FN];
+    uint64_t acc2[FN / 2];
 #pragma unroll
-    for (int i = 0; i < FN; ++i) acc[i] = 0.f;
+    for (int i = 0; i < FN / 2; ++i) acc2[i] = 0ull;
     bool ok = true;
     for (int kb = 0; kb < num_kb; ++kb) {
       const int part = kb & 1, buf = (kb / F_GROUP) & 1;
@@ -215,22 +222,31 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       if (!ok) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + part * FN + (static_cast<uint32_t>(q * 32) << 16);
-      // 16 columns are on their way while the 16 before them are added
+      // 16 columns are on their way while the 16 before them are added, two per instruction (32 columns at a time without the
+      // overlap: a tenth slower than the sums one by one; in pairs this way: 7168 x 18432, 4000 tokens 666 -> 614 us)
       uint32_t r[2][16];
       tmem_ld_32x32b_x16(t_row, r[0]);
 #pragma unroll
       for (int c = 0; c < FN; c += 16) {
         tmem_ld_wait();
         if (c + 16 < FN) tmem_ld_32x32b_x16(t_row + c + 16, r[((c >> 4) + 1) & 1]);
-        const float sc = c < 64 ? s0 : s1;
+        const uint32_t sc = __float_as_uint(c < 64 ? s0 : s1);
+        const uint64_t sc2 = (static_cast<uint64_t>(sc) << 32) | sc;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(__uint_as_float(r[(c >> 4) & 1][j]), sc, acc[c + j]);
+        for (int j = 0; j < 16; j += 2) {
+          uint64_t x;
+          asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(r[(c >> 4) & 1][j]), "r"(r[(c >> 4) & 1][j + 1]));
+          acc2[(c + j) >> 1] = fma2(x, sc2, acc2[(c + j) >> 1]);
+        }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(pempty0 + 8 * part);
     }
     cp_async_wait<0>();
+    float acc[FN];
+#pragma unroll
+    for (int i = 0; i < FN / 2; ++i) acc[2 * i] = __uint_as_float(static_cast<uint32_t>(acc2[i])), acc[2 * i + 1] = __uint_as_float(static_cast<uint32_t>(acc2[i] >> 32));
     if constexpr (SPLIT) {
       // every load and product of this CTA is done: its stages take the partial sums
       if (ok) {
@@ -381,10 +397,12 @@ __global__ void __launch_bounds__(256) quant_fp8_rows_kernel(const bf16* __restr
   if (l == 0) s[i] = scale;
 }
 
-int launch_fp8(const void* A, const void* W, const Fp8Args& g, uint64_t a_rows, uint64_t w_rows, int lda, int ldw,
+int launch_fp8(const void* A, const void* W, Fp8Args g, uint64_t a_rows, uint64_t w_rows, int lda, int ldw,
                int tiles, int* status, cudaStream_t stream) {
   CUtensorMap ta, tb;
-  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, a_rows, g.K, lda, FM, FK)) return PXL_ERR_TENSORMAP;
+  const int box = a_rows < FM ? pxl::ceil_div(static_cast<int>(a_rows), 8) * 8 : FM;
+  g.stage_bytes = (box + FN) * FK;
+  if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, a_rows, g.K, lda, box, FK)) return PXL_ERR_TENSORMAP;
   if (!pxl_host::make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, W, w_rows, g.K, ldw, FN, FK)) return PXL_ERR_TENSORMAP;
   static bool configured[64] = {false};
   int dev = 0;

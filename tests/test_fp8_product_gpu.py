@@ -61,3 +61,38 @@ def test_row_quantisation_into_words():
                                             torch.cuda.current_stream().cuda_stream) == 0
     assert torch.equal(buf[4:-4], want.view(torch.uint8).flatten()) and torch.equal(s, scales)
     assert int(buf[:4].sum()) == 0 and int(buf[-4:].sum()) == 0
+
+
+@pytest.mark.parametrize("M", [1, 7, 31, 32, 33, 64, 97, 127, 128])
+@pytest.mark.parametrize("N,K,epi", [(39168, 256, "glu"), (128, 2048, "plain")])
+def test_fp8_product_of_part_of_a_tile(M, N, K, epi):
+    """Boxes of fewer than 128 rows and warps without a row, with a tile per CTA and split over a cluster; rows of A that follow the
+    last one in memory are no numbers."""
+    from parallax_b200.loader.quant import quantize_fp8_block
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(M + N)
+    x = torch.full((136, K), float("nan")).bfloat16().cuda()
+    x[:M] = torch.randn(M, K).bfloat16().cuda()
+    w, s = quantize_fp8_block(torch.randn(N, K, device="cuda") * 0.05, (64, 128))
+    kw = dict(epi=ref.EPI_SILU_MUL) if epi == "glu" else {}
+    want, got = ref.linear_fp8(x[:M], w, s, **kw), cu.linear_fp8(x[:M], w, s, **kw)
+    cu.check_status(torch.device("cuda", 0))
+    assert float((got.float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("M", [5, 8, 61, 120, 128])
+def test_gated_bf16_product_of_part_of_a_tile(M):
+    """The same for bf16 gate / up products, whose rows stay in the first operand's place."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(M)
+    x = torch.full((136, 512), float("nan")).bfloat16().cuda()
+    x[:M] = torch.randn(M, 512).bfloat16().cuda()
+    w = (torch.randn(38400, 512) * 0.05).bfloat16().cuda()
+    y = x[:M].float() @ w.float().t()
+    y = y.view(M, -1, 2, 64)
+    want = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(M, -1)
+    got = cu.linear(x[:M], w, epi=ref.EPI_SILU_MUL)
+    cu.check_status(torch.device("cuda", 0))
+    assert float((got.float() - want).norm() / want.norm()) < 2 ** -8
