@@ -1273,10 +1273,11 @@ int gemm_small_m(const void* A, const void* W, void* C, bool f32_out, const void
       while (c > 1 && small_m_max_clusters(bn_tok, c) < tiles) --c;
     }
     const bool launchable = small_m_max_clusters(bn_tok, c) > 0;
-    // few tiles and a long K: more K ranges than a cluster holds put more SMs to work - but the CTA that finishes a tile
-    // then adds all of its slabs alone, which for one or two tiles (routers, gates) takes longer than it saves
-    const bool prefer_scratch = auto_split && splitk > c && tiles > 2 && tiles * c * 2 < pxl_host::num_sms();
-    if (launchable && (mode == 2 || !prefer_scratch)) {
+    // (More K ranges than a cluster holds would put more SMs to work where there are few tiles, but the CTA that finishes a tile
+    // adds all of its slabs alone: 576 x 7168 takes 12.4 / 32.5 / 58.1 us for 8 / 64 / 128 rows with 28 ranges and 7.3 / 8.5 / 11.2
+    // with a cluster of eight. Up to 18432 wide no shape of 128 to 1536 columns was faster with slabs: they are for devices or
+    // contexts that do not take the cluster.)
+    if (launchable) {
       splitk = c;
       mode = 2;
     } else if (mode == 2) {
