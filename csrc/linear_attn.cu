@@ -47,6 +47,50 @@ __global__ void __launch_bounds__(128) conv1d_silu_kernel(const bf16* __restrict
   for (int j = 0; j < K - 1; ++j) st[j] = __float2bfloat16(win[j]);
 }
 
+// The same for windows of three (K = 4) and a pair of channels per thread: 12 bytes of window, 16 of weights and 4 of input are
+// three independent vector loads, and the loops are known, so that nothing is kept in local memory. One token of 96 sequences x
+// 8192 channels: 12.1 -> 5.5 us.
+__global__ void __launch_bounds__(128) conv1d_silu_pair_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ w,
+                                                               const bf16* __restrict__ bias, bf16* __restrict__ conv_state,
+                                                               const int* __restrict__ seq_cu, const int* __restrict__ seq_slots,
+                                                               const int* __restrict__ positions, bf16* __restrict__ out, int64_t ldo,
+                                                               int C) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 2, b = blockIdx.y;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (c >= C) return;
+  const int t0 = seq_cu[b], t1 = seq_cu[b + 1];
+  if (t1 <= t0) return;
+  const bool fresh = positions[t0] == 0;
+  uint32_t* st = reinterpret_cast<uint32_t*>(conv_state + (static_cast<size_t>(seq_slots[b]) * C + c) * 3);
+  const uint4 wr = *reinterpret_cast<const uint4*>(w + static_cast<size_t>(c) * 4);
+  const uint32_t br = bias ? *reinterpret_cast<const uint32_t*>(bias + c) : 0u;
+  uint32_t sr[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) sr[j] = fresh ? 0u : st[j];
+  const float2 w0 = unpack_bf16x2(wr.x), w1 = unpack_bf16x2(wr.y), w2 = unpack_bf16x2(wr.z), w3 = unpack_bf16x2(wr.w);
+  const float wk[2][4] = {{w0.x, w0.y, w1.x, w1.y}, {w2.x, w2.y, w3.x, w3.y}};
+  const float2 bs = unpack_bf16x2(br), s0 = unpack_bf16x2(sr[0]), s1 = unpack_bf16x2(sr[1]), s2 = unpack_bf16x2(sr[2]);
+  float win[2][3] = {{s0.x, s0.y, s1.x}, {s1.y, s2.x, s2.y}};  // oldest first
+  for (int t = t0; t < t1; ++t) {
+    const float2 in = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(x + t * ldx + c));
+    float y[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float xin = e ? in.y : in.x;
+      float acc = (e ? bs.y : bs.x) + wk[e][3] * xin;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc += wk[e][j] * win[e][j];
+      win[e][0] = win[e][1], win[e][1] = win[e][2], win[e][2] = xin;
+      y[e] = acc / (1.f + __expf(-acc));
+    }
+    *reinterpret_cast<uint32_t*>(out + t * ldo + c) = pack_bf16x2(y[0], y[1]);
+  }
+  st[0] = pack_bf16x2(win[0][0], win[0][1]);
+  st[1] = pack_bf16x2(win[0][2], win[1][0]);
+  st[2] = pack_bf16x2(win[1][1], win[1][2]);
+}
+
 // Prompts: a thread walks a run of tokens of 8 channels, weights and last inputs in registers, inputs four tokens ahead. The
 // walk of a whole sequence by one thread (above) is a chain of as many loads as it has tokens (2.0 ms for 5900 tokens x 8192
 // channels); runs make it a streaming pass (57 us, 3.4 TB/s read and written). The slots are rewritten by a launch of its own, because the first tokens of a
@@ -250,9 +294,18 @@ PXL_EXPORT int pxl_causal_conv1d_silu(const void* x_, int64_t ldx, const void* w
   if (prefill_seqs > 0 && prefill_tokens > 0 &&
       launch_conv_run(x, ldx, w, bias, conv_state, seq_cu, seq_slots, positions, out, ldo, C, K, prefill_seqs, prefill_tokens, stream))
     done = prefill_seqs;
-  if (done < B)
-    pxl_host::launch(conv1d_silu_kernel, dim3(pxl::ceil_div(C, 128), B - done), 128, 0, stream, x, ldx, w, bias, conv_state, seq_cu + done,
-                                                                                 seq_slots + done, positions, out, ldo, C, K);
+  if (done < B) {
+    // pairs of channels where rows and the tables start on the bytes that they take
+    const bool pairs = K == 4 && C % 2 == 0 && ldx % 2 == 0 && ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
+                       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(conv_state) |
+                         reinterpret_cast<uintptr_t>(out)) & 3) == 0;
+    if (pairs)
+      pxl_host::launch(conv1d_silu_pair_kernel, dim3(pxl::ceil_div(C, 256), B - done), 128, 0, stream, x, ldx, w, bias, conv_state,
+                       seq_cu + done, seq_slots + done, positions, out, ldo, C);
+    else
+      pxl_host::launch(conv1d_silu_kernel, dim3(pxl::ceil_div(C, 128), B - done), 128, 0, stream, x, ldx, w, bias, conv_state,
+                       seq_cu + done, seq_slots + done, positions, out, ldo, C, K);
+  }
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
