@@ -206,6 +206,7 @@ int pxl_moe_route(const void* logits, int64_t ld, int logits_bf16, const float* 
                   int mode, int renorm, int n_group, int topk_group, int group_top, float routed_scale,
                   int* out_ids, float* out_w, pxl_stream_t stream);
 
+int pxl_moe_align_alone(int T, int k);  // non-zero: pxl_moe_align needs no zeros in `counts` for this many pairs
 int pxl_moe_align(const int* ids, int T, int k, int E, int e_lo, int e_hi, int* counts,
                   int* offsets, int* cursor, int* mt_expert, int* mt_row0, int* mt_row_end,
                   int* num_mt, int max_mt, int* pos_of, int* src_tok, pxl_stream_t stream);

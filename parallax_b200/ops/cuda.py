@@ -653,7 +653,9 @@ def moe_align(ids: torch.Tensor, num_experts: int, e_lo: int = 0, e_hi: Optional
     dev = ids.device
     max_rows = T * k
     max_mt = (max_rows + 127) // 128 + n_local
-    ints = torch.zeros(n_local * 2 + (n_local + 1) + 3 * max_mt + 1 + 2 * max_rows, dtype=torch.int32, device=dev)
+    alone = _lib.lib().pxl_moe_align_alone(T, k)      # one kernel, whose counters need no zeros
+    ints = (torch.empty if alone else torch.zeros)(n_local * 2 + (n_local + 1) + 3 * max_mt + 1 + 2 * max_rows, dtype=torch.int32,
+                                                   device=dev)
     o = 0
 
     def take(n):
@@ -671,7 +673,7 @@ def moe_align(ids: torch.Tensor, num_experts: int, e_lo: int = 0, e_hi: Optional
                                    offsets.data_ptr(), cursor.data_ptr(), p.mt_expert.data_ptr(),
                                    p.mt_row0.data_ptr(), p.mt_row_end.data_ptr(), p.num_mt.data_ptr(), max_mt,
                                    p.pos_of.data_ptr(), p.src_tok.data_ptr(), _stream(dev)), "pxl_moe_align")
-    _count(4)
+    _count(1 if alone else 3)
     return p
 
 

@@ -163,3 +163,29 @@ def test_routed_experts_record_on_gpu():
     from parallax_b200.ops import cuda as cu
 
     cu.check_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("T,k,E,lo,hi", [(1, 1, 1, 0, 1), (48, 8, 128, 0, 128), (1023, 8, 128, 32, 64), (1024, 8, 1024, 0, 1024),
+                                         (1025, 8, 1000, 0, 1000), (700, 4, 60, 0, 60)])
+def test_expert_order_of_the_pairs(T, k, E, lo, hi):
+    """Both forms (one block; three launches for more than 8192 pairs), some ids out of range, one expert with many rows."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(T + E)
+    ids = torch.randint(-1, E + 1, (T, k), dtype=torch.int32)
+    ids[T // 2:, 0] = lo
+    p = cu.moe_align(ids.cuda(), E, lo, hi)
+    flat, pos = ids.flatten().long(), p.pos_of.cpu().long()
+    mine = (flat >= lo) & (flat < hi)
+    counts = torch.bincount(flat[mine] - lo, minlength=hi - lo)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    assert torch.equal(p.offsets.cpu().long(), offsets)
+    assert torch.equal(pos >= 0, mine)
+    assert torch.equal(pos[mine].sort().values, torch.arange(int(mine.sum())))      # every row once
+    e = flat[mine] - lo
+    assert ((pos[mine] >= offsets[e]) & (pos[mine] < offsets[e + 1])).all()
+    assert torch.equal(p.src_tok.cpu().long()[pos[mine]], torch.arange(T * k)[mine] // k)
+    tiles = [(x, int(offsets[x]) + i, int(offsets[x + 1])) for x in range(hi - lo) for i in range(0, int(counts[x]), 128)]
+    n = int(p.num_mt)
+    assert n == len(tiles)
+    assert [tuple(t) for t in torch.stack([p.mt_expert[:n], p.mt_row0[:n], p.mt_row_end[:n]], 1).cpu().tolist()] == tiles
