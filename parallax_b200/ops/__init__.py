@@ -32,15 +32,24 @@ def _first_tensor(args, kwargs):
     raise TypeError("op called without tensor arguments")
 
 
+_cuda = None      # the module of the kernels' wrappers, once an op was called with tensors on a device
+
+
+def _load_cuda():
+    global _cuda
+    from . import cuda
+
+    _cuda = cuda
+    return cuda
+
+
 def _make(name):
     ref_fn = getattr(reference, name)
 
     def op(*args, **kwargs):
-        t = _first_tensor(args, kwargs)
+        t = args[0] if args and isinstance(args[0], torch.Tensor) else _first_tensor(args, kwargs)
         if t.is_cuda:
-            from . import cuda
-
-            return getattr(cuda, name)(*args, **kwargs)
+            return getattr(_cuda or _load_cuda(), name)(*args, **kwargs)
         return ref_fn(*args, **kwargs)
 
     op.__name__ = name
