@@ -29,8 +29,9 @@ __device__ __forceinline__ uint64_t widen(uint32_t two) {  // two bf16 -> two fp
 }
 
 // MM rows of A (the last ones repeated where M is smaller), R rows of W per warp, U steps of 256 columns in flight.
+// ONE: K fits one round of U steps, and the rows are held in registers.
 // EPI: PXL_EPI_NONE, _RESIDUAL, _F32 or _SILU_MUL (R rows = R / 2 gate / up pairs, 64 rows apart in groups of 128)
-template <int MM, int R, int U, int EPI, bool NORM>
+template <int MM, int R, int U, int EPI, bool NORM, bool ONE>
 __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
   constexpr bool kGlu = EPI == PXL_EPI_SILU_MUL;
   const int lane = threadIdx.x & 31, wid = blockIdx.x * kWarps + (threadIdx.x >> 5);
@@ -53,22 +54,61 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
     }
   };
   load(0);
+  // What no kernel of the chain writes goes out ahead of the wait, what the kernel before wrote right behind it and all at once: in a
+  // chain of small layers the products are a handful of load latencies one after the other.
+  uint4 nw[NORM ? U : 1];
+  if constexpr (NORM) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = u * 256 + lane * 8;
+      nw[u] = k < a.K ? *reinterpret_cast<const uint4*>(a.norm_w + k) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  constexpr int V = MM * R, kSpan = 32 / V;  // number i of the results ends in lanes [i * kSpan, (i + 1) * kSpan)
+  const int oi = lane / kSpan, om = oi / R, orow = oi % R;
+  const bool stores = lane % kSpan == 0 && om < a.M && !(kGlu && (orow & 1));
+  const int col = kGlu ? (n0 + orow) / 2 : n0 + orow;
+  const int64_t at = static_cast<int64_t>(om) * a.ldc + col;
+  float add_bias = 0.f, add_res = 0.f;
+  constexpr bool kEarly = V <= 8;  // (registers)
+  if (kEarly && !kGlu && stores && a.bias) add_bias = __bfloat162float(a.bias[col]);
   pdl_wait();
   pdl_launch_dependents();
+  const bf16* rows_a[MM];
+#pragma unroll
+  for (int m = 0; m < MM; ++m) rows_a[m] = a.A + static_cast<int64_t>(m < a.M ? m : a.M - 1) * a.lda;
+  constexpr bool kHeld = ONE && MM == 1;  // (more rows would not fit the registers)
+  uint4 held[kHeld ? U : 1];
+  if constexpr (kHeld) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = u * 256 + lane * 8;
+      held[u] = k < a.K ? *reinterpret_cast<const uint4*>(rows_a[0] + k) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  if constexpr (EPI == PXL_EPI_RESIDUAL && kEarly) {
+    if (stores) add_res = __bfloat162float(a.residual[at]);
+  }
   float inv[MM];
   if constexpr (NORM) {
 #pragma unroll
     for (int m = 0; m < MM; ++m) {
-      const bf16* x = a.A + static_cast<int64_t>(m < a.M ? m : a.M - 1) * a.lda;
       float ss = 0.f;
-      for (int k = lane * 8; k < a.K; k += 256) {
-        const bf16x8 v = ld_bf16x8(x + k);
+      auto squares = [&](const uint4& v) {
+        const uint32_t* p = &v.x;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float2 f = unpack_bf16x2(v.u[j]);
+          const float2 f = unpack_bf16x2(p[j]);
           ss += f.x * f.x + f.y * f.y;
         }
+      };
+      int k = lane * 8;
+      if constexpr (kHeld) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) squares(held[u]);
+        k += U * 256;
       }
+      for (; k < a.K; k += 256) squares(*reinterpret_cast<const uint4*>(rows_a[m] + k));
       inv[m] = rsqrtf(warp_reduce_sum(ss) / static_cast<float>(a.K) + a.norm_eps);
     }
   }
@@ -84,13 +124,14 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
         wv[r][0] = widen(w[u][r].x), wv[r][1] = widen(w[u][r].y), wv[r][2] = widen(w[u][r].z), wv[r][3] = widen(w[u][r].w);
 #pragma unroll
       for (int m = 0; m < MM; ++m) {
-        uint4 xr = *reinterpret_cast<const uint4*>(a.A + static_cast<int64_t>(m < a.M ? m : a.M - 1) * a.lda + k);
+        uint4 xr = kHeld && k0 == 0 ? held[kHeld ? u : 0] : *reinterpret_cast<const uint4*>(rows_a[m] + k);
         if constexpr (NORM) {
-          const bf16x8 nw = ld_bf16x8(a.norm_w + k);
+          const uint4 nv = k0 == 0 ? nw[u] : *reinterpret_cast<const uint4*>(a.norm_w + k);
+          const uint32_t* nx = &nv.x;
           uint32_t* xw = &xr.x;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const float2 f = unpack_bf16x2(xw[j]), g = unpack_bf16x2(nw.u[j]);
+            const float2 f = unpack_bf16x2(xw[j]), g = unpack_bf16x2(nx[j]);
             xw[j] = pack_bf16x2(f.x * inv[m] * (g.x + a.norm_offset), f.y * inv[m] * (g.y + a.norm_offset));
           }
         }
@@ -101,10 +142,10 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
           for (int j = 0; j < 4; ++j) acc[m][r] = fma2(wv[r][j], x[j], acc[m][r]);
       }
     }
+    if (ONE) break;
     if (k0 + U * 256 < a.K) load(k0 + U * 256);
   }
   // sums over the lanes: every exchange halves the numbers a lane holds, lanes V = MM * R apart end with the same one
-  constexpr int V = MM * R;
   float v[V];
 #pragma unroll
   for (int m = 0; m < MM; ++m)
@@ -122,28 +163,27 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
   }
 #pragma unroll
   for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-  constexpr int kSpan = 32 / V;  // number i is in lanes [i * kSpan, (i + 1) * kSpan)
-  const int i = lane / kSpan, m = i / R, r = i % R;
   float sum = v[0];
-  int col = n0 + r;
   if constexpr (kGlu) {  // the up product sits kSpan lanes further
     const float up = __shfl_down_sync(0xffffffffu, sum, kSpan);
     sum = sum / (1.f + __expf(-sum)) * up;
-    col = (n0 + r) / 2;
   }
-  if (lane % kSpan || m >= a.M || (kGlu && (r & 1))) return;
-  if (!kGlu && a.bias) sum += __bfloat162float(a.bias[col]);
-  const int64_t at = static_cast<int64_t>(m) * a.ldc + col;
+  if (!stores) return;
+  if constexpr (!kEarly) {
+    if (!kGlu && a.bias) add_bias = __bfloat162float(a.bias[col]);
+    if constexpr (EPI == PXL_EPI_RESIDUAL) add_res = __bfloat162float(a.residual[at]);
+  }
+  sum += add_bias;
   if constexpr (EPI == PXL_EPI_F32) {
     static_cast<float*>(a.C)[at] = sum;
   } else {
-    if constexpr (EPI == PXL_EPI_RESIDUAL) sum += __bfloat162float(a.residual[at]);
+    if constexpr (EPI == PXL_EPI_RESIDUAL) sum += add_res;
     static_cast<bf16*>(a.C)[at] = __float2bfloat16(sum);
   }
 }
 
-template <int MM, int R, int U>
-int launch_epi(const GemvArgs& a, int epi, cudaStream_t stream) {
+template <int MM, int R, int U, bool ONE>
+int launch_one(const GemvArgs& a, int epi, cudaStream_t stream) {
   const dim3 grid(ceil_div(ceil_div(a.N, R), kWarps)), block(kWarps * 32);
   auto go = [&](auto kern) {
     pxl_host::launch(kern, grid, block, 0, stream, a);
@@ -151,20 +191,25 @@ int launch_epi(const GemvArgs& a, int epi, cudaStream_t stream) {
   };
   if (a.norm_w) {
     if constexpr (MM <= PXL_GEMV_NORM_MAX_M) {
-      if (epi == PXL_EPI_NONE) return go(gemv_kernel<MM, R, U, PXL_EPI_NONE, true>);
+      if (epi == PXL_EPI_NONE) return go(gemv_kernel<MM, R, U, PXL_EPI_NONE, true, ONE>);
       if constexpr (R > 1)
-        if (epi == PXL_EPI_SILU_MUL) return go(gemv_kernel<MM, R, U, PXL_EPI_SILU_MUL, true>);
+        if (epi == PXL_EPI_SILU_MUL) return go(gemv_kernel<MM, R, U, PXL_EPI_SILU_MUL, true, ONE>);
     }
     return PXL_ERR_INVALID_ARG;
   }
   switch (epi) {
-    case PXL_EPI_NONE: return go(gemv_kernel<MM, R, U, PXL_EPI_NONE, false>);
-    case PXL_EPI_RESIDUAL: return go(gemv_kernel<MM, R, U, PXL_EPI_RESIDUAL, false>);
-    case PXL_EPI_F32: return go(gemv_kernel<MM, R, U, PXL_EPI_F32, false>);
+    case PXL_EPI_NONE: return go(gemv_kernel<MM, R, U, PXL_EPI_NONE, false, ONE>);
+    case PXL_EPI_RESIDUAL: return go(gemv_kernel<MM, R, U, PXL_EPI_RESIDUAL, false, ONE>);
+    case PXL_EPI_F32: return go(gemv_kernel<MM, R, U, PXL_EPI_F32, false, ONE>);
     case PXL_EPI_SILU_MUL:
-      if constexpr (R > 1) return go(gemv_kernel<MM, R, U, PXL_EPI_SILU_MUL, false>);
+      if constexpr (R > 1) return go(gemv_kernel<MM, R, U, PXL_EPI_SILU_MUL, false, ONE>);
     default: return PXL_ERR_INVALID_ARG;
   }
+}
+
+template <int MM, int R, int U>
+int launch_epi(const GemvArgs& a, int epi, cudaStream_t stream) {
+  return MM == 1 && a.K <= U * 256 ? launch_one<MM, R, U, MM == 1>(a, epi, stream) : launch_one<MM, R, U, false>(a, epi, stream);
 }
 
 template <int MM>
@@ -173,6 +218,8 @@ int launch_rows(const GemvArgs& a, int epi, cudaStream_t stream) {
   const int want = 12 * pxl_host::num_sms();
   if (a.N >= 4 * want) return launch_epi<MM, 4, 2>(a, epi, stream);
   if (a.N >= 2 * want || epi == PXL_EPI_SILU_MUL) return launch_epi<MM, 2, 4>(a, epi, stream);
+  // one row of W: the whole of it in flight up to K = 3072
+  if (MM == 1 && a.K > 2048 && a.K <= 3072) return launch_epi<MM, 1, 12>(a, epi, stream);
   return launch_epi<MM, 1, 8>(a, epi, stream);
 }
 
