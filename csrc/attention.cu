@@ -1242,15 +1242,44 @@ int set_smem(K kern, int bytes) {
 
 }  // namespace
 
-PXL_EXPORT int pxl_attn_decode_splits(int B, int Hkv, int max_ctx) {
-  const int blocks = B * Hkv;
-  const int target = 2 * pxl_host::num_sms();
-  int s = blocks >= target ? 1 : pxl::ceil_div(target, blocks);
-  const int max_by_ctx = pxl::ceil_div(max_ctx > 0 ? max_ctx : 1, 256);
-  if (s > max_by_ctx) s = max_by_ctx;
-  if (s > 64) s = 64;
-  if (s < 1) s = 1;
-  return s;
+// Splits of a decode step: the count with the lowest estimate, us = (tiles of the longest split + start) x waves of CTAs + adding.
+// A last wave of few CTAs costs nearly as much as a full one, which ceil(2 SMs / CTAs), the rule before, did not see.
+//
+// Pages the TMA unit reads (head dim 128): 2 CTAs per SM; a tile of 64 keys takes 1.2 us while the memory is not full and 1.4 us
+// beside a full chip of others, start and end about one tile's time. Adding costs 1.3 us inside a cluster; through the workspace 1.5,
+// 0.1 per split and 2 per wave of partial results. Over 26 sizes of 1 to 150 rows and 100 to 100000 keys, bf16 and e4m3, the count is
+// the fastest measured or within 2 % (8 key heads, splits: us):
+//   rows x keys   before   now             rows x keys   before   now
+//   1 x 777       4:  8.1  7:  6.7         36 x 1280     2: 37.1  1:  31.9
+//   8 x 2100      5: 21.0  4: 16.7         40 x 4000     1: 136   4: 110
+//   16 x 1280     3: 24.6  2: 18.1         20 x 8192     2: 144   5: 105
+// The kernel for other pages and head dim 64: 5 CTAs per SM (3 at 128), 1.0 us per tile either way, through the workspace 1 + 0.03 per
+// split and 1 per 296 CTAs (head dim 64): 16 x 1280 3: 18.3, 5: 16.3; 40 x 4000 1: 118, 2: 80.1; 36 x 1280 2: 26.3 both.
+PXL_EXPORT int pxl_attn_decode_splits(int B, int Hkv, int D, int page_size, int max_ctx) {
+  const bool tma = D == 128 && (page_size == 16 || page_size == 32 || page_size == 64);
+  const int64_t pairs = static_cast<int64_t>(B) * Hkv;
+  const int slots = (tma ? 2 : D == 64 ? 5 : 3) * pxl_host::num_sms();
+  const int tiles = pxl::ceil_div(max_ctx > 0 ? max_ctx : 1, TILE);
+  int best = 1, last = 0;
+  float best_us = 0.f;
+  for (int s = 1; s <= 64 && s <= tiles; ++s) {
+    const int per = pxl::ceil_div(tiles, s);
+    if (per == last) continue;  // no fewer tiles for the longest split
+    last = per;
+    const int64_t ctas = pairs * s, full = ctas / slots, rest = ctas % slots;
+    const float waves = static_cast<float>(ctas) / (2 * pxl_host::num_sms());
+    float us;
+    if (tma) {
+      const float part = static_cast<float>(rest) / slots;
+      us = static_cast<float>(per + 1) * (1.4f * static_cast<float>(full) + (rest ? fmaxf(1.2f, 1.4f * part) : 0.f));
+      if (s > 1) us += s <= kMaxClusterSplits && waves <= 0.9375f ? 1.3f : 1.5f + 0.1f * s + 2.f * waves;
+    } else {
+      us = static_cast<float>(per) * static_cast<float>(full + (rest ? 1 : 0));
+      if (s > 1) us += 1.f + 0.03f * s + waves;
+    }
+    if (s == 1 || us < best_us) best = s, best_us = us;
+  }
+  return best;
 }
 
 namespace {
@@ -1333,7 +1362,7 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
   const ScoreArgs sa = score_args(scale, softcap, sig_bias);
   if (cache_fp8 && mode != kPlain) return PXL_ERR_INVALID_ARG;
   if (Hkv <= 0 || Hq % Hkv || Hq / Hkv > 16 || page_size <= 0) return PXL_ERR_INVALID_ARG;
-  if (num_splits <= 0) num_splits = pxl_attn_decode_splits(B, Hkv, max_ctx);
+  if (num_splits <= 0) num_splits = pxl_attn_decode_splits(B, Hkv, D, page_size, max_ctx);
   if (num_splits > 1 && workspace == nullptr) return PXL_ERR_INVALID_ARG;
   const float scale_log2 = scale * kLog2e;
   dim3 grid(Hkv, B, num_splits);

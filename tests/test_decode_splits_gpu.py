@@ -33,3 +33,25 @@ def test_splits(B, splits, kernels, fp8, kw):
     want = ref.attn_decode(q, k, v, table, ctx, D ** -0.5, **kw)
     # probabilities and outputs are rounded to bf16 (2^-9 each)
     assert float((got.cpu().float() - want.float()).norm() / want.float().norm()) < 2 ** -7
+
+
+@pytest.mark.parametrize("D,page", [(128, 16), (128, 8), (64, 16)])
+@pytest.mark.parametrize("B,most", [(1, 64), (1, 65), (1, 777), (9, 129), (75, 640)])
+def test_chosen_splits(D, page, B, most):
+    from parallax_b200.ops import _lib
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(B + most)
+    Hq, Hkv, blocks = 8, 2, -(-most // page)
+    s = _lib.lib().pxl_attn_decode_splits(B, Hkv, D, page, most)
+    tiles = -(-most // 64)
+    assert 1 <= s <= min(64, tiles) and (s == 1 or -(-tiles // s) < -(-tiles // (s - 1)))
+    ctx = torch.tensor([most - 41 * i % most for i in range(B)]).int()
+    table = torch.randperm(B * blocks).int().view(B, blocks)
+    k, v = (torch.randn(B * blocks, Hkv, page, D).bfloat16() for _ in range(2))
+    q = torch.randn(B, Hq, D).bfloat16()
+    got = cu.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), ctx.cuda(), D ** -0.5, max_ctx=most)
+    cu.check_status(torch.device("cuda", 0))
+    want = ref.attn_decode(q, k, v, table, ctx, D ** -0.5)
+    # probabilities and outputs are rounded to bf16 (2^-9 each)
+    assert float((got.cpu().float() - want.float()).norm() / want.float().norm()) < 2 ** -7
