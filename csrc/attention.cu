@@ -426,6 +426,41 @@ __device__ __forceinline__ void add_splits(const float* part_o, const float* par
   cluster_sync_all();  // nobody leaves while its parts are being read
 }
 
+// Producer warp: the blocks of the pages of 32 / (pages per tile) tiles at a time, one per lane, the next ones read while these are
+// used. Read tile by tile, the latency of a table read was the time of a tile: 1.2 us (e4m3 0.7) with one CTA per SM, whatever the
+// consumers did.
+struct TileBlocks {
+  const int* bt;
+  KeyTiles tiles;
+  int t_begin, n_tiles, page_size, shift, hi, max_blocks;  // shift: log2(pages per tile)
+  int64_t num_blocks;
+  int* status;
+  int now = 0, ahead = 0;
+
+  __device__ __forceinline__ int look(int it) const {
+    const int lane = threadIdx.x & 31;
+    it += lane >> shift;
+    if (it >= n_tiles) return 0;
+    int bi = (tiles[t_begin + it] << shift) + (lane & ((1 << shift) - 1));
+    if (bi * page_size >= hi) bi = (hi - 1) / page_size;  // beyond the context: re-read the last page (masked)
+    return bi < max_blocks ? bt[bi] : -1;
+  }
+  __device__ __forceinline__ void begin() { ahead = look(0); }
+  // block of page lane % ppt of tile `it`; called by the whole warp, tile after tile
+  __device__ __forceinline__ int operator()(int it) {
+    const int per = 32 >> shift, i = it & (per - 1);
+    if (i == 0) {
+      now = ahead;
+      ahead = look(it + per);  // not looked at before it is needed
+      if (now < 0 || now >= num_blocks) {
+        if (status) atomicCAS(status, 0, PXL_DEV_BAD_BLOCK_DECODE);
+        now = 0;
+      }
+    }
+    return __shfl_sync(0xffffffffu, now, (i << shift) + (threadIdx.x & ((1 << shift) - 1)));
+  }
+};
+
 constexpr int kDecStages = 3;
 constexpr int kDecThreads = 160;  // 4 consumer warps + 1 producer warp
 
@@ -447,9 +482,6 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kDecStages);
   const uint32_t full0 = smem_u32(bars);
   const uint32_t empty0 = smem_u32(bars + kDecStages);
-  pdl_wait();
-  pdl_launch_dependents();
-
   const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int G = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -462,7 +494,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   const int t_end = min(tiles.total, t_begin + per_split);
   const int n_tiles = t_end > t_begin ? t_end - t_begin : 0;
   const int* bt = block_tables + static_cast<size_t>(b) * max_blocks;
-  const int ppt = TILE / page_size;  // pages per tile
+  const int shift = page_size == 16 ? 2 : page_size == 32 ? 1 : 0, ppt = 1 << shift;  // pages per tile
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -475,25 +507,19 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
   }
+  // the tables and the lengths of a step are there before its first kernel, the queries and the new keys after the wait
+  TileBlocks blocks{bt, tiles, t_begin, n_tiles, page_size, shift, hi, max_blocks, num_blocks, status};
+  if (warp == 4) blocks.begin();
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
 
   int failed = 0;
   if (warp == 4) {
-    // ---- producer warp, up to kDecStages tiles ahead of the consumers. Lane p looks up the block of
-    // page p of the tile and issues that page's four box loads: the block-table reads of a tile are in
-    // flight together and are issued before the wait for the stage.
+    // ---- producer warp, up to kDecStages tiles ahead of the consumers. Lane p issues the four box loads of page p of the tile.
     for (int it = 0; it < n_tiles; ++it) {
       const int stage = it % kDecStages;
-      int blk = 0;
-      if (lane < ppt) {
-        int bi = tiles[t_begin + it] * ppt + lane;
-        if (bi * page_size >= hi) bi = (hi - 1) / page_size;  // beyond the context: re-read the last page (masked)
-        blk = bi < max_blocks ? bt[bi] : -1;
-        if (blk < 0 || blk >= num_blocks) {
-          if (status) atomicCAS(status, 0, PXL_DEV_BAD_BLOCK_DECODE);
-          blk = 0;
-        }
-      }
+      const int blk = blocks(it);
       int okf = 1;
       if (it >= kDecStages && lane == 0)
         okf = mbar_wait_bounded(empty0 + 8 * stage, ((it / kDecStages) - 1) & 1, abort_flag, status,
@@ -702,7 +728,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 // The pages stay bytes up to the fragments: a tile of 64 tokens is 8 KB of K and 8 KB of V (one 128-byte swizzled row per
 // token), so the same shared memory holds twice the tiles of the kernel above, and an operand is converted once, by the thread
 // that multiplies it. Widening 8 bytes at a time into shared memory on the way in (the kernel without TMA) took 1170 us for 128
-// rows x 3600 keys x 8 heads, 0.8 TB/s, bound by issue; this one takes 224 us, 4.2 TB/s.
+// rows x 3600 keys x 8 heads, 0.8 TB/s, bound by issue. One full wave (37 rows x 4096 keys x 8 heads) takes 52 us, 6.0 TB/s; 64 us
+// when the block table was read tile by tile (TileBlocks) and each warp took 16 tokens of every tile, two chains of dependent
+// products, one softmax and twice the shuffles, instead of 32 of every other one. Rows 8 to 15 of the products are nobody's with up
+// to 8 query heads per key head: HIGH = false leaves their softmax out.
 //
 // e4m3 becomes f16 with one instruction per two values, exactly, and the products are f16 ones. What the other operands lose in
 // range against bf16 they make up for in mantissa: a row of q is scaled by a power of two that puts its largest value at 2^13
@@ -735,7 +764,7 @@ __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-template <bool CLUSTER>
+template <bool CLUSTER, bool HIGH>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                         const bf16* __restrict__ q, int64_t q_stride, const int* __restrict__ block_tables,
@@ -749,9 +778,6 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kE4Stages * 2 * kE4Tile);  // full[S], empty[S]
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kE4Stages);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kE4Stages);
-  pdl_wait();
-  pdl_launch_dependents();
-
   const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int G = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -763,35 +789,31 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   const int t_end = min(tiles.total, t_begin + per_split);
   const int n_tiles = t_end > t_begin ? t_end - t_begin : 0;
   const int* bt = block_tables + static_cast<size_t>(b) * max_blocks;
-  const int ppt = TILE / page_size;  // pages per tile
+  const int shift = page_size == 16 ? 2 : page_size == 32 ? 1 : 0, ppt = 1 << shift;  // pages per tile
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < kE4Stages; ++s) {
       mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 4);  // one arrival per consumer warp
+      mbar_init(empty0 + 8 * s, 2);  // one arrival per consumer warp
     }
     mbar_fence_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
   }
+  // the tables and the lengths of a step are there before its first kernel, the queries and the new keys after the wait
+  TileBlocks blocks{bt, tiles, t_begin, n_tiles, page_size, shift, hi, max_blocks, num_blocks, status};
+  if (warp == 4) blocks.begin();
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
 
   int failed = 0;
-  if (warp == 4) {  // producer: lane p looks up the block of page p of the tile and issues its two boxes
+  if (warp == 4) {  // producer: lane p issues the two boxes of page p of the tile
     for (int it = 0; it < n_tiles; ++it) {
       const int stage = it % kE4Stages;
-      int blk = 0;
-      if (lane < ppt) {
-        int bi = tiles[t_begin + it] * ppt + lane;
-        if (bi * page_size >= hi) bi = (hi - 1) / page_size;  // beyond the context: re-read the last page (masked)
-        blk = bi < max_blocks ? bt[bi] : -1;
-        if (blk < 0 || blk >= num_blocks) {
-          if (status) atomicCAS(status, 0, PXL_DEV_BAD_BLOCK_DECODE);
-          blk = 0;
-        }
-      }
+      const int blk = blocks(it);
       int okf = 1;
       if (it >= kE4Stages && lane == 0)
         okf = mbar_wait_bounded(empty0 + 8 * stage, ((it / kE4Stages) - 1) & 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY) ? 1 : 0;
@@ -819,7 +841,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   for (int h = 0; h < 2; ++h) {
     const int r = g8 + h * 8;
     float mx = 0.f;
-    if (r < G) {
+    if ((HIGH || h == 0) && r < G) {
       const bf16* row = q + static_cast<size_t>(b) * q_stride + (kvh * G + r) * D + t4 * 32;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
@@ -832,6 +854,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) qf[ks][h] = qf[ks][2 + h] = 0u;
     }
+    if (!HIGH && h == 1) break;
     mx = quad_max(mx);
     int up = 267 - static_cast<int>(__float_as_uint(mx) >> 23);  // exponent bits of the factor: the largest value to [2^13, 2^14)
     up = up < 1 ? 1 : up > 253 ? 253 : up;
@@ -851,97 +874,103 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   float m_run[2] = {-INFINITY, -INFINITY};
   float l_run[2] = {0.f, 0.f};
 
-  for (int it = 0; warp < 4 && it < n_tiles; ++it) {
+  // Warps 0 and 1 take the even tiles, 2 and 3 the odd ones, 32 tokens each. A stage has to belong to one pair (an even number of
+  // them): another pair that is a use ahead would take the parity of the use before last for its own.
+  static_assert(kE4Stages % 2 == 0);
+  constexpr int kRows = HIGH ? 2 : 1, kKeys = 32;  // kRows: of this thread, g8 and g8 + 8
+  for (int it = warp >> 1; warp < 4 && it < n_tiles; it += 2) {
     const int stage = it % kE4Stages;
     if (!mbar_wait_bounded(full0 + 8 * stage, (it / kE4Stages) & 1, abort_flag, status, PXL_DEV_TIMEOUT_FULL)) {
       failed = 1;
       break;  // reported to the whole CTA at the barrier behind the loop
     }
     const uint32_t k_smem = stage0 + stage * 2 * kE4Tile, v_smem = k_smem + kE4Tile;
-    const int r0 = warp * 16;
+    const int r0 = (warp & 1) * kKeys;
     const int tok_base = tiles[t_begin + it] * TILE + r0;
-    if (tok_base < hi && (tok_base + 16 > lo || tok_base < keep)) {  // warp-uniform
-      float s[2][4];
+    if (tok_base < hi && (tok_base + kKeys > lo || tok_base < keep)) {  // warp-uniform
+      float s[kKeys / 8][4];  // 8 tokens each
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {  // 8 tokens each
-        s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-        const int row = r0 + j * 8 + g8;
+      for (int j = 0; j < kKeys / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t w[4];
+      for (int c = 0; c < 2; ++c) {
+        uint32_t w[kKeys / 8][4];
+#pragma unroll
+        for (int j = 0; j < kKeys / 8; ++j) {
+          const int row = r0 + j * 8 + g8;
           asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                       : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                       : "=r"(w[j][0]), "=r"(w[j][1]), "=r"(w[j][2]), "=r"(w[j][3])
                        : "r"(k_smem + row * 128 + (((t4 * 2 + c) ^ (row & 7)) << 4)));
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            mma_m16n8k16_f16(s[j], qf[c * 4 + i], e4m3x2_to_f16x2(w[i] & 0xffffu), e4m3x2_to_f16x2(w[i] >> 16));
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < kKeys / 8; ++j)
+            mma_m16n8k16_f16(s[j], qf[c * 4 + i], e4m3x2_to_f16x2(w[j][i] & 0xffffu), e4m3x2_to_f16x2(w[j][i] >> 16));
       }
-      float mx[2] = {-INFINITY, -INFINITY};
+      const bool whole = tok_base + kKeys <= hi && (tok_base >= lo || tok_base + kKeys <= keep);  // every token is seen
+      float corr[2] = {1.f, 1.f}, ps[2] = {0.f, 0.f};
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
+      for (int h = 0; h < kRows; ++h) {
+        float mx = -INFINITY;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int tok = tok_base + j * 8 + 2 * t4 + (e & 1);
-          const bool valid = tok < hi && (tok >= lo || tok < keep);
-          s[j][e] = valid ? s[j][e] * row_scale[e >> 1] : -INFINITY;
-          mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
-        }
-      }
-      float corr[2], m_use[2];
+        for (int j = 0; j < kKeys / 8; ++j)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        mx[h] = quad_max(mx[h]);
-        const float m_new = fmaxf(m_run[h], mx[h]);
-        m_use[h] = (m_new == -INFINITY) ? 0.f : m_new;
-        corr[h] = exp2f(m_run[h] - m_use[h]);
+          for (int e = 2 * h; e < 2 * h + 2; ++e) {
+            s[j][e] *= row_scale[h];
+            if (!whole) {
+              const int tok = tok_base + j * 8 + 2 * t4 + (e & 1);
+              if (!(tok < hi && (tok >= lo || tok < keep))) s[j][e] = -INFINITY;
+            }
+            mx = fmaxf(mx, s[j][e]);
+          }
+        const float m_new = fmaxf(m_run[h], quad_max(mx));
+        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+        corr[h] = exp2f(m_run[h] - m_use);
         m_run[h] = m_new;
+#pragma unroll
+        for (int j = 0; j < kKeys / 8; ++j)
+#pragma unroll
+          for (int e = 2 * h; e < 2 * h + 2; ++e) {
+            s[j][e] = exp2f(s[j][e] - m_use + kPShift);
+            ps[h] += s[j][e];
+          }
+        l_run[h] = l_run[h] * corr[h] + ps[h];
       }
-      float ps[2] = {0.f, 0.f};
+      if (__any_sync(0xffffffffu, corr[0] != 1.f || (HIGH && corr[1] != 1.f))) {
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+        for (int i = 0; i < D / 8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[j][e] = exp2f(s[j][e] - m_use[e >> 1] + kPShift);
-          ps[e >> 1] += s[j][e];
-        }
-      l_run[0] = l_run[0] * corr[0] + ps[0];
-      l_run[1] = l_run[1] * corr[1] + ps[1];
-      if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-          o[i][0] *= corr[0];
-          o[i][1] *= corr[0];
-          o[i][2] *= corr[1];
-          o[i][3] *= corr[1];
-        }
+          for (int e = 0; e < 2 * kRows; ++e) o[i][e] *= corr[e >> 1];
       }
-      uint32_t pf[4];
-      pf[0] = pack_f16x2(s[0][0], s[0][1]);
-      pf[1] = pack_f16x2(s[0][2], s[0][3]);
-      pf[2] = pack_f16x2(s[1][0], s[1][1]);
-      pf[3] = pack_f16x2(s[1][2], s[1][3]);
-      if (tok_base + 16 > hi || (tok_base < lo && tok_base + 16 > keep)) {
+      if (!whole) {
         // The pages come whole. A probability of 0 times a NaN byte of a token that is not seen (what the page's last owner left
         // behind the context) would be NaN: this warp's rows of such tokens become zeros, in the first and last tiles only.
-        for (int i = lane; i < 16 * 8; i += 32) {
+        for (int i = lane; i < kKeys * 8; i += 32) {
           const int tok = tok_base + (i >> 3);
           if (!(tok < hi && (tok >= lo || tok < keep))) st_shared_zero16(v_smem + (r0 + (i >> 3)) * 128 + (i & 7) * 16);
         }
         fence_proxy_async_smem();  // the stage is loaded again
         __syncwarp();
       }
-      const int mi = lane >> 3, row = r0 + (mi & 1) * 8 + (lane & 7);
 #pragma unroll
-      for (int c = 0; c < 8; c += 2) {  // 16 columns per 16-byte chunk
-        uint32_t r[4];  // chunk c: tokens 0-7, 8-15; chunk c + 1: the same
-        ldmatrix_x4_trans(r, v_smem + row * 128 + (((c + (mi >> 1)) ^ (row & 7)) << 4));
+      for (int k = 0; k < kKeys / 16; ++k) {
+        uint32_t pf[4];
+        pf[0] = pack_f16x2(s[2 * k][0], s[2 * k][1]);
+        pf[1] = HIGH ? pack_f16x2(s[2 * k][2], s[2 * k][3]) : 0u;
+        pf[2] = pack_f16x2(s[2 * k + 1][0], s[2 * k + 1][1]);
+        pf[3] = HIGH ? pack_f16x2(s[2 * k + 1][2], s[2 * k + 1][3]) : 0u;
+        const int mi = lane >> 3, row = r0 + k * 16 + (mi & 1) * 8 + (lane & 7);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);  // even column of both tokens | odd column
+        for (int c = 0; c < 8; c += 2) {  // 16 columns per 16-byte chunk
+          uint32_t r[4];  // chunk c: tokens 0-7, 8-15; chunk c + 1: the same
+          ldmatrix_x4_trans(r, v_smem + row * 128 + (((c + (mi >> 1)) ^ (row & 7)) << 4));
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          mma_m16n8k16_f16(o[(c + h) * 2], pf, e4m3x2_to_f16x2(r[2 * h] & 0xffffu), e4m3x2_to_f16x2(r[2 * h + 1] & 0xffffu));
-          mma_m16n8k16_f16(o[(c + h) * 2 + 1], pf, e4m3x2_to_f16x2(r[2 * h] >> 16), e4m3x2_to_f16x2(r[2 * h + 1] >> 16));
+          for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);  // even column of both tokens | odd column
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            mma_m16n8k16_f16(o[(c + h) * 2], pf, e4m3x2_to_f16x2(r[2 * h] & 0xffffu), e4m3x2_to_f16x2(r[2 * h + 1] & 0xffffu));
+            mma_m16n8k16_f16(o[(c + h) * 2 + 1], pf, e4m3x2_to_f16x2(r[2 * h] >> 16), e4m3x2_to_f16x2(r[2 * h + 1] >> 16));
+          }
         }
       }
     }
@@ -1393,10 +1422,15 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
     if (!pxl_host::make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k_cache, rows, 128, 128, page_size, 128) ||
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, v_cache, rows, 128, 128, page_size, 128))
       return PXL_ERR_TENSORMAP;
-    return launch_decode_splits<attn_decode_e4m3_kernel<false>, attn_decode_e4m3_kernel<true>, attn_decode_reduce_kernel<128, kPlain>>(
+    auto go = [&](auto high) {
+      constexpr bool H = decltype(high)::value;
+      return launch_decode_splits<attn_decode_e4m3_kernel<false, H>, attn_decode_e4m3_kernel<true, H>,
+                                  attn_decode_reduce_kernel<128, kPlain>>(
         grid, kE4Smem, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
         static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2 * k_scale, window, keep_first,
         num_splits, v_scale, status);
+    };
+    return Hq / Hkv > 8 ? go(std::true_type{}) : go(std::false_type{});
   }
 #define PXL_DEC(DD, F8, M)                                                                       \
   {                                                                                              \
@@ -1440,7 +1474,7 @@ PXL_EXPORT int pxl_attn_decode_launches(int B, int Hkv, int D, int page_size, in
   if (num_splits <= 1) return 1;
   if (D != 128 || (page_size != 16 && page_size != 32 && page_size != 64)) return 2;
   const int64_t pairs = static_cast<int64_t>(B) * Hkv;
-  const bool one = cache_fp8       ? splits_together<attn_decode_e4m3_kernel<true>>(pairs, num_splits, kE4Smem)
+  const bool one = cache_fp8       ? splits_together<attn_decode_e4m3_kernel<true, true>>(pairs, num_splits, kE4Smem)
                    : sigmoid       ? splits_together<attn_decode_tma_kernel<kSigmoid, true>>(pairs, num_splits, kDecSmem)
                    : softcap > 0.f ? splits_together<attn_decode_tma_kernel<kCapped, true>>(pairs, num_splits, kDecSmem)
                                    : splits_together<attn_decode_tma_kernel<kPlain, true>>(pairs, num_splits, kDecSmem);
