@@ -461,11 +461,108 @@ struct TileBlocks {
   }
 };
 
+// The 16 rows of a warp's products (rows >= G of a key head's query heads are zero; rows 8 to 15 are left out of the softmax where
+// HIGH is false): queries, running softmax and output of the keys that it has seen.
+template <int SM, bool HIGH>
+struct RowsBf16 {
+  static constexpr int D = 128, kRows = HIGH ? 2 : 1, kKeys = 16;  // kRows: of this thread, lane / 4 and lane / 4 + 8; keys per step
+  uint32_t qf[D / 16][4];
+  float bias2[2], o[D / 8][4], m_run[2], l_run[2];
+
+  // q: first query head of the key head
+  __device__ __forceinline__ void begin(const bf16* q, int G, int head0, float, const ScoreArgs& sa) {
+    const int lane = threadIdx.x & 31, r_lo = lane >> 2, r_hi = r_lo + 8;
+    const bf16 *q_lo = q + r_lo * D, *q_hi = q + r_hi * D;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+      const int c = ks * 16 + 2 * (lane & 3);
+      qf[ks][0] = r_lo < G ? *reinterpret_cast<const uint32_t*>(q_lo + c) : 0u;
+      qf[ks][1] = HIGH && r_hi < G ? *reinterpret_cast<const uint32_t*>(q_hi + c) : 0u;
+      qf[ks][2] = r_lo < G ? *reinterpret_cast<const uint32_t*>(q_lo + c + 8) : 0u;
+      qf[ks][3] = HIGH && r_hi < G ? *reinterpret_cast<const uint32_t*>(q_hi + c + 8) : 0u;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      bias2[h] = 0.f;
+      if constexpr (SM == kSigmoid)
+        if (r_lo + h * 8 < G) bias2[h] = sa.bias[head0 + r_lo + h * 8] * kLog2e;
+      m_run[h] = -INFINITY;
+      l_run[h] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  }
+
+  // Keys r0 .. r0 + 15 of a tile; the first is token tok_base.
+  __device__ __forceinline__ void step(uint32_t k_smem, uint32_t v_smem, int r0, int tok_base, int lo, int hi, int keep, float scale_log2,
+                                       const ScoreArgs& sa) {
+    if (!(tok_base < hi && (tok_base + kKeys > lo || tok_base < keep))) return;  // warp-uniform
+    const int lane = threadIdx.x & 31;
+    float s[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+    qk_16x16<D, true>(qf, k_smem, r0, s[0], s[1]);
+    const bool whole = tok_base + kKeys <= hi && (tok_base >= lo || tok_base + kKeys <= keep);  // every token is seen
+    float corr[2] = {1.f, 1.f};
+#pragma unroll
+    for (int h = 0; h < kRows; ++h) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 2 * h; e < 2 * h + 2; ++e) {
+          if constexpr (SM == kSigmoid) s[j][e] = sigmoid_weight(s[j][e], scale_log2, bias2[h]);
+          else s[j][e] = score_log2<SM>(s[j][e], scale_log2, sa);
+          if (!whole) {
+            const int tok = tok_base + j * 8 + 2 * (lane & 3) + (e & 1);
+            if (!(tok < hi && (tok >= lo || tok < keep))) s[j][e] = SM == kSigmoid ? 0.f : -INFINITY;
+          }
+          if constexpr (SM != kSigmoid) mx = fmaxf(mx, s[j][e]);
+        }
+      if constexpr (SM != kSigmoid) {
+        const float m_new = fmaxf(m_run[h], quad_max(mx));
+        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+        corr[h] = exp2f(m_run[h] - m_use);
+        m_run[h] = m_new;
+        float ps = 0.f;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 2 * h; e < 2 * h + 2; ++e) {
+            s[j][e] = exp2f(s[j][e] - m_use);
+            ps += s[j][e];
+          }
+        l_run[h] = l_run[h] * corr[h] + ps;
+      }
+    }
+    if (SM != kSigmoid && __any_sync(0xffffffffu, corr[0] != 1.f || (HIGH && corr[1] != 1.f))) {
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 2 * kRows; ++e) o[i][e] *= corr[e >> 1];
+    }
+    uint32_t pf[4];
+    pf[0] = pack_bf16x2(s[0][0], s[0][1]);
+    pf[1] = HIGH ? pack_bf16x2(s[0][2], s[0][3]) : 0u;
+    pf[2] = pack_bf16x2(s[1][0], s[1][1]);
+    pf[3] = HIGH ? pack_bf16x2(s[1][2], s[1][3]) : 0u;
+    pv_16x16<D, true>(pf, v_smem, r0, o);
+  }
+
+  // columns of the accumulator registers o[i][0], o[i][1], o[i + 1][0], o[i + 1][1] (i even): two pairs, 8 apart
+  template <typename F>
+  static __device__ __forceinline__ void columns(const float (&o)[D / 8][4], int i, int row, F put) {
+    const int c = i * 8 + 2 * (threadIdx.x & 3);
+    put(c, o[i][2 * row], o[i][2 * row + 1]);
+    put(c + 8, o[i + 1][2 * row], o[i + 1][2 * row + 1]);
+  }
+};
+
 constexpr int kDecStages = 3;
 constexpr int kDecThreads = 160;  // 4 consumer warps + 1 producer warp
 
 // CLUSTER: the splits of a (sequence, key head) are a cluster and add their results (add_splits); else through the workspace
-template <int SM, bool CLUSTER>
+template <int SM, bool CLUSTER, bool HIGH>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const bf16* __restrict__ q, int64_t q_stride, const int* __restrict__ block_tables,
@@ -544,33 +641,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     }
   }
 
-  uint32_t qf[D / 16][4];
-  {
-    const int r_lo = lane >> 2, r_hi = r_lo + 8;
-    const bf16* q_lo = q + static_cast<size_t>(b) * q_stride + (kvh * G + r_lo) * D;
-    const bf16* q_hi = q + static_cast<size_t>(b) * q_stride + (kvh * G + r_hi) * D;
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-      const int c = ks * 16 + 2 * (lane & 3);
-      qf[ks][0] = r_lo < G ? *reinterpret_cast<const uint32_t*>(q_lo + c) : 0u;
-      qf[ks][1] = r_hi < G ? *reinterpret_cast<const uint32_t*>(q_hi + c) : 0u;
-      qf[ks][2] = r_lo < G ? *reinterpret_cast<const uint32_t*>(q_lo + c + 8) : 0u;
-      qf[ks][3] = r_hi < G ? *reinterpret_cast<const uint32_t*>(q_hi + c + 8) : 0u;
-    }
-  }
-  float bias2[2] = {0.f, 0.f};  // of this thread's two rows
-  if constexpr (SM == kSigmoid) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = (lane >> 2) + h * 8;
-      if (r < G) bias2[h] = sa.bias[kvh * G + r] * kLog2e;
-    }
-  }
-  float o[D / 8][4];
-#pragma unroll
-  for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY};
-  float l_run[2] = {0.f, 0.f};
+  RowsBf16<SM, HIGH> rows;
+  rows.begin(q + static_cast<size_t>(b) * q_stride + kvh * G * D, G, kvh * G, scale_log2, sa);
+  float (&o)[D / 8][4] = rows.o;
+  float (&m_run)[2] = rows.m_run, (&l_run)[2] = rows.l_run;
 
   for (int it = 0; warp < 4 && it < n_tiles; ++it) {
     const int stage = it % kDecStages;
@@ -578,64 +652,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       failed = 1;
       break;  // reported to the whole CTA at the barrier behind the loop
     }
-    const uint32_t k_smem = stage0 + stage * 2 * TILE_BYTES, v_smem = k_smem + TILE_BYTES;
-    const int r0 = warp * 16;
-    const int tok_base = tiles[t_begin + it] * TILE + r0;
-    if (tok_base < hi && (tok_base + 16 > lo || tok_base < keep)) {  // warp-uniform
-      float s[2][4];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-      qk_16x16<D, true>(qf, k_smem, r0, s[0], s[1]);
-      float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int tok = tok_base + j * 8 + 2 * (lane & 3) + (e & 1);
-          const bool valid = tok < hi && (tok >= lo || tok < keep);
-          if constexpr (SM == kSigmoid) {
-            s[j][e] = valid ? sigmoid_weight(s[j][e], scale_log2, bias2[e >> 1]) : 0.f;
-          } else {
-            s[j][e] = valid ? score_log2<SM>(s[j][e], scale_log2, sa) : -INFINITY;
-            mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
-          }
-        }
-      }
-      if constexpr (SM != kSigmoid) {
-        float corr[2], m_use[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          mx[h] = quad_max(mx[h]);
-          const float m_new = fmaxf(m_run[h], mx[h]);
-          m_use[h] = (m_new == -INFINITY) ? 0.f : m_new;
-          corr[h] = exp2f(m_run[h] - m_use[h]);
-          m_run[h] = m_new;
-        }
-        float ps[2] = {0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s[j][e] = exp2f(s[j][e] - m_use[e >> 1]);
-            ps[e >> 1] += s[j][e];
-          }
-        l_run[0] = l_run[0] * corr[0] + ps[0];
-        l_run[1] = l_run[1] * corr[1] + ps[1];
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-          o[i][0] *= corr[0];
-          o[i][1] *= corr[0];
-          o[i][2] *= corr[1];
-          o[i][3] *= corr[1];
-        }
-      }
-      uint32_t pf[4];
-      pf[0] = pack_bf16x2(s[0][0], s[0][1]);
-      pf[1] = pack_bf16x2(s[0][2], s[0][3]);
-      pf[2] = pack_bf16x2(s[1][0], s[1][1]);
-      pf[3] = pack_bf16x2(s[1][2], s[1][3]);
-      pv_16x16<D, true>(pf, v_smem, r0, o);
-    }
+    const uint32_t k_smem = stage0 + stage * 2 * TILE_BYTES;
+    rows.step(k_smem, k_smem + TILE_BYTES, warp * 16, tiles[t_begin + it] * TILE + warp * 16, lo, hi, keep, scale_log2, sa);
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * stage);  // this warp is done with the stage
   }
@@ -764,6 +782,153 @@ __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+template <bool HIGH>
+struct RowsE4m3 {
+  static constexpr int D = 128, kRows = HIGH ? 2 : 1, kKeys = 32;
+  uint32_t qf[D / 16][4];
+  float row_scale[2], o[D / 8][4], m_run[2], l_run[2];
+
+  // q: first query head of the key head; each row is scaled by a power of two
+  __device__ __forceinline__ void begin(const bf16* q, int G, int, float scale_log2, const ScoreArgs&) {
+    const int lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g8 + h * 8;
+      float mx = 0.f;
+      if ((HIGH || h == 0) && r < G) {
+        const bf16* row = q + r * D + t4 * 32;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          qf[ks][h] = *reinterpret_cast<const uint32_t*>(row + ks * 4);
+          qf[ks][2 + h] = *reinterpret_cast<const uint32_t*>(row + ks * 4 + 2);
+          const float2 x = unpack_bf16x2(qf[ks][h]), y = unpack_bf16x2(qf[ks][2 + h]);
+          mx = fmaxf(fmaxf(fmaxf(mx, fabsf(x.x)), fabsf(x.y)), fmaxf(fabsf(y.x), fabsf(y.y)));
+        }
+      } else {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) qf[ks][h] = qf[ks][2 + h] = 0u;
+      }
+      if (!HIGH && h == 1) break;
+      mx = quad_max(mx);
+      int up = 267 - static_cast<int>(__float_as_uint(mx) >> 23);  // exponent bits of the factor: the largest value to [2^13, 2^14)
+      up = up < 1 ? 1 : up > 253 ? 253 : up;
+      const float f = __uint_as_float(static_cast<uint32_t>(up) << 23);
+      row_scale[h] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23) * scale_log2;
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const float2 x = unpack_bf16x2(qf[ks][2 * p + h]);
+          qf[ks][2 * p + h] = pack_f16x2(x.x * f, x.y * f);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    m_run[0] = m_run[1] = -INFINITY;
+    l_run[0] = l_run[1] = 0.f;
+  }
+
+  // Keys r0 .. r0 + 31 of a tile; the first is token tok_base.
+  __device__ __forceinline__ void step(uint32_t k_smem, uint32_t v_smem, int r0, int tok_base, int lo, int hi, int keep, float,
+                                       const ScoreArgs&) {
+    if (!(tok_base < hi && (tok_base + kKeys > lo || tok_base < keep))) return;  // warp-uniform
+    const int lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+    float s[kKeys / 8][4];  // 8 tokens each
+#pragma unroll
+    for (int j = 0; j < kKeys / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t w[kKeys / 8][4];
+#pragma unroll
+      for (int j = 0; j < kKeys / 8; ++j) {
+        const int row = r0 + j * 8 + g8;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w[j][0]), "=r"(w[j][1]), "=r"(w[j][2]), "=r"(w[j][3])
+                     : "r"(k_smem + row * 128 + (((t4 * 2 + c) ^ (row & 7)) << 4)));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < kKeys / 8; ++j)
+          mma_m16n8k16_f16(s[j], qf[c * 4 + i], e4m3x2_to_f16x2(w[j][i] & 0xffffu), e4m3x2_to_f16x2(w[j][i] >> 16));
+    }
+    const bool whole = tok_base + kKeys <= hi && (tok_base >= lo || tok_base + kKeys <= keep);  // every token is seen
+    float corr[2] = {1.f, 1.f}, ps[2] = {0.f, 0.f};
+#pragma unroll
+    for (int h = 0; h < kRows; ++h) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < kKeys / 8; ++j)
+#pragma unroll
+        for (int e = 2 * h; e < 2 * h + 2; ++e) {
+          s[j][e] *= row_scale[h];
+          if (!whole) {
+            const int tok = tok_base + j * 8 + 2 * t4 + (e & 1);
+            if (!(tok < hi && (tok >= lo || tok < keep))) s[j][e] = -INFINITY;
+          }
+          mx = fmaxf(mx, s[j][e]);
+        }
+      const float m_new = fmaxf(m_run[h], quad_max(mx));
+      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+      corr[h] = exp2f(m_run[h] - m_use);
+      m_run[h] = m_new;
+#pragma unroll
+      for (int j = 0; j < kKeys / 8; ++j)
+#pragma unroll
+        for (int e = 2 * h; e < 2 * h + 2; ++e) {
+          s[j][e] = exp2f(s[j][e] - m_use + kPShift);
+          ps[h] += s[j][e];
+        }
+      l_run[h] = l_run[h] * corr[h] + ps[h];
+    }
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || (HIGH && corr[1] != 1.f))) {
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 2 * kRows; ++e) o[i][e] *= corr[e >> 1];
+    }
+    if (!whole) {
+      // The pages come whole. A probability of 0 times a NaN byte of a token that is not seen (what the page's last owner left
+      // behind the context) would be NaN: this warp's rows of such tokens become zeros, in the first and last tiles only.
+      for (int i = lane; i < kKeys * 8; i += 32) {
+        const int tok = tok_base + (i >> 3);
+        if (!(tok < hi && (tok >= lo || tok < keep))) st_shared_zero16(v_smem + (r0 + (i >> 3)) * 128 + (i & 7) * 16);
+      }
+      fence_proxy_async_smem();  // the stage is loaded again
+      __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < kKeys / 16; ++k) {
+      uint32_t pf[4];
+      pf[0] = pack_f16x2(s[2 * k][0], s[2 * k][1]);
+      pf[1] = HIGH ? pack_f16x2(s[2 * k][2], s[2 * k][3]) : 0u;
+      pf[2] = pack_f16x2(s[2 * k + 1][0], s[2 * k + 1][1]);
+      pf[3] = HIGH ? pack_f16x2(s[2 * k + 1][2], s[2 * k + 1][3]) : 0u;
+      const int mi = lane >> 3, row = r0 + k * 16 + (mi & 1) * 8 + (lane & 7);
+#pragma unroll
+      for (int c = 0; c < 8; c += 2) {  // 16 columns per 16-byte chunk
+        uint32_t r[4];  // chunk c: tokens 0-7, 8-15; chunk c + 1: the same
+        ldmatrix_x4_trans(r, v_smem + row * 128 + (((c + (mi >> 1)) ^ (row & 7)) << 4));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);  // even column of both tokens | odd column
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          mma_m16n8k16_f16(o[(c + h) * 2], pf, e4m3x2_to_f16x2(r[2 * h] & 0xffffu), e4m3x2_to_f16x2(r[2 * h + 1] & 0xffffu));
+          mma_m16n8k16_f16(o[(c + h) * 2 + 1], pf, e4m3x2_to_f16x2(r[2 * h] >> 16), e4m3x2_to_f16x2(r[2 * h + 1] >> 16));
+        }
+      }
+    }
+  }
+
+  // columns of the accumulator registers o[i][0], o[i + 1][0], o[i][1], o[i + 1][1] (i even): four in a row
+  template <typename F>
+  static __device__ __forceinline__ void columns(const float (&o)[D / 8][4], int i, int row, F put) {
+    const int c = i * 8 + 4 * (threadIdx.x & 3);
+    put(c, o[i][2 * row], o[i + 1][2 * row]);
+    put(c + 2, o[i][2 * row + 1], o[i + 1][2 * row + 1]);
+  }
+};
+
 template <bool CLUSTER, bool HIGH>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -833,147 +998,24 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     }
   }
 
-  // Q fragments: row r of the MMA tile is q head kvh * G + r (rows >= G are zero), scaled per row
   const int g8 = lane >> 2, t4 = lane & 3;
-  uint32_t qf[D / 16][4];
-  float row_scale[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int r = g8 + h * 8;
-    float mx = 0.f;
-    if ((HIGH || h == 0) && r < G) {
-      const bf16* row = q + static_cast<size_t>(b) * q_stride + (kvh * G + r) * D + t4 * 32;
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        qf[ks][h] = *reinterpret_cast<const uint32_t*>(row + ks * 4);
-        qf[ks][2 + h] = *reinterpret_cast<const uint32_t*>(row + ks * 4 + 2);
-        const float2 x = unpack_bf16x2(qf[ks][h]), y = unpack_bf16x2(qf[ks][2 + h]);
-        mx = fmaxf(fmaxf(fmaxf(mx, fabsf(x.x)), fabsf(x.y)), fmaxf(fabsf(y.x), fabsf(y.y)));
-      }
-    } else {
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) qf[ks][h] = qf[ks][2 + h] = 0u;
-    }
-    if (!HIGH && h == 1) break;
-    mx = quad_max(mx);
-    int up = 267 - static_cast<int>(__float_as_uint(mx) >> 23);  // exponent bits of the factor: the largest value to [2^13, 2^14)
-    up = up < 1 ? 1 : up > 253 ? 253 : up;
-    const float f = __uint_as_float(static_cast<uint32_t>(up) << 23);
-    row_scale[h] = __uint_as_float(static_cast<uint32_t>(254 - up) << 23) * scale_log2;
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks)
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const float2 x = unpack_bf16x2(qf[ks][2 * p + h]);
-        qf[ks][2 * p + h] = pack_f16x2(x.x * f, x.y * f);
-      }
-  }
-  float o[D / 8][4];
-#pragma unroll
-  for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY};
-  float l_run[2] = {0.f, 0.f};
+  RowsE4m3<HIGH> rows;
+  rows.begin(q + static_cast<size_t>(b) * q_stride + kvh * G * D, G, kvh * G, scale_log2, ScoreArgs{});
+  float (&o)[D / 8][4] = rows.o;
+  float (&m_run)[2] = rows.m_run, (&l_run)[2] = rows.l_run;
 
   // Warps 0 and 1 take the even tiles, 2 and 3 the odd ones, 32 tokens each. A stage has to belong to one pair (an even number of
   // them): another pair that is a use ahead would take the parity of the use before last for its own.
   static_assert(kE4Stages % 2 == 0);
-  constexpr int kRows = HIGH ? 2 : 1, kKeys = 32;  // kRows: of this thread, g8 and g8 + 8
   for (int it = warp >> 1; warp < 4 && it < n_tiles; it += 2) {
     const int stage = it % kE4Stages;
     if (!mbar_wait_bounded(full0 + 8 * stage, (it / kE4Stages) & 1, abort_flag, status, PXL_DEV_TIMEOUT_FULL)) {
       failed = 1;
       break;  // reported to the whole CTA at the barrier behind the loop
     }
-    const uint32_t k_smem = stage0 + stage * 2 * kE4Tile, v_smem = k_smem + kE4Tile;
-    const int r0 = (warp & 1) * kKeys;
-    const int tok_base = tiles[t_begin + it] * TILE + r0;
-    if (tok_base < hi && (tok_base + kKeys > lo || tok_base < keep)) {  // warp-uniform
-      float s[kKeys / 8][4];  // 8 tokens each
-#pragma unroll
-      for (int j = 0; j < kKeys / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t w[kKeys / 8][4];
-#pragma unroll
-        for (int j = 0; j < kKeys / 8; ++j) {
-          const int row = r0 + j * 8 + g8;
-          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                       : "=r"(w[j][0]), "=r"(w[j][1]), "=r"(w[j][2]), "=r"(w[j][3])
-                       : "r"(k_smem + row * 128 + (((t4 * 2 + c) ^ (row & 7)) << 4)));
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < kKeys / 8; ++j)
-            mma_m16n8k16_f16(s[j], qf[c * 4 + i], e4m3x2_to_f16x2(w[j][i] & 0xffffu), e4m3x2_to_f16x2(w[j][i] >> 16));
-      }
-      const bool whole = tok_base + kKeys <= hi && (tok_base >= lo || tok_base + kKeys <= keep);  // every token is seen
-      float corr[2] = {1.f, 1.f}, ps[2] = {0.f, 0.f};
-#pragma unroll
-      for (int h = 0; h < kRows; ++h) {
-        float mx = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < kKeys / 8; ++j)
-#pragma unroll
-          for (int e = 2 * h; e < 2 * h + 2; ++e) {
-            s[j][e] *= row_scale[h];
-            if (!whole) {
-              const int tok = tok_base + j * 8 + 2 * t4 + (e & 1);
-              if (!(tok < hi && (tok >= lo || tok < keep))) s[j][e] = -INFINITY;
-            }
-            mx = fmaxf(mx, s[j][e]);
-          }
-        const float m_new = fmaxf(m_run[h], quad_max(mx));
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-        corr[h] = exp2f(m_run[h] - m_use);
-        m_run[h] = m_new;
-#pragma unroll
-        for (int j = 0; j < kKeys / 8; ++j)
-#pragma unroll
-          for (int e = 2 * h; e < 2 * h + 2; ++e) {
-            s[j][e] = exp2f(s[j][e] - m_use + kPShift);
-            ps[h] += s[j][e];
-          }
-        l_run[h] = l_run[h] * corr[h] + ps[h];
-      }
-      if (__any_sync(0xffffffffu, corr[0] != 1.f || (HIGH && corr[1] != 1.f))) {
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i)
-#pragma unroll
-          for (int e = 0; e < 2 * kRows; ++e) o[i][e] *= corr[e >> 1];
-      }
-      if (!whole) {
-        // The pages come whole. A probability of 0 times a NaN byte of a token that is not seen (what the page's last owner left
-        // behind the context) would be NaN: this warp's rows of such tokens become zeros, in the first and last tiles only.
-        for (int i = lane; i < kKeys * 8; i += 32) {
-          const int tok = tok_base + (i >> 3);
-          if (!(tok < hi && (tok >= lo || tok < keep))) st_shared_zero16(v_smem + (r0 + (i >> 3)) * 128 + (i & 7) * 16);
-        }
-        fence_proxy_async_smem();  // the stage is loaded again
-        __syncwarp();
-      }
-#pragma unroll
-      for (int k = 0; k < kKeys / 16; ++k) {
-        uint32_t pf[4];
-        pf[0] = pack_f16x2(s[2 * k][0], s[2 * k][1]);
-        pf[1] = HIGH ? pack_f16x2(s[2 * k][2], s[2 * k][3]) : 0u;
-        pf[2] = pack_f16x2(s[2 * k + 1][0], s[2 * k + 1][1]);
-        pf[3] = HIGH ? pack_f16x2(s[2 * k + 1][2], s[2 * k + 1][3]) : 0u;
-        const int mi = lane >> 3, row = r0 + k * 16 + (mi & 1) * 8 + (lane & 7);
-#pragma unroll
-        for (int c = 0; c < 8; c += 2) {  // 16 columns per 16-byte chunk
-          uint32_t r[4];  // chunk c: tokens 0-7, 8-15; chunk c + 1: the same
-          ldmatrix_x4_trans(r, v_smem + row * 128 + (((c + (mi >> 1)) ^ (row & 7)) << 4));
-#pragma unroll
-          for (int i = 0; i < 4; ++i) r[i] = __byte_perm(r[i], 0u, 0x3120);  // even column of both tokens | odd column
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            mma_m16n8k16_f16(o[(c + h) * 2], pf, e4m3x2_to_f16x2(r[2 * h] & 0xffffu), e4m3x2_to_f16x2(r[2 * h + 1] & 0xffffu));
-            mma_m16n8k16_f16(o[(c + h) * 2 + 1], pf, e4m3x2_to_f16x2(r[2 * h] >> 16), e4m3x2_to_f16x2(r[2 * h + 1] >> 16));
-          }
-        }
-      }
-    }
+    const uint32_t k_smem = stage0 + stage * 2 * kE4Tile;
+    const int r0 = (warp & 1) * 32;
+    rows.step(k_smem, k_smem + kE4Tile, r0, tiles[t_begin + it] * TILE + r0, lo, hi, keep, scale_log2, ScoreArgs{});
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * stage);  // this warp is done with the stage
   }
@@ -1044,6 +1086,341 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   if constexpr (CLUSTER) {
     __syncwarp();
     add_splits<kPlain>(part_o, part_m, part_l, num_splits, split, G, kvh * G, sinks, kPShift, v_scale, out + static_cast<size_t>(b) * Hq * D);
+  }
+}
+
+// ---- decode of many rows: every CTA the same number of tiles ------------------------------------------------------
+// The tiles of all (sequence, key head) pairs stand in a row, and CTA c of n takes the c-th n-th of it: rows of any lengths end
+// together, where a grid of pairs has a last wave (1024 pairs on 296 places are 3.46 waves) and waits for its longest row. The loads
+// run on from one pair into the next: the ring of stages is filled with the next pair's keys, and its table read, while the results of
+// the one before are put together, which by CTA per pair is 2 to 4 us in which a CTA loads nothing. A pair that lies in several CTAs is
+// added up from the workspace by a second kernel: each CTA leaves at most the end of one pair (place 0) and the start of another (1).
+// Against a grid of pairs (8 key heads, us): e4m3 128 x 4096 keys 169 and 154 (0.94 of the bandwidth), 40 x 4000 81 and 56; bf16 40 x
+// 4000 121 and 95, 296 x 512 104 and 93, 512 x 100 78 and 47. Bounds: memory; over e4m3 pages and short rows the consumers, two warps
+// per scheduler that convert and multiply one behind the other.
+struct DecodeWork {
+  const int* ctx_lens;
+  int B, Hkv, window, keep;
+
+  __device__ __forceinline__ KeyTiles tiles(int b, int& lo, int& hi) const {
+    hi = __ldg(ctx_lens + b);
+    lo = (window > 0 && hi > window) ? hi - window : 0;
+    return KeyTiles(lo, hi, keep);
+  }
+  __device__ __forceinline__ int weight(int b) const {  // a pair without keys has a result too
+    int lo, hi;
+    const int n = tiles(b, lo, hi).total;
+    return n > 0 ? n : 1;
+  }
+  __device__ __forceinline__ int64_t total() const {  // whole warp
+    int sum = 0;
+    for (int b = threadIdx.x & 31; b < B; b += 32) sum += weight(b);
+    return static_cast<int64_t>(__reduce_add_sync(0xffffffffu, sum)) * Hkv;
+  }
+  // The pair that tile `pos` of the row belongs to, and which of its tiles it is; whole warp.
+  __device__ __forceinline__ void find(int64_t pos, int& b, int& kvh, int& t) const {
+    const int lane = threadIdx.x & 31;
+    int64_t before = 0;  // of the chunk of 32 sequences
+    for (int b0 = 0; b0 < B; b0 += 32) {
+      const int w = b0 + lane < B ? weight(b0 + lane) : 0;
+      int incl = w;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += up;
+      }
+      const uint32_t past = __ballot_sync(0xffffffffu, before + static_cast<int64_t>(incl) * Hkv > pos);
+      if (past) {
+        const int at = __ffs(past) - 1;
+        const int rest = static_cast<int>(pos - before - static_cast<int64_t>(__shfl_sync(0xffffffffu, incl - w, at)) * Hkv);
+        const int wa = __shfl_sync(0xffffffffu, w, at);
+        b = b0 + at;
+        kvh = rest / wa;
+        t = rest % wa;
+        return;
+      }
+      before += static_cast<int64_t>(__shfl_sync(0xffffffffu, incl, 31)) * Hkv;
+    }
+    b = B, kvh = 0, t = 0;
+  }
+};
+
+// Where the CTAs' shares begin: the first total % ctas of them are one tile longer.
+struct DecodeShares {
+  int64_t each;
+  int longer;
+  __device__ __forceinline__ DecodeShares(int64_t total, int ctas) : each(total / ctas), longer(static_cast<int>(total % ctas)) {}
+  __device__ __forceinline__ int64_t operator[](int cta) const { return each * cta + min(cta, longer); }
+};
+
+// One CTA's way along the row, a pair (or the part of one that is its share) at a time.
+struct DecodeWalk {
+  DecodeWork work;
+  int left, b, kvh, t, weight, take, lo, hi;  // tiles left; of the pair, tiles t .. t + take of `weight`
+  KeyTiles tiles;
+
+  __device__ __forceinline__ DecodeWalk(const DecodeWork& w, int cta, int ctas) : work(w), tiles(0, 0, 0) {
+    const DecodeShares at(work.total(), ctas);
+    left = static_cast<int>(at[cta + 1] - at[cta]);
+    b = kvh = t = weight = take = lo = hi = 0;
+    if (left > 0) {
+      work.find(at[cta], b, kvh, t);
+      enter();
+    }
+  }
+  __device__ __forceinline__ void enter() {
+    tiles = work.tiles(b, lo, hi);
+    weight = tiles.total > 0 ? tiles.total : 1;
+    take = min(left, weight - t);
+  }
+  __device__ __forceinline__ int count() const { return tiles.total > 0 ? take : 0; }
+  __device__ __forceinline__ bool whole() const { return take == weight; }
+  __device__ __forceinline__ void next() {
+    left -= take;
+    t += take;
+    if (t == weight) {
+      t = 0;
+      if (++kvh == work.Hkv) kvh = 0, ++b;
+    }
+    if (left > 0) enter();
+  }
+};
+
+template <bool F8, int SM>
+using DecodeRows = std::conditional_t<F8, RowsE4m3<false>, RowsBf16<SM, false>>;
+template <bool F8>
+constexpr int kEvenSmem = 1024 + (F8 ? kE4Stages * 2 * kE4Tile : kDecStages * 4 * TILE * 128) + 3 * 4096 + 3 * 2 * 32 * 4 + 128;
+
+template <bool F8, int SM>
+__global__ void __launch_bounds__(kDecThreads, 2)
+attn_decode_even_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const bf16* __restrict__ q,
+                        int64_t q_stride, const int* __restrict__ block_tables, const int* __restrict__ ctx_lens,
+                        bf16* __restrict__ out, float* __restrict__ workspace, const float* __restrict__ sinks, int B, int Hq, int Hkv,
+                        int page_size, int max_blocks, int64_t num_blocks, float scale_log2, int window, int keep, float v_scale,
+                        const ScoreArgs sa, int* status) {
+  constexpr int D = 128, STAGES = F8 ? kE4Stages : kDecStages, TILE_BYTES = TILE * D * (F8 ? 1 : 2);
+  using Rows = DecodeRows<F8, SM>;
+  constexpr float kShift = F8 ? kPShift : 0.f;  // log2 of the factor on the probabilities
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const uint32_t stage0 = smem_u32(smem);                                     // stage s: K at s * 2 * TILE_BYTES, V behind it
+  float4* parts = reinterpret_cast<float4*>(smem + STAGES * 2 * TILE_BYTES);  // [3][8][32]: outputs of a warp, lane by lane
+  float* part_m = reinterpret_cast<float*>(parts + 3 * 8 * 32);               // [3][32]
+  float* part_l = part_m + 3 * 32;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(part_l + 3 * 32);  // full[S], empty[S]
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * STAGES);
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
+  const int G = Hq / Hkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int shift = page_size == 16 ? 2 : page_size == 32 ? 1 : 0, ppt = 1 << shift;  // pages per tile
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, F8 ? 2 : 4);  // one arrival per warp that reads the stage
+    }
+    mbar_fence_init();
+    fence_proxy_async_smem();
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  // the lengths and the tables of a step are there before its first kernel, the queries and the new keys after the wait
+  const DecodeWork work{ctx_lens, B, Hkv, window, keep};
+  DecodeWalk walk(work, blockIdx.x, gridDim.x);
+  auto blocks_of = [&](const DecodeWalk& w) {
+    return TileBlocks{block_tables + static_cast<size_t>(w.left > 0 ? w.b : 0) * max_blocks, w.tiles, w.t, w.left > 0 ? w.count() : 0,
+                      page_size, shift, w.hi, max_blocks, num_blocks, status};
+  };
+  TileBlocks blocks = blocks_of(walk);
+  if (warp == 4) blocks.begin();
+  __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
+
+  int failed = 0;
+  int g = 0;  // tiles so far: tile g is in stage g % STAGES
+  if (warp == 4) {  // producer: lane p issues the boxes of page p of the tile
+    while (walk.left > 0 && !failed) {
+      const int n = walk.count(), kvh = walk.kvh;
+      walk.next();
+      TileBlocks ahead = blocks_of(walk);
+      ahead.begin();  // in flight during this pair
+      for (int it = 0; it < n; ++it, ++g) {
+        const int stage = g % STAGES;
+        const int blk = blocks(it);
+        int okf = 1;
+        if (g >= STAGES && lane == 0)
+          okf = mbar_wait_bounded(empty0 + 8 * stage, ((g / STAGES) - 1) & 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY) ? 1 : 0;
+        okf = __shfl_sync(0xffffffffu, okf, 0);
+        if (!okf) {
+          failed = 1;
+          break;
+        }
+        const uint32_t bar = full0 + 8 * stage;
+        const uint32_t dst = stage0 + stage * 2 * TILE_BYTES + lane * page_size * 128;
+        if (lane == 0) mbar_arrive_expect_tx(bar, 2 * TILE_BYTES);
+        __syncwarp();
+        if (lane < ppt) {
+          const int row0 = (blk * Hkv + kvh) * page_size;
+          tma_load_2d(dst, &tm_k, bar, 0, row0);
+          if constexpr (!F8) tma_load_2d(dst + TILE * 128, &tm_k, bar, 64, row0);
+          tma_load_2d(dst + TILE_BYTES, &tm_v, bar, 0, row0);
+          if constexpr (!F8) tma_load_2d(dst + TILE_BYTES + TILE * 128, &tm_v, bar, 64, row0);
+        }
+      }
+      blocks = ahead;
+    }
+  } else {
+    Rows rows;
+    const int r0 = (F8 ? warp & 1 : warp) * Rows::kKeys;
+    // after a failed wait the warp goes on to the end without loads or products: the others meet it at the barriers
+    for (; walk.left > 0; walk.next()) {
+      const int n = walk.count(), head0 = walk.kvh * G;
+      rows.begin(q + static_cast<size_t>(walk.b) * q_stride + head0 * D, G, head0, scale_log2, sa);
+      if (lane < 2 * G && walk.left > walk.take) {  // the next pair's queries, to be near when they are wanted
+        const int kvh = walk.kvh + 1 < Hkv ? walk.kvh + 1 : 0, b = walk.b + (kvh == 0 ? 1 : 0);
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(q + static_cast<size_t>(b) * q_stride + kvh * G * D + lane * 64));
+      }
+      for (int it = 0; it < n; ++it, ++g) {
+        if (F8 && (g & 1) != (warp >> 1)) continue;  // warps 0 and 1 take the even stages, 2 and 3 the odd ones (attn_decode_e4m3_kernel)
+        const int stage = g % STAGES;
+        if (!failed)
+          failed = __any_sync(0xffffffffu, !mbar_wait_bounded(full0 + 8 * stage, (g / STAGES) & 1, abort_flag, status, PXL_DEV_TIMEOUT_FULL));
+        if (failed) continue;
+        const uint32_t k_smem = stage0 + stage * 2 * TILE_BYTES;
+        rows.step(k_smem, k_smem + TILE_BYTES, r0, walk.tiles[walk.t + it] * TILE + r0, walk.lo, walk.hi, keep, scale_log2, sa);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8 * stage);
+      }
+
+      // warps 2 and 3 hand their results to 0 and 1, 1 to 0; a register goes to the same lane
+      auto give = [&](int p) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          parts[(p * 8 + i) * 32 + lane] = make_float4(rows.o[2 * i][0], rows.o[2 * i][1], rows.o[2 * i + 1][0], rows.o[2 * i + 1][1]);
+        part_m[p * 32 + lane] = rows.m_run[0];
+        part_l[p * 32 + lane] = rows.l_run[0];
+      };
+      auto add = [&](int p) {
+        float fa = 1.f, fb = 1.f;
+        if constexpr (SM != kSigmoid) {
+          const float m = part_m[p * 32 + lane], M = fmaxf(rows.m_run[0], m), Mu = M == -INFINITY ? 0.f : M;
+          fa = exp2f(rows.m_run[0] - Mu);
+          fb = exp2f(m - Mu);
+          rows.m_run[0] = M;
+          rows.l_run[0] = rows.l_run[0] * fa + part_l[p * 32 + lane] * fb;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 x = parts[(p * 8 + i) * 32 + lane];
+          rows.o[2 * i][0] = rows.o[2 * i][0] * fa + x.x * fb;
+          rows.o[2 * i][1] = rows.o[2 * i][1] * fa + x.y * fb;
+          rows.o[2 * i + 1][0] = rows.o[2 * i + 1][0] * fa + x.z * fb;
+          rows.o[2 * i + 1][1] = rows.o[2 * i + 1][1] * fa + x.w * fb;
+        }
+      };
+      if (warp >= 2) give(warp - 2);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (warp < 2) add(warp);
+      if (warp == 1) give(2);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (warp == 0) {
+        add(2);
+        const int r = lane >> 2;
+        const float M = rows.m_run[0], L = quad_sum(rows.l_run[0]);
+        if (r < G && !failed) {
+          if (walk.whole()) {
+            float f = 1.f;
+            if constexpr (SM != kSigmoid) {
+              const float sink = sinks ? sinks[head0 + r] * kLog2e : -INFINITY;
+              const float Mx = fmaxf(M, sink), Mu = Mx == -INFINITY ? 0.f : Mx;
+              const float e = exp2f(M - Mu), denom = L * e + exp2f(sink - Mu + kShift);
+              f = denom > 0.f ? e / denom * v_scale : 0.f;
+            }
+            bf16* dst = out + (static_cast<size_t>(walk.b) * Hq + head0 + r) * D;
+#pragma unroll
+            for (int i = 0; i < D / 8; i += 2)
+              Rows::columns(rows.o, i, 0, [&](int c, float x, float y) { *reinterpret_cast<uint32_t*>(dst + c) = pack_bf16x2(x * f, y * f); });
+          } else {
+            const size_t place = static_cast<size_t>(blockIdx.x) * 2 + (walk.t == 0 ? 1 : 0);
+            float* po = workspace + place * G * (D + 2);
+#pragma unroll
+            for (int i = 0; i < D / 8; i += 2)
+              Rows::columns(rows.o, i, 0, [&](int c, float x, float y) { *reinterpret_cast<float2*>(po + r * D + c) = make_float2(x, y); });
+            if ((lane & 3) == 0) po[G * D + r] = M, po[G * D + G + r] = L;
+          }
+        }
+      }
+    }
+  }
+  if (__syncthreads_or(failed)) __nanosleep(200000);  // loads that are still in flight must land before the shared memory is released
+}
+
+// Adds up the pairs that lie in several CTAs of attn_decode_even_kernel. Block x: the pair that the border between CTAs x and x + 1 cuts,
+// if no border before it does. Four query heads at a time, so that their loads are in flight together.
+template <int SM>
+__global__ void __launch_bounds__(128)
+attn_decode_even_reduce_kernel(const float* __restrict__ workspace, const float* __restrict__ sinks, const int* __restrict__ ctx_lens,
+                               bf16* __restrict__ out, int B, int Hq, int Hkv, int window, int keep, float shift, float v_scale) {
+  constexpr int D = 128, R = 4;
+  const DecodeWork work{ctx_lens, B, Hkv, window, keep};
+  const int ctas = gridDim.x + 1, cut = blockIdx.x + 1, d = threadIdx.x, G = Hq / Hkv;
+  const DecodeShares at(work.total(), ctas);
+  const int64_t pos = at[cut];
+  int b, kvh, t;
+  work.find(pos, b, kvh, t);
+  const int64_t begin = pos - t;
+  const bool mine = t > 0 && b < B && at[cut - 1] <= begin;
+  int last = cut;  // CTA that ends the pair; all of them up to it have tiles of it
+  if (mine)
+    for (const int64_t end = begin + work.weight(b); at[last + 1] < end;) ++last;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (!mine) return;
+  const size_t place = static_cast<size_t>(G) * (D + 2);
+  auto part = [&](int x) { return workspace + (static_cast<size_t>(x) * 2 + (x < cut ? 1 : 0)) * place; };
+  for (int r0 = 0; r0 < G; r0 += R) {
+    float acc[R], denom[R], M[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      acc[i] = 0.f;
+      M[i] = sinks && r0 + i < G ? sinks[kvh * G + r0 + i] * kLog2e : -INFINITY;
+      denom[i] = M[i] == -INFINITY ? 0.f : exp2f(shift);  // the sink's share, relative to M
+    }
+    for (int x = cut - 1; x <= last; ++x) {
+      const float* p = part(x) + r0 * D + d;
+      const float *pm = part(x) + G * D + r0, *pl = pm + G;
+      float o[R], m[R], l[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const bool in = r0 + i < G;
+        o[i] = in ? p[i * D] : 0.f;
+        if constexpr (SM != kSigmoid) {
+          m[i] = in ? pm[i] : -INFINITY;
+          l[i] = in ? pl[i] : 0.f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        if constexpr (SM == kSigmoid) {
+          acc[i] += o[i];
+        } else {
+          const float Mn = fmaxf(M[i], m[i]), Mu = Mn == -INFINITY ? 0.f : Mn;
+          const float f = exp2f(M[i] - Mu), g = exp2f(m[i] - Mu);
+          acc[i] = acc[i] * f + o[i] * g;
+          denom[i] = denom[i] * f + l[i] * g;
+          M[i] = Mn;
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (r0 + i >= G) break;
+      float res = acc[i];
+      if constexpr (SM != kSigmoid) res = denom[i] > 0.f ? res / denom[i] * v_scale : 0.f;
+      out[(static_cast<size_t>(b) * Hq + kvh * G + r0 + i) * D + d] = __float2bfloat16(res);
+    }
   }
 }
 
@@ -1274,21 +1651,32 @@ int set_smem(K kern, int bytes) {
 // Splits of a decode step: the count with the lowest estimate, us = (tiles of the longest split + start) x waves of CTAs + adding.
 // A last wave of few CTAs costs nearly as much as a full one, which ceil(2 SMs / CTAs), the rule before, did not see.
 //
-// Pages the TMA unit reads (head dim 128): 2 CTAs per SM; a tile of 64 keys takes 1.2 us while the memory is not full and 1.4 us
-// beside a full chip of others, start and end about one tile's time. Adding costs 1.3 us inside a cluster; through the workspace 1.5,
-// 0.1 per split and 2 per wave of partial results. Over 26 sizes of 1 to 150 rows and 100 to 100000 keys, bf16 and e4m3, the count is
-// the fastest measured or within 2 % (8 key heads, splits: us):
-//   rows x keys   before   now             rows x keys   before   now
-//   1 x 777       4:  8.1  7:  6.7         36 x 1280     2: 37.1  1:  31.9
-//   8 x 2100      5: 21.0  4: 16.7         40 x 4000     1: 136   4: 110
-//   16 x 1280     3: 24.6  2: 18.1         20 x 8192     2: 144   5: 105
+// Pages the TMA unit reads (head dim 128): 2 CTAs per SM; `part` us per tile of 64 keys while the memory is not full (over bf16 pages
+// less behind a full wave, whose rows do not end together), `full` beside a full chip of others. Adding is cheaper inside a cluster than
+// through the workspace. Tiles dealt out evenly (attn_decode_even_kernel, asked for by splits that give two places per CTA) take
+// `full` for each and a start, a sum and a share per pair. Fitted to 36 sizes of 1 to 512 rows and 100 to 100000 keys per type; the
+// choice is the fastest measured or within 3 % in all but six, within 12 % in all (8 key heads, splits or even: us, before and now):
+//   rows x keys   bf16                          e4m3
+//   1 x 777       4:  8.1      7:    6.7        4:  7.5     7:     6.4
+//   8 x 2100      5: 21.0      4:   16.2        5: 27       4:    12.1
+//   16 x 1280     3: 24.6      2:   17.8        3: 18.6     2:    12.9
+//   40 x 4000     1: 121       even: 95         1: 81       even: 56
+//   128 x 4096    1: 278       1:   278         1: 169      even: 154
+//   512 x 100     1: 78        even: 47         1: 71       even: 57
 // The kernel for other pages and head dim 64: 5 CTAs per SM (3 at 128), 1.0 us per tile either way, through the workspace 1 + 0.03 per
 // split and 1 per 296 CTAs (head dim 64): 16 x 1280 3: 18.3, 5: 16.3; 40 x 4000 1: 118, 2: 80.1; 36 x 1280 2: 26.3 both.
-PXL_EXPORT int pxl_attn_decode_splits(int B, int Hkv, int D, int page_size, int max_ctx) {
+PXL_EXPORT int pxl_attn_decode_splits(int B, int Hq, int Hkv, int D, int page_size, int cache_fp8, int max_ctx) {
+  struct Line {
+    float start, part, part_behind, full, cluster, add, add_split, add_wave, even, even_pair, even_margin;
+  };
+  static constexpr Line kLines[2] = {{2.f, 1.f, 0.85f, 1.4f, 1.1f, 1.3f, 0.13f, 0.8f, 9.f, 0.7f, 0.95f},
+                                     {2.7f, 0.59f, 0.59f, 0.66f, 2.5f, 1.4f, 0.09f, 2.4f, 9.f, 0.4f, 1.f}};
+  const Line& c = kLines[cache_fp8 ? 1 : 0];
   const bool tma = D == 128 && (page_size == 16 || page_size == 32 || page_size == 64);
   const int64_t pairs = static_cast<int64_t>(B) * Hkv;
-  const int slots = (tma ? 2 : D == 64 ? 5 : 3) * pxl_host::num_sms();
+  const int chip = 2 * pxl_host::num_sms(), slots = tma ? chip : (D == 64 ? 5 : 3) * pxl_host::num_sms();
   const int tiles = pxl::ceil_div(max_ctx > 0 ? max_ctx : 1, TILE);
+  const bool even = tma && Hkv > 0 && Hq / Hkv <= 8 && pairs > 0 && pairs * 64 >= 2 * chip;
   int best = 1, last = 0;
   float best_us = 0.f;
   for (int s = 1; s <= 64 && s <= tiles; ++s) {
@@ -1296,17 +1684,23 @@ PXL_EXPORT int pxl_attn_decode_splits(int B, int Hkv, int D, int page_size, int 
     if (per == last) continue;  // no fewer tiles for the longest split
     last = per;
     const int64_t ctas = pairs * s, full = ctas / slots, rest = ctas % slots;
-    const float waves = static_cast<float>(ctas) / (2 * pxl_host::num_sms());
+    if (even && s > 1 && ctas >= 2 * chip) break;  // asks for the even kernel
+    const float waves = static_cast<float>(ctas) / static_cast<float>(chip);
     float us;
     if (tma) {
-      const float part = static_cast<float>(rest) / slots;
-      us = static_cast<float>(per + 1) * (1.4f * static_cast<float>(full) + (rest ? fmaxf(1.2f, 1.4f * part) : 0.f));
-      if (s > 1) us += s <= kMaxClusterSplits && waves <= 0.9375f ? 1.3f : 1.5f + 0.1f * s + 2.f * waves;
+      const float part = rest ? fmaxf(full ? c.part_behind : c.part, c.full * static_cast<float>(rest) / slots) : 0.f;
+      us = (static_cast<float>(per) + c.start) * (c.full * static_cast<float>(full) + part);
+      if (s > 1) us += s <= kMaxClusterSplits && waves <= 0.9375f ? c.cluster : c.add + c.add_split * s + c.add_wave * waves;
     } else {
       us = static_cast<float>(per) * static_cast<float>(full + (rest ? 1 : 0));
       if (s > 1) us += 1.f + 0.03f * s + waves;
     }
     if (s == 1 || us < best_us) best = s, best_us = us;
+  }
+  if (even) {
+    const float waves = static_cast<float>(pairs) / static_cast<float>(chip);
+    if (c.full * waves * static_cast<float>(tiles) + c.even + c.even_pair * waves < c.even_margin * best_us)
+      best = pairs >= chip ? 2 : static_cast<int>((2 * chip + pairs - 1) / pairs);
   }
   return best;
 }
@@ -1346,6 +1740,31 @@ int resident_clusters(int splits, int smem) {
 template <auto Together>
 bool splits_together(int64_t pairs, int splits, int smem) {
   return splits > 1 && splits <= kMaxClusterSplits && pairs <= resident_clusters<Together>(splits, smem);
+}
+
+// Whether a step's tiles are dealt out evenly (attn_decode_even_kernel): the workspace of `splits` holds two results per CTA.
+bool decode_even(int64_t pairs, int splits, int group, const float* workspace) {
+  return splits > 1 && group <= 8 && pairs * splits >= 4ll * pxl_host::num_sms() && (reinterpret_cast<uintptr_t>(workspace) & 7) == 0;
+}
+
+template <bool F8, int SM>
+int launch_decode_even(const CUtensorMap& tk, const CUtensorMap& tv, const bf16* q, int64_t q_stride, const int* block_tables,
+                       const int* ctx_lens, bf16* out, float* workspace, const float* sinks, int B, int Hq, int Hkv, int page_size,
+                       int max_blocks, int64_t num_blocks, float scale_log2, int window, int keep, float v_scale, const ScoreArgs& sa,
+                       int* status, cudaStream_t stream) {
+  static bool done[64] = {false};  // function attributes are per device
+  const int dev = pxl_host::current_device_slot();
+  if (!done[dev]) {
+    if (set_smem(attn_decode_even_kernel<F8, SM>, kEvenSmem<F8>)) return PXL_ERR_CUDA;
+    done[dev] = true;
+  }
+  const int ctas = 2 * pxl_host::num_sms();
+  pxl_host::launch(attn_decode_even_kernel<F8, SM>, dim3(ctas), kDecThreads, kEvenSmem<F8>, stream, tk, tv, q, q_stride, block_tables,
+                   ctx_lens, out, workspace, sinks, B, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2, window, keep, v_scale, sa,
+                   status);
+  pxl_host::launch(attn_decode_even_reduce_kernel<SM>, dim3(ctas - 1), 128, 0, stream, workspace, sinks, ctx_lens, out, B, Hq,
+                   Hkv, window, keep, F8 ? kPShift : 0.f, v_scale);
+  return check_launch();
 }
 
 // One kernel of the splits (grid.z): alone, as clusters that add their results, or with the reduction behind it.
@@ -1391,7 +1810,7 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
   const ScoreArgs sa = score_args(scale, softcap, sig_bias);
   if (cache_fp8 && mode != kPlain) return PXL_ERR_INVALID_ARG;
   if (Hkv <= 0 || Hq % Hkv || Hq / Hkv > 16 || page_size <= 0) return PXL_ERR_INVALID_ARG;
-  if (num_splits <= 0) num_splits = pxl_attn_decode_splits(B, Hkv, D, page_size, max_ctx);
+  if (num_splits <= 0) num_splits = pxl_attn_decode_splits(B, Hq, Hkv, D, page_size, cache_fp8, max_ctx);
   if (num_splits > 1 && workspace == nullptr) return PXL_ERR_INVALID_ARG;
   const float scale_log2 = scale * kLog2e;
   dim3 grid(Hkv, B, num_splits);
@@ -1403,13 +1822,19 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
     if (!pxl_host::make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k_cache, rows, 128, 128, page_size, 64) ||
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v_cache, rows, 128, 128, page_size, 64))
       return PXL_ERR_TENSORMAP;
-    auto go = [&](auto sm) {
+    auto run = [&](auto sm, auto high) {
       constexpr int M = decltype(sm)::value;
-      return launch_decode_splits<attn_decode_tma_kernel<M, false>, attn_decode_tma_kernel<M, true>, attn_decode_reduce_kernel<128, M>>(
+      constexpr bool H = decltype(high)::value;
+      if (decode_even(static_cast<int64_t>(B) * Hkv, num_splits, Hq / Hkv, workspace))
+        return launch_decode_even<false, M>(tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
+                                            static_cast<bf16*>(out), workspace, sinks, B, Hq, Hkv, page_size, max_blocks, num_blocks,
+                                            scale_log2, window, keep_first, 1.f, sa, status, stream);
+      return launch_decode_splits<attn_decode_tma_kernel<M, false, H>, attn_decode_tma_kernel<M, true, H>, attn_decode_reduce_kernel<128, M>>(
           grid, kDecSmem, B, Hq, workspace, sinks, out, stream, tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
           static_cast<bf16*>(out), workspace, sinks, Hq, Hkv, page_size, max_blocks, num_blocks, scale_log2, window, keep_first,
           num_splits, sa, status);
     };
+    auto go = [&](auto sm) { return Hq / Hkv > 8 ? run(sm, std::true_type{}) : run(sm, std::false_type{}); };
     if (mode == kSigmoid) return go(std::integral_constant<int, kSigmoid>{});
     if (mode == kCapped) return go(std::integral_constant<int, kCapped>{});
     return go(std::integral_constant<int, kPlain>{});
@@ -1422,6 +1847,10 @@ int attn_decode_impl(const void* q, int64_t q_stride, const void* k_cache, const
     if (!pxl_host::make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k_cache, rows, 128, 128, page_size, 128) ||
         !pxl_host::make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, v_cache, rows, 128, 128, page_size, 128))
       return PXL_ERR_TENSORMAP;
+    if (decode_even(static_cast<int64_t>(B) * Hkv, num_splits, Hq / Hkv, workspace))
+      return launch_decode_even<true, kPlain>(tk, tv, static_cast<const bf16*>(q), q_stride, block_tables, ctx_lens,
+                                              static_cast<bf16*>(out), workspace, sinks, B, Hq, Hkv, page_size, max_blocks, num_blocks,
+                                              scale_log2 * k_scale, window, keep_first, v_scale, sa, status, stream);
     auto go = [&](auto high) {
       constexpr bool H = decltype(high)::value;
       return launch_decode_splits<attn_decode_e4m3_kernel<false, H>, attn_decode_e4m3_kernel<true, H>,
@@ -1475,9 +1904,9 @@ PXL_EXPORT int pxl_attn_decode_launches(int B, int Hkv, int D, int page_size, in
   if (D != 128 || (page_size != 16 && page_size != 32 && page_size != 64)) return 2;
   const int64_t pairs = static_cast<int64_t>(B) * Hkv;
   const bool one = cache_fp8       ? splits_together<attn_decode_e4m3_kernel<true, true>>(pairs, num_splits, kE4Smem)
-                   : sigmoid       ? splits_together<attn_decode_tma_kernel<kSigmoid, true>>(pairs, num_splits, kDecSmem)
-                   : softcap > 0.f ? splits_together<attn_decode_tma_kernel<kCapped, true>>(pairs, num_splits, kDecSmem)
-                                   : splits_together<attn_decode_tma_kernel<kPlain, true>>(pairs, num_splits, kDecSmem);
+                   : sigmoid       ? splits_together<attn_decode_tma_kernel<kSigmoid, true, true>>(pairs, num_splits, kDecSmem)
+                   : softcap > 0.f ? splits_together<attn_decode_tma_kernel<kCapped, true, true>>(pairs, num_splits, kDecSmem)
+                                   : splits_together<attn_decode_tma_kernel<kPlain, true, true>>(pairs, num_splits, kDecSmem);
   return one ? 1 : 2;
 }
 

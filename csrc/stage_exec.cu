@@ -116,7 +116,7 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
                           st->num_blocks * Hkv * st->page < (1ll << 31);
   int splits = 0;
   if (sp->Bd > 0) {
-    splits = pxl_attn_decode_splits(sp->Bd, Hkv, D, st->page, sp->d_max_ctx);
+    splits = pxl_attn_decode_splits(sp->Bd, Hq, Hkv, D, st->page, 0, sp->d_max_ctx);
     if (splits > 1 && static_cast<int64_t>(sp->Bd) * Hq * splits * (D + 2) > ws->decode_floats) return PXL_ERR_TOO_LARGE;
   }
   // every kernel of the sequence waits (griddepcontrol.wait) before it touches global memory, so each

@@ -89,7 +89,7 @@ class NativeDenseStage:
             w.xn, w.qkv, w.attn, w.act, w.h_a, w.h_b = [b.data_ptr() for b in self._bufs]
             self._cap = cap
         if Bd > 0:
-            splits = self._splits(Bd, d.Hkv, d.D, d.page, d_max_ctx)
+            splits = self._splits(Bd, d.Hq, d.Hkv, d.D, d.page, 0, d_max_ctx)
             need = Bd * d.Hq * splits * (d.D + 2) if splits > 1 else 0
             if self._dec is None or self._dec.numel() < need:
                 self._dec = torch.empty(max(need, 1), dtype=torch.float32, device=self.device)

@@ -81,7 +81,7 @@ _SIGS = {
     "pxl_patch_i32": [_P, _P, _P, _P, c_int, c_int, c_int, _P, _P],
     "pxl_attn_decode": [_P, c_int64, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
                         c_int64, c_float, c_int, c_int, c_int, c_int, c_float, _P, _P, _P],
-    "pxl_attn_decode_splits": [c_int] * 5,
+    "pxl_attn_decode_splits": [c_int] * 7,
     "pxl_attn_decode_launches": [c_int] * 6 + [c_float, c_int],
     "pxl_attn_prefill": [_P, c_int64, _P, _P, _P, _P, _P, _P, c_int64, _P, c_int, c_int, c_int,
                          c_int, c_int, c_int, c_int, c_int64, c_float, c_int, c_int, c_float, _P, _P, _P],

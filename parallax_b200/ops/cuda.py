@@ -477,7 +477,7 @@ def attn_decode(
     if num_splits <= 0:
         # keys a query reads: whole tiles of 64 of the window and of the kept ones
         span = min(max_ctx, window + keep_first + 128) if window > 0 else max_ctx
-        num_splits = _lib.lib().pxl_attn_decode_splits(B, Hkv, D, page, span)
+        num_splits = _lib.lib().pxl_attn_decode_splits(B, Hq, Hkv, D, page, _is_fp8_cache(k_cache), span)
     ws = None
     if num_splits > 1:
         ws = workspace(q.device, "attn_decode", B * Hq * num_splits * (D + 2) * 4)
