@@ -390,11 +390,13 @@ __device__ __forceinline__ void st_shared_cluster_f32x4(uint32_t addr, float a, 
 __device__ __forceinline__ void st_shared_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
-// Every thread of every CTA of the cluster must call this the same number of times (the wait has
-// no timeout); writes made before it are visible cluster-wide after it.
+// Every thread of every CTA of the cluster must call these the same number of times (the wait has
+// no timeout); writes made before the arrival are visible cluster-wide after the wait.
+__device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive_all();
+  cluster_wait_all();
 }
 
 // --- untiled bulk copies (TMA engine, one contiguous span per instruction) -----------------

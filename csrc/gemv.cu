@@ -12,7 +12,9 @@
 namespace {
 using namespace pxl;
 
-constexpr int kWarps = 4;
+constexpr int kWarps = 4, kHeadWarps = 8;
+constexpr int kEpiHeads = 1000;  // a head's norm, rotation and place in the cache behind its product (HeadArgs)
+constexpr int kHeadDim = 128, kHeadCtas = kHeadDim / 2 / kHeadWarps;
 
 struct GemvArgs {
   const bf16 *A, *W, *residual, *bias;
@@ -20,6 +22,19 @@ struct GemvArgs {
   int M, N, K, lda, ldw, ldc;
   const bf16* norm_w;  // NORM: [K]; rows of A times norm_w + norm_offset over their root mean square, rounded to bf16
   float norm_eps, norm_offset;
+};
+
+// The query, key and value heads of a layer, all of 128 columns and rotated over the whole of them: the product's columns i and i + 64
+// of a head are one warp's, so the rotation stays in it, and the eight CTAs of a head, a cluster, pass the warps' sums of squares round.
+struct HeadArgs : GemvArgs {  // C: [M, N], the query heads' columns are written; keys and values go to the cache
+  const bf16 *q_norm, *k_norm;  // [128] or null
+  const float* cos_sin;         // [positions][128]
+  const int* positions;
+  const int64_t* slots;  // or null: no cache
+  bf16 *k_cache, *v_cache;
+  int Hq, Hkv, page_size, max_pos;
+  int64_t num_slots;
+  int* status;
 };
 
 __device__ __forceinline__ uint64_t widen(uint32_t two) {  // two bf16 -> two fp32 in a register pair
@@ -31,17 +46,18 @@ __device__ __forceinline__ uint64_t widen(uint32_t two) {  // two bf16 -> two fp
 // MM rows of A (the last ones repeated where M is smaller), R rows of W per warp, U steps of 256 columns in flight.
 // ONE: K fits one round of U steps, and the rows are held in registers.
 // EPI: PXL_EPI_NONE, _RESIDUAL, _F32 or _SILU_MUL (R rows = R / 2 gate / up pairs, 64 rows apart in groups of 128)
-template <int MM, int R, int U, int EPI, bool NORM, bool ONE>
-__global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
-  constexpr bool kGlu = EPI == PXL_EPI_SILU_MUL;
+template <int MM, int R, int U, int EPI, bool NORM, bool ONE, typename Args>
+__device__ __forceinline__ void gemv_body(const Args& a) {
+  constexpr bool kGlu = EPI == PXL_EPI_SILU_MUL, kHeads = EPI == kEpiHeads;
   const int lane = threadIdx.x & 31, wid = blockIdx.x * kWarps + (threadIdx.x >> 5);
-  const int n0 = wid * R;  // first row of W; pairs: 2 x first output column
+  const int head = blockIdx.x / kHeadCtas, in_head = blockIdx.x % kHeadCtas * kHeadWarps + (threadIdx.x >> 5);  // kHeads
+  const int n0 = kHeads ? head * kHeadDim + in_head : wid * R;  // first row of W; pairs: 2 x first output column
   if (n0 >= a.N) return;
   int row[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int c = n0 / 2 + r / 2;
-    row[r] = kGlu ? c / 64 * 128 + c % 64 + (r & 1) * 64 : n0 + r;
+    row[r] = kHeads ? n0 + r * (kHeadDim / 2) : kGlu ? c / 64 * 128 + c % 64 + (r & 1) * 64 : n0 + r;
   }
   uint4 w[U][R];
   auto load = [&](int k0) {
@@ -67,11 +83,32 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
   constexpr int V = MM * R, kSpan = 32 / V;  // number i of the results ends in lanes [i * kSpan, (i + 1) * kSpan)
   const int oi = lane / kSpan, om = oi / R, orow = oi % R;
   const bool stores = lane % kSpan == 0 && om < a.M && !(kGlu && (orow & 1));
-  const int col = kGlu ? (n0 + orow) / 2 : n0 + orow;
+  const int col = kHeads ? n0 + orow * (kHeadDim / 2) : kGlu ? (n0 + orow) / 2 : n0 + orow;
   const int64_t at = static_cast<int64_t>(om) * a.ldc + col;
   float add_bias = 0.f, add_res = 0.f;
   constexpr bool kEarly = V <= 8;  // (registers)
   if (kEarly && !kGlu && stores && a.bias) add_bias = __bfloat162float(a.bias[col]);
+  [[maybe_unused]] float head_w = 0.f, cs = 1.f, sn = 0.f;
+  [[maybe_unused]] int64_t slot = -1;
+  [[maybe_unused]] bool head_normed = false;
+  if constexpr (kHeads) {
+    const bf16* w = head < a.Hq ? a.q_norm : head < a.Hq + a.Hkv ? a.k_norm : nullptr;
+    head_normed = w != nullptr;
+    // the other CTAs' shared memory is written to later on: they have to have begun
+    if (head_normed) cluster_arrive_all();
+    if (head_normed) head_w = __bfloat162float(w[col - head * kHeadDim]) + a.norm_offset;
+    const int m = om < a.M ? om : a.M - 1, p = a.positions[m];
+    const bool p_ok = p >= 0 && (a.max_pos <= 0 || p < a.max_pos);
+    slot = a.slots ? a.slots[m] : -1;
+    if (p_ok && head < a.Hq + a.Hkv) {  // a position outside the table is reported, its row is left unrotated
+      cs = a.cos_sin[static_cast<int64_t>(p) * kHeadDim + in_head];
+      sn = a.cos_sin[static_cast<int64_t>(p) * kHeadDim + kHeadDim / 2 + in_head];
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 32 && stores && orow == 0 && a.status) {
+      if (slot >= a.num_slots) atomicCAS(a.status, 0, PXL_DEV_BAD_SLOT);
+      if (!p_ok) atomicCAS(a.status, 0, PXL_DEV_BAD_POSITION);
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
   const bf16* rows_a[MM];
@@ -168,6 +205,37 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
     const float up = __shfl_down_sync(0xffffffffu, sum, kSpan);
     sum = sum / (1.f + __expf(-sum)) * up;
   }
+  if constexpr (kHeads) {
+    __shared__ float squares[MM][kHeadDim / 2];  // of columns i and i + 64 of the head
+    float x = __bfloat162float(__float2bfloat16(sum + __shfl_sync(0xffffffffu, add_bias, lane / kSpan * kSpan)));
+    float other = __shfl_xor_sync(0xffffffffu, x, kSpan);
+    if (head_normed) {  // the same in all CTAs of the cluster
+      cluster_wait_all();
+      if (orow == 0 && lane % kSpan < kHeadCtas)
+        st_shared_cluster_f32(cluster_map_shared(smem_u32(&squares[om][in_head]), lane % kSpan), x * x + other * other);
+      cluster_sync_all();
+      float total = 0.f;
+#pragma unroll
+      for (int m = 0; m < MM; ++m) {
+        const float t = warp_reduce_sum(squares[m][lane] + squares[m][lane + 32]);
+        if (m == om) total = t;
+      }
+      const float inv_rms = rsqrtf(total / static_cast<float>(kHeadDim) + a.norm_eps);
+      x = __bfloat162float(__float2bfloat16(x * inv_rms * head_w));  // rounded before the rotation, as a bf16 module does
+      other = __shfl_xor_sync(0xffffffffu, x, kSpan);
+    }
+    const bf16 y = __float2bfloat16(x * cs + (orow == 0 ? -other : other) * sn);
+    if (!stores) return;
+    if (head < a.Hq) {
+      static_cast<bf16*>(a.C)[at] = y;
+    } else if (slot >= 0 && slot < a.num_slots) {
+      const bool is_k = head < a.Hq + a.Hkv;
+      const int kvh = head - a.Hq - (is_k ? 0 : a.Hkv);
+      const int64_t line = (slot / a.page_size * a.Hkv + kvh) * a.page_size + slot % a.page_size;
+      (is_k ? a.k_cache : a.v_cache)[line * kHeadDim + in_head + orow * (kHeadDim / 2)] = y;
+    }
+    return;
+  }
   if (!stores) return;
   if constexpr (!kEarly) {
     if (!kGlu && a.bias) add_bias = __bfloat162float(a.bias[col]);
@@ -180,6 +248,15 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
     if constexpr (EPI == PXL_EPI_RESIDUAL) sum += add_res;
     static_cast<bf16*>(a.C)[at] = __float2bfloat16(sum);
   }
+}
+
+template <int MM, int R, int U, int EPI, bool NORM, bool ONE>
+__global__ void __launch_bounds__(kWarps * 32) gemv_kernel(const GemvArgs a) {
+  gemv_body<MM, R, U, EPI, NORM, ONE>(a);
+}
+template <int MM, bool ONE>
+__global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadWarps * 32, 2) gemv_heads_kernel(const HeadArgs a) {
+  gemv_body<MM, 2, 4, kEpiHeads, true, ONE>(a);
 }
 
 template <int MM, int R, int U, bool ONE>
@@ -258,4 +335,37 @@ PXL_EXPORT int pxl_gemv_bf16_norm(const void* A, const void* norm_w, float eps, 
   return run(GemvArgs{static_cast<const pxl::bf16*>(A), static_cast<const pxl::bf16*>(W), nullptr, static_cast<const pxl::bf16*>(bias),
                       C, M, N, K, lda, ldw, ldc, static_cast<const pxl::bf16*>(norm_w), eps, offset},
              epi, stream);
+}
+
+// One launch for the norm, the product of the q, k and v heads and pxl_qk_norm_rope_cache behind it. The launches are what a layer of one
+// row costs: six of them take the host 3.9 us each, longer than the chip needs; behind the product the rotation is 1 us of a cluster's
+// barrier, where its own kernel takes 2.9.
+PXL_EXPORT int pxl_gemv_bf16_qkv_takes(int M, int K, int Hq, int Hkv, int D, int rot_dim) {
+  return M <= PXL_GEMV_NORM_MAX_M && D == kHeadDim && rot_dim == kHeadDim && Hq > 0 && Hkv > 0 &&
+         pxl_gemv_bf16_takes(M, (Hq + 2 * Hkv) * D, K, PXL_EPI_NONE);
+}
+
+PXL_EXPORT int pxl_gemv_bf16_qkv(const void* A, const void* norm_w, float eps, float offset, const void* W, const void* bias, void* qkv,
+                                 const void* q_norm_w, const void* k_norm_w, const float* cos_sin, const int* positions,
+                                 const int64_t* slot_mapping, void* k_cache, void* v_cache, int M, int K, int Hq, int Hkv, int D,
+                                 int rot_dim, int page_size, int64_t num_slots, int max_pos, int* status, cudaStream_t stream) {
+  using pxl::bf16;
+  if (!pxl_gemv_bf16_qkv_takes(M, K, Hq, Hkv, D, rot_dim) || norm_w == nullptr || page_size <= 0 ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(norm_w)) & 15))
+    return PXL_ERR_INVALID_ARG;
+  HeadArgs a{};
+  a.A = static_cast<const bf16*>(A), a.W = static_cast<const bf16*>(W), a.bias = static_cast<const bf16*>(bias), a.C = qkv;
+  a.M = M, a.N = (Hq + 2 * Hkv) * D, a.K = a.lda = a.ldw = K, a.ldc = a.N;
+  a.norm_w = static_cast<const bf16*>(norm_w), a.norm_eps = eps, a.norm_offset = offset;
+  a.q_norm = static_cast<const bf16*>(q_norm_w), a.k_norm = static_cast<const bf16*>(k_norm_w);
+  a.cos_sin = cos_sin, a.positions = positions, a.slots = slot_mapping;
+  a.k_cache = static_cast<bf16*>(k_cache), a.v_cache = static_cast<bf16*>(v_cache);
+  a.Hq = Hq, a.Hkv = Hkv, a.page_size = page_size, a.max_pos = max_pos, a.num_slots = num_slots, a.status = status;
+  const dim3 grid((Hq + 2 * Hkv) * kHeadCtas), block(kHeadWarps * 32);
+  auto go = [&](auto kern) {
+    pxl_host::launch(kern, grid, block, 0, stream, a);
+    return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
+  };
+  if (M == 1) return K <= 1024 ? go(gemv_heads_kernel<1, true>) : go(gemv_heads_kernel<1, false>);
+  return go(gemv_heads_kernel<2, false>);
 }

@@ -135,7 +135,13 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
     const PxlDenseLayer& L = st->layers[li];
     int op_ = 0;  // 1 norm, 2 qkv, 3 rope+cache, 4 prefill, 5 decode (4 if no prefill), then o_proj, norm, gate_up, down
     void* h_mid = (h == ws->h_a) ? ws->h_b : ws->h_a;
-    if (normed(qkv_n, PXL_EPI_NONE)) {
+    const bool heads = H % 8 == 0 && pxl_gemv_bf16_qkv_takes(T, H, Hq, Hkv, D, st->rot_dim);
+    if (heads) {  // one or two rows: norm, product, rotation and cache in one kernel
+      PXL_TRY(pxl_gemv_bf16_qkv(h, L.ln1, st->eps, st->norm_offset, L.w_qkv, L.b_qkv, qkv, L.q_norm, L.k_norm, st->cos_sin, sp->positions,
+                                sp->slots, L.k_cache, L.v_cache, T, H, Hq, Hkv, D, st->rot_dim, st->page, num_slots, st->max_pos, status,
+                                stream));
+      ++n;
+    } else if (normed(qkv_n, PXL_EPI_NONE)) {
       PXL_TRY(pxl_gemv_bf16_norm(h, L.ln1, st->eps, st->norm_offset, L.w_qkv, qkv, L.b_qkv, T, qkv_n, H, H, H, qkv_n, PXL_EPI_NONE,
                                  stream));
       --n;
@@ -143,10 +149,12 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
       PXL_TRY(pxl_rmsnorm(h, L.ln1, ws->xn, nullptr, T, H, st->eps, st->norm_offset, stream));
       PXL_TRY(pxl_gemm_bf16(ws->xn, L.w_qkv, qkv, nullptr, L.b_qkv, T, qkv_n, H, H, H, qkv_n, PXL_EPI_NONE, 0, status, stream));
     }
-    PXL_TRY(pxl_qk_norm_rope_cache(qkv, L.q_norm, L.k_norm, st->cos_sin, sp->positions, sp->slots, L.k_cache,
-                                   L.v_cache, T, Hq, Hkv, D, st->rot_dim, st->page, num_slots, st->eps,
-                                   st->norm_offset, st->max_pos, status, stream));
-    n += 2 + pxl_gemm_bf16_launches(T, qkv_n, H, PXL_EPI_NONE);
+    if (!heads) {
+      PXL_TRY(pxl_qk_norm_rope_cache(qkv, L.q_norm, L.k_norm, st->cos_sin, sp->positions, sp->slots, L.k_cache,
+                                     L.v_cache, T, Hq, Hkv, D, st->rot_dim, st->page, num_slots, st->eps,
+                                     st->norm_offset, st->max_pos, status, stream));
+      n += 2 + pxl_gemm_bf16_launches(T, qkv_n, H, PXL_EPI_NONE);
+    }
     if (sp->Tp > 0) {
       if (prefill_tc) {
         PXL_TRY(pxl_attn_prefill_tc(qkv, qkv_n, L.k_cache, L.v_cache, sp->p_bt, sp->p_cu_q, sp->p_ctx, attn,
