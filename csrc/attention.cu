@@ -378,53 +378,64 @@ attn_decode_kernel(const bf16* __restrict__ q, int64_t q_stride, const void* __r
 // consumer warp), so the consumer warps never meet at a CTA-wide barrier inside the loop: with the
 // producer inside warp 0 and a __syncthreads per tile the top stall was that barrier.
 // ---- split-KV results met inside a thread-block cluster (2 to 8 splits of few sequences: splits_together): the CTAs of a
-// (sequence, key head) leave their partial outputs, maxima and sums in shared memory, and each adds a share of the columns over all
-// of them. Saves the workspace's round trip and a kernel whose launch is most of its 4 to 5 us, once per layer of a chat.
+// (sequence, key head) write their partial outputs, maxima and sums into each other's shared memory, a share of the columns to each,
+// and each adds up what it got. Saves the workspace's round trip and a kernel whose launch is most of its 4 to 5 us, once per layer of
+// a chat. Written rather than read: one barrier instead of two and no remote load's latency (1 x 777 keys in 7 splits: 6.5 us, 5.5 now).
 constexpr int kMaxClusterSplits = 8;
 
-__device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_map_shared(smem_u32(p), rank)) : "memory");
-  return v;
-}
+struct SplitParts {  // in shared memory that nothing else uses: the other CTAs write to it while this one is still at its keys
+  float* base;       // [splits][share], then maxima and sums [kMaxClusterSplits][16]
+  int splits, rank, share;
+  static constexpr int kOut = 16 * 128 + kMaxClusterSplits, kFloats = kOut + 2 * kMaxClusterSplits * 16;
 
-// part_o [G][128] relative to the maxima part_m [G], sums part_l [G] (scaled by 2^shift, like part_o). Every thread of every CTA of
-// the cluster calls this, also after a failed wait.
-template <int SM>
-__device__ __forceinline__ void add_splits(const float* part_o, const float* part_m, const float* part_l, int splits, int rank, int G,
-                                           int head0, const float* sinks, float shift, float v_scale, bf16* out) {
-  constexpr int D = 128;
-  cluster_sync_all();
-  const int share = ceil_div(G * D, splits), end = min(G * D, (rank + 1) * share);
-  for (int idx = rank * share + threadIdx.x; threadIdx.x < 128 && idx < end; idx += 128) {
-    const int r = idx / D, head = head0 + r;
-    float acc = 0.f;
-    if constexpr (SM == kSigmoid) {
-      for (int s = 0; s < splits; ++s) acc += ld_cluster_f32(part_o + idx, s);
-      out[static_cast<size_t>(head) * D + idx % D] = __float2bfloat16(acc);
-    } else {
-      const float sink = sinks ? sinks[head] * kLog2e : -INFINITY;
-      float m[kMaxClusterSplits], M = sink;
-#pragma unroll
-      for (int s = 0; s < kMaxClusterSplits; ++s) {
-        m[s] = s < splits ? ld_cluster_f32(part_m + r, s) : -INFINITY;
-        M = fmaxf(M, m[s]);
-      }
-      const float Mu = (M == -INFINITY) ? 0.f : M;
-      float denom = exp2f(sink - Mu + shift);
-#pragma unroll
-      for (int s = 0; s < kMaxClusterSplits; ++s) {
-        if (s >= splits) break;
-        const float f = exp2f(m[s] - Mu);
-        denom += ld_cluster_f32(part_l + r, s) * f;
-        acc += ld_cluster_f32(part_o + idx, s) * f;
-      }
-      out[static_cast<size_t>(head) * D + idx % D] = __float2bfloat16(denom > 0.f ? acc / denom * v_scale : 0.f);
+  __device__ __forceinline__ SplitParts(void* at, int splits, int rank, int G)
+      : base(static_cast<float*>(at)), splits(splits), rank(rank), share(ceil_div(G * 128, splits)) {}
+  __device__ __forceinline__ void put(int at, int to, float v) const { st_shared_cluster_f32(cluster_map_shared(smem_u32(base + at), to), v); }
+  // element d of row r of this CTA's partial output, relative to the row's maximum M, and its sum L (both scaled by 2^shift)
+  __device__ __forceinline__ void give(int r, int d, float acc, float M, float L) const {
+    const int idx = r * 128 + d, to = idx / share;
+    put(rank * share + idx - to * share, to, acc);
+    if (d < splits) {
+      put(kOut + rank * 16 + r, d, M);
+      put(kOut + (kMaxClusterSplits + rank) * 16 + r, d, L);
     }
   }
-  __syncwarp();
-  cluster_sync_all();  // nobody leaves while its parts are being read
-}
+  // Every thread of every CTA of the cluster calls this, also after a failed wait.
+  template <int SM>
+  __device__ __forceinline__ void add(int G, int head0, const float* sinks, float shift, float v_scale, bf16* out, bool failed) const {
+    constexpr int D = 128;
+    __syncwarp();
+    cluster_sync_all();
+    if (failed || threadIdx.x >= 128) return;
+    const int end = min(share, G * D - rank * share);
+    for (int j = threadIdx.x; j < end; j += 128) {
+      const int idx = rank * share + j, r = idx / D, head = head0 + r;
+      float acc = 0.f;
+      if constexpr (SM == kSigmoid) {
+        for (int s = 0; s < splits; ++s) acc += base[s * share + j];
+        out[static_cast<size_t>(head) * D + idx % D] = __float2bfloat16(acc);
+      } else {
+        const float sink = sinks ? sinks[head] * kLog2e : -INFINITY;
+        float m[kMaxClusterSplits], M = sink;
+#pragma unroll
+        for (int s = 0; s < kMaxClusterSplits; ++s) {
+          m[s] = s < splits ? base[kOut + s * 16 + r] : -INFINITY;
+          M = fmaxf(M, m[s]);
+        }
+        const float Mu = (M == -INFINITY) ? 0.f : M;
+        float denom = exp2f(sink - Mu + shift);
+#pragma unroll
+        for (int s = 0; s < kMaxClusterSplits; ++s) {
+          if (s >= splits) break;
+          const float f = exp2f(m[s] - Mu);
+          denom += base[kOut + (kMaxClusterSplits + s) * 16 + r] * f;
+          acc += base[s * share + j] * f;
+        }
+        out[static_cast<size_t>(head) * D + idx % D] = __float2bfloat16(denom > 0.f ? acc / denom * v_scale : 0.f);
+      }
+    }
+  }
+};
 
 // Producer warp: the blocks of the pages of 32 / (pages per tile) tiles at a time, one per lane, the next ones read while these are
 // used. Read tile by tile, the latency of a table read was the time of a tile: 1.2 us (e4m3 0.7) with one CTA per SM, whatever the
@@ -593,6 +604,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   const int* bt = block_tables + static_cast<size_t>(b) * max_blocks;
   const int shift = page_size == 16 ? 2 : page_size == 32 ? 1 : 0, ppt = 1 << shift;  // pages per tile
 
+  if constexpr (CLUSTER) cluster_arrive_all();  // its shared memory may be written to from here on
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < kDecStages; ++s) {
@@ -657,12 +669,13 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * stage);  // this warp is done with the stage
   }
+  const SplitParts parts(bars + 16, num_splits, split, G);
   if (__syncthreads_or(failed)) {
     // loads that are still in flight must land before the CTA's shared memory is released
     __nanosleep(200000);
     if constexpr (CLUSTER) {  // the other CTAs of the cluster wait for this one
-      cluster_sync_all();
-      cluster_sync_all();
+      cluster_wait_all();
+      parts.add<SM>(G, kvh * G, sinks, 0.f, 1.f, out, true);
     }
     return;
   }
@@ -679,10 +692,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) {
       const int c = i * 8 + 2 * (lane & 3);
-      ow[r_lo * D + c] = o[i][0];
-      ow[r_lo * D + c + 1] = o[i][1];
-      ow[r_hi * D + c] = o[i][2];
-      ow[r_hi * D + c + 1] = o[i][3];
+      *reinterpret_cast<float2*>(ow + r_lo * D + c) = make_float2(o[i][0], o[i][1]);
+      if constexpr (HIGH) *reinterpret_cast<float2*>(ow + r_hi * D + c) = make_float2(o[i][2], o[i][3]);
     }
     if ((lane & 3) == 0) {
       m_sm[warp * 16 + r_lo] = m_run[0];
@@ -691,8 +702,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       l_sm[warp * 16 + r_hi] = l_run[1];
     }
   }
-  float* part_o = l_sm + 4 * 16;  // [16][D]: behind the warps' results
-  float *part_m = part_o + 16 * D, *part_l = part_m + 16;
+  __syncwarp();
+  if constexpr (CLUSTER) cluster_wait_all();
   __syncthreads();
   for (int idx = threadIdx.x; warp < 4 && idx < G * D; idx += 128) {
     const int r = idx / D, d = idx % D;
@@ -702,7 +713,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 #pragma unroll
       for (int w = 0; w < 4; ++w) acc += o_sm[(w * 16 + r) * D + d];
       if constexpr (CLUSTER) {
-        part_o[idx] = acc;
+        parts.give(r, d, acc, 0.f, 0.f);
         continue;
       }
       if (num_splits == 1) out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(acc);
@@ -723,8 +734,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       acc += o_sm[(w * 16 + r) * D + d] * f;
     }
     if constexpr (CLUSTER) {
-      part_o[idx] = acc;
-      if (d == 0) part_m[r] = M, part_l[r] = L;
+      parts.give(r, d, acc, M, L);
     } else if (num_splits == 1) {
       const float denom = L + exp2f(sink - Mu);
       out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(denom > 0.f ? acc / denom : 0.f);
@@ -736,10 +746,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       if (d == 0) plse[row] = L > 0.f ? Mu + log2f(L) : -INFINITY;
     }
   }
-  if constexpr (CLUSTER) {
-    __syncwarp();
-    add_splits<SM>(part_o, part_m, part_l, num_splits, split, G, kvh * G, sinks, 0.f, 1.f, out + static_cast<size_t>(b) * Hq * D);
-  }
+  if constexpr (CLUSTER) parts.add<SM>(G, kvh * G, sinks, 0.f, 1.f, out + static_cast<size_t>(b) * Hq * D, false);
 }
 
 // ---- decode over e4m3 pages, TMA-fed (D = 128; page_size 16, 32 or 64) -------------------------------------
@@ -956,6 +963,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   const int* bt = block_tables + static_cast<size_t>(b) * max_blocks;
   const int shift = page_size == 16 ? 2 : page_size == 32 ? 1 : 0, ppt = 1 << shift;  // pages per tile
 
+  if constexpr (CLUSTER) cluster_arrive_all();  // its shared memory may be written to from here on
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < kE4Stages; ++s) {
@@ -1019,12 +1027,13 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     __syncwarp();
     if (lane == 0) mbar_arrive(empty0 + 8 * stage);  // this warp is done with the stage
   }
+  const SplitParts parts(bars + 16, num_splits, split, G);
   if (__syncthreads_or(failed)) {
     // loads that are still in flight must land before the CTA's shared memory is released
     __nanosleep(200000);
     if constexpr (CLUSTER) {  // the other CTAs of the cluster wait for this one
-      cluster_sync_all();
-      cluster_sync_all();
+      cluster_wait_all();
+      parts.add<kPlain>(G, kvh * G, sinks, 0.f, 1.f, out, true);
     }
     return;
   }
@@ -1041,7 +1050,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     for (int i = 0; i < D / 8; i += 2) {  // accumulator columns 2 t, 2 t + 1 of an even and an odd tile: columns 4 t .. 4 t + 3
       const int c = i * 8 + t4 * 4;
       *reinterpret_cast<float4*>(ow + g8 * D + c) = make_float4(o[i][0], o[i + 1][0], o[i][1], o[i + 1][1]);
-      *reinterpret_cast<float4*>(ow + (g8 + 8) * D + c) = make_float4(o[i][2], o[i + 1][2], o[i][3], o[i + 1][3]);
+      if constexpr (HIGH) *reinterpret_cast<float4*>(ow + (g8 + 8) * D + c) = make_float4(o[i][2], o[i + 1][2], o[i][3], o[i + 1][3]);
     }
     if (t4 == 0) {
       m_sm[warp * 16 + g8] = m_run[0];
@@ -1050,8 +1059,8 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       l_sm[warp * 16 + g8 + 8] = l_run[1];
     }
   }
-  float* part_o = l_sm + 4 * 16;  // [16][D]: behind the warps' results
-  float *part_m = part_o + 16 * D, *part_l = part_m + 16;
+  __syncwarp();
+  if constexpr (CLUSTER) cluster_wait_all();
   __syncthreads();
   for (int idx = threadIdx.x; warp < 4 && idx < G * D; idx += 128) {
     const int r = idx / D, d = idx % D;
@@ -1070,8 +1079,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       acc += o_sm[(w * 16 + r) * D + d] * f;
     }
     if constexpr (CLUSTER) {
-      part_o[idx] = acc;
-      if (d == 0) part_m[r] = M, part_l[r] = L;
+      parts.give(r, d, acc, M, L);
     } else if (num_splits == 1) {
       const float denom = L + exp2f(sink - Mu + kPShift);
       out[(static_cast<size_t>(b) * Hq + head) * D + d] = __float2bfloat16(denom > 0.f ? acc / denom * v_scale : 0.f);
@@ -1083,10 +1091,7 @@ attn_decode_e4m3_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       if (d == 0) plse[row] = L > 0.f ? Mu + log2f(L) - kPShift : -INFINITY;
     }
   }
-  if constexpr (CLUSTER) {
-    __syncwarp();
-    add_splits<kPlain>(part_o, part_m, part_l, num_splits, split, G, kvh * G, sinks, kPShift, v_scale, out + static_cast<size_t>(b) * Hq * D);
-  }
+  if constexpr (CLUSTER) parts.add<kPlain>(G, kvh * G, sinks, kPShift, v_scale, out + static_cast<size_t>(b) * Hq * D, false);
 }
 
 // ---- decode of many rows: every CTA the same number of tiles ------------------------------------------------------
@@ -1706,7 +1711,8 @@ PXL_EXPORT int pxl_attn_decode_splits(int B, int Hq, int Hkv, int D, int page_si
 }
 
 namespace {
-constexpr int kDecSmem = 1024 + kDecStages * 2 * TILE * 128 * 2 + 128, kE4Smem = 1024 + kE4Stages * 2 * kE4Tile + 128;
+constexpr int kDecSmem = 1024 + kDecStages * 2 * TILE * 128 * 2 + 128 + SplitParts::kFloats * 4,
+              kE4Smem = 1024 + kE4Stages * 2 * kE4Tile + 128 + SplitParts::kFloats * 4;
 
 // Clusters of `splits` CTAs of a kernel that are on the chip at once; asked for once per device and size.
 template <auto Kernel>
