@@ -1150,10 +1150,37 @@ namespace {
 int box_rows(int M) { return M < BM ? pxl::ceil_div(M, 8) * 8 : BM; }
 }  // namespace
 
+namespace {
+constexpr int kMidMaxM = 1024;
+
+// Cost model (microseconds) of one launch of up to kMidMaxM rows, fitted to CUDA-event timings of eleven shapes at 144 to 1016 rows in a
+// chain of launches (weights streamed from HBM):
+//   plain persistent kernel   rounds x (k-blocks x t_kb) + fixed
+//   cluster split-K           k-blocks per CTA x t_kb + exchange (of partial sums)
+// t_kb = time of one 64-deep k-block per CTA, set by what the SM can pull from L2, 64 bytes a clock (48 KB per k-block for a
+// 128 x 256 tile, 32 KB for 128 x 128). Split variants are only considered when all clusters are resident at once (a second round
+// pays the fixed cost again and was always slower: 144 CTAs in clusters of 3, which pack the GPCs badly, are one).
+// The choice is within 5 % of the fastest of all variants in all 132. Against the figures before the issuing warps' loops
+// were shortened (0.43, 0.29, 0.36 and 7; no clusters of 3, no 64 columns): 256 rows x 2112 x 7168 18.8 -> 16.0 us, 4096 x 12288
+// 34.2 -> 31.7, gated 24576 x 4096 60.2 -> 53.4.
+struct MidWidth {
+  int bn;
+  double kb, fixed, exchange, exchange_each;  // exchange < 0: no cluster variant of this width
+};
+constexpr MidWidth kMidWidths[4] = {{256, 0.365, 4.0, 9.0, 1.5}, {128, 0.228, 2.7, 7.5, 0.0}, {192, 0.345, 3.0, -1.0, 0.0}, {64, 0.19, 2.7, -1.0, 0.0}};
+
+double mid_plain_cost(int M, int N, int K, const MidWidth& w) {
+  const int tiles = pxl::ceil_div(M, BM) * pxl::ceil_div(N, w.bn);
+  return pxl::ceil_div(tiles, pxl_host::num_sms()) * (pxl::ceil_div(K, BK) * w.kb) + w.fixed;
+}
+}  // namespace
+
 // Tile width heuristic: estimated time = waves over the SMs x tile width / relative throughput of
 // that width (measured on compute-bound shapes: a 256-wide tile keeps the tensor pipe busiest, a
 // 64-wide one reaches about a third of it). Large problems take the width that wastes the least of
-// the last wave; problems with few tiles end up with narrow ones, which put more SMs to work.
+// the last wave; problems with few tiles end up with narrow ones, which put more SMs to work. Up to kMidMaxM rows the figures of the
+// cost model above are taken (at K = 4096: its fixed parts weigh little): gated 24576 x 4096, 256 rows 60.2 us in tiles of 256 columns,
+// 53.4 in tiles of 128.
 PXL_EXPORT int pxl_gemm_bf16_pick_bn(int M, int N, int epi) {
   const int sms = pxl_host::num_sms();
   const int num_m = pxl::ceil_div(M, BM);
@@ -1167,7 +1194,10 @@ PXL_EXPORT int pxl_gemm_bf16_pick_bn(int M, int N, int epi) {
     if (epi == PXL_EPI_SILU_MUL && ((N % bn) != 0 || bn < 128 || bn == 192)) continue;
     if (bn == 192 && !plain) continue;
     const int tiles = num_m * pxl::ceil_div(N, bn);
-    const double cost = static_cast<double>(pxl::ceil_div(tiles, sms)) * bn / eff[i];
+    double cost = static_cast<double>(pxl::ceil_div(tiles, sms)) * bn / eff[i];
+    if (M <= kMidMaxM)
+      for (const MidWidth& w : kMidWidths)
+        if (w.bn == bn) cost = mid_plain_cost(M, N, 4096, w);
     if (cost < best_cost) {
       best_cost = cost;
       best = bn;
@@ -1354,7 +1384,6 @@ int gemm_small_m(const void* A, const void* W, void* C, bool f32_out, const void
 
 namespace {
 // ---- mid-M path: 129 .. kMidMaxM tokens, operands in their usual slots, K split inside a cluster ----
-constexpr int kMidMaxM = 1024;
 
 int mid_m_max_clusters(int bn, int cluster) {
   static int cache[64][2][9];
@@ -1378,45 +1407,35 @@ int mid_m_max_clusters(int bn, int cluster) {
   return cache[dev][bi][cluster];
 }
 
-// Cost model (microseconds) of one launch, fitted to CUDA-event timings of the four Qwen3-8B projection
-// shapes at 192 / 320 / 512 rows (weights streamed from HBM):
-//   plain persistent kernel   rounds x (k-blocks x t_kb) + 7
-//   cluster split-K           k-blocks per CTA x t_kb + 8 + splitk x bn / 128   (exchange of partial sums)
-// t_kb = time of one 64-deep k-block per CTA, set by what the SM can pull from L2 (48 KB per k-block for a
-// 128 x 256 tile, 32 KB for 128 x 128). Split variants are only considered when all clusters are resident at
-// once (a second round pays the fixed cost again and was always slower) and for 2 or 4 K ranges (clusters of
-// 3 pack the GPCs badly: 144 CTAs in clusters of 3 ran as slowly as two rounds).
 struct MidPlan {
   int bn, splitk;
   double cost;
 };
-constexpr int kPlanBns[3] = {256, 128, 192};
-constexpr double kPlanKb[3] = {0.43, 0.29, 0.36};  // t_kb
-
-double plain_cost(int M, int N, int K, int i) {  // tiles of kPlanBns[i] columns
-  const int tiles = pxl::ceil_div(M, BM) * pxl::ceil_div(N, kPlanBns[i]);
-  return pxl::ceil_div(tiles, pxl_host::num_sms()) * (pxl::ceil_div(K, BK) * kPlanKb[i]) + 7.0;
-}
-
 MidPlan mid_m_plan(int M, int N, int K) {
   const int num_kb = pxl::ceil_div(K, BK);
   const int num_m = pxl::ceil_div(M, BM);
   MidPlan best{0, 1, 1e300};
-  for (int i = 0; i < 3; ++i) {
-    const int bn = kPlanBns[i], tiles = num_m * pxl::ceil_div(N, bn);
-    const double plain = plain_cost(M, N, K, i);
-    if (plain < best.cost) best = MidPlan{bn, 1, plain};
-    if (bn == 192) continue;  // the cluster variant exists for 128- and 256-wide tiles
-    for (int sk = 2; sk <= 4; sk += 2) {
+  for (const MidWidth& w : kMidWidths) {
+    const int tiles = num_m * pxl::ceil_div(N, w.bn);
+    const double plain = mid_plain_cost(M, N, K, w);
+    if (plain < best.cost) best = MidPlan{w.bn, 1, plain};
+    if (w.exchange < 0) continue;
+    for (int sk = 2; sk <= 4; ++sk) {
       if (num_kb / sk < 4) break;
       const int kb_per = pxl::ceil_div(num_kb, sk);
       if (pxl::ceil_div(num_kb, kb_per) != sk) continue;  // no empty K range
-      if (tiles > mid_m_max_clusters(bn, sk)) continue;
-      const double cost = kb_per * kPlanKb[i] + 8.0 + sk * (bn / 128);
-      if (cost < best.cost) best = MidPlan{bn, sk, cost};
+      if (tiles > mid_m_max_clusters(w.bn, sk)) continue;
+      const double cost = kb_per * w.kb + w.exchange + sk * w.exchange_each;
+      if (cost < best.cost) best = MidPlan{w.bn, sk, cost};
     }
   }
   return best;
+}
+
+// Many rounds, where all SMs pull at once and the tensor cores and the power limit are near: us per k-block of 256 and 192 columns.
+double plain_cost(int M, int N, int K, int bn) {
+  const int tiles = pxl::ceil_div(M, BM) * pxl::ceil_div(N, bn);
+  return pxl::ceil_div(tiles, pxl_host::num_sms()) * (pxl::ceil_div(K, BK) * (bn == 256 ? 0.43 : 0.36)) + 7.0;
 }
 
 bool mid_m_disabled() {
@@ -1430,7 +1449,7 @@ bool mid_m_disabled() {
 int rows_ahead_of_the_tail(int M, int N, int K, int epi) {
   if (M <= kMidMaxM || (epi != PXL_EPI_NONE && epi != PXL_EPI_RESIDUAL && epi != PXL_EPI_F32) || mid_m_disabled()) return M;
   const int sms = pxl_host::num_sms(), num_n = pxl::ceil_div(N, 256);
-  auto plain = [&](int rows) { return std::min(plain_cost(rows, N, K, 0), plain_cost(rows, N, K, 2)); };
+  auto plain = [&](int rows) { return std::min(plain_cost(rows, N, K, 256), plain_cost(rows, N, K, 192)); };
   const int ahead = pxl::ceil_div(M, BM) * num_n / sms * sms / num_n * BM;
   const int tail = M - ahead;
   if (ahead <= 0 || tail <= 0 || tail > kMidMaxM) return M;
@@ -1514,6 +1533,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
     if (plan > 0 && (plan & 15) > 1)
       return gemm_mid_m(A, W, C, epi == PXL_EPI_F32, epi == PXL_EPI_RESIDUAL ? residual : nullptr, bias, M, N, K, lda,
                         ldw, ldc, plan >> 4, plan & 15, status, stream);
+    if (plan > 0) bn = plan >> 4;
   }
   if (bn == 0) {
     const int ahead = rows_ahead_of_the_tail(M, N, K, epi);
