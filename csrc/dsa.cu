@@ -9,6 +9,7 @@
 // without sorting.
 #include "common.cuh"
 #include "pxl_api.h"
+#include "tc_issue.cuh"
 
 namespace {
 using namespace pxl;
@@ -30,7 +31,7 @@ __device__ __forceinline__ int find_seq(const int* cu_q, int B, int t) {
 // One CTA scores 128 keys for a group of consecutive tokens. Keys are the rows of the products and index heads the columns: a
 // warp keeps the fragments of its 32 keys in registers for as long as the tokens are of one sequence (a token costs its queries,
 // 16 KB of shared memory, and no key is read again), and the weighted sum over the heads stays inside a thread up to two
-// shuffles. With a CTA per token and 64 keys, queries and keys were loaded anew for each 64 x 64 product and the sum over the
+// shuffles. (Decoded tokens, other numbers of heads; prompts of 32 or 64 heads: dsa_scores_tc_kernel.) With a CTA per token and 64 keys, queries and keys were loaded anew for each 64 x 64 product and the sum over the
 // heads went through shuffles of every accumulator and shared-memory atomics: 640 us for 1000 tokens x 5500 keys beside 16 x 8000,
 // 324 us this way.
 constexpr int kScoreKeys = 128, kScoreThreads = 128;
@@ -142,6 +143,203 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
       }
   }
   cp_async_wait<0>();
+}
+
+// ---- the same on the 5th-generation tensor cores: prompts, 32 or 64 index heads -----------------------------------
+// 256 keys, two accumulators of 128 rows, stay in shared memory; the queries of 128 / HI tokens are the 128 columns of a product and
+// stream past them, 32 KB per 1024 clocks of products (a single accumulator of keys would take 64 bytes a clock, all that an SM gets
+// from L2). A thread of the sixteen warps behind the products has one key and half of the tokens: 64 columns of its row, clipped, times the heads'
+// weights, no exchange. Two pairs of accumulators, so that sums and products overlap: 256 columns x 2 of tensor memory. Warp 0 loads queries,
+// warp 1 issues products; the keys come through the other warps, whose waits for the last product also free them. Bound by the
+// products, 54 us for the 90 GFLOP of 1000 tokens x 5500 keys at the rate of plain ones, and by the 2.5 instructions per score of the
+// other warps, which take as long: 287 us with mma.sync, 115 with eight such warps, 99 now (0.91 PFLOP/s); 4096 x 14336 2909 and 992;
+// 32 heads 284 and 60.
+constexpr int kTcTokens = 16;  // smallest prompt
+constexpr int kTcKeys = 256, kTcCols = 128, kTcStages = 3, kTcWarps = 16, kTcThreads = 64 + 32 * kTcWarps;
+struct TcScoreSmem {
+  uint8_t k[2][2][128 * 128];             // [accumulator][half of the columns]: 128-byte swizzled rows
+  uint8_t q[kTcStages][2][kTcCols * 128];
+  uint64_t qfull[kTcStages], qempty[kTcStages], afull[2], aempty[2], keys;
+  uint32_t tmem;
+  int abort_flag;
+};
+
+// The tokens [first, last) of a CTA: runs of one sequence, and of those, tiles of TOK tokens that see some key of the CTA.
+template <int TOK, typename Run, typename Tile>
+__device__ __forceinline__ void score_tiles(const int* positions, const int* cu_q, int B, int first, int last, int j0, Run run, Tile tile) {
+  for (int t = first; t < last;) {
+    const int seq = find_seq(cu_q, B, t), end = min(max(cu_q[seq + 1], t + 1), last);
+    if (!run(seq, t, end)) return;
+    for (int i = t; i < end; i += TOK) {
+      bool seen = false;
+#pragma unroll
+      for (int e = 0; e < TOK; ++e) seen |= i + e < end && __ldg(positions + i + e) >= j0;
+      if (!tile(i, min(TOK, end - i), seen)) return;
+    }
+    t = end;
+  }
+}
+
+template <int HI>
+__global__ void __launch_bounds__(kTcThreads, 1)
+dsa_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const float* __restrict__ w, const bf16* __restrict__ cache,
+                     const int* __restrict__ block_tables, const int* __restrict__ cu_q, const int* __restrict__ positions,
+                     float* __restrict__ scores, int64_t ld_scores, int width, int T, int B, int max_blocks, int page, int group,
+                     int* status) {
+  constexpr int TOK = kTcCols / HI;
+  extern __shared__ uint8_t raw[];
+  TcScoreSmem& sm = *reinterpret_cast<TcScoreSmem*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j0 = blockIdx.x * kTcKeys;
+  const int first = (gridDim.y - 1 - blockIdx.y) * group, last = min(T, first + group);  // late tokens, which see the most, begin
+  volatile int* abort_flag = &sm.abort_flag;
+  if (threadIdx.x == 0) {
+    sm.abort_flag = 0;
+    for (int i = 0; i < kTcStages; ++i) mbar_init(smem_u32(&sm.qfull[i]), 1), mbar_init(smem_u32(&sm.qempty[i]), 1);
+    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&sm.afull[i]), 1), mbar_init(smem_u32(&sm.aempty[i]), kTcWarps);
+    mbar_init(smem_u32(&sm.keys), kTcWarps);
+    mbar_fence_init();
+    fence_proxy_async_smem();
+    tma_prefetch_desc(&tm_q);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&sm.tmem), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = sm.tmem;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  bool ok = true;
+  if (warp == 0) {
+    const uint32_t leader = elect_leader();
+    int stage = 0;
+    uint32_t phase = 1;
+    score_tiles<TOK>(positions, cu_q, B, first, last, j0, [&](int, int, int) { return true; }, [&](int t, int, bool seen) {
+      if (!seen) return true;
+      const uint32_t full = smem_u32(&sm.qfull[stage]);
+      ok = wait_warp(smem_u32(&sm.qempty[stage]), phase, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY);
+      if (!ok) return false;
+      expect_tx(full, 2 * kTcCols * 128, leader);
+      tma_box(smem_u32(sm.q[stage][0]), &tm_q, full, 0, t * HI, leader);
+      tma_box(smem_u32(sm.q[stage][1]), &tm_q, full, 64, t * HI, leader);
+      if (++stage == kTcStages) stage = 0, phase ^= 1;
+      return true;
+    });
+  } else if (warp == 1) {
+    const uint32_t leader = elect_leader();
+    constexpr uint32_t idesc = umma_idesc(128, kTcCols, 1, 1);
+    const uint64_t dk = umma_desc_k_sw128(smem_u32(sm.k)), dq = umma_desc_k_sw128(smem_u32(sm.q));
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, aphase = 1, kphase = 0;
+    bool fresh = true;
+    score_tiles<TOK>(positions, cu_q, B, first, last, j0,
+                     [&](int, int, int) {
+                       fresh = true;
+                       return true;
+                     },
+                     [&](int, int, bool seen) {
+                       if (!seen) return true;
+                       if (fresh) {
+                         ok = wait_warp(smem_u32(&sm.keys), kphase, abort_flag, status, PXL_DEV_TIMEOUT_FULL);
+                         kphase ^= 1;
+                         fresh = false;
+                       }
+                       ok = ok && wait_warp(smem_u32(&sm.aempty[buf]), aphase, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_EMPTY);
+                       ok = ok && wait_warp(smem_u32(&sm.qfull[stage]), phase, abort_flag, status, PXL_DEV_TIMEOUT_FULL);
+                       if (!ok) return false;
+                       tc_fence_after_sync();
+                       const uint64_t b = dq + stage * (2 * kTcCols * 128 >> 4);
+#pragma unroll
+                       for (int m = 0; m < 2; ++m)
+#pragma unroll
+                         for (int k = 0; k < 8; ++k)
+                           mma_ss(tmem + (buf * 2 + m) * kTcCols, dk + ((m * 2 + k / 4) * 128 * 128 >> 4) + (k & 3) * 2,
+                                  b + ((k / 4) * kTcCols * 128 >> 4) + (k & 3) * 2, idesc, k > 0 ? 1u : 0u, leader);
+                       commit(smem_u32(&sm.qempty[stage]), leader);
+                       commit(smem_u32(&sm.afull[buf]), leader);
+                       if (++stage == kTcStages) stage = 0, phase ^= 1;
+                       buf ^= 1;
+                       if (buf == 0) aphase ^= 1;
+                       return true;
+                     });
+  } else {
+    const int m = (warp - 2) >> 2 & 1, e0 = (warp - 2) / 8 * (TOK / 2), row = m * 128 + (warp & 3) * 32 + lane, j = j0 + row;  // warp % 4: the lanes of tensor memory
+    const int tid = threadIdx.x - 64;
+    int buf = 0;
+    uint32_t aphase = 0;
+    score_tiles<TOK>(
+        positions, cu_q, B, first, last, j0,
+        [&](int seq, int t, int end) {  // the keys of a sequence, as far as these tokens see; all products with the last ones are done
+          int limit = -1;
+          for (int i = t + lane; i < end; i += 32) limit = max(limit, positions[i]);
+          limit = __reduce_max_sync(0xffffffffu, limit);
+          if (limit < j0) return true;
+          const int* bt = block_tables + static_cast<size_t>(seq) * max_blocks;
+#pragma unroll 4
+          for (int c = tid; c < kTcKeys * (kDi / 8); c += 32 * kTcWarps) {
+            const int r = c / (kDi / 8), ch = c % (kDi / 8), kp = j0 + r;
+            const bf16* src = cache;
+            if (kp <= limit) src = cache + (static_cast<size_t>(bt[kp / page]) * page + kp % page) * kDi + ch * 8;
+            cp_async_16(smem_u32(sm.k[r >> 7][ch >> 3]) + (r & 127) * 128 + (((ch & 7) ^ (r & 7)) << 4), src, kp <= limit);
+          }
+          cp_async_commit();
+          cp_async_wait<0>();
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sm.keys));
+          return true;
+        },
+        [&](int t, int n, bool seen) {
+          float* out = scores + static_cast<size_t>(t) * ld_scores + j;
+          if (!seen) {
+            for (int e = e0; e < e0 + TOK / 2; ++e)
+              if (e < n && j < width) out[e * ld_scores] = -INFINITY;
+            return true;
+          }
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sm.afull[buf]), aphase, abort_flag, status, PXL_DEV_TIMEOUT_TMEM_FULL)) != 0;
+          if (!ok) return false;
+          tc_fence_after_sync();
+          const uint32_t acc = tmem + (buf * 2 + m) * kTcCols + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll
+          for (int i = 0; i < TOK / 2; ++i) {
+            const int e = e0 + i, te = min(t + e, T - 1);
+            const float4* wt = reinterpret_cast<const float4*>(w + static_cast<size_t>(te) * HI);
+            float sum[4] = {};
+#pragma unroll
+            for (int c = 0; c < HI; c += 32) {
+              uint32_t r[32];
+              tmem_ld_32x32b_x32(acc + e * HI + c, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int v = 0; v < 8; ++v) {
+                const float4 f = __ldg(wt + c / 4 + v);
+                sum[0] = fmaf(fmaxf(__uint_as_float(r[4 * v]), 0.f), f.x, sum[0]);
+                sum[1] = fmaf(fmaxf(__uint_as_float(r[4 * v + 1]), 0.f), f.y, sum[1]);
+                sum[2] = fmaf(fmaxf(__uint_as_float(r[4 * v + 2]), 0.f), f.z, sum[2]);
+                sum[3] = fmaf(fmaxf(__uint_as_float(r[4 * v + 3]), 0.f), f.w, sum[3]);
+              }
+            }
+            if (i == TOK / 2 - 1) {  // the accumulator is read
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&sm.aempty[buf]));
+            }
+            if (e < n && j < width) out[e * ld_scores] = j <= __ldg(positions + te) ? (sum[0] + sum[1]) + (sum[2] + sum[3]) : -INFINITY;
+          }
+          buf ^= 1;
+          if (buf == 0) aphase ^= 1;
+          return true;
+        });
+  }
+  __syncwarp();
+  if (!ok || *abort_flag) __nanosleep(200000);  // loads that are still in flight must land before the shared memory is released
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 __device__ __forceinline__ uint32_t order_key(float x) {
@@ -324,6 +522,54 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
   pxl_host::launch(dsa_scores_kernel, dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream, static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
       ld_scores, width, T, B, Hi, max_blocks, page, group);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
+}
+
+namespace {
+template <int HI>
+int launch_scores_tc(const void* q, const float* w, const void* cache, const int* block_tables, const int* cu_q, const int* positions,
+                     float* scores, int64_t ld_scores, int width, int T, int B, int max_blocks, int page, int max_ctx, int* status,
+                     cudaStream_t stream) {
+  constexpr int smem = 1024 + sizeof(TcScoreSmem);
+  static bool done[64] = {false};
+  const int dev = pxl_host::current_device_slot();
+  if (!done[dev]) {
+    if (cudaFuncSetAttribute(dsa_scores_tc_kernel<HI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return PXL_ERR_CUDA;
+    done[dev] = true;
+  }
+  CUtensorMap tq;
+  if (!pxl_host::make_tmap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, static_cast<uint64_t>(T) * HI, kDi, kDi, kTcCols, 64))
+    return PXL_ERR_TENSORMAP;
+  // A prompt without a cached part leaves half of the tiles empty: eight waves where a CTA still has 48 tokens for its keys, two
+  // otherwise, and the late tokens' begin (4096 tokens of 4096: 329 us in two waves, 238 in eight).
+  const int tiles = pxl::ceil_div(max_ctx, kTcKeys), tok = kTcCols / HI;
+  int groups = 8 * pxl_host::num_sms() / tiles;
+  if (groups < 1 || T / groups < 48) groups = 2 * pxl_host::num_sms() / tiles;
+  groups = groups < 1 ? 1 : groups;
+  const int group = pxl::ceil_div(pxl::ceil_div(T, groups), tok) * tok;
+  pxl_host::launch(dsa_scores_tc_kernel<HI>, dim3(tiles, pxl::ceil_div(T, group)), kTcThreads, smem, stream, tq, w,
+                   static_cast<const pxl::bf16*>(cache), block_tables, cu_q, positions, scores, ld_scores, width, T, B, max_blocks, page,
+                   group, status);
+  return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
+}
+}  // namespace
+
+// pxl_dsa_index_scores with a status word: prompts of 32 or 64 index heads go to the tensor cores' kernel from 16 tokens on
+// (16 tokens x 6000 keys 16.6 and 14.6 us, 64 x 2000 18.9 and 14.6; below, both are as long as their launch).
+PXL_EXPORT int pxl_dsa_index_scores_status(const void* q, const float* w, const void* index_cache, const int* block_tables, const int* cu_q,
+                                           const int* positions, float* scores, int64_t ld_scores, int T, int B, int Hi, int Di,
+                                           int max_blocks, int page, int max_ctx, int* status, cudaStream_t stream) {
+  const int width = max_ctx > 0 ? pxl::ceil_div(max_ctx, kKeyTile) * kKeyTile : 0;
+  if (cu_q != nullptr && T >= kTcTokens && Di == kDi && (Hi == 32 || Hi == 64) && width > 0 && width <= ld_scores && page > 0 &&
+      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(index_cache)) & 15) == 0 &&
+      static_cast<int64_t>(T) * Hi < (1ll << 31)) {
+    if (Hi == 64)
+      return launch_scores_tc<64>(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, width, T, B, max_blocks, page,
+                                  max_ctx, status, stream);
+    return launch_scores_tc<32>(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, width, T, B, max_blocks, page, max_ctx,
+                                status, stream);
+  }
+  return pxl_dsa_index_scores(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, T, B, Hi, Di, max_blocks, page, max_ctx,
+                              stream);
 }
 
 PXL_EXPORT int pxl_topk_select(const float* scores, int64_t ld, const int* positions, int T, int k, int* out,

@@ -68,3 +68,31 @@ def test_tokens_in_any_order():
     seen = torch.isfinite(want)
     assert torch.equal(torch.isfinite(got), seen)
     assert float((got[seen] - want[seen]).norm() / want[seen].norm()) < 1e-5      # fp32 sums in another order
+
+
+@pytest.mark.parametrize("Hi", [32, 64])
+@pytest.mark.parametrize("lens,ctx,shuffled", [([2], [2], False), ([1, 130, 3], [300, 130, 512], False), ([257], [257], True),
+                                               ([600], [1700], False), ([40, 1, 90], [255, 256, 1030], True)])
+def test_scores_of_32_and_64_heads(Hi, lens, ctx, shuffled):
+    """256 keys per CTA and tiles of 128 / heads tokens: ends of sequences, groups and tiles, keys nobody sees."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(sum(lens) + Hi)
+    page = 16
+    need = [-(-c // page) for c in ctx]
+    ids, at = torch.randperm(sum(need)).int(), 0
+    table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+    for i, n in enumerate(need):
+        table[i, :n], at = ids[at:at + n], at + n
+    T, most = sum(lens), max(ctx)
+    pos = torch.cat([(torch.arange(c - n, c)[torch.randperm(n)] if shuffled else torch.arange(c - n, c)) for n, c in zip(lens, ctx)]).int()
+    cache = torch.randn(sum(need), 1, page, 128).bfloat16()
+    q, w = torch.randn(T, Hi, 128).bfloat16(), torch.randn(T, Hi)
+    cu_q = torch.tensor([0] + lens).cumsum(0).int()
+    got = cu.dsa_index_scores(*[t.cuda() for t in (q, w, cache, table, cu_q, pos)], most).cpu()
+    cu.check_status(torch.device("cuda", 0))
+    want = ref.dsa_index_scores(q, w, cache, table.clamp(min=0), cu_q, pos, most)
+    seen = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), seen)
+    # bf16 products are exact in fp32; sums of 128 and of Hi terms in another order
+    assert float((got[seen] - want[seen]).norm() / want[seen].norm()) < 1e-5
