@@ -2,7 +2,7 @@
 //
 // Every weight is read once and used M times: bound by memory, so nothing of a tensor-core product helps and its costs remain
 // (tiles of 128 rows for M = 1, partial sums exchanged between the K ranges, TMA and TMEM set up per launch). Here a warp takes
-// R rows of W over the whole of K, 16 bytes a lane and eight such loads in flight, and the sums of its lanes meet in one
+// R rows of W over the whole of K, 16 bytes a lane and eight to twelve such loads in flight, and the sums of its lanes meet in one
 // transposing shuffle reduction. The rows of A are shared by all warps and come from L1. Weights are not written by the kernel
 // before, so the first loads go out ahead of the wait for it (programmatic dependent launch): in a chain of small layers they
 // run under its tail.
@@ -312,9 +312,9 @@ int run(const GemvArgs& a, int epi, cudaStream_t stream) {
 }  // namespace
 
 // Where it beats the tensor cores: the rows of A cost it a load and an unpacking each per 16 bytes of W, so it is ahead for one
-// row (4096 x 4096: 9.0 us against 11.8; 151936 x 1024: 46 against 63) and stays so up to four where K is short (4096 x 1024, four
-// rows: 4.4 against 7.2) but not where the split along K of the other kernel pays (6144 x 4096, four rows: 17.3 against 15.2).
-// Gated products have no such split: four rows at 24576 x 4096 take 41 us against 50, six 67 against 49.
+// row (4096 x 4096: 9.0 us against 10.7; 151936 x 1024: 46 against 55) and stays so up to four where K is short (4096 x 1024, four
+// rows: 4.4 against 7.2) but not where the split along K of the other kernel pays (6144 x 4096, four rows: 17.3 against 12.3).
+// Gated products have no such split: four rows at 24576 x 4096 take 39 us, six on the tensor cores 40.
 PXL_EXPORT int pxl_gemv_bf16_takes(int M, int N, int K, int epi) {
   if (M <= 0 || M > PXL_GEMV_MAX_M || N % 8 || K % 8) return 0;
   if (epi == PXL_EPI_SILU_MUL) return N % 128 == 0;
