@@ -90,7 +90,7 @@ __device__ __forceinline__ void gemv_body(const Args& a) {
   if (kEarly && !kGlu && stores && a.bias) add_bias = __bfloat162float(a.bias[col]);
   [[maybe_unused]] float head_w = 0.f, cs = 1.f, sn = 0.f;
   [[maybe_unused]] int64_t slot = -1;
-  [[maybe_unused]] bool head_normed = false;
+  [[maybe_unused]] bool head_normed = false, turned = false;
   if constexpr (kHeads) {
     const bf16* w = head < a.Hq ? a.q_norm : head < a.Hq + a.Hkv ? a.k_norm : nullptr;
     head_normed = w != nullptr;
@@ -100,7 +100,8 @@ __device__ __forceinline__ void gemv_body(const Args& a) {
     const int m = om < a.M ? om : a.M - 1, p = a.positions[m];
     const bool p_ok = p >= 0 && (a.max_pos <= 0 || p < a.max_pos);
     slot = a.slots ? a.slots[m] : -1;
-    if (p_ok && head < a.Hq + a.Hkv) {  // a position outside the table is reported, its row is left unrotated
+    turned = p_ok && head < a.Hq + a.Hkv;  // a position outside the table is reported, its row is left unrotated
+    if (turned) {
       cs = a.cos_sin[static_cast<int64_t>(p) * kHeadDim + in_head];
       sn = a.cos_sin[static_cast<int64_t>(p) * kHeadDim + kHeadDim / 2 + in_head];
     }
@@ -224,7 +225,8 @@ __device__ __forceinline__ void gemv_body(const Args& a) {
       x = __bfloat162float(__float2bfloat16(x * inv_rms * head_w));  // rounded before the rotation, as a bf16 module does
       other = __shfl_xor_sync(0xffffffffu, x, kSpan);
     }
-    const bf16 y = __float2bfloat16(x * cs + (orow == 0 ? -other : other) * sn);
+    // (a branch: cosine 1 and sine 0 would make NaN of what has an infinity or a NaN for its other half)
+    const bf16 y = __float2bfloat16(turned ? x * cs + (orow == 0 ? -other : other) * sn : x);
     if (!stores) return;
     if (head < a.Hq) {
       static_cast<bf16*>(a.C)[at] = y;

@@ -57,6 +57,42 @@ def test_heads(M, K, Hq, Hkv, normed, bias):
     assert not gk.cpu().transpose(1, 2).reshape(-1, Hkv, D)[rows].any()
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_values_that_are_no_numbers(bad):
+    """Value heads, and rows whose position is outside the table, are not rotated: a column that is no number leaves its other half alone."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(1)
+    dev, D, Hq, Hkv, K, page = torch.device("cuda", 0), 128, 2, 1, 256, 16
+    N = (Hq + 2 * Hkv) * D
+    x, w_ln = torch.randn(1, K, device=dev).bfloat16(), torch.ones(K, device=dev).bfloat16()
+    w, b = (torch.randn(N, K, device=dev) / K ** 0.5).bfloat16(), torch.randn(N, device=dev).bfloat16()
+    marked = b.view(-1, D).clone()
+    marked[:, 5] = bad
+    cos_sin = torch.randn(8, D, device=dev)
+    st = cu.status_tensor(dev).data_ptr()
+    for pos, turned in ((3, True), (8, False)):
+        p, slot = torch.tensor([pos], device=dev).int(), torch.tensor([1], device=dev).long()
+        rows = []
+        for bias in (marked, b):
+            out = torch.zeros(1, N, dtype=torch.bfloat16, device=dev)
+            k, v = (torch.zeros(1, Hkv, page, D, dtype=torch.bfloat16, device=dev) for _ in range(2))
+            assert _fn()(x.data_ptr(), w_ln.data_ptr(), 1e-6, 0.0, w.data_ptr(), bias.data_ptr(), out.data_ptr(), None, None,
+                         cos_sin.data_ptr(), p.data_ptr(), slot.data_ptr(), k.data_ptr(), v.data_ptr(), 1, K, Hq, Hkv, D, D, page, page, 8,
+                         st, torch.cuda.current_stream().cuda_stream) == 0
+            torch.cuda.synchronize()
+            if not turned:
+                with pytest.raises(RuntimeError):
+                    cu.check_status(dev)
+            rows.append(torch.cat([out[0, :Hq * D].view(Hq, D), k[0, :, 1], v[0, :, 1]]))
+        got, want = (t.cpu() for t in rows)
+        away = torch.zeros(Hq + 2 * Hkv, D, dtype=torch.bool)
+        away[:, 5] = True
+        away[:Hq + Hkv, 5 + D // 2] = turned
+        assert not got[away].isfinite().any()
+        assert torch.equal(got[~away], want[~away])
+
+
 def test_refused_and_reported():
     from parallax_b200.ops import _lib
     from parallax_b200.ops import cuda as cu
