@@ -28,6 +28,17 @@ __device__ __forceinline__ int find_seq(const int* cu_q, int B, int t) {
   return lo;
 }
 
+// Row of the index cache that holds key kp of a sequence. An entry outside the cache or behind the table is reported and read as block 0.
+__device__ __forceinline__ int64_t key_row(const int* bt, int kp, int page, int max_blocks, int64_t num_blocks, int* status) {
+  const int bi = kp / page;
+  int blk = bi < max_blocks ? bt[bi] : -1;
+  if (blk < 0 || blk >= num_blocks) {
+    if (status) atomicCAS(status, 0, PXL_DEV_BAD_INDEX);
+    blk = 0;
+  }
+  return static_cast<int64_t>(blk) * page + kp % page;
+}
+
 // One CTA scores 128 keys for a group of consecutive tokens. Keys are the rows of the products and index heads the columns: a
 // warp keeps the fragments of its 32 keys in registers for as long as the tokens are of one sequence (a token costs its queries,
 // 16 KB of shared memory, and no key is read again), and the weighted sum over the heads stays inside a thread up to two
@@ -48,7 +59,8 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
                                                                    const int* __restrict__ cu_q,
                                                                    const int* __restrict__ positions,
                                                                    float* __restrict__ scores, int64_t ld_scores, int width, int T,
-                                                                   int B, int Hi, int max_blocks, int page, int group) {
+                                                                   int B, int Hi, int max_blocks, int page, int group,
+                                                                   int64_t num_blocks, int* status) {
   pdl_wait();
   pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t raw[];
@@ -83,12 +95,14 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
       int limit = pos;  // what the group's tokens of the sequence see, in whatever order they are
       for (int i = t + 1; i < seq_end && i < last; ++i) limit = max(limit, positions[i]);
       const int* bt = block_tables + static_cast<size_t>(seq) * max_blocks;
-      for (int c = tid; c < kScoreKeys * (kDi / 8); c += kScoreThreads) {
-        const int r = c / (kDi / 8), ch = c % (kDi / 8);
-        const int kp = j0 + r;
-        const bf16* src = cache;
-        if (kp <= limit) src = cache + (static_cast<size_t>(bt[kp / page]) * page + kp % page) * kDi + ch * 8;
-        cp_async_16(smem_u32(&sm.k[r * kPitch + ch * 8]), src, kp <= limit);
+      constexpr int kStep = kScoreThreads / 16;  // keys per step, two of a warp; lane l looks up one of them for step l / 2
+      const int mine = j0 + (lane >> 1) * kStep + warp * 2 + (lane & 1);
+      const int64_t at = mine <= limit ? key_row(bt, mine, page, max_blocks, num_blocks, status) : 0;
+#pragma unroll 4
+      for (int i = 0; i < kScoreKeys / kStep; ++i) {
+        const int r = i * kStep + warp * 2 + (lane >> 4), ch = lane & 15;
+        const int64_t key = __shfl_sync(0xffffffffu, at, 2 * i + (lane >> 4));
+        cp_async_16(smem_u32(&sm.k[r * kPitch + ch * 8]), cache + key * kDi + ch * 8, j0 + r <= limit);
       }
       cp_async_commit();
       cp_async_wait<0>();
@@ -185,7 +199,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 dsa_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const float* __restrict__ w, const bf16* __restrict__ cache,
                      const int* __restrict__ block_tables, const int* __restrict__ cu_q, const int* __restrict__ positions,
                      float* __restrict__ scores, int64_t ld_scores, int width, int T, int B, int max_blocks, int page, int group,
-                     int* status) {
+                     int64_t num_blocks, int* status) {
   constexpr int TOK = kTcCols / HI;
   extern __shared__ uint8_t raw[];
   TcScoreSmem& sm = *reinterpret_cast<TcScoreSmem*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -268,7 +282,6 @@ dsa_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const float* __re
                      });
   } else {
     const int m = (warp - 2) >> 2 & 1, e0 = (warp - 2) / 8 * (TOK / 2), row = m * 128 + (warp & 3) * 32 + lane, j = j0 + row;  // warp % 4: the lanes of tensor memory
-    const int tid = threadIdx.x - 64;
     int buf = 0;
     uint32_t aphase = 0;
     score_tiles<TOK>(
@@ -279,12 +292,15 @@ dsa_scores_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const float* __re
           limit = __reduce_max_sync(0xffffffffu, limit);
           if (limit < j0) return true;
           const int* bt = block_tables + static_cast<size_t>(seq) * max_blocks;
+          constexpr int kStep = 2 * kTcWarps;  // keys per step, two of a warp; lane l looks up one of them for step l / 2
+          const int first_key = (warp - 2) * 2, mine = j0 + (lane >> 1) * kStep + first_key + (lane & 1);
+          const int64_t at = lane < 2 * kTcKeys / kStep && mine <= limit ? key_row(bt, mine, page, max_blocks, num_blocks, status) : 0;
 #pragma unroll 4
-          for (int c = tid; c < kTcKeys * (kDi / 8); c += 32 * kTcWarps) {
-            const int r = c / (kDi / 8), ch = c % (kDi / 8), kp = j0 + r;
-            const bf16* src = cache;
-            if (kp <= limit) src = cache + (static_cast<size_t>(bt[kp / page]) * page + kp % page) * kDi + ch * 8;
-            cp_async_16(smem_u32(sm.k[r >> 7][ch >> 3]) + (r & 127) * 128 + (((ch & 7) ^ (r & 7)) << 4), src, kp <= limit);
+          for (int i = 0; i < kTcKeys / kStep; ++i) {
+            const int r = i * kStep + first_key + (lane >> 4), ch = lane & 15;
+            const int64_t key = __shfl_sync(0xffffffffu, at, 2 * i + (lane >> 4));
+            cp_async_16(smem_u32(sm.k[r >> 7][ch >> 3]) + (r & 127) * 128 + (((ch & 7) ^ (r & 7)) << 4), cache + key * kDi + ch * 8,
+                        j0 + r <= limit);
           }
           cp_async_commit();
           cp_async_wait<0>();
@@ -557,10 +573,10 @@ PXL_EXPORT int pxl_dsa_index_prep(void* q_idx, int64_t ldq, const void* kv, int6
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
-PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* index_cache,
-                                    const int* block_tables, const int* cu_q, const int* positions,
-                                    float* scores, int64_t ld_scores, int T, int B, int Hi, int Di,
-                                    int max_blocks, int page, int max_ctx, cudaStream_t stream) {
+namespace {
+int launch_scores(const void* q, const float* w, const void* index_cache, const int* block_tables, const int* cu_q, const int* positions,
+                  float* scores, int64_t ld_scores, int T, int B, int Hi, int Di, int max_blocks, int page, int max_ctx,
+                  int64_t num_blocks, int* status, cudaStream_t stream) {
   if (T <= 0) return PXL_OK;
   if (Di != kDi || Hi <= 0 || Hi > kHiMax || max_ctx <= 0) return PXL_ERR_INVALID_ARG;
   const int width = pxl::ceil_div(max_ctx, kKeyTile) * kKeyTile;  // (the last tile of 128 keys may reach past it)
@@ -578,16 +594,16 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
   int group = cu_q ? static_cast<int>(static_cast<int64_t>(T) * tiles / (3 * pxl_host::num_sms())) : 1;
   group = group < 1 ? 1 : group > 16 ? 16 : group;
   while (pxl::ceil_div(T, group) > 65535) group *= 2;
-  pxl_host::launch(dsa_scores_kernel, dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream, static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
-      ld_scores, width, T, B, Hi, max_blocks, page, group);
+  pxl_host::launch(dsa_scores_kernel, dim3(tiles, pxl::ceil_div(T, group)), kScoreThreads, sizeof(ScoreSmem), stream,
+                   static_cast<const pxl::bf16*>(q), w, static_cast<const pxl::bf16*>(index_cache), block_tables, cu_q, positions, scores,
+                   ld_scores, width, T, B, Hi, max_blocks, page, group, num_blocks, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
-namespace {
 template <int HI>
 int launch_scores_tc(const void* q, const float* w, const void* cache, const int* block_tables, const int* cu_q, const int* positions,
-                     float* scores, int64_t ld_scores, int width, int T, int B, int max_blocks, int page, int max_ctx, int* status,
-                     cudaStream_t stream) {
+                     float* scores, int64_t ld_scores, int width, int T, int B, int max_blocks, int page, int max_ctx,
+                     int64_t num_blocks, int* status, cudaStream_t stream) {
   constexpr int smem = 1024 + sizeof(TcScoreSmem);
   static bool done[64] = {false};
   const int dev = pxl_host::current_device_slot();
@@ -607,28 +623,35 @@ int launch_scores_tc(const void* q, const float* w, const void* cache, const int
   const int group = pxl::ceil_div(pxl::ceil_div(T, groups), tok) * tok;
   pxl_host::launch(dsa_scores_tc_kernel<HI>, dim3(tiles, pxl::ceil_div(T, group)), kTcThreads, smem, stream, tq, w,
                    static_cast<const pxl::bf16*>(cache), block_tables, cu_q, positions, scores, ld_scores, width, T, B, max_blocks, page,
-                   group, status);
+                   group, num_blocks, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 }  // namespace
+
+PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* index_cache, const int* block_tables, const int* cu_q,
+                                    const int* positions, float* scores, int64_t ld_scores, int T, int B, int Hi, int Di,
+                                    int max_blocks, int page, int max_ctx, cudaStream_t stream) {
+  return launch_scores(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, T, B, Hi, Di, max_blocks, page, max_ctx,
+                       INT64_MAX, nullptr, stream);  // (the size of the cache is not known)
+}
 
 // pxl_dsa_index_scores with a status word: prompts of 32 or 64 index heads go to the tensor cores' kernel from 16 tokens on
 // (16 tokens x 6000 keys 16.6 and 14.6 us, 64 x 2000 18.9 and 14.6; below, both are as long as their launch).
 PXL_EXPORT int pxl_dsa_index_scores_status(const void* q, const float* w, const void* index_cache, const int* block_tables, const int* cu_q,
                                            const int* positions, float* scores, int64_t ld_scores, int T, int B, int Hi, int Di,
-                                           int max_blocks, int page, int max_ctx, int* status, cudaStream_t stream) {
+                                           int max_blocks, int page, int max_ctx, int64_t num_blocks, int* status, cudaStream_t stream) {
   const int width = max_ctx > 0 ? pxl::ceil_div(max_ctx, kKeyTile) * kKeyTile : 0;
   if (cu_q != nullptr && T >= kTcTokens && Di == kDi && (Hi == 32 || Hi == 64) && width > 0 && width <= ld_scores && page > 0 &&
       ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(index_cache)) & 15) == 0 &&
       static_cast<int64_t>(T) * Hi < (1ll << 31)) {
     if (Hi == 64)
       return launch_scores_tc<64>(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, width, T, B, max_blocks, page,
-                                  max_ctx, status, stream);
+                                  max_ctx, num_blocks, status, stream);
     return launch_scores_tc<32>(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, width, T, B, max_blocks, page, max_ctx,
-                                status, stream);
+                                num_blocks, status, stream);
   }
-  return pxl_dsa_index_scores(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, T, B, Hi, Di, max_blocks, page, max_ctx,
-                              stream);
+  return launch_scores(q, w, index_cache, block_tables, cu_q, positions, scores, ld_scores, T, B, Hi, Di, max_blocks, page, max_ctx,
+                       num_blocks, status, stream);
 }
 
 PXL_EXPORT int pxl_topk_select(const float* scores, int64_t ld, const int* positions, int T, int k, int* out,

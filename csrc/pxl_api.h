@@ -266,10 +266,11 @@ int pxl_dsa_index_scores(const void* q, const float* w, const void* index_cache,
                          const int* block_tables, const int* cu_q, const int* positions,
                          float* scores, int64_t ld_scores, int T, int B, int Hi, int Di,
                          int max_blocks, int page, int max_ctx, pxl_stream_t stream);
-// The same; prompts (cu_q) of 32 or 64 heads on the tensor cores' kernel, whose waits report to `status`.
+// The same; prompts (cu_q) of 32 or 64 heads on the tensor cores' kernel, whose waits report to `status`. Table entries outside
+// [0, num_blocks) and positions behind the table are reported there too, and read block 0.
 int pxl_dsa_index_scores_status(const void* q, const float* w, const void* index_cache, const int* block_tables, const int* cu_q,
                                 const int* positions, float* scores, int64_t ld_scores, int T, int B, int Hi, int Di, int max_blocks,
-                                int page, int max_ctx, int* status, pxl_stream_t stream);
+                                int page, int max_ctx, int64_t num_blocks, int* status, pxl_stream_t stream);
 // Positions of the k largest scores among [0, positions[t]] per row (unordered); rows with at
 // most k candidates are filled with -1 ("attend densely").
 int pxl_topk_select(const float* scores, int64_t ld, const int* positions, int T, int k, int* out,

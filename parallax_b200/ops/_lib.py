@@ -100,7 +100,8 @@ _SIGS = {
                      c_int, c_int, c_float, _P],
     "pxl_mla_rotate": [_P, c_int64, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P],
     "pxl_mla_prefill": [_P] * 5 + [c_int] * 8 + [c_float, _P, _P],
-    "pxl_dsa_index_scores_status": [_P, _P, _P, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P],
+    "pxl_dsa_index_scores_status": [_P, _P, _P, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int64,
+                                    _P, _P],
     "pxl_dsa_index_scores": [_P, _P, _P, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P],
     "pxl_topk_select": [_P, c_int64, _P, c_int, c_int, _P, c_int64, _P],
     "pxl_store_rows": [_P, c_int64, _P, _P, c_int, c_int, c_int64, _P, _P],

@@ -975,7 +975,7 @@ def dsa_index_scores(q_idx, w, index_cache, block_tables, cu_q, positions, max_c
     check(_lib.lib().pxl_dsa_index_scores_status(q_idx.data_ptr(), w.data_ptr(), index_cache.data_ptr(),
                                                  block_tables.data_ptr(), _ptr(cu_q), positions.data_ptr(),
                                                  scores.data_ptr(), ld, T, block_tables.shape[0], Hi, Di,
-                                                 block_tables.shape[1], index_cache.shape[-2], max_ctx,
+                                                 block_tables.shape[1], index_cache.shape[-2], max_ctx, index_cache.shape[0],
                                                  status_tensor(q_idx.device).data_ptr(), _stream(q_idx.device)), "pxl_dsa_index_scores")
     _count()
     return scores

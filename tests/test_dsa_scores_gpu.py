@@ -96,3 +96,33 @@ def test_scores_of_32_and_64_heads(Hi, lens, ctx, shuffled):
     assert torch.equal(torch.isfinite(got), seen)
     # bf16 products are exact in fp32; sums of 128 and of Hi terms in another order
     assert float((got[seen] - want[seen]).norm() / want[seen].norm()) < 1e-5
+
+
+@pytest.mark.parametrize("Hi,prompt", [(64, True), (32, True), (24, True), (64, False)])
+@pytest.mark.parametrize("entry", [-1, 20, 1 << 30])
+def test_entries_outside_the_cache(Hi, prompt, entry):
+    """A table entry that is no block of the cache, where a token sees it: reported, and block 0 in its place."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(Hi)
+    dev, page, pages, T = torch.device("cuda", 0), 16, 20, 40 if prompt else 3
+    B, ctx = (1, 310) if prompt else (T, 310)
+    table = torch.arange(pages).int().repeat(B, 1)
+    bad = table.clone()
+    bad[0, 7], table[0, 7] = entry, 0
+    cache = torch.randn(pages, 1, page, 128).bfloat16()
+    q, w = torch.randn(T, Hi, 128).bfloat16(), torch.randn(T, Hi)
+    pos = (torch.arange(ctx - T, ctx) if prompt else torch.full((T,), ctx - 1)).int()
+    cu_q = torch.tensor([0, T]).int().cuda() if prompt else None
+    a = [t.cuda() for t in (q, w, cache)]
+    want = cu.dsa_index_scores(*a, table.cuda(), cu_q, pos.cuda(), ctx)
+    cu.check_status(dev)
+    got = cu.dsa_index_scores(*a, bad.cuda(), cu_q, pos.cuda(), ctx)
+    with pytest.raises(RuntimeError):
+        cu.check_status(dev)
+    assert torch.equal(got, want)
+    if entry < 0:       # a position behind the table
+        got = cu.dsa_index_scores(*a, table.cuda()[:, :7].contiguous(), cu_q, pos.cuda(), ctx)
+        with pytest.raises(RuntimeError):
+            cu.check_status(dev)
+        assert bool(torch.isfinite(got[:, :ctx - T]).all())
