@@ -439,7 +439,8 @@ __device__ __forceinline__ bool flag_wait_bounded(const uint32_t* flag, uint32_t
 // A kernel launched with the programmatic-stream-serialization attribute may start while the
 // kernel before it in the stream is still draining. pdl_wait() blocks until that kernel has
 // completed and its writes are visible (a no-op for launches without the attribute), so it must
-// run before the first access to global memory that an earlier kernel wrote or still reads.
+// run before the first access to global memory that a kernel of the chain wrote or still reads (what is complete
+// ahead of the chain: see pxl_host::launch_chain).
 // pdl_launch_dependents() lets the next kernel of the stream begin its own prologue early. It comes after pdl_wait(), so that
 // what the kernels before the last one wrote is visible without a wait, and in kernels with tensor memory after their allocation:
 // the next kernel's blocks take theirs as soon as they run, and would keep it from a block of this one that still needs some.
@@ -487,11 +488,17 @@ namespace pxl_host {
 
 // Launch chain of the calling thread: a sequence of layers whose launches carry the programmatic-stream-serialization attribute
 // (every kernel started through launch() waits with pdl_wait()). The first launch of a chain goes without it: it follows whatever
-// the caller had in the stream, so that weights and batch arrays are complete before any kernel of the chain starts.
+// the caller had in the stream. Kernels read ahead of their wait what is complete by then: weights (the second operand of a product,
+// biases, norm weights) and the step's index arrays (block tables, lengths, positions, slots). A launcher inside a chain that writes
+// one of these calls next_launch_follows_whole() behind its kernel.
 enum Chain : int { kNoChain = 0, kChainBegun = 1, kInChain = 2 };
 inline int& launch_chain() {
   static thread_local int state = kNoChain;
   return state;
+}
+// The next launch of the chain goes without the attribute, as the first one did.
+inline void next_launch_follows_whole() {
+  if (launch_chain() == kInChain) launch_chain() = kChainBegun;
 }
 // whether the next launch carries the attribute
 inline bool chained() {

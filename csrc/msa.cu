@@ -180,8 +180,6 @@ PXL_EXPORT int pxl_msa_select(const float* scores, int64_t ld, const int* positi
   if (ld_vt < static_cast<int64_t>(topk) * (sparse_block / page)) return PXL_ERR_INVALID_ARG;
   msa_select_kernel<<<T, 32, 0, stream>>>(scores, ld, positions, block_tables, cu_q, B, max_blocks, page, sparse_block,
                                           topk, init_blocks, local_blocks, v_tables, ld_vt, v_ctx);
-  // decode attention reads its tables and lengths ahead of its wait, as arrays that were there before the chain: these were not, so the
-  // kernel behind this one follows it whole
-  if (pxl_host::launch_chain() == pxl_host::kInChain) pxl_host::launch_chain() = pxl_host::kChainBegun;
+  pxl_host::next_launch_follows_whole();  // decode attention reads its tables and lengths ahead of its wait
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

@@ -111,9 +111,11 @@ def workspace(device: torch.device, tag: str, nbytes: int) -> torch.Tensor:
 
 
 class launch_chain:
-    """``with launch_chain():`` - the kernels that this thread launches inside overlap their prologue, and the first loads of
-    weights, with the tail of the kernel before them on the stream (programmatic dependent launch; every kernel waits before it
-    touches anything else). Weights and the step's index arrays are written before the chain, on the same stream."""
+    """``with launch_chain():`` - the kernels that this thread launches inside overlap their prologue with the tail of the kernel
+    before them on the stream (programmatic dependent launch). Ahead of their wait for that kernel they read weights (second
+    operands of products, biases, norm weights) and the step's index arrays (block tables, lengths, positions, slots): these are
+    complete before the chain begins, on the same stream. What makes one of them inside a chain has the next launch follow it whole
+    (``pxl_host::next_launch_follows_whole`` in its launcher, as block selection does)."""
 
     def __enter__(self):
         self.before = _lib.lib().pxl_launch_chain(1)
