@@ -699,8 +699,6 @@ __global__ void patch_i32_kernel(int* __restrict__ dst, const int* __restrict__ 
                                  const int* __restrict__ src_idx, int n, int dst_len, int src_len, int* status) {
   pdl_wait();
   pdl_launch_dependents();
-  pdl_wait();
-  pdl_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int d = dst_idx[i], s = src_idx[i];
