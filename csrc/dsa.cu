@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kScoreThreads) dsa_scores_kernel(const bf16* _
 // products, 54 us for the 90 GFLOP of 1000 tokens x 5500 keys at the rate of plain ones, and by the 2.5 instructions per score of the
 // other warps, which take as long: 287 us with mma.sync, 115 with eight such warps, 99 now (0.91 PFLOP/s); 4096 x 14336 2909 and 992;
 // 32 heads 284 and 60.
-constexpr int kTcTokens = 16;  // smallest prompt
+constexpr int kTcTokens = 16;  // fewest tokens of a step's prompts
 constexpr int kTcKeys = 256, kTcCols = 128, kTcStages = 3, kTcWarps = 16, kTcThreads = 64 + 32 * kTcWarps;
 struct TcScoreSmem {
   uint8_t k[2][2][128 * 128];             // [accumulator][half of the columns]: 128-byte swizzled rows
@@ -636,12 +636,16 @@ PXL_EXPORT int pxl_dsa_index_scores(const void* q, const float* w, const void* i
 }
 
 // pxl_dsa_index_scores with a status word: prompts of 32 or 64 index heads go to the tensor cores' kernel from 16 tokens on
-// (16 tokens x 6000 keys 16.6 and 14.6 us, 64 x 2000 18.9 and 14.6; below, both are as long as their launch).
+// (16 tokens x 6000 keys 16.6 and 14.6 us, 64 x 2000 18.9 and 14.6; below, both are as long as their launch), if there is a tile of
+// tokens, 128 / heads, for each: a prompt of fewer loads its 256 keys for a product that is mostly padding. us, other kernel and this one:
+//   prompts x tokens x keys   16 x 1 x 2000   16 x 1 x 6000   32 x 1 x 6000   16 x 2 x 6000   32 x 2 x 6000   16 x 4 x 6000
+//   64 heads                   8.4 12.3        16.2 22.6       36.5 40.8       28.7 22.8       47.7 32.8       39.7 25.5
+//   32 heads                  12.2 31.6        24.3 34.3       36.4 41.7       31.1 34.1       46.7 41.7       40.0 27.2
 PXL_EXPORT int pxl_dsa_index_scores_status(const void* q, const float* w, const void* index_cache, const int* block_tables, const int* cu_q,
                                            const int* positions, float* scores, int64_t ld_scores, int T, int B, int Hi, int Di,
                                            int max_blocks, int page, int max_ctx, int64_t num_blocks, int* status, cudaStream_t stream) {
   const int width = max_ctx > 0 ? pxl::ceil_div(max_ctx, kKeyTile) * kKeyTile : 0;
-  if (cu_q != nullptr && T >= kTcTokens && Di == kDi && (Hi == 32 || Hi == 64) && width > 0 && width <= ld_scores && page > 0 &&
+  if (cu_q != nullptr && T >= kTcTokens && Di == kDi && (Hi == 32 || Hi == 64) && T >= static_cast<int64_t>(kTcCols / Hi) * B && width > 0 && width <= ld_scores && page > 0 &&
       ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(index_cache)) & 15) == 0 &&
       static_cast<int64_t>(T) * Hi < (1ll << 31)) {
     if (Hi == 64)

@@ -126,3 +126,23 @@ def test_entries_outside_the_cache(Hi, prompt, entry):
         with pytest.raises(RuntimeError):
             cu.check_status(dev)
         assert bool(torch.isfinite(got[:, :ctx - T]).all())
+
+
+@pytest.mark.parametrize("Hi,each", [(64, 1), (64, 2), (32, 3), (32, 4)])
+def test_many_short_prompts(Hi, each):
+    """Fewer tokens per prompt than a tile of the tensor cores' kernel (128 / heads), and as many."""
+    from parallax_b200.ops import cuda as cu
+
+    torch.manual_seed(each)
+    page, ctx, B = 16, 300, 20
+    pages = -(-ctx // page)
+    table, cache = torch.randperm(B * pages).int().view(B, pages), torch.randn(B * pages, 1, page, 128).bfloat16()
+    T = B * each
+    pos = torch.cat([torch.arange(ctx - 7 * i - each, ctx - 7 * i) for i in range(B)]).int()
+    q, w, cu_q = torch.randn(T, Hi, 128).bfloat16(), torch.randn(T, Hi), (torch.arange(B + 1) * each).int()
+    got = cu.dsa_index_scores(*[t.cuda() for t in (q, w, cache, table, cu_q, pos)], ctx).cpu()
+    cu.check_status(torch.device("cuda", 0))
+    want = ref.dsa_index_scores(q, w, cache, table, cu_q, pos, ctx)
+    seen = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), seen)
+    assert float((got[seen] - want[seen]).norm() / want[seen].norm()) < 1e-5      # fp32 sums in another order
