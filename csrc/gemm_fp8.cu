@@ -52,6 +52,7 @@ struct Fp8Args {
   // SPLIT: CTAs of a cluster, one per K range; K blocks per range (a multiple of F_GROUP)
   int splits, kb_per;
   int stage_bytes;  // of a stage that are loaded
+  int early;        // launched in a chain: the weights of the first stages go out ahead of the wait
 };
 
 constexpr int kPartPitch = FN + 4;  // floats of a row of partial sums: 16-byte stores of a quarter warp hit distinct banks
@@ -121,7 +122,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   // weights of the first stages, under the tail of the kernel before (no kernel of a launch chain writes weights)
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && lane == 0 && g.early) {
     for (int kb = 0; kb < F_STAGES && kb < num_kb; ++kb) {
       mbar_arrive_expect_tx(full0 + 8 * kb, g.stage_bytes);
       tma_load_2d(smem_u32(smem + kb * F_STAGE_BYTES + FM * FK), &tmap_b, full0 + 8 * kb, (kb_base + kb) * FK, b_row);
@@ -137,7 +138,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     uint32_t phase = 0;
     for (int kb = 0; kb < num_kb; ++kb) {
       const uint32_t fb = full0 + 8 * stage, at = s0 + stage * F_STAGE_BYTES;
-      if (kb >= F_STAGES) {
+      if (kb >= F_STAGES || !g.early) {
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1, abort_flag, status, PXL_DEV_TIMEOUT_EMPTY))) break;
         expect_tx(fb, g.stage_bytes, leader);
         tma_box(at + FM * FK, &tmap_b, fb, (kb_base + kb) * FK, b_row, leader);
@@ -426,9 +427,11 @@ int launch_fp8(const void* A, const void* W, Fp8Args g, uint64_t a_rows, uint64_
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pxl_host::chained() ? 2 : 1;
+    g.early = pxl_host::chained();
+    cfg.numAttrs = g.early ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gemm_fp8_kernel<true>, ta, tb, g, status) == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
   }
+  g.early = pxl_host::launch_chain() == pxl_host::kInChain;
   pxl_host::launch(gemm_fp8_kernel<false>, tiles, F_THREADS, F_SMEM, stream, ta, tb, g, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }

@@ -61,6 +61,7 @@ struct GemmEpilogueArgs {
   float* C_f32;          // EPI_F32 output
   int ldc;
   int a_rows;            // rows of A that a stage loads (0: all 128)
+  int early;             // launched in a chain: the first weights go out ahead of the wait
   bf16* const* row_ptrs; // EPI_SCATTER: destination of every output row (null = drop), N elements each
   uint32_t* done_counter;  // EPI_SCATTER: local counter for the "last CTA publishes the flags" step
   float act_limit;           // EPI_CLIP_GLU
@@ -328,11 +329,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   // of the previous kernel. So do the first loads of weights, which no kernel of a launch chain writes: what the ring of stages
   // takes. A product of a few rows is bound by these bytes, and the SMs that the previous kernel (a norm, a rotation, the tail
   // of an attention) leaves idle fetch them: five layers of 57 rows 800 -> 780 us, a layer's weights 59 us of each 160. (More of
-  // the tile into L2 by prefetches brings nothing, or delays the rows that queue behind them: 8 boxes 780, 24 boxes 803 us.)
+  // the tile into L2 by prefetches brings nothing, or delays the rows that queue behind them: 8 boxes 780, 24 boxes 803 us.) Outside
+  // of a chain there is nothing to wait for, and the first rows would queue behind all of these weights: 57 rows x 6144 x 4096 15.2 us
+  // with them and 14.5 without, gated 24576 x 4096 40.6 and 39.9.
   const uint32_t stage_bytes = (ep.a_rows > 0 ? ep.a_rows * BK * 2 : A_STAGE_BYTES) + Cfg::B_STAGE_BYTES;
   constexpr bool kSwapped = EPI == PXL_EPI_SPLITK_T || EPI == PXL_EPI_SPLITK_C;  // the weights take A's slot
   int ahead = 0;
-  if (warp == 0 && lane == 0 && grp.num_mt == nullptr && comm.tp <= 1 && static_cast<int>(blockIdx.x) < num_items) {
+  if (warp == 0 && lane == 0 && ep.early && grp.num_mt == nullptr && comm.tp <= 1 && static_cast<int>(blockIdx.x) < num_items) {
     const TileCoord tc = tile_coord<BN>(item_tile(blockIdx.x), num_m, num_n, M, grp, comm);
     const int kb0 = item_ks(blockIdx.x) * kb_per, kb1 = kb0 + kb_per < num_kb ? kb0 + kb_per : num_kb;
     for (int kb = kb0; kb < kb1 && ahead < STAGES; ++kb, ++ahead) {
@@ -1071,7 +1074,9 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmEpilogue
     grid = grid + comm.ag_ncopy <= pxl_host::num_sms() ? grid + comm.ag_ncopy : pxl_host::num_sms();
     if (grid <= comm.ag_ncopy) return PXL_ERR_INVALID_ARG;
   }
-  pxl_host::launch(kern, grid, kGemmThreads, gemm_smem_bytes<BN, EPI>(), stream, ta, tb, ep, grp, comm, M, N, K, status);
+  GemmEpilogueArgs e = ep;
+  e.early = pxl_host::launch_chain() == pxl_host::kInChain;
+  pxl_host::launch(kern, grid, kGemmThreads, gemm_smem_bytes<BN, EPI>(), stream, ta, tb, e, grp, comm, M, N, K, status);
   return cudaGetLastError() == cudaSuccess ? PXL_OK : PXL_ERR_CUDA;
 }
 
@@ -1116,7 +1121,9 @@ int launch_gemm_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm
   }
   GemmGroupArgs grp{};
   GemmCommArgs comm{};
-  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, ep, grp, comm, M, N, K, status) != cudaSuccess) {
+  GemmEpilogueArgs e = ep;
+  e.early = cfg.numAttrs == 2;
+  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, e, grp, comm, M, N, K, status) != cudaSuccess) {
     cudaGetLastError();
     return PXL_ERR_CUDA;
   }
