@@ -1418,11 +1418,12 @@ struct MidPlan {
   int bn, splitk;
   double cost;
 };
-MidPlan mid_m_plan(int M, int N, int K) {
+template <int W>
+MidPlan mid_m_plan(int M, int N, int K, const MidWidth (&widths)[W]) {
   const int num_kb = pxl::ceil_div(K, BK);
   const int num_m = pxl::ceil_div(M, BM);
   MidPlan best{0, 1, 1e300};
-  for (const MidWidth& w : kMidWidths) {
+  for (const MidWidth& w : widths) {
     const int tiles = num_m * pxl::ceil_div(N, w.bn);
     const double plain = mid_plain_cost(M, N, K, w);
     if (plain < best.cost) best = MidPlan{w.bn, 1, plain};
@@ -1439,11 +1440,10 @@ MidPlan mid_m_plan(int M, int N, int K) {
   return best;
 }
 
-// Many rounds, where all SMs pull at once and the tensor cores and the power limit are near: us per k-block of 256 and 192 columns.
-double plain_cost(int M, int N, int K, int bn) {
-  const int tiles = pxl::ceil_div(M, BM) * pxl::ceil_div(N, bn);
-  return pxl::ceil_div(tiles, pxl_host::num_sms()) * (pxl::ceil_div(K, BK) * (bn == 256 ? 0.43 : 0.36)) + 7.0;
-}
+// The model's figures where a product has many rounds: all SMs pull at once, and the tensor cores and the power limit are near. Both
+// sides of the decision on a tail are in these. With the tail in the figures of a launch of its own, which are a sixth to a half lower,
+// it was cut off too readily (1551 rows x 5120 x 8192 116.8 us in two launches, 107.7 in one; 5409 x 1024 x 3072 36.8 and 33.3).
+constexpr MidWidth kTailWidths[3] = {{256, 0.43, 7.0, 8.0, 2.0}, {128, 0.29, 7.0, 8.0, 1.0}, {192, 0.36, 7.0, -1.0, 0.0}};
 
 bool mid_m_disabled() {
   static const bool off = getenv("PXL_NO_MID_M_GEMM") != nullptr;
@@ -1456,11 +1456,11 @@ bool mid_m_disabled() {
 int rows_ahead_of_the_tail(int M, int N, int K, int epi) {
   if (M <= kMidMaxM || (epi != PXL_EPI_NONE && epi != PXL_EPI_RESIDUAL && epi != PXL_EPI_F32) || mid_m_disabled()) return M;
   const int sms = pxl_host::num_sms(), num_n = pxl::ceil_div(N, 256);
-  auto plain = [&](int rows) { return std::min(plain_cost(rows, N, K, 256), plain_cost(rows, N, K, 192)); };
+  auto plain = [&](int rows) { return std::min(mid_plain_cost(rows, N, K, kTailWidths[0]), mid_plain_cost(rows, N, K, kTailWidths[2])); };
   const int ahead = pxl::ceil_div(M, BM) * num_n / sms * sms / num_n * BM;
   const int tail = M - ahead;
   if (ahead <= 0 || tail <= 0 || tail > kMidMaxM) return M;
-  const double alone = tail <= kSmallMaxM ? 2.0 * N * K / 5.0e6 + 8.0 : mid_m_plan(tail, N, K).cost;
+  const double alone = tail <= kSmallMaxM ? 2.0 * N * K / 5.0e6 + 8.0 : mid_m_plan(tail, N, K, kTailWidths).cost;
   return plain(ahead) + alone < 0.97 * plain(M) ? ahead : M;
 }
 
@@ -1500,7 +1500,7 @@ int gemm_mid_m(const void* A, const void* W, void* C, bool f32_out, const void* 
 PXL_EXPORT int pxl_gemm_bf16_mid_m_plan(int M, int N, int K, int epi) {
   if (mid_m_disabled() || M <= BM || M > kMidMaxM) return 0;
   if (epi != PXL_EPI_NONE && epi != PXL_EPI_RESIDUAL && epi != PXL_EPI_F32) return 0;
-  const MidPlan p = mid_m_plan(M, N, K);
+  const MidPlan p = mid_m_plan(M, N, K, kMidWidths);
   return p.bn * 16 + p.splitk;
 }
 

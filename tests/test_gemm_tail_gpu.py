@@ -34,3 +34,11 @@ def test_tail_in_a_launch_of_its_own(M, N, K):
         # the same fp32 products in another order, rounded to bf16 (2^-9) where the result is: row by row, so that the tail's count
         err = (out[:M, :N].float() - one[:M, :N].float()).norm(dim=1) / one[:M, :N].float().norm(dim=1)
         assert float(err.max()) < (1e-5 if epi else 2 ** -8)
+
+
+@pytest.mark.parametrize("M,N,K", [(1551, 5120, 8192), (2252, 5120, 8192), (5409, 1024, 3072)])
+def test_tails_that_are_cheaper_in_the_last_wave(M, N, K):
+    """Tails of hundreds of rows whose product is longer on its own than the wave that they share."""
+    from parallax_b200.ops import _lib
+
+    assert _lib.lib().pxl_gemm_bf16_launches(M, N, K, 0) == 1
