@@ -1186,9 +1186,9 @@ double mid_plain_cost(int M, int N, int K, const MidWidth& w) {
 // that width (measured on compute-bound shapes: a 256-wide tile keeps the tensor pipe busiest, a
 // 64-wide one reaches about a third of it). Large problems take the width that wastes the least of
 // the last wave; problems with few tiles end up with narrow ones, which put more SMs to work. Up to kMidMaxM rows the figures of the
-// cost model above are taken (at K = 4096: its fixed parts weigh little): gated 24576 x 4096, 256 rows 60.2 us in tiles of 256 columns,
-// 53.4 in tiles of 128.
-PXL_EXPORT int pxl_gemm_bf16_pick_bn(int M, int N, int epi) {
+// cost model above are taken: gated 24576 x 4096, 256 rows 60.2 us in tiles of 256 columns, 53.4 in tiles of 128; with a short K the
+// fixed parts decide, 11008 x 256, 800 rows 13.5 and 12.2, 6144 x 768, 400 rows 10.7 and 10.2.
+static int pick_bn(int M, int N, int K, int epi) {
   const int sms = pxl_host::num_sms();
   const int num_m = pxl::ceil_div(M, BM);
   const int cands[4] = {256, 192, 128, 64};
@@ -1204,7 +1204,7 @@ PXL_EXPORT int pxl_gemm_bf16_pick_bn(int M, int N, int epi) {
     double cost = static_cast<double>(pxl::ceil_div(tiles, sms)) * bn / eff[i];
     if (M <= kMidMaxM)
       for (const MidWidth& w : kMidWidths)
-        if (w.bn == bn) cost = mid_plain_cost(M, N, 4096, w);
+        if (w.bn == bn) cost = mid_plain_cost(M, N, K, w);
     if (cost < best_cost) {
       best_cost = cost;
       best = bn;
@@ -1212,6 +1212,9 @@ PXL_EXPORT int pxl_gemm_bf16_pick_bn(int M, int N, int epi) {
   }
   return best ? best : 128;
 }
+
+// The width at K = 4096, for callers that have no K at hand.
+PXL_EXPORT int pxl_gemm_bf16_pick_bn(int M, int N, int epi) { return pick_bn(M, N, 4096, epi); }
 
 namespace {
 // fp32 scratch of the small-M path: one per (device, stream) so that GEMMs on different streams
@@ -1545,7 +1548,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
   if (bn == 0) {
     const int ahead = rows_ahead_of_the_tail(M, N, K, epi);
     if (ahead < M) {
-      const int rc = pxl_gemm_bf16(A, W, C, residual, bias, ahead, N, K, lda, ldw, ldc, epi, pxl_gemm_bf16_pick_bn(ahead, N, epi), status,
+      const int rc = pxl_gemm_bf16(A, W, C, residual, bias, ahead, N, K, lda, ldw, ldc, epi, pick_bn(ahead, N, K, epi), status,
                                    stream);
       if (rc != PXL_OK) return rc;
       const size_t out = static_cast<size_t>(ahead) * ldc;
@@ -1555,7 +1558,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
                            lda, ldw, ldc, epi, 0, status, stream);
     }
   }
-  if (bn == 0) bn = pxl_gemm_bf16_pick_bn(M, N, epi);
+  if (bn == 0) bn = pick_bn(M, N, K, epi);
   if (epi == PXL_EPI_SILU_MUL && ((N % bn) != 0 || bn < 128)) return PXL_ERR_INVALID_ARG;
 
   CUtensorMap ta, tb;
@@ -1598,7 +1601,7 @@ int gemm_glu(const void* A, const void* W, void* C, int M, int N, int K, int lda
   if ((K % 8) || (lda % 8) || (ldw % 8) || (ldc % 8) || (N % 128)) return PXL_ERR_INVALID_ARG;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C)) & 15)
     return PXL_ERR_INVALID_ARG;
-  if (bn == 0) bn = pxl_gemm_bf16_pick_bn(M, N, PXL_EPI_SILU_MUL);
+  if (bn == 0) bn = pick_bn(M, N, K, PXL_EPI_SILU_MUL);
   if ((bn != 128 && bn != 256) || (N % bn)) return PXL_ERR_INVALID_ARG;
   CUtensorMap ta, tb;
   if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, box_rows(M), BK) ||
@@ -1640,7 +1643,7 @@ PXL_EXPORT int pxl_gemm_bf16_act(const void* A, const void* W, void* C, int M, i
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C) |
        reinterpret_cast<uintptr_t>(table)) & 15)
     return PXL_ERR_INVALID_ARG;
-  const int bn = pxl_gemm_bf16_pick_bn(M, N, PXL_EPI_ACT);
+  const int bn = pick_bn(M, N, K, PXL_EPI_ACT);
   CUtensorMap ta, tb;
   if (!pxl_host::make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, M, K, lda, box_rows(M), BK) ||
       !pxl_host::make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, N, K, ldw, bn, BK))
