@@ -9,7 +9,6 @@ import torch
 
 from parallax_b200.engine.batch import BatchBuilder
 from parallax_b200.engine.worker import StageWorker
-from parallax_b200.loader.lora import LoRAStack
 from parallax_b200.models.config import config_from_hf, named_config
 
 pytestmark = pytest.mark.gpu
@@ -24,19 +23,12 @@ def _config(name):
             num_attention_heads=8, num_key_value_heads=2, head_dim=128, intermediate_size=2048, vocab_size=512, rope_theta=1e4,
             partial_rotary_factor=0.25, full_attention_interval=4, max_position_embeddings=4096, linear_num_key_heads=4,
             linear_num_value_heads=8, linear_key_head_dim=128, linear_value_head_dim=128, linear_conv_kernel_dim=4))
-    if name == "gpt-oss":       # attention sinks, windows, expert biases (mxfp4 experts are expanded when they are loaded)
-        return config_from_hf(dict(
-            architectures=["GptOssForCausalLM"], model_type="gpt_oss", hidden_size=512, num_hidden_layers=4, num_attention_heads=8,
-            num_key_value_heads=2, head_dim=64, intermediate_size=512, moe_intermediate_size=512, num_local_experts=8,
-            num_experts_per_tok=2, sliding_window=128, layer_types=["sliding_attention", "full_attention"] * 2, attention_bias=True,
-            vocab_size=512, rope_theta=1e4, max_position_embeddings=4096))
-    return named_config("qwen3-8b" if name == "lora" else name)
+    return named_config(name)
 
 
 @pytest.mark.parametrize("name,start,layers,kv", [("qwen3-30b-a3b", 8, 2, "bf16"), ("deepseek-v3", 1, 2, "bf16"),
                                                   ("deepseek-v3.2", 1, 2, "bf16"), ("hybrid", 4, 4, "bf16"),
-                                                  ("qwen3-8b", 8, 2, "fp8_e4m3"), ("lora", 8, 2, "bf16"),
-                                                  ("gpt-oss", 1, 2, "bf16"), ("small-msa", 1, 2, "bf16")])
+                                                  ("qwen3-8b", 8, 2, "fp8_e4m3")])
 def test_chained_layers_give_the_same_bits(name, start, layers, kv):
     from parallax_b200.ops import cuda as cu
 
@@ -66,15 +58,6 @@ def test_chained_layers_give_the_same_bits(name, start, layers, kv):
         for t in layer:
             t.copy_((torch.randn(t.shape, device=DEV, generator=g) * 0.5).to(t.dtype))
     kept = [[t.clone() for t in layer] for layer in caches]
-    if name == "lora":
-        m = worker.model
-        m.lora = LoRAStack(m, 2, 16)
-        for per in m.lora.layers:
-            for ab in per.values():
-                for t in ab:
-                    t.normal_(0, 0.05, generator=g)
-        m.lora.scale.fill_(0.7)
-        fb.extras["lora_ids"] = (torch.arange(len(pos), device=DEV) % 3 - 1).int()
 
     def step():
         for layer, old in zip(caches, kept):
@@ -88,14 +71,13 @@ def test_chained_layers_give_the_same_bits(name, start, layers, kv):
     del worker.model.chained
     for _ in range(4):
         y = step()
-        for i, (layer, old) in enumerate(zip([*caches, [y]], [*after, [want]])):
+        if cfg.index_topk:      # lists of chosen keys come in any order, and sums over them in the order of the list: bf16 roundings
+            assert float((y.float() - want.float()).norm() / want.float().norm()) < 1e-2
+            continue
+        assert torch.equal(y, want)
+        for layer, old in zip(caches, after):
             for t, o in zip(layer, old):
-                # lists of chosen keys come in any order, and sums over them in the order of the list: bf16 roundings (behind the
-                # first layer's caches, which no list has touched)
-                if cfg.index_topk and i > 0:
-                    assert float((t.float() - o.float()).norm() / o.float().norm()) < 1e-2
-                else:
-                    assert torch.equal(t.view(torch.uint8), o.view(torch.uint8))
+                assert torch.equal(t.view(torch.uint8), o.view(torch.uint8))
     cu.check_status(DEV)
 
 
