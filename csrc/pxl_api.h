@@ -167,6 +167,8 @@ int pxl_attn_decode(const void* q, int64_t q_stride, const void* k_cache, const 
                     int max_blocks, int64_t num_blocks, float scale, int window, int keep_first, int num_splits,
                     int max_ctx, float softcap, const float* sig_bias, int* status, pxl_stream_t stream);
 int pxl_attn_decode_splits(int B, int Hq, int Hkv, int D, int page_size, int cache_fp8, int max_ctx);
+// for rows of `total_ctx` keys together, of which the longest has max_ctx (the one above: all as long as that)
+int pxl_attn_decode_splits_of(int B, int Hq, int Hkv, int D, int page_size, int cache_fp8, int max_ctx, int64_t total_ctx);
 // kernels that pxl_attn_decode / pxl_attn_decode_fp8 launch: one where the splits add their results inside clusters
 int pxl_attn_decode_launches(int B, int Hkv, int D, int page_size, int num_splits, int cache_fp8, float softcap, int sigmoid);
 

@@ -43,6 +43,7 @@ struct PxlStageDesc {
 
 struct PxlStepDesc {
   int T, Tp, Bp, Bd, p_max_q, d_max_ctx, p_max_blocks, d_max_blocks;
+  int64_t d_total_ctx;  // keys of all decoding rows, 0: not known
   const int* positions;
   const int64_t* slots;
   const int* p_cu_q;
@@ -116,7 +117,7 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
                           st->num_blocks * Hkv * st->page < (1ll << 31);
   int splits = 0;
   if (sp->Bd > 0) {
-    splits = pxl_attn_decode_splits(sp->Bd, Hq, Hkv, D, st->page, 0, sp->d_max_ctx);
+    splits = pxl_attn_decode_splits_of(sp->Bd, Hq, Hkv, D, st->page, 0, sp->d_max_ctx, sp->d_total_ctx);
     if (splits > 1 && static_cast<int64_t>(sp->Bd) * Hq * splits * (D + 2) > ws->decode_floats) return PXL_ERR_TOO_LARGE;
   }
   // every kernel of the sequence waits (griddepcontrol.wait) before it touches global memory, so each

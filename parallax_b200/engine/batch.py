@@ -35,6 +35,7 @@ class ForwardBatch:
     d_ctx_lens: Optional[torch.Tensor] = None     # int32 [Bd]
     d_block_tables: Optional[torch.Tensor] = None  # int32 [Bd, MB]
     d_max_ctx: int = 0
+    d_total_ctx: int = 0                          # sum of d_ctx_lens (0: not known)
     # rows whose logits are needed (last token of finished prefills + every decode row)
     logit_rows: Optional[torch.Tensor] = None     # int32 [n_logits]
     num_logits: int = 0
@@ -156,6 +157,7 @@ class BatchBuilder:
             fb.d_ctx_lens = view("d_ctx")
             fb.d_block_tables = view("d_bt").view(Bd, -1)
             fb.d_max_ctx = int(d_ctx_lens.max())
+            fb.d_total_ctx = int(d_ctx_lens.sum(dtype=np.int64))
         fb.logit_rows = view("rows")
         if seq_rows is not None:
             fb.seq_cu = view("seq_cu")

@@ -27,7 +27,7 @@ class _StageDesc(Structure):
 
 class _StepDesc(Structure):
     _fields_ = [(n, c_int) for n in ("T", "Tp", "Bp", "Bd", "p_max_q", "d_max_ctx", "p_max_blocks", "d_max_blocks")] + \
-               [(n, c_void_p) for n in ("positions", "slots", "p_cu_q", "p_ctx", "p_bt", "d_ctx", "d_bt")]
+               [("d_total_ctx", c_int64)] + [(n, c_void_p) for n in ("positions", "slots", "p_cu_q", "p_ctx", "p_bt", "d_ctx", "d_bt")]
 
 
 class _Workspace(Structure):
@@ -66,7 +66,7 @@ class NativeDenseStage:
         self._dec = None
         self._fn = _lib.bind("pxl_stage_forward_dense", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                                          c_void_p, c_void_p])
-        self._splits = _lib.lib().pxl_attn_decode_splits
+        self._splits = _lib.lib().pxl_attn_decode_splits_of
 
     @staticmethod
     def supported(stage) -> bool:
@@ -78,7 +78,7 @@ class NativeDenseStage:
             return False
         return all(lw.moe is None and lw.w_gu is not None and isinstance(lw.w_gu, torch.Tensor) for lw in stage.layers)
 
-    def _ensure(self, T: int, Bd: int, d_max_ctx: int) -> None:
+    def _ensure(self, T: int, Bd: int, d_max_ctx: int, d_total_ctx: int) -> None:
         d = self.desc
         if T > self._cap:
             cap = max(T, 256)
@@ -89,7 +89,7 @@ class NativeDenseStage:
             w.xn, w.qkv, w.attn, w.act, w.h_a, w.h_b = [b.data_ptr() for b in self._bufs]
             self._cap = cap
         if Bd > 0:
-            splits = self._splits(Bd, d.Hq, d.Hkv, d.D, d.page, 0, d_max_ctx)
+            splits = self._splits(Bd, d.Hq, d.Hkv, d.D, d.page, 0, d_max_ctx, d_total_ctx)
             need = Bd * d.Hq * splits * (d.D + 2) if splits > 1 else 0
             if self._dec is None or self._dec.numel() < need:
                 self._dec = torch.empty(max(need, 1), dtype=torch.float32, device=self.device)
@@ -97,10 +97,10 @@ class NativeDenseStage:
 
     def forward(self, h_in: torch.Tensor, fb) -> torch.Tensor:
         T = fb.num_tokens
-        self._ensure(T, fb.num_decode, fb.d_max_ctx)
+        self._ensure(T, fb.num_decode, fb.d_max_ctx, fb.d_total_ctx)
         s = _StepDesc()
         s.T, s.Tp, s.Bp, s.Bd = T, fb.num_prefill_tokens, fb.num_prefill_seqs, fb.num_decode
-        s.p_max_q, s.d_max_ctx = fb.p_max_q, fb.d_max_ctx
+        s.p_max_q, s.d_max_ctx, s.d_total_ctx = fb.p_max_q, fb.d_max_ctx, fb.d_total_ctx
         s.positions, s.slots = fb.positions.data_ptr(), fb.slot_mapping.data_ptr()
         if s.Bp:
             s.p_cu_q, s.p_ctx, s.p_bt = fb.p_cu_q.data_ptr(), fb.p_ctx_lens.data_ptr(), fb.p_block_tables.data_ptr()

@@ -453,7 +453,8 @@ class DecoderStage(ExpertParallelMixin):
                              self.scale, window=lw.window, sinks=lw.sinks, out=attn[:Tp], kv_scale=kvs)
         if fb.num_decode:
             ops.attn_decode(q[Tp:], kc, vc, fb.d_block_tables, fb.d_ctx_lens, self.scale,
-                            window=lw.window, sinks=lw.sinks, max_ctx=fb.d_max_ctx, out=attn[Tp:], kv_scale=kvs)
+                            window=lw.window, sinks=lw.sinks, max_ctx=fb.d_max_ctx, total_ctx=fb.d_total_ctx, out=attn[Tp:],
+                            kv_scale=kvs)
         if lw.w_g is not None:      # head-wise gate: every head's output times sigmoid of that head's gate logit
             return ops.gate_mul_grouped(attn.view(T, Hq * D), ops.linear(xn, lw.w_g), D)
         return attn.view(T, Hq * D)

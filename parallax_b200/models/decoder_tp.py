@@ -161,7 +161,7 @@ class TPDecoderStage(TPStageMixin, DecoderStage):
                                  self.scale, window=lw.window, sinks=lw.sinks, out=attn[:Tp], kv_scale=kvs)
             if fb.num_decode:
                 ops.attn_decode(q[Tp:], kc, vc, fb.d_block_tables, fb.d_ctx_lens, self.scale, window=lw.window,
-                                sinks=lw.sinks, max_ctx=fb.d_max_ctx, out=attn[Tp:T], kv_scale=kvs)
+                                sinks=lw.sinks, max_ctx=fb.d_max_ctx, total_ctx=fb.d_total_ctx, out=attn[Tp:T], kv_scale=kvs)
             h_shard = comm.linear_rs(attn.view(T_pad, hq * D), lw.w_o, residual=h_shard)
             if lora is not None:
                 h_shard = lora.apply_tp("o", li, attn.view(T_pad, hq * D), h_shard, fb, comm)

@@ -227,7 +227,7 @@ class LoopedStage(LayerListStage):
                              window=m.window, keep_first=m.keep_first, out=heads[:Tp])
         if fb.num_decode:
             ops.attn_decode(q[Tp:], cache.k, cache.v, fb.d_block_tables, fb.d_ctx_lens, m.scale, window=m.window,
-                            max_ctx=fb.d_max_ctx, keep_first=m.keep_first, out=heads[Tp:])
+                            max_ctx=fb.d_max_ctx, total_ctx=fb.d_total_ctx, keep_first=m.keep_first, out=heads[Tp:])
         return heads
 
     def _mixer(self, lw: LoopedLayer, cache, h: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:

@@ -158,5 +158,5 @@ class MSAStage(DecoderStage):
                 sparse(slice(Tp, T), fb.d_block_tables, None, fb.d_max_ctx)
             else:
                 ops.attn_decode(q[Tp:], kc, vc, fb.d_block_tables, fb.d_ctx_lens, self.scale, max_ctx=fb.d_max_ctx,
-                                out=attn[Tp:], kv_scale=kvs)
+                                total_ctx=fb.d_total_ctx, out=attn[Tp:], kv_scale=kvs)
         return attn.view(T, Hq * D)

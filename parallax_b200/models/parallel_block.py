@@ -154,7 +154,7 @@ class ParallelBlockStage(LayerListStage):
                              sinks=lw.sinks, out=heads[:Tp])
         if fb.num_decode:
             ops.attn_decode(q[Tp:], src.k, src.v, fb.d_block_tables, fb.d_ctx_lens, m.scale, sinks=lw.sinks,
-                            max_ctx=fb.d_max_ctx, out=heads[Tp:])
+                            max_ctx=fb.d_max_ctx, total_ctx=fb.d_total_ctx, out=heads[Tp:])
         ops.gated_rows(heads, m.vdim, proj[:, offs["g"]:offs["g"] + m.out_width], out)
 
     def _lightning(self, lw: ParallelLayer, li: int, h: torch.Tensor, fb: ForwardBatch, out: torch.Tensor) -> None:

@@ -180,7 +180,7 @@ class PreNormStage(LayerListStage):
                              out=heads[:Tp], **score)
         if fb.num_decode:
             ops.attn_decode(q[Tp:], cache.k, cache.v, fb.d_block_tables, fb.d_ctx_lens, m.scale, max_ctx=fb.d_max_ctx,
-                            out=heads[Tp:], **score)
+                            total_ctx=fb.d_total_ctx, out=heads[Tp:], **score)
         return heads
 
     def _convolve(self, lw: PreNormLayer, cache, x, fb: ForwardBatch) -> torch.Tensor:

@@ -82,6 +82,7 @@ _SIGS = {
     "pxl_attn_decode": [_P, c_int64, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
                         c_int64, c_float, c_int, c_int, c_int, c_int, c_float, _P, _P, _P],
     "pxl_attn_decode_splits": [c_int] * 7,
+    "pxl_attn_decode_splits_of": [c_int] * 7 + [c_int64],
     "pxl_attn_decode_launches": [c_int] * 6 + [c_float, c_int],
     "pxl_attn_prefill": [_P, c_int64, _P, _P, _P, _P, _P, _P, c_int64, _P, c_int, c_int, c_int,
                          c_int, c_int, c_int, c_int, c_int64, c_float, c_int, c_int, c_float, _P, _P, _P],

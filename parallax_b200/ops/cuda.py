@@ -463,9 +463,11 @@ def attn_decode(
     keep_first: int = 0,
     softcap: float = 0.0,
     sigmoid_bias: Optional[torch.Tensor] = None,
+    total_ctx: int = 0,
 ) -> torch.Tensor:
     """q ``[B, Hq, D]`` (may be a strided view into a packed qkv buffer) vs the paged cache (bf16, or e4m3
-    with ``kv_scale``). With a ``window`` the first ``keep_first`` keys of a sequence stay visible."""
+    with ``kv_scale``). With a ``window`` the first ``keep_first`` keys of a sequence stay visible. The work is split as
+    suits ``total_ctx`` keys of all sequences together, of which the longest has ``max_ctx`` (0: all as long as that)."""
     B, Hq, D = q.shape
     assert q.stride(2) == 1 and q.stride(1) == D
     Hkv, page = k_cache.shape[1], k_cache.shape[2]
@@ -479,7 +481,7 @@ def attn_decode(
     if num_splits <= 0:
         # keys a query reads: whole tiles of 64 of the window and of the kept ones
         span = min(max_ctx, window + keep_first + 128) if window > 0 else max_ctx
-        num_splits = _lib.lib().pxl_attn_decode_splits(B, Hq, Hkv, D, page, _is_fp8_cache(k_cache), span)
+        num_splits = _lib.lib().pxl_attn_decode_splits_of(B, Hq, Hkv, D, page, _is_fp8_cache(k_cache), span, total_ctx)
     ws = None
     if num_splits > 1:
         ws = workspace(q.device, "attn_decode", B * Hq * num_splits * (D + 2) * 4)

@@ -211,7 +211,8 @@ def _attend(q, k, v, scale, q_pos, window, sinks, keep_first=0, softcap=0.0, sig
 
 
 def attn_decode(q, k_cache, v_cache, block_tables, ctx_lens, scale, window=0, sinks=None,
-                max_ctx=0, num_splits=0, out=None, kv_scale=(1.0, 1.0), keep_first=0, softcap=0.0, sigmoid_bias=None):
+                max_ctx=0, num_splits=0, out=None, kv_scale=(1.0, 1.0), keep_first=0, softcap=0.0, sigmoid_bias=None,
+                total_ctx=0):
     """One query per sequence over the paged cache; ``window`` keys per query (0: all) and the sequence's first
     ``keep_first``. ``softcap``: scores become ``softcap * tanh(score / softcap)``. ``sigmoid_bias [Hq]``: the weight of a
     key is ``sigmoid(score + bias)``, not a softmax, and nothing normalises the weights."""
