@@ -572,7 +572,7 @@ struct RowsBf16 {
 constexpr int kDecStages = 3;
 constexpr int kDecThreads = 160;  // 4 consumer warps + 1 producer warp
 
-// CLUSTER: the splits of a (sequence, key head) are a cluster and add their results (add_splits); else through the workspace
+// CLUSTER: the splits of a (sequence, key head) are a cluster and add their results (SplitParts); else through the workspace
 template <int SM, bool CLUSTER, bool HIGH>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
