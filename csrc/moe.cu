@@ -287,26 +287,28 @@ moe_align_kernel(const int* __restrict__ ids, int n, int k, int E, int e_lo, int
   }
 }
 
-// x_perm[p, :] = x[src_tok[p], :]   for p < *n_rows. A warp per row, eight vectors of a lane in flight: a block per row spends
-// as long on starting blocks as on the copy (38400 rows x 2048: 42 -> 28 us).
+// x_perm[p, :] = x[src_tok[p], :]   for p < *n_rows. A warp per U x 32 vectors of a row, all in flight: a block per row spends as long
+// on starting blocks as on the copy (38400 rows x 2048: 42 us, now 31), a warp for the whole of a wide row is a chain of loads and stores.
+// Few rows are bound by latency, many by their bytes (block per row, warp per row, now, us): 8 rows x 7168 2.8, 4.1, 2.1; 384 x 7168
+// 3.4, 4.7, 2.9; 1024 x 2048 2.9, 2.6, 2.6; 8192 x 7168 24.4, 28.3, 23.2.
+template <int U>
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ src_tok,
-                  const int* __restrict__ n_rows, bf16* __restrict__ x_perm, int H) {
+                   const int* __restrict__ n_rows, bf16* __restrict__ x_perm, int H, int per_row) {
   pdl_wait();
   pdl_launch_dependents();
-  const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int part = blockIdx.x * 8 + (threadIdx.x >> 5), p = part / per_row;
+  const int v0 = part % per_row * (32 * U) + (threadIdx.x & 31), nvec = H >> 3;
   if (p >= *n_rows) return;
   const bf16* src = x + static_cast<size_t>(src_tok[p]) * H;
   bf16* dst = x_perm + static_cast<size_t>(p) * H;
-  for (int v0 = lane; v0 < (H >> 3); v0 += 256) {
-    bf16x8 w[8];
+  bf16x8 w[U];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (v0 + 32 * i < (H >> 3)) w[i] = ld_bf16x8(src + (v0 + 32 * i) * 8);
+  for (int i = 0; i < U; ++i)
+    if (v0 + 32 * i < nvec) w[i] = ld_bf16x8(src + (v0 + 32 * i) * 8);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (v0 + 32 * i < (H >> 3)) st_bf16x8(dst + (v0 + 32 * i) * 8, w[i]);
-  }
+  for (int i = 0; i < U; ++i)
+    if (v0 + 32 * i < nvec) st_bf16x8(dst + (v0 + 32 * i) * 8, w[i]);
 }
 
 // x_perm[pos_of[t, j], :] = weights[t, j] * x[t, :]: rows in expert order whose routing weight is part of the input. One CTA
@@ -464,8 +466,15 @@ PXL_EXPORT int pxl_moe_gather(const void* x, const int* src_tok, const int* n_ro
                               int max_rows, int H, pxl_stream_t stream) {
   if (max_rows <= 0) return PXL_OK;
   if (H % 8) return PXL_ERR_INVALID_ARG;
-  pxl_host::launch(moe_gather_kernel, pxl::ceil_div(max_rows, 8), 256, 0, stream, static_cast<const bf16*>(x), src_tok, n_rows,
-                                                  static_cast<bf16*>(x_perm), H);
+  const int nvec = H >> 3;
+  auto go = [&](auto kern, int u) {
+    const int per_row = pxl::ceil_div(nvec, 32 * u);
+    pxl_host::launch(kern, pxl::ceil_div(max_rows * per_row, 8), 256, 0, stream, static_cast<const bf16*>(x), src_tok, n_rows,
+                     static_cast<bf16*>(x_perm), H, per_row);
+  };
+  // four vectors per lane once they give the SMs a few warps each (2400 parts of four: 2.93 us with two, 3.07; 7168: 5.53 and 4.83)
+  if (static_cast<int64_t>(max_rows) * pxl::ceil_div(nvec, 128) >= 4096) go(moe_gather_kernel<4>, 4);
+  else go(moe_gather_kernel<2>, 2);
   return check_launch();
 }
 
