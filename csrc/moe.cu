@@ -355,6 +355,11 @@ __global__ void __launch_bounds__(512) moe_scatter_rows_kernel(const T* __restri
 }
 
 // out[t, :] = (base ? base[t, :] : 0) + sum_j w[t, j] * y_perm[pos_of[t*k + j], :]
+// U rows at a time: their places first, then their vectors, then the sums in order. Four are fewer latencies one after the other, one
+// leaves room for eight blocks per SM instead of five (one and four, us: 48 tokens x 2048, 8 experts each, 3.8 and 3.1; 512 x 7168, 8
+// experts 24.8 and 18.2; 2000 of them 55.3 and 52.4; a single wave of eight blocks, 1024 of them, 30.3 and 32.5; two experts never gain,
+// 1024 x 4096 8.4 and 11.1).
+template <int U>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ pos_of,
                    const float* __restrict__ w, const bf16* __restrict__ base,
@@ -376,18 +381,16 @@ moe_combine_kernel(const bf16* __restrict__ y_perm, const int* __restrict__ pos_
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0.f;
     }
-    // Four rows at a time: their places first, then their vectors, then the sums in order (48 tokens x 2048, 8 experts each: 7.1 ->
-    // 5.1 us, 4800 tokens 40.0 -> 38.8; eight at a time 4.0 and 44.7, for want of threads).
-    for (int s0 = 0; s0 < k; s0 += 4) {
-      int p[4];
-      bf16x8 y[4];
+    for (int s0 = 0; s0 < k; s0 += U) {
+      int p[U];
+      bf16x8 y[U];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = s0 + i < k ? pos_of[t * k + s0 + i] : -1;
+      for (int i = 0; i < U; ++i) p[i] = s0 + i < k ? pos_of[t * k + s0 + i] : -1;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < U; ++i)
         if (p[i] >= 0) y[i] = ld_bf16x8(y_perm + static_cast<size_t>(p[i]) * H + v * 8);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < U; ++i) {
         if (p[i] < 0) continue;
         const float ws = w[t * k + s0 + i];
 #pragma unroll
@@ -501,8 +504,12 @@ PXL_EXPORT int pxl_moe_combine(const void* y_perm, const int* pos_of, const floa
                                pxl_stream_t stream) {
   if (T <= 0) return PXL_OK;
   if (H % 8) return PXL_ERR_INVALID_ARG;
-  pxl_host::launch(moe_combine_kernel, T, 256, 0, stream, static_cast<const bf16*>(y_perm), pos_of, w,
-                                            static_cast<const bf16*>(base),
-                                            static_cast<bf16*>(out), k, H);
+  auto go = [&](auto kern) {
+    pxl_host::launch(kern, T, 256, 0, stream, static_cast<const bf16*>(y_perm), pos_of, w, static_cast<const bf16*>(base),
+                     static_cast<bf16*>(out), k, H);
+  };
+  const int sms = pxl_host::num_sms();
+  if (k <= 2 || (T > 5 * sms && T <= 8 * sms)) go(moe_combine_kernel<1>);  // (one wave of eight blocks per SM, more than one of five)
+  else go(moe_combine_kernel<4>);
   return check_launch();
 }
