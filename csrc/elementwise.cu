@@ -562,9 +562,10 @@ PXL_EXPORT int pxl_rmsnorm(const void* x, const void* weight, void* out, void* r
   const bf16* wp = static_cast<const bf16*>(weight);
   bf16* op = static_cast<bf16*>(out);
   bf16* rp = static_cast<bf16*>(residual);
-  if (H <= 2048 && T >= 2048) {
+  if (H <= 2048 && T >= (H <= 512 ? 1536 : 2048)) {
     // short rows by the thousand: blocks of eight rows, a block for each would be bound by their number (8192 x 1024: 7.2 us
-    // against 9.6; 4096 x 1536: 5.9 against 6.1; 1024 rows are better off with a block each, 2.5 against 3.2)
+    // against 9.6; 4096 x 1536: 5.9 against 6.1; 1024 rows are better off with a block each, 2.5 against 3.2, and up to 512 columns
+    // 1536 rows are as fast either way, 2047 x 256 2.6 and 3.1)
     const unsigned grid = static_cast<unsigned>((T + 7) / 8);
     if (residual)
       pxl_host::launch(rmsnorm_warp_kernel<true, 8>, grid, 256, 0, stream, xp, wp, op, rp, T, H, eps, w_offset);
@@ -573,22 +574,18 @@ PXL_EXPORT int pxl_rmsnorm(const void* x, const void* weight, void* out, void* r
     return check_launch();
   }
   const int nvec = H >> 3;
-  if (H <= 16384) {
+  if (H <= 16384 && !(residual && H > 8192 && T >= 1024)) {
     // vectors per thread: two for the shortest chain while the SMs are not full, four once throughput counts (128 x 4096: 2.1 us
-    // with two, 2.3 with four; 1016 x 7168: 8.6 and 6.9; 8192 x 4096: 28.7 and 23.2)
-    int nv = T < 512 ? 2 : 4;
+    // with two, 2.3 with four; 1016 x 7168: 8.6 and 6.9; 8192 x 4096: 28.7 and 23.2). With a residual a thread has two rows' loads
+    // in flight anyway, and a store ahead of the sum: one (16 x 1024: 2.0 us, 2.5 with two; 4096 x 4096: 22.4, and 26.2 with four), up
+    // to the width at which that is a block of 1024 threads and many rows want several blocks per SM: 4096 x 12288 71 us, rows read
+    // twice 66.
+    int nv = residual ? 1 : T < 512 ? 2 : 4;
     while (nvec > nv * 1024) nv *= 2;
     const int threads = pxl::ceil_div(pxl::ceil_div(nvec, nv), 32) * 32;
-#define PXL_RMS(NV)                                                                                                      \
-  do {                                                                                                                   \
-    if (residual)                                                                                                        \
-      pxl_host::launch(rmsnorm_kernel<true, NV>, T, threads, 0, stream, xp, wp, op, rp, H, eps, w_offset);               \
-    else                                                                                                                 \
-      pxl_host::launch(rmsnorm_kernel<false, NV>, T, threads, 0, stream, xp, wp, op, rp, H, eps, w_offset);              \
-  } while (0)
-    if (nv == 2) PXL_RMS(2);
-    else PXL_RMS(4);
-#undef PXL_RMS
+    auto go = [&](auto kern) { pxl_host::launch(kern, T, threads, 0, stream, xp, wp, op, rp, H, eps, w_offset); };
+    if (residual) nv == 1 ? go(rmsnorm_kernel<true, 1>) : go(rmsnorm_kernel<true, 2>);
+    else nv == 2 ? go(rmsnorm_kernel<false, 2>) : go(rmsnorm_kernel<false, 4>);
     return check_launch();
   }
   if (residual)
