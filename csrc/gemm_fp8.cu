@@ -203,9 +203,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       cp_async_commit();
     };
     fetch(0);
-    uint64_t acc2[FN / 2];
+    float acc[FN];
 #pragma unroll
-    for (int i = 0; i < FN / 2; ++i) acc2[i] = 0ull;
+    for (int i = 0; i < FN; ++i) acc[i] = 0.f;
     bool ok = true;
     for (int kb = 0; kb < num_kb; ++kb) {
       const int part = kb & 1, buf = (kb / F_GROUP) & 1;
@@ -224,7 +224,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + part * FN + (static_cast<uint32_t>(q * 32) << 16);
       // 16 columns are on their way while the 16 before them are added, two per instruction (32 columns at a time without the
-      // overlap: a tenth slower than the sums one by one; in pairs this way: 7168 x 18432, 4000 tokens 666 -> 614 us)
+      // overlap: a tenth slower than the sums one by one; in pairs this way: 7168 x 18432, 4000 tokens 666 -> 614 us).
+      // The sums stay single numbers that are put into pairs here: held as pairs and taken apart behind the loop they cost registers and a
+      // microsecond at its end (100 tokens x 1024 x 512 9.5 us, 7.5 this way; 7.6 one by one).
       uint32_t r[2][16];
       tmem_ld_32x32b_x16(t_row, r[0]);
 #pragma unroll
@@ -237,7 +239,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         for (int j = 0; j < 16; j += 2) {
           uint64_t x;
           asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(r[(c >> 4) & 1][j]), "r"(r[(c >> 4) & 1][j + 1]));
-          acc2[(c + j) >> 1] = fma2(x, sc2, acc2[(c + j) >> 1]);
+          uint64_t y;
+          asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(acc[c + j]), "f"(acc[c + j + 1]));
+          y = fma2(x, sc2, y);
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[c + j]), "=f"(acc[c + j + 1]) : "l"(y));
         }
       }
       tc_fence_before_sync();
@@ -245,9 +250,6 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       if (lane == 0) mbar_arrive(pempty0 + 8 * part);
     }
     cp_async_wait<0>();
-    float acc[FN];
-#pragma unroll
-    for (int i = 0; i < FN / 2; ++i) acc[2 * i] = __uint_as_float(static_cast<uint32_t>(acc2[i])), acc[2 * i + 1] = __uint_as_float(static_cast<uint32_t>(acc2[i] >> 32));
     if constexpr (SPLIT) {
       // every load and product of this CTA is done: its stages take the partial sums
       if (ok) {
