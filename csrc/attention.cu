@@ -1658,38 +1658,41 @@ int set_smem(K kern, int bytes) {
 // ceil(2 SMs / CTAs), the rule before, did not see; where rows differ in length it is filled by the rows behind (`behind`: the part
 // of that cost that stays).
 //
-// Pages the TMA unit reads (head dim 128): 2 CTAs per SM; `part` us per tile of 64 keys while the memory is not full (over bf16 pages
-// less behind a full wave, whose rows do not end together), `full` beside a full chip of others, `alone` where the others are done.
-// Adding is cheaper inside a cluster than through the workspace. Tiles dealt out evenly (attn_decode_even_kernel, asked for by splits
-// that give two places per CTA) take `full` for each and a start, a sum and a share per pair (more where short pairs stand beside long
-// ones, for CTAs that have many: even_short), and the reduction 0.4 per four query heads and CTA that the longest row lies in. Fitted
-// to 36 sizes of 1 to 512 rows and 100 to 100000 keys per type, rows alike (8 key heads, splits or even: us, before and now):
-//   rows x keys   bf16                          e4m3
-//   1 x 777       4:  8.1      7:    6.7        4:  7.5     7:     6.4
-//   8 x 2100      5: 21.0      4:   16.2        5: 27       4:    12.1
-//   16 x 1280     3: 24.6      2:   17.8        3: 18.6     2:    12.9
-//   40 x 4000     1: 121       even: 95         1: 81       even: 56
-//   128 x 4096    1: 278       1:   278         1: 169      even: 154
-//   512 x 100     1: 78        even: 47         1: 71       even: 57
-// and to 780 batches of 2 to 256 rows and 1 to 8 key heads, alike, one row of up to 60 times the others, spread evenly or over their
-// logarithm: time over the fastest measured with the rule before, every row taken for as long as the longest, and now: bf16 1.34,
-// 1.27, 1.02; e4m3 1.43, 1.15, 1.02 (mean; 6.1, 8.2, 1.4 and 6.7, 5.8, 1.6 at most). 32 rows of which one has 32768 keys and the others
-// 1000: 2: 183, 1: 284, even: 62.
-// The kernel for other pages and head dim 64: 5 CTAs per SM (3 at 128), 1.0 us per tile either way, 0.8 alone, through the workspace 3 +
-// 0.03 per split and 1 per 296 CTAs: rows alike, head dim 64, 16 x 1280 3: 18.3, 5: 16.3; 40 x 4000 1: 118, 2: 80.1; 36 x 1280 2: 26.3
-// both; the 780 batches 1.89, 1.16, 1.02.
+// Pages the TMA unit reads (head dim 128): 2 CTAs per SM; `part` us per tile of 64 keys while the memory is not full (less behind a
+// full wave, whose rows do not end together), `full` beside a full chip of others, `alone` where the others are done. Adding is cheaper
+// inside a cluster than through the workspace, whose bytes grow with the query heads per key head. Tiles dealt out evenly (attn_decode_even_kernel, asked for by splits that give two
+// places per CTA) take `full` for each and a start, a sum and a share per pair (more where short pairs stand beside long ones: even_short
+// per pair, for CTAs that have many, and even_each per tile), and the reduction a time per four query heads and CTA that the longest row lies in. The kernel for
+// other pages and head dim 64: 5 CTAs per SM (3 at 128), 1.2 us per tile (1.5 at 128, 2 of e4m3 bytes), always through the workspace.
+//
+// Fitted to the times of every count, in a chain of launches, for 1370 batches (TMA; 750 of the other kernel) of 1 to 512 rows, 16 to 100000 keys, 1 to 8
+// key heads and 1 to 16 query heads for each: rows alike, within a quarter, one of up to 60 times the others, spread evenly or over their
+// logarithm. Time over the fastest measured, mean and worst, with the rule before, with every row taken for as long as the longest,
+// and now:
+//   bf16, TMA          1.27 4.8   1.20 6.4   1.01 1.2     e4m3, TMA          1.34 7.4   1.14 7.9   1.01 1.4
+//   bf16, head dim 64  1.59 8.5   1.09 3.3   1.02 1.2     e4m3, head dim 64  1.77 7.7   1.13 3.7   1.02 1.2
+//   bf16, other pages  1.54 6.5   1.17 5.8   1.03 1.3     e4m3, other pages  1.75 7.5   1.27 6.9   1.03 1.4
+// 8 key heads, splits or even (us, with the rule before and now):
+//   rows x keys        bf16                       e4m3
+//   1 x 777            4:  8.1      7:    6.7     4:  7.5     7:     6.4
+//   16 x 1280          3: 24.6      2:   17.8     3: 18.6     2:    12.9
+//   40 x 4000          1: 121       even: 95      1: 81       even: 56
+//   512 x 100          1: 78        even: 47      1: 71       even: 57
+//   1 x 32768 and
+//     31 x 1000        2: 183       even: 62      2: 167      even: 48   (every row for as long as the longest: bf16 1: 284)
 //
 // total_ctx: keys of all rows together, 0 where it is not known: rows as long as the longest.
 PXL_EXPORT int pxl_attn_decode_splits_of(int B, int Hq, int Hkv, int D, int page_size, int cache_fp8, int max_ctx, int64_t total_ctx) {
   struct Line {
-    float start, part, part_behind, full, cluster, add, add_split, add_wave, even, even_pair, even_short, even_margin, alone;
+    float start, part, part_behind, full, cluster, add, add_split, add_wave, even, even_pair, even_short, even_each, even_part, even_margin, alone;
   };
-  static constexpr Line kLines[2] = {{2.f, 1.f, 0.85f, 1.4f, 1.1f, 1.3f, 0.13f, 0.8f, 9.f, 0.7f, 0.f, 0.95f, 0.55f},
-                                     {2.7f, 0.59f, 0.59f, 0.66f, 2.5f, 1.4f, 0.09f, 2.4f, 9.f, 0.4f, 8.f, 1.f, 0.45f}};
+  static constexpr Line kLines[2] = {{1.9f, 0.9f, 0.65f, 1.4f, 1.45f, 2.5f, 0.14f, 0.23f, 8.9f, 0.85f, 0.f, 0.35f, 0.5f, 0.95f, 0.65f},
+                                     {2.3f, 0.61f, 0.7f, 0.68f, 2.4f, 1.4f, 0.23f, 0.49f, 9.f, 0.3f, 7.f, 0.16f, 0.4f, 0.98f, 0.55f}};
   const Line& c = kLines[cache_fp8 ? 1 : 0];
   const bool tma = D == 128 && (page_size == 16 || page_size == 32 || page_size == 64);
   const int64_t pairs = static_cast<int64_t>(B) * Hkv;
   const int chip = 2 * pxl_host::num_sms(), slots = tma ? chip : (D == 64 ? 5 : 3) * pxl_host::num_sms();
+  const float tile = cache_fp8 ? 2.f : D == 64 ? 1.2f : 1.5f;  // of the other kernel
   if (max_ctx < 1) max_ctx = 1;
   const int tiles = pxl::ceil_div(max_ctx, TILE);
   // a mean row, as a part of the longest (its last tile is half full)
@@ -1697,7 +1700,8 @@ PXL_EXPORT int pxl_attn_decode_splits_of(int B, int Hq, int Hkv, int D, int page
   if (total_ctx > 0 && total_ctx < static_cast<int64_t>(B) * max_ctx)
     mean = fminf(1.f, (static_cast<float>(total_ctx) / (static_cast<float>(B) * TILE) + 0.5f) / static_cast<float>(tiles));
   const float behind = fmaxf(0.f, 1.f - 4.f * (1.f - mean));
-  const bool even = tma && Hkv > 0 && Hq / Hkv <= 8 && pairs > 0 && pairs * 64 >= 2 * chip;
+  const int group = Hkv > 0 ? Hq / Hkv : 0;
+  const bool even = tma && group > 0 && group <= 8 && pairs > 0 && pairs * 64 >= 2 * chip;
   int best = 1, last = 0;
   float best_us = 0.f;
   for (int s = 1; s <= 64 && s <= tiles; ++s) {
@@ -1714,18 +1718,18 @@ PXL_EXPORT int pxl_attn_decode_splits_of(int B, int Hq, int Hkv, int D, int page
       const float share = c.full * wave;
       us = (mine + c.start) * (c.full * static_cast<float>(full) + last_wave(fmaxf(full ? c.part_behind : c.part, share), share));
       us += longer * c.alone;
-      if (s > 1) us += s <= kMaxClusterSplits && waves <= 0.9375f ? c.cluster : c.add + c.add_split * s + c.add_wave * waves;
+      if (s > 1) us += s <= kMaxClusterSplits && waves <= 0.9375f ? c.cluster : c.add + c.add_split * s + c.add_wave * group * waves;
     } else {
-      us = mine * (static_cast<float>(full) + last_wave(1.f, wave)) + longer * 0.8f;
-      if (s > 1) us += 3.f + 0.03f * s + waves;
+      us = (mine * (static_cast<float>(full) + last_wave(1.f, wave)) + longer) * tile;
+      if (s > 1) us += 2.f + 0.08f * s + 0.8f * waves;
     }
     if (s == 1 || us < best_us) best = s, best_us = us;
   }
   if (even) {
     const float waves = static_cast<float>(pairs) / static_cast<float>(chip), each = waves * mean * static_cast<float>(tiles);  // tiles per CTA
     const float parts = fmaxf(0.f, static_cast<float>(tiles) / fmaxf(each, 1.f) - 1.f);
-    const float us = c.full * each + c.even + c.even_pair * waves + 0.41f * pxl::ceil_div(Hq / Hkv, 4) * parts +
-                     (1.f - mean) * (c.even_short * waves + 0.1f * each);
+    const float us = c.full * each + c.even + c.even_pair * waves + c.even_part * pxl::ceil_div(group, 4) * parts +
+                     (1.f - mean) * (c.even_short * waves + c.even_each * each);
     if (us < c.even_margin * best_us) best = pairs >= chip ? 2 : static_cast<int>((2 * chip + pairs - 1) / pairs);
   }
   return best;
