@@ -1464,7 +1464,9 @@ int rows_ahead_of_the_tail(int M, int N, int K, int epi) {
   const int tail = M - ahead;
   if (ahead <= 0 || tail <= 0 || tail > kMidMaxM) return M;
   const double alone = tail <= kSmallMaxM ? 2.0 * N * K / 5.0e6 + 8.0 : mid_m_plan(tail, N, K, kTailWidths).cost;
-  return plain(ahead) + alone < 0.97 * plain(M) ? ahead : M;
+  // 220 products of 1031 to 9000 rows: 1.004 of the faster way on average, 1.08 at most; with 0.97 the same, but 2461 x 4096 x 12288
+  // 217 us in one launch, 204 in two; never in two 1.032 and 1.30
+  return plain(ahead) + alone < 0.98 * plain(M) ? ahead : M;
 }
 
 int gemm_mid_m(const void* A, const void* W, void* C, bool f32_out, const void* residual, const void* bias, int M,
