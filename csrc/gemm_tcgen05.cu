@@ -1164,10 +1164,13 @@ constexpr int kMidMaxM = 1024;
 // chain of launches (weights streamed from HBM):
 //   plain persistent kernel   rounds x (k-blocks x t_kb) + fixed
 //   cluster split-K           k-blocks per CTA x t_kb + exchange (of partial sums)
+// each with what the last tile's residual, bias or fp32 results take per column and thread, which the CTAs of a cluster share.
 // t_kb = time of one 64-deep k-block per CTA, set by what the SM can pull from L2, 64 bytes a clock (48 KB per k-block for a
 // 128 x 256 tile, 32 KB for 128 x 128). Split variants are only considered when all clusters are resident at once (a second round
 // pays the fixed cost again and was always slower: 144 CTAs in clusters of 3, which pack the GPCs badly, are one).
-// The choice is within 5 % of the fastest of all variants in all 132. Against the figures before the issuing warps' loops
+// The choice is within 5 % of the fastest of all variants in all 132 without a residual; with one, over 25 shapes of 129 to 1024 rows,
+// 1.006 of the fastest on average, 1.13 at most (without its term 1.018 and 1.15: 256 x 512 x 2048 9.6 us in 64 columns, 8.4 in clusters
+// of four). Against the figures before the issuing warps' loops
 // were shortened (0.43, 0.29, 0.36 and 7; no clusters of 3, no 64 columns): 256 rows x 2112 x 7168 18.8 -> 16.0 us, 4096 x 12288
 // 34.2 -> 31.7, gated 24576 x 4096 60.2 -> 53.4.
 struct MidWidth {
@@ -1422,13 +1425,13 @@ struct MidPlan {
   double cost;
 };
 template <int W>
-MidPlan mid_m_plan(int M, int N, int K, const MidWidth (&widths)[W]) {
+MidPlan mid_m_plan(int M, int N, int K, const MidWidth (&widths)[W], double column = 0.0) {
   const int num_kb = pxl::ceil_div(K, BK);
   const int num_m = pxl::ceil_div(M, BM);
   MidPlan best{0, 1, 1e300};
   for (const MidWidth& w : widths) {
     const int tiles = num_m * pxl::ceil_div(N, w.bn);
-    const double plain = mid_plain_cost(M, N, K, w);
+    const double plain = mid_plain_cost(M, N, K, w) + w.bn * column;
     if (plain < best.cost) best = MidPlan{w.bn, 1, plain};
     if (w.exchange < 0) continue;
     for (int sk = 2; sk <= 4; ++sk) {
@@ -1436,7 +1439,7 @@ MidPlan mid_m_plan(int M, int N, int K, const MidWidth (&widths)[W]) {
       const int kb_per = pxl::ceil_div(num_kb, sk);
       if (pxl::ceil_div(num_kb, kb_per) != sk) continue;  // no empty K range
       if (tiles > mid_m_max_clusters(w.bn, sk)) continue;
-      const double cost = kb_per * w.kb + w.exchange + sk * w.exchange_each;
+      const double cost = kb_per * w.kb + w.exchange + sk * w.exchange_each + 0.7 * w.bn * column / sk;
       if (cost < best.cost) best = MidPlan{w.bn, sk, cost};
     }
   }
@@ -1502,12 +1505,15 @@ int gemm_mid_m(const void* A, const void* W, void* C, bool f32_out, const void* 
 
 // Which (tile width, K ranges) pxl_gemm_bf16 picks for a shape with 128 < M <= 1024: returns
 // bn * 16 + splitk, splitk == 1 meaning the plain persistent kernel.
-PXL_EXPORT int pxl_gemm_bf16_mid_m_plan(int M, int N, int K, int epi) {
+static int mid_plan(int M, int N, int K, int epi, bool bias) {
   if (mid_m_disabled() || M <= BM || M > kMidMaxM) return 0;
   if (epi != PXL_EPI_NONE && epi != PXL_EPI_RESIDUAL && epi != PXL_EPI_F32) return 0;
-  const MidPlan p = mid_m_plan(M, N, K, kMidWidths);
+  const MidPlan p = mid_m_plan(M, N, K, kMidWidths, epi == PXL_EPI_RESIDUAL ? 0.02 : bias || epi == PXL_EPI_F32 ? 0.016 : 0.0);
   return p.bn * 16 + p.splitk;
 }
+
+// (without a bias)
+PXL_EXPORT int pxl_gemm_bf16_mid_m_plan(int M, int N, int K, int epi) { return mid_plan(M, N, K, epi, false); }
 
 // Explicit entry to the mid-M cluster split-K kernel (tests and benchmarks; pxl_gemm_bf16 picks it by itself).
 PXL_EXPORT int pxl_gemm_bf16_mid_m(const void* A, const void* W, void* C, const void* residual, const void* bias,
@@ -1541,7 +1547,7 @@ PXL_EXPORT int pxl_gemm_bf16(const void* A, const void* W, void* C, const void* 
     return gemm_small_m(A, W, C, epi == PXL_EPI_F32, epi == PXL_EPI_RESIDUAL ? residual : nullptr, bias, M, N, K,
                         lda, ldw, ldc, 0, 0, status, stream);
   if (bn == 0 && !((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(bias)) & 15)) {
-    const int plan = pxl_gemm_bf16_mid_m_plan(M, N, K, epi);
+    const int plan = mid_plan(M, N, K, epi, bias != nullptr);
     if (plan > 0 && (plan & 15) > 1)
       return gemm_mid_m(A, W, C, epi == PXL_EPI_F32, epi == PXL_EPI_RESIDUAL ? residual : nullptr, bias, M, N, K, lda,
                         ldw, ldc, plan >> 4, plan & 15, status, stream);
