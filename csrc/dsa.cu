@@ -366,7 +366,7 @@ __device__ __forceinline__ uint32_t order_key(float x) {
 // One CTA per query row: radix select of the k largest scores among positions [0, pos], eight bits a pass. Rows of up to 8192 scores
 // are read once and stay in registers (HELD). What it takes is chains, not bytes (24 KB a row): lanes that fall into one bin add once
 // (the first bits of scores are few different ones), a warp finds the bin of the k-th score with one scan, and places in the list are
-// given out a warp at a time. One thread per score and per bin, 1000 rows of 5500 scores and k = 2048 took 65 us, 16 of 8000 31 us;
+// given out a warp at a time. One thread per score and per bin, 1000 rows of 5500 scores and k = 2048 took 62 us, 16 of 8000 35 us;
 // 40 and 17 us now (64 rows of 60000, which do not fit the registers: 125 and 97).
 constexpr int kTopkThreads = 512, kTopkHeld = 16;
 template <bool HELD>

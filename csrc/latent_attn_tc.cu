@@ -324,12 +324,6 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
       const int next_row = listed ? listed_row(list_tile(it + 1) * NK + lane) : tile_row(it + 1);
       const int next_row2 = listed ? listed_row(list_tile(it + 1) * NK + 32 + lane) : 0;
       if (listed) spread(row, row2);
-      auto key_chunk = [&](int j, uint32_t dst, uint32_t bar) {
-        if (listed) gather(dst, bar, k_chunk(j) * 64);
-        else
-          for (int p = 0; p < pieces; ++p)
-            tma_box(dst + p * box * 128, &tm_kv, bar, k_chunk(j) * 64, __shfl_sync(0xffffffffu, row, p), leader);
-      };
       if constexpr (WIDE) {  // two groups of chunks, a barrier each
         if (keys) {
           ok = acquire(k_empty, k_full, it, kWideFirst * kKvChunk);
@@ -358,6 +352,12 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
           }
         }
       } else {
+        auto key_chunk = [&](int j, uint32_t dst, uint32_t bar) {
+          if (listed) gather(dst, bar, k_chunk(j) * 64);
+          else
+            for (int p = 0; p < pieces; ++p)
+              tma_box(dst + p * box * 128, &tm_kv, bar, k_chunk(j) * 64, __shfl_sync(0xffffffffu, row, p), leader);
+        };
         for (int j = 0; ok && keys && j < nkc; ++j) {
           ok = acquire(k_empty + 8 * slot, k_full + 8 * slot, slot_use, kKvChunk);
           if (ok) key_chunk(j, sm_k + slot * kKvChunk, k_full + 8 * slot);
@@ -368,7 +368,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q_map, const __grid
         }
       }
       if (ok && values) ok = acquire(v_empty + 8 * vb, v_full + 8 * vb, vb_use, nv * kKvChunk);
-      if (ok && values && listed)
+      if (!WIDE && ok && values && listed)  // (WIDE: copies, above)
         for (int c = 0; c < nv; ++c) gather(sm_v + (vb * per + c) * kKvChunk, v_full + 8 * vb, (v0 + c) * 64);
       else if (ok && values)
         for (int p = 0; p < pieces; ++p) {
