@@ -350,6 +350,15 @@ PXL_EXPORT int pxl_gemv_bf16_qkv_takes(int M, int K, int Hq, int Hkv, int D, int
          pxl_gemv_bf16_takes(M, (Hq + 2 * Hkv) * D, K, PXL_EPI_NONE);
 }
 
+// Where that is faster than the product and the rotation apart: with a wave of clusters (of the 37 that two blocks per SM are, the GPCs
+// take 32 to 36), and one row only if they are on every SM. Layers of one row, us, together and apart: 16 + 2 x 8 heads, 1024 wide 18.2
+// and 18.5, 4096 wide 49.6 and 58.6; 32 + 2 x 8 heads, 4096 wide 98 and 96; 64 + 2 x 8, 5120 wide 198 and 181; 32 + 2 x 4, 2048 wide 34.0
+// and 31.7; 8 + 2 x 2, 2048 wide 29.9 and 28.3 (two rows 35.1 and 36.4).
+PXL_EXPORT int pxl_gemv_bf16_qkv_pays(int M, int Hq, int Hkv) {
+  const int ctas = (Hq + 2 * Hkv) * kHeadCtas, sms = pxl_host::num_sms();
+  return ctas * 8 <= 2 * sms * 7 && (M > 1 || ctas >= sms);
+}
+
 PXL_EXPORT int pxl_gemv_bf16_qkv(const void* A, const void* norm_w, float eps, float offset, const void* W, const void* bias, void* qkv,
                                  const void* q_norm_w, const void* k_norm_w, const float* cos_sin, const int* positions,
                                  const int64_t* slot_mapping, void* k_cache, void* v_cache, int M, int K, int Hq, int Hkv, int D,

@@ -56,6 +56,7 @@ int pxl_gemv_bf16_norm(const void* A, const void* norm_w, float eps, float offse
 // and the q, k and v heads of a layer with pxl_qk_norm_rope_cache behind it (head dim 128, rotated over all of it): the query heads'
 // columns of qkv [M, (Hq + 2 Hkv) 128] are written, keys and values go to the cache only.
 int pxl_gemv_bf16_qkv_takes(int M, int K, int Hq, int Hkv, int D, int rot_dim);
+int pxl_gemv_bf16_qkv_pays(int M, int Hq, int Hkv);  // whether it is the faster way
 int pxl_gemv_bf16_qkv(const void* A, const void* norm_w, float eps, float offset, const void* W, const void* bias, void* qkv,
                       const void* q_norm_w, const void* k_norm_w, const float* cos_sin, const int* positions, const int64_t* slot_mapping,
                       void* k_cache, void* v_cache, int M, int K, int Hq, int Hkv, int D, int rot_dim, int page_size, int64_t num_slots,

@@ -136,7 +136,7 @@ PXL_EXPORT int pxl_stage_forward_dense(const PxlStageDesc* st, const PxlStepDesc
     const PxlDenseLayer& L = st->layers[li];
     int op_ = 0;  // 1 norm, 2 qkv, 3 rope+cache, 4 prefill, 5 decode (4 if no prefill), then o_proj, norm, gate_up, down
     void* h_mid = (h == ws->h_a) ? ws->h_b : ws->h_a;
-    const bool heads = H % 8 == 0 && pxl_gemv_bf16_qkv_takes(T, H, Hq, Hkv, D, st->rot_dim);
+    const bool heads = H % 8 == 0 && pxl_gemv_bf16_qkv_takes(T, H, Hq, Hkv, D, st->rot_dim) && pxl_gemv_bf16_qkv_pays(T, Hq, Hkv);
     if (heads) {  // one or two rows: norm, product, rotation and cache in one kernel
       PXL_TRY(pxl_gemv_bf16_qkv(h, L.ln1, st->eps, st->norm_offset, L.w_qkv, L.b_qkv, qkv, L.q_norm, L.k_norm, st->cos_sin, sp->positions,
                                 sp->slots, L.k_cache, L.v_cache, T, H, Hq, Hkv, D, st->rot_dim, st->page, num_slots, st->max_pos, status,
