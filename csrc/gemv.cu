@@ -297,7 +297,8 @@ template <int MM>
 int launch_rows(const GemvArgs& a, int epi, cudaStream_t stream) {
   // rows of W per warp: as many as still give every SM a dozen warps
   const int want = 12 * pxl_host::num_sms();
-  if (a.N >= 4 * want) return launch_epi<MM, 4, 2>(a, epi, stream);
+  // (two rows with a norm, whose squares every warp adds up for itself: four rows of W from fewer warps on; 6144 x 4096 20.6 us with two, 15.9)
+  if (a.N >= 4 * want || (MM == 2 && a.norm_w && a.N >= 3 * want)) return launch_epi<MM, 4, 2>(a, epi, stream);
   if (a.N >= 2 * want || epi == PXL_EPI_SILU_MUL) return launch_epi<MM, 2, 4>(a, epi, stream);
   // one row of W: the whole of it in flight up to K = 3072 (1024 x 2304 3.8 us in rounds of eight, 2.2 in one of twelve; 2048 x 3072 5.4 and
   // 4.1; longer rows take two rounds either way, 1024 x 3584 4.9 and 5.1, and sixteen steps beside the norm's weights spill)
