@@ -1659,17 +1659,19 @@ int set_smem(K kern, int bytes) {
 // of that cost that stays).
 //
 // Pages the TMA unit reads (head dim 128): 2 CTAs per SM; `part` us per tile of 64 keys while the memory is not full (less behind a
-// full wave, whose rows do not end together), `full` beside a full chip of others, `alone` where the others are done. Adding is cheaper
-// inside a cluster than through the workspace, whose bytes grow with the query heads per key head. Tiles dealt out evenly (attn_decode_even_kernel, asked for by splits that give two
-// places per CTA) take `full` for each and a start, a sum and a share per pair (more where short pairs stand beside long ones: even_short
-// per pair, for CTAs that have many, and even_each per tile), and the reduction a time per four query heads and CTA that the longest row lies in. The kernel for
-// other pages and head dim 64: 5 CTAs per SM (3 at 128), 1.2 us per tile (1.5 at 128, 2 of e4m3 bytes), always through the workspace.
+// full wave, whose rows do not end together), `full` beside a full chip of others, `alone` where the others are done. Adding is
+// cheaper inside a cluster than through the workspace, whose bytes grow with the query heads per key head. Tiles dealt out evenly
+// (attn_decode_even_kernel, asked for by splits that give two places per CTA) take `full` for each and a start, a sum and a share per
+// pair (more where short pairs stand beside long ones: even_short per pair, for CTAs that have many, and even_each per tile), and the
+// reduction a time per four query heads and CTA that the longest row lies in. The kernel for other pages and head dim 64: 5 CTAs per
+// SM (3 at 128), 1.2 us per tile (1.5 at 128, 2 of e4m3 bytes), always through the workspace.
 //
-// Fitted to the times of every count, in a chain of launches, for 1370 batches (TMA; 750 of the other kernel) of 1 to 512 rows, 16 to 100000 keys, 1 to 8
-// key heads and 1 to 16 query heads for each: rows alike, within a quarter, one of up to 60 times the others, spread evenly or over their
-// logarithm. Time over the fastest measured, mean and worst, with the rule before, with every row taken for as long as the longest,
-// and now:
-//   bf16, TMA          1.27 4.8   1.20 6.4   1.01 1.2     e4m3, TMA          1.34 7.4   1.14 7.9   1.01 1.4
+// Fitted to the times of every count, in a chain of launches, for 2410 batches (TMA, pages of 64 and of 16; 750 of the other kernel)
+// of 1 to 512 rows, 16 to 100000 keys, 1 to 8 key heads and 1 to 16 query heads for each: rows alike, within a quarter, one of up to
+// 60 times the others, spread evenly or over their logarithm. Time over the fastest measured, mean and worst, with the rule before,
+// with every row taken for as long as the longest, and now:
+//   bf16, pages of 64  1.27 4.8   1.20 6.4   1.01 1.2     e4m3, pages of 64  1.34 7.4   1.14 7.9   1.01 1.4
+//   bf16, pages of 16  1.38 12.7  1.30 13.9  1.01 1.2     e4m3, pages of 16  1.43 13.5  1.16 13.5  1.01 1.3
 //   bf16, head dim 64  1.59 8.5   1.09 3.3   1.02 1.2     e4m3, head dim 64  1.77 7.7   1.13 3.7   1.02 1.2
 //   bf16, other pages  1.54 6.5   1.17 5.8   1.03 1.3     e4m3, other pages  1.75 7.5   1.27 6.9   1.03 1.4
 // 8 key heads, splits or even (us, with the rule before and now):
@@ -1684,11 +1686,14 @@ int set_smem(K kern, int bytes) {
 // total_ctx: keys of all rows together, 0 where it is not known: rows as long as the longest.
 PXL_EXPORT int pxl_attn_decode_splits_of(int B, int Hq, int Hkv, int D, int page_size, int cache_fp8, int max_ctx, int64_t total_ctx) {
   struct Line {
-    float start, part, part_behind, full, cluster, add, add_split, add_wave, even, even_pair, even_short, even_each, even_part, even_margin, alone;
+    float start, part, part_behind, full, cluster, add, add_split, add_wave;
+    float even, even_pair, even_short, even_each, even_part, even_margin, alone;
   };
-  static constexpr Line kLines[2] = {{1.9f, 0.9f, 0.65f, 1.4f, 1.45f, 2.5f, 0.14f, 0.23f, 8.9f, 0.85f, 0.f, 0.35f, 0.5f, 0.95f, 0.65f},
-                                     {2.3f, 0.61f, 0.7f, 0.68f, 2.4f, 1.4f, 0.23f, 0.49f, 9.f, 0.3f, 7.f, 0.16f, 0.4f, 0.98f, 0.55f}};
-  const Line& c = kLines[cache_fp8 ? 1 : 0];
+  static constexpr Line kLines[2][2] = {{{1.9f, 0.9f, 0.65f, 1.4f, 1.45f, 2.5f, 0.14f, 0.23f, 8.9f, 0.85f, 0.f, 0.35f, 0.5f, 0.95f, 0.65f},
+                                         {1.9f, 1.04f, 1.f, 1.4f, 1.6f, 2.1f, 0.12f, 0.3f, 8.9f, 0.46f, 0.f, 0.52f, 0.37f, 0.96f, 0.88f}},
+                                        {{2.3f, 0.61f, 0.7f, 0.68f, 2.4f, 1.4f, 0.23f, 0.49f, 9.f, 0.3f, 7.f, 0.16f, 0.4f, 0.98f, 0.55f},
+                                         {3.f, 0.61f, 0.64f, 0.72f, 2.05f, 1.7f, 0.12f, 0.27f, 8.f, 0.f, 4.3f, 0.02f, 0.4f, 0.99f, 0.46f}}};
+  const Line& c = kLines[cache_fp8 ? 1 : 0][page_size < 64 ? 1 : 0];  // (a tile of four pages is four times the boxes)
   const bool tma = D == 128 && (page_size == 16 || page_size == 32 || page_size == 64);
   const int64_t pairs = static_cast<int64_t>(B) * Hkv;
   const int chip = 2 * pxl_host::num_sms(), slots = tma ? chip : (D == 64 ? 5 : 3) * pxl_host::num_sms();
